@@ -224,6 +224,18 @@ def tolerance(case):
 # ---- what a user's program has in hand -------------------------------------------------------------------
 
 
+def _normal(gen, dtype, n):
+    return torch.empty(n, device="cuda", dtype=dtype).normal_(generator=gen)
+
+
+def _fills(who, counts):
+    """The steps in which cached rows are put in place, at most 128 Ki tokens each where a sequence allows it."""
+    while who:
+        n = max(1, sum(sum(counts[:i + 1]) <= 1 << 17 for i in range(len(counts))))
+        yield who[:n], counts[:n]
+        who, counts = who[n:], counts[n:]
+
+
 class State:
     def __init__(self):
         self.arena = self.rope = None
@@ -244,7 +256,7 @@ def prepare(case, seed):
     longest = max(c + m for c, m in zip(ctx, most))
 
     def normal(n):
-        return torch.empty(n, device="cuda", dtype=dtype).normal_(generator=gen)
+        return _normal(gen, dtype, n)
 
     st = State()
     if case["api"] == "cache":
@@ -257,12 +269,10 @@ def prepare(case, seed):
     arena.set_free_list(torch.randperm(arena.num_pages, generator=torch.Generator().manual_seed(int(seed))).numpy())
 
     def fill(who, counts):  # cached rows, and with them every layer's pages
-        while who:
-            n = max(1, sum(sum(counts[:i + 1]) <= 1 << 17 for i in range(len(counts))))
-            arena.begin_step(who[:n], counts[:n])
+        for part, rows in _fills(who, counts):
+            arena.begin_step(part, rows)
             for layer in range(layers):
-                arena.append(layer, normal(sum(counts[:n]) * n_kv * d), normal(sum(counts[:n]) * n_kv * d))
-            who, counts = who[n:], counts[n:]
+                arena.append(layer, normal(sum(rows) * n_kv * d), normal(sum(rows) * n_kv * d))
 
     if case["api"] != "cache":
         root = arena.new_seq()
@@ -334,3 +344,101 @@ def run(st):
     for s, n in st.rollback:
         s.popn(n)
     return outputs
+
+
+# ---- the same in 64 bits ---------------------------------------------------------------------------------
+
+
+def exact(case, seed):
+    """What `run` returns, in plain torch and 64 bits.  Rounded are only the values that the cache holds by
+    definition: table entries, normed and rotated rows (in the case's type), and int8 pages' bytes and scales."""
+    gen = torch.Generator(device="cuda").manual_seed(int(seed))
+    dtype, f64 = DTYPES[case["dtype"]], torch.float64
+    n_q, n_kv, d, layers, wins = case["n_q"], case["n_kv"], case["d"], case["layers"], _windows(case)
+    ctx, most = _contexts(case), _grown(case)[0]
+    longest = max(c + m for c, m in zip(ctx, most))
+
+    def normal(n):
+        return _normal(gen, dtype, n)
+
+    def stored(x):
+        return x.to(dtype).to(f64)
+
+    def quantised(x):  # one scale for 32 values
+        g = x.view(-1, 32)
+        s = (g.abs().amax(1, keepdim=True) / 127).clamp(min=1e-8)
+        return ((g / s).round().clamp(-127, 127) * stored(s)).view(x.shape)
+
+    # the draws of `prepare`, in its order: cached[layer][sequence] = [k, v], each (heads, tokens, d)
+    def cached_rows(who, counts, into):
+        for part, rows in _fills(who, counts):
+            for layer in range(layers):
+                kv = [normal(sum(rows) * n_kv * d).split([n * n_kv * d for n in rows]) for _ in range(2)]
+                for i, n, k, v in zip(part, rows, *kv):
+                    into[layer][i] = [k.view(n_kv, n, d), v.view(n_kv, n, d)]
+
+    shared, cached = [{} for _ in wins], [{} for _ in wins]
+    if case["prefix"]:
+        cached_rows([0], [case["prefix"]], shared)
+    old = [(i, n - case["prefix"]) for i, n in enumerate(ctx) if n > case["prefix"]]
+    if old:
+        cached_rows([i for i, _ in old], [n for _, n in old], cached)
+    else:
+        cached_rows([0], [1], [{} for _ in wins])
+    norms = [[0.1 * normal(d), 0.1 * normal(d)] for _ in wins] if case["rope"] == 2 else None
+    passes = []
+    for who, new, reject in _schedule(case):
+        q, k, v = (normal(layers * sum(new) * h * d).view(layers, -1) for h in (n_q, n_kv, n_kv))
+        passes.append((who, new, reject, q, k, v, torch.zeros(q.shape, dtype=f64, device="cuda")))
+
+    if case["rope"]:
+        angle = torch.arange(longest, device="cuda", dtype=f64)[:, None] * 500000.0 ** (-torch.arange(0, d, 2, device="cuda", dtype=f64) / d)
+        cos, sin = stored(angle.cos()), stored(angle.sin())
+
+    def normed_rotated(x, weight, pos):
+        if weight is not None:
+            x = stored(x * (x.square().mean(-1, keepdim=True) + 1e-6).rsqrt() * stored(weight.to(f64) + 1))
+        if case["rope"]:
+            c, s = cos[pos:pos + x.shape[1]], sin[pos:pos + x.shape[1]]
+            a, b = x[..., :d // 2], x[..., d // 2:]
+            x = stored(torch.cat([a * c - b * s, b * c + a * s], -1))
+        return x
+
+    for layer, w in enumerate(wins):
+        int8 = case["int8"] and w is None
+
+        def kept(x):
+            return quantised(x).to(torch.float32) if int8 else x.to(dtype)
+
+        held = []
+        for i, n in enumerate(ctx):
+            rows = torch.empty(2, n_kv, n + most[i], d, device="cuda", dtype=torch.float32 if int8 else dtype)
+            at = 0
+            for part in (shared[layer].get(0) if case["prefix"] else None, cached[layer].pop(i, None)):
+                for j in range(2 if part else 0):
+                    rows[j, :, at:at + part[j].shape[1]] = kept(part[j].to(f64).contiguous())
+                at += part[0].shape[1] if part else 0
+            held.append(rows)
+        lengths = list(ctx)
+        for who, new, reject, q, k, v, out in passes:
+            off = 0
+            for i, n in zip(who, new):
+                pos, end = lengths[i], lengths[i] + n
+                qi, ki, vi = (x[layer, off * h * d:(off + n) * h * d].view(h, n, d).to(f64) for x, h in ((q, n_q), (k, n_kv), (v, n_kv)))
+                weights = norms[layer] if norms else (None, None)
+                qi, ki = (normed_rotated(x, wt, pos) for x, wt in zip((qi, ki), weights))
+                held[i][0, :, pos:end], held[i][1, :, pos:end] = kept(ki.contiguous()), kept(vi.contiguous())
+                first = 0 if w is None else max(0, pos - w + 1)
+                keys, values = held[i][:, :, first:end].to(f64)
+                score = (qi.reshape(n_kv, -1, d) @ keys.transpose(1, 2) * d ** -0.5).view(n_q, n, -1)
+                if n > 1:
+                    p, t = torch.arange(pos, end, device="cuda")[:, None], torch.arange(first, end, device="cuda")
+                    score.masked_fill_((t > p) | (t <= p - (w or end + 1)), -math.inf)
+                prob = score.softmax(-1).view(n_kv, -1, end - first)
+                out[layer, off * n_q * d:(off + n) * n_q * d] = (prob @ values).view(-1)
+                lengths[i] = end - reject
+                off += n
+    outs = [p[-1] for p in passes]
+    if case["api"] == "cache":
+        return [x.view(1, n_q, -1, d) for o, p in zip(outs, passes) for x in o]
+    return [o.cpu() for o in outs] if case["api"] == "host" else outs
