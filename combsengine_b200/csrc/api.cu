@@ -108,10 +108,8 @@ struct DeviceState {
     const int32_t* chunk_item_begin = nullptr;
     bool tc_ok = false;       // the tcgen05 chunk kernel covers this geometry
     int chunk_mode = 0;       // cbkv_set_chunk_kernel: 0 = choose, 1 = mma.sync, 2 = tcgen05 one tile, 3 = two tiles, 4 = two tiles, int8 records converted in the kernel
-    bool tile_plan_ok = false;
-    int tile_plan_tokens = 0;  // tokens per work item the tile plan was built for
-    ChunkPlan tile_host;
-    const int32_t* tile_item_begin = nullptr;
+    struct TilePlanDev { ChunkPlan host; const TileItem* tiles = nullptr; };
+    std::map<std::pair<int64_t, int>, TilePlanDev> tile_plans;  // of the step, by (window, tokens per work item)
     float* part_o = nullptr;
     float* part_ml = nullptr;
     size_t part_cap = 0;
@@ -122,12 +120,12 @@ struct DeviceState {
     bool pdl = true;
     bool host_direct = true;  // cbkv_set_host_route
     bool zero_pending = false; // the step's first unit-table kernel still has to zero the decode kernels' counters
-    // two-tile chunk kernel: slices of the items of a launch's last, mostly empty wave (ChunkArgs::split_*)
-    int chunk_split = 4;               // most slices per item, 1 = never cut (cbkv_set_chunk_split)
+    // tcgen05 chunk kernels: partial results of items cut along K/V (ChunkArgs::split_*)
+    int chunk_split = 64;              // most slices per item, 1 = never cut (cbkv_set_chunk_split)
     float* split_o = nullptr;
     float2* split_ml = nullptr;
     int32_t* split_counter = nullptr;
-    int split_cap = 0;                 // slices the buffers hold
+    size_t split_cap = 0, split_cut_cap = 0;  // slots the buffers hold, counters
     int last_kv_writer = -1;  // layer whose pages the most recent launch wrote (-1: none since the last upload)
     // host-buffer entry point staging
     uint8_t* io = nullptr;
@@ -326,7 +324,7 @@ int32_t slot_upload(DeviceState* d, const void* src, size_t bytes, cudaStream_t 
                 p = pd.items; fix(p); pd.items = (const ItemInfo*)p;
             }
             p = d->chunk_item_begin; fix(p); d->chunk_item_begin = (const int32_t*)p;
-            p = d->tile_item_begin; fix(p); d->tile_item_begin = (const int32_t*)p;
+            for (auto& kv : d->tile_plans) { p = kv.second.tiles; fix(p); kv.second.tiles = (const TileItem*)p; }
             cudaFreeHost(s.host);
             cudaFree(s.dev);
         }
@@ -361,15 +359,14 @@ int32_t upload_step(Arena* a, cudaStream_t st) {
     d->decode_plans.clear();
     d->chunk_plan_ok = false;
     d->chunk_item_begin = nullptr;
-    d->tile_plan_ok = false;
-    d->tile_item_begin = nullptr;
+    d->tile_plans.clear();
     d->step = StepDev{};
     d->last_kv_writer = -1;  // the upload is a full stream dependency
     d->unit_rows_used = 0;
     // tickets and claim counters start every step at zero, whatever an earlier launch that gave up left behind:
     // the decode kernels' by the step's first unit-table kernel (get_decode_plan), the chunk kernel's here
     d->zero_pending = true;
-    if (d->split_counter && !a->step_is_decode) CU_TRY(cudaMemsetAsync(d->split_counter, 0, (size_t)d->split_cap * sizeof(int32_t), st));
+    if (d->split_counter && !a->step_is_decode) CU_TRY(cudaMemsetAsync(d->split_counter, 0, d->split_cut_cap * sizeof(int32_t), st));
     if (a->step_meta.empty()) {  // an empty step: nothing to upload, nothing will launch
         d->uploaded_step = a->step_id;
         return CBKV_OK;
@@ -485,16 +482,56 @@ int rep_slots_of(int n_rep) {
     return rs;
 }
 
-int32_t get_tile_plan(Arena* a, int tokens_per_item, cudaStream_t st) {
+// Room for the partial results of a chunk launch's cut items.  False (nothing is cut then) when there is no memory
+// for it, or when the buffers would have to move while the stream is being captured.
+bool ensure_split(Arena* a, size_t slots, size_t cuts, cudaStream_t st) {
     DeviceState* d = dev_of(a);
-    if (d->tile_plan_ok && d->tile_plan_tokens == tokens_per_item) return CBKV_OK;
-    build_chunk_tile_plan(*a, tokens_per_item, &d->tile_host);
-    d->tile_plan_tokens = tokens_per_item;
+    if (slots <= d->split_cap && cuts <= d->split_cut_cap) return true;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) { cudaGetLastError(); return false; }
+    if (cudaStreamSynchronize(st) != cudaSuccess) return false;  // the launch that follows reports it
+    if (d->split_o) cudaFree(d->split_o);
+    if (d->split_ml) cudaFree(d->split_ml);
+    if (d->split_counter) cudaFree(d->split_counter);
+    d->split_o = nullptr; d->split_ml = nullptr; d->split_counter = nullptr;
+    d->split_cap = d->split_cut_cap = 0;
+    const size_t ncap = std::max(slots + slots / 4, (size_t)d->sm_count), ccap = std::max(2 * cuts, (size_t)d->sm_count);
+    const size_t rows = chunk_tc2_supported(a->cfg.head_dim) ? 256 : 128;  // of a slot, whichever kernel comes later
+    if (cudaMalloc(&d->split_o, ncap * rows * a->cfg.head_dim * sizeof(float)) != cudaSuccess ||
+        cudaMalloc(&d->split_ml, ncap * rows * sizeof(float2)) != cudaSuccess ||
+        cudaMalloc(&d->split_counter, ccap * sizeof(int32_t)) != cudaSuccess ||
+        cudaMemsetAsync(d->split_counter, 0, ccap * sizeof(int32_t), st) != cudaSuccess) {
+        cudaGetLastError();
+        if (d->split_o) cudaFree(d->split_o);
+        if (d->split_ml) cudaFree(d->split_ml);
+        if (d->split_counter) cudaFree(d->split_counter);
+        d->split_o = nullptr; d->split_ml = nullptr; d->split_counter = nullptr;
+        return false;
+    }
+    d->split_cap = ncap; d->split_cut_cap = ccap;
+    return true;
+}
+
+// Work list of a tcgen05 chunk launch: tokens_per_item new tokens per item in tiles of tile_tokens, K/V tiles of
+// kv_tile tokens.  Built once per step and window; the partial-result buffers grow with it.
+int32_t get_tile_plan(Arena* a, int64_t window, int tokens_per_item, int tile_tokens, int kv_tile, cudaStream_t st, DeviceState::TilePlanDev** out) {
+    DeviceState* d = dev_of(a);
+    const auto key = std::make_pair(window, tokens_per_item);
+    auto it = d->tile_plans.find(key);
+    if (it != d->tile_plans.end()) { *out = &it->second; return CBKV_OK; }
+    DeviceState::TilePlanDev pd;
+    TileCut cut{window, kv_tile, tile_tokens, d->sm_count, d->chunk_split};
+    build_chunk_tile_plan(*a, tokens_per_item, &pd.host, cut);
+    if (!ensure_split(a, (size_t)pd.host.n_slots, (size_t)pd.host.n_cut, st)) {
+        cut.max_parts = 1;
+        build_chunk_tile_plan(*a, tokens_per_item, &pd.host, cut);
+    }
     const void* p = nullptr;
-    int32_t rc = slot_upload(d, d->tile_host.item_begin.data(), d->tile_host.item_begin.size() * sizeof(int32_t), st, &p);
+    int32_t rc = slot_upload(d, pd.host.tiles.data(), pd.host.tiles.size() * sizeof(TileItem), st, &p);
     if (rc) return rc;
-    d->tile_item_begin = (const int32_t*)p;
-    d->tile_plan_ok = true;
+    pd.tiles = (const TileItem*)p;
+    auto ins = d->tile_plans.emplace(key, std::move(pd));
+    *out = &ins.first->second;
     return CBKV_OK;
 }
 
@@ -549,12 +586,13 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
     if (w != 0 && w < 2) { set_error("sliding window must be >= 2, got " + std::to_string(w)); return CBKV_ERR_ARG; }
     LayerArena& L = d->layers[(size_t)layer];
     const float scale_log2 = (float)(scale * 1.4426950408889634);
-    // tensor-core chunk kernels: worth it once the step has enough new tokens to fill 128-row tiles
+    // tensor-core chunk kernels, whatever the number of new tokens: a few tokens leave most of a tile's rows empty,
+    // but their items are cut along K/V until the chip is full, so the step runs at the rate its K/V arrives
     // (their softmax takes row maxima before scaling, which needs a positive scale)
     const bool tc_able = d->fast && d->tc_ok && scale > 0 && !a->step_is_decode;
     const bool use_tc2 = tc_able && chunk_tc2_supported(a->cfg.head_dim) &&
-                         (d->chunk_mode == 3 || d->chunk_mode == 4 || (d->chunk_mode == 0 && a->step_tokens >= 128));
-    const bool use_tc = tc_able && !use_tc2 && (d->chunk_mode == 2 || (d->chunk_mode == 0 && a->step_tokens >= 64));
+                         (d->chunk_mode == 3 || d->chunk_mode == 4 || d->chunk_mode == 0);
+    const bool use_tc = tc_able && !use_tc2 && (d->chunk_mode == 2 || d->chunk_mode == 0);
     // int8 pages: decode steps stream the records through the decode kernel; the chunk kernels read a float
     // copy made per layer and step (mode 4: the two-tile kernel converts the records itself, slower so far);
     // shapes outside the fast path de-quantise on the fly in the generic kernel
@@ -623,51 +661,27 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
         return CBKV_OK;
     }
     if (use_tc || use_tc2) {
-        const int rs = rep_slots_of(a->n_rep());
-        int32_t rc = get_tile_plan(a, (use_tc2 ? 2 : 1) * (128 / rs), st);
+        const int tile_tokens = 128 / rep_slots_of(a->n_rep());
+        DeviceState::TilePlanDev* pd = nullptr;
+        int32_t rc = get_tile_plan(a, w, (use_tc2 ? 2 : 1) * tile_tokens, tile_tokens, !use_tc2 && a->cfg.head_dim == 256 ? 64 : 128, st, &pd);
         if (rc) return rc;
         ChunkArgs args{};
-        args.step = d->step; args.geo = geom(a); args.item_begin = d->tile_item_begin; args.n_items = d->tile_host.n_items;
-        args.q = q; args.out = out; args.status = d->status; args.window = (int32_t)w; args.scale_log2 = scale_log2; args.rep_slots = rs;
+        args.step = d->step; args.geo = geom(a); args.tiles = pd->tiles; args.n_items = (int32_t)pd->host.tiles.size();
+        args.q = q; args.out = out; args.status = d->status; args.window = (int32_t)w; args.scale_log2 = scale_log2;
+        args.rep_slots = 128 / tile_tokens;
         args.q8_arena = q8_direct ? L.base : nullptr;
-        if (use_tc2 && d->chunk_split > 1) {
-            // The grid runs one CTA per SM at a time.  When the last wave would fill at most half of the SMs, its
-            // items are cut along K/V so that the wave is full and ends sooner (the slices are merged by whichever
-            // CTA of an item finishes last).  Only worth it when every slice still has a few K/V tiles.
-            const int n_items = d->tile_host.n_items, rem = n_items % d->sm_count;
-            int parts = rem > 0 ? std::min(d->chunk_split, d->sm_count / rem) : 1;
-            int64_t min_keys = INT64_MAX;
-            for (const auto& m : a->step_meta) {
-                const int64_t keys = w > 0 ? std::min<int64_t>(w, (int64_t)m.pos + m.snew) : (int64_t)m.pos + m.snew;
-                min_keys = std::min(min_keys, keys);
-            }
-            while (parts > 1 && min_keys < (int64_t)parts * 8 * 128) parts--;  // measured: below 8 tiles per slice the merge costs more than the wave saves
-            if (parts > 1) {
-                const int slices = rem * parts;
-                if (slices > d->split_cap) {
-                    CU_TRY(cudaStreamSynchronize(st));
-                    if (d->split_o) { cudaFree(d->split_o); cudaFree(d->split_ml); cudaFree(d->split_counter); }
-                    d->split_cap = std::max(slices, d->sm_count);
-                    CU_TRY(cudaMalloc(&d->split_o, (size_t)d->split_cap * 2 * 128 * 128 * sizeof(float)));
-                    CU_TRY(cudaMalloc(&d->split_ml, (size_t)d->split_cap * 2 * 128 * sizeof(float2)));
-                    CU_TRY(cudaMalloc(&d->split_counter, (size_t)d->split_cap * sizeof(int32_t)));
-                    CU_TRY(cudaMemsetAsync(d->split_counter, 0, (size_t)d->split_cap * sizeof(int32_t), st));
-                }
-                args.split_first = n_items - rem; args.split_parts = parts;
-                args.split_o = d->split_o; args.split_ml = d->split_ml; args.split_counter = d->split_counter;
-            }
-        }
+        args.split_o = d->split_o; args.split_ml = d->split_ml; args.split_counter = d->split_counter;
 #ifdef CBKV_MEASURE
         if (debug_flags() & 8) {  // per-role cycle counters of the first 4096 CTAs
             if (!d->dbg_buf) { CU_TRY(cudaMalloc(&d->dbg_buf, 4096 * 16 * sizeof(unsigned long long))); }
             CU_TRY(cudaMemsetAsync(d->dbg_buf, 0, 4096 * 16 * sizeof(unsigned long long), st));
-            if (d->tile_host.n_items + d->sm_count * 4 <= 4096) { args.dbg_buf = d->dbg_buf; d->dbg_ctas = -d->tile_host.n_items; }
+            if (args.n_items <= 4096) { args.dbg_buf = d->dbg_buf; d->dbg_ctas = -args.n_items; }
         }
 #endif
         ProfScope ps(d, st);
         { int32_t frc = flush_uploads(d, st); if (frc) return frc; }
         if (use_tc2) CU_TRY(q8_direct ? launch_chunk_tc2(L.map_k16, L.map_sc, args, bf16, st) : launch_chunk_tc2(KV->map_kv, KV->map_kv, args, bf16, st));
-        else CU_TRY(launch_chunk_tc(KV->map_k16, KV->map_kv, args, bf16, st));
+        else CU_TRY(launch_chunk_tc(KV->map_kv, args, bf16, st));
         g_launches++;
         d->last_kv_writer = -1;
         return CBKV_OK;
@@ -1525,6 +1539,7 @@ int32_t cbkv_set_chunk_split(cbkv_arena* arena, int32_t max_parts) {
     int32_t rc = ensure_device(a);
     if (rc) return rc;
     dev_of(a)->chunk_split = max_parts;
+    dev_of(a)->tile_plans.clear();
     return CBKV_OK;
     });
 }
@@ -1562,6 +1577,23 @@ int64_t cbkv_debug_decode_plan(cbkv_arena* arena, int64_t window, int32_t n_ctas
     flat.insert(flat.end(), sp32, sp32 + pl.segs.size() * 8);
     const int32_t* ip32 = reinterpret_cast<const int32_t*>(pl.items.data());
     flat.insert(flat.end(), ip32, ip32 + pl.items.size() * 4);
+    for (int64_t i = 0; i < (int64_t)flat.size() && i < cap; i++) out[i] = flat[(size_t)i];
+    return (int64_t)flat.size();
+    });
+}
+
+// Host-only view of a tcgen05 chunk launch's work list (used by the CPU tests of the cut): out = [n_ctas, n_slots,
+// n_cut, TileItem records of 8 ints in launch order].
+int64_t cbkv_debug_tile_plan(cbkv_arena* arena, int64_t window, int32_t tokens_per_item, int32_t tile_tokens, int32_t kv_tile,
+                             int32_t sm_count, int32_t max_parts, int32_t* out, int64_t cap) {
+    return fenced64([&]() -> int64_t {
+    Arena* a = reinterpret_cast<Arena*>(arena);
+    if (!a || a->step_meta.empty() || !out || tokens_per_item < 1 || tile_tokens < 1 || kv_tile < 16) return -1;
+    ChunkPlan pl;
+    build_chunk_tile_plan(*a, tokens_per_item, &pl, TileCut{window, kv_tile, tile_tokens, sm_count, max_parts});
+    std::vector<int32_t> flat = {(int32_t)pl.tiles.size(), pl.n_slots, pl.n_cut};
+    const int32_t* tp = reinterpret_cast<const int32_t*>(pl.tiles.data());
+    flat.insert(flat.end(), tp, tp + pl.tiles.size() * 8);
     for (int64_t i = 0; i < (int64_t)flat.size() && i < cap; i++) out[i] = flat[(size_t)i];
     return (int64_t)flat.size();
     });

@@ -127,14 +127,12 @@ struct ChunkArgs {
     float scale_log2;
     int32_t rep_slots;  // tcgen05 kernel: q heads per kv head rounded up to a power of two (rows per token in a tile)
     const void* q8_arena;  // two-tile tcgen05 kernel: non-null = the layer's int8 records, read and converted by the kernel itself
-    // two-tile tcgen05 kernel: the items from split_first on are cut along K/V into split_parts CTAs each (the
-    // last wave of a launch would otherwise leave most SMs idle); each writes its un-normalised rows and their
-    // (reference exponent, sum) to split_o / split_ml and draws a ticket from split_counter, the last one
-    // merges.  split_parts <= 1: no item is cut.  n_items counts items, the grid has
-    // split_first + (n_items - split_first) * split_parts CTAs.
-    int32_t split_first, split_parts;
-    float* split_o;         // float4 [(item - split_first) * split_parts + part][tile 2][column group 32][row 128]
-    float2* split_ml;       // [(item - split_first) * split_parts + part][tile 2][row 128]
+    // tcgen05 kernels: one record per CTA (n_items of them).  The CTAs of an item that is cut along K/V write their
+    // un-normalised rows and their (reference exponent, sum) to the slots of split_o / split_ml and draw a ticket
+    // from split_counter; the last one merges.
+    const TileItem* tiles;
+    float* split_o;         // float4 [slot][query tile][column group D / 4][row 128]; rows: q head * valid tokens + token
+    float2* split_ml;       // [slot][query tile][row 128]
     int32_t* split_counter; // per cut item, zero between launches
 #ifdef CBKV_MEASURE
     unsigned long long* dbg_buf;  // per-CTA cycle counters of the tcgen05 kernel
@@ -206,10 +204,10 @@ cudaError_t launch_rope_append(const RopeArgs& a, bool bf16, cudaStream_t st);
 // host side of the rotary tables (rope.cu): frequencies, then [max_position][head_dim] f32 tables
 int32_t rope_inv_freq(const cbkv_rope_config& c, std::vector<double>* inv, double* mscale);
 void rope_tables(const cbkv_rope_config& c, const std::vector<double>& inv, double mscale, float* cos_out, float* sin_out);
-// tcgen05 chunk kernel (prefill_tc.cu): head_dim 64 or 128; `map` is the 16-row box view
+// tcgen05 chunk kernel (prefill_tc.cu): head_dim 64, 128 or 256; `map32` is the layer's map_kv
 bool chunk_tc_supported(int d);
 cudaError_t chunk_tc_init();
-cudaError_t launch_chunk_tc(const CUtensorMap& map16, const CUtensorMap& map32, const ChunkArgs& a, bool bf16, cudaStream_t st);
+cudaError_t launch_chunk_tc(const CUtensorMap& map32, const ChunkArgs& a, bool bf16, cudaStream_t st);
 // two query tiles per CTA, P in tensor memory (head_dim 128)
 bool chunk_tc2_supported(int d);
 // int8 layer (a.q8_arena non-null): `map32` = the layer's map_k16, `map_sc` = its map_sc; float layer: map_sc is not used

@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 
 namespace cbkv {
 
@@ -327,17 +328,137 @@ void build_chunk_plan(const Arena& a, int32_t cols_per_item, ChunkPlan* pl) {
     pl->n_items = (int32_t)items;
 }
 
-void build_chunk_tile_plan(const Arena& a, int32_t tokens_per_tile, ChunkPlan* pl) {
+namespace {
+
+// Launch model of the tcgen05 chunk kernels, in units of one K/V tile of a full item: a CTA costs kCtaCost
+// besides its tiles (tensor-memory allocation, first loads, epilogue), a K/V tile of an item that fills one of
+// its two query tiles kHalfTile, a slice kSliceCost more (its partial rows), and the merge at the end
+// kMergeCost for each slice of the full 256 rows.
+constexpr float kCtaCost = 3.f, kHalfTile = 0.7f, kSliceCost = 0.7f, kMergeCost = 0.7f;
+
+struct TileWork { int32_t seq, h, qt, n_tiles; float per_tile, rows; };  // an uncut item
+
+// End of the last CTA when `sm_count` SMs take the CTAs in launch order.
+float launch_end(const std::vector<float>& cost, int sm_count, std::vector<float>* heap) {
+    heap->assign((size_t)sm_count, 0.f);
+    float end = 0.f;
+    for (float c : cost) {
+        std::pop_heap(heap->begin(), heap->end(), std::greater<float>());
+        const float e = heap->back() + c;
+        heap->back() = e;
+        std::push_heap(heap->begin(), heap->end(), std::greater<float>());
+        end = std::max(end, e);
+    }
+    return end;
+}
+
+}  // namespace
+
+// CTAs are launched longest (sequence, kv head) first; the items of one (sequence, kv head) stay together, slice
+// by slice, because they read the same K/V.  Whether and how finely items are cut is decided by running the
+// launch model over a few candidates: no cut, the remainder of the last wave cut in equal parts (a launch of
+// several waves whose last is mostly empty), and every item longer than a limit cut into slices of at most that
+// (a launch that has too few items for the chip: a few tokens of a few sequences over long contexts).
+void build_chunk_tile_plan(const Arena& a, int32_t tokens_per_tile, ChunkPlan* pl, const TileCut& cut) {
     const int n = (int)a.step_meta.size();
+    const int tile_tokens = cut.tile_tokens > 0 ? cut.tile_tokens : tokens_per_tile;
     pl->cols_per_item = tokens_per_tile;
     pl->item_begin.assign((size_t)n + 1, 0);
+    pl->tiles.clear();
+    pl->n_slots = pl->n_cut = 0;
     int64_t items = 0;
+    struct Group { int32_t seq, first, n_qt; float cost; };
+    std::vector<TileWork> work;    // of one kv head, per sequence and block of query tokens
+    std::vector<Group> groups;
     for (int b = 0; b < n; b++) {
+        const SeqMeta& m = a.step_meta[(size_t)b];
+        const int n_qt = (m.snew + tokens_per_tile - 1) / tokens_per_tile;
         pl->item_begin[(size_t)b] = (int32_t)items;
-        items += (int64_t)a.cfg.n_kv_heads * ((a.step_meta[(size_t)b].snew + tokens_per_tile - 1) / tokens_per_tile);
+        items += (int64_t)a.cfg.n_kv_heads * n_qt;
+        if (n_qt == 0) continue;
+        Group g{b, (int32_t)work.size(), n_qt, 0.f};
+        for (int qt = 0; qt < n_qt; qt++) {
+            const int r0 = qt * tokens_per_tile, toks = std::min(tokens_per_tile, m.snew - r0);
+            const int64_t q_first = m.pos + r0, q_last = q_first + toks - 1;
+            const int64_t lo_key = cut.window > 0 ? std::max<int64_t>(0, q_first - cut.window + 1) : 0;
+            const int32_t pages = (int32_t)((q_last >> 4) - (lo_key >> 4) + 1), ppt = cut.kv_tile / 16;
+            TileWork w{b, 0, qt, (pages + ppt - 1) / ppt, toks > tile_tokens ? 1.f : kHalfTile, (float)toks / (float)tokens_per_tile};
+            if (tile_tokens == tokens_per_tile) w.per_tile = 1.f;  // one query tile per CTA
+            g.cost = std::max(g.cost, w.per_tile * w.n_tiles);
+            work.push_back(w);
+        }
+        groups.push_back(g);
     }
     pl->item_begin[(size_t)n] = (int32_t)items;
     pl->n_items = (int32_t)items;
+    std::stable_sort(groups.begin(), groups.end(), [](const Group& x, const Group& y) { return x.cost > y.cost; });
+
+    // parts of an item: ceil(cost / limit), and for the last `rem` items of the launch order at least rem_parts
+    std::vector<float> cost, heap;
+    auto emit = [&](float limit, int64_t rem, int rem_parts, std::vector<TileItem>* out, int32_t* n_slots, int32_t* n_cut) -> float {
+        cost.clear();
+        int32_t slots = 0, cuts = 0;
+        float merge = 0.f;
+        int64_t at = 0;
+        std::vector<int32_t> parts, base, id;
+        for (const Group& g : groups) {
+            for (int h = 0; h < a.cfg.n_kv_heads; h++) {
+                int most = 1;
+                parts.assign((size_t)g.n_qt, 1); base.assign((size_t)g.n_qt, -1); id.assign((size_t)g.n_qt, -1);
+                for (int qt = 0; qt < g.n_qt; qt++, at++) {
+                    const TileWork& w = work[(size_t)(g.first + qt)];
+                    int p = limit > 0.f ? (int)std::min(1e6f, w.per_tile * (float)w.n_tiles / limit + 0.999f) : 1;
+                    if (at >= items - rem) p = std::max(p, rem_parts);
+                    p = std::max(1, std::min(std::min(p, cut.max_parts), w.n_tiles));
+                    const int per = (w.n_tiles + p - 1) / p;
+                    p = (w.n_tiles + per - 1) / per;  // no empty slices
+                    parts[(size_t)qt] = p;
+                    most = std::max(most, p);
+                    if (p > 1) {
+                        base[(size_t)qt] = slots; id[(size_t)qt] = cuts;
+                        slots += p; cuts++;
+                        merge = std::max(merge, kMergeCost * (0.5f + (float)p * w.rows));
+                    }
+                }
+                for (int p = 0; p < most; p++)
+                    for (int qt = 0; qt < g.n_qt; qt++) {
+                        const int np = parts[(size_t)qt];
+                        if (p >= np) continue;
+                        const TileWork& w = work[(size_t)(g.first + qt)];
+                        const int per = (w.n_tiles + np - 1) / np, t0 = p * per, t1 = std::min(w.n_tiles, t0 + per);
+                        if (out) out->push_back({g.seq, h, qt, t0, t1, p | (np << 16), base[(size_t)qt], id[(size_t)qt]});
+                        else cost.push_back(kCtaCost + w.per_tile * (float)(t1 - t0) + (np > 1 ? kSliceCost : 0.f));
+                    }
+            }
+        }
+        if (n_slots) { *n_slots = slots; *n_cut = cuts; }
+        return out ? 0.f : launch_end(cost, cut.sm_count, &heap) + merge;
+    };
+
+    float limit = 0.f;
+    int64_t rem = 0;
+    int rem_parts = 1;
+    if (cut.sm_count > 0 && cut.max_parts > 1 && items > 0 && items <= 8192) {
+        float best = emit(0.f, 0, 1, nullptr, nullptr, nullptr);
+        const int64_t r = items % cut.sm_count;
+        if (items > cut.sm_count && r > 0)
+            for (int p = 2; p <= std::min<int64_t>(4, cut.sm_count / r); p++) {
+                const float e = emit(0.f, r, p, nullptr, nullptr, nullptr);
+                if (e < best) { best = e; rem = r; rem_parts = p; limit = 0.f; }
+            }
+        double total = 0.;
+        float longest = 0.f;
+        for (const TileWork& w : work) { total += (double)w.per_tile * w.n_tiles; longest = std::max(longest, w.per_tile * w.n_tiles); }
+        const float even = (float)(total * a.cfg.n_kv_heads / cut.sm_count);  // tiles per SM
+        if (items <= 4 * cut.sm_count)
+            for (float f : {1.3f, 1.f, 0.75f, 0.5f, 0.35f}) {
+                const float lim = std::max(1.f, even * f);
+                if (lim >= longest) continue;
+                const float e = emit(lim, 0, 1, nullptr, nullptr, nullptr);
+                if (e < best) { best = e; limit = lim; rem = 0; rem_parts = 1; }
+            }
+    }
+    emit(limit, rem, rem_parts, &pl->tiles, &pl->n_slots, &pl->n_cut);
 }
 
 }  // namespace cbkv

@@ -123,7 +123,20 @@ struct ChunkPlan {
     int32_t cols_per_item = 0;
     int32_t n_items = 0;
     std::vector<int32_t> item_begin;  // n_seqs + 1
+    std::vector<struct TileItem> tiles;  // tcgen05 kernels: one record per CTA, in launch order
+    int32_t n_slots = 0, n_cut = 0;      // partial-result slots and tickets that the cut items take
 };
+
+// One CTA of a tcgen05 chunk launch: K/V tiles [t0, t1) of one (sequence, kv head, block of query tokens).  An
+// item may be cut along K/V into `nparts` CTAs; part p leaves its rows in slot slot_base + p, draws a ticket of
+// counter `cut`, and whoever draws the last one merges.
+struct TileItem {  // 32 bytes, read by the kernels as two 16-byte words
+    int32_t seq, h, qt, t0;
+    int32_t t1, part_nparts /* part | nparts << 16 */, slot_base, cut;
+};
+// How a tcgen05 chunk launch may be cut: `window` of the layer, tokens per K/V tile, query tokens per 128-row
+// tile, SMs (one CTA each at a time; 0 = never cut), most slices per item.
+struct TileCut { int64_t window = 0; int32_t kv_tile = 128, tile_tokens = 0, sm_count = 0, max_parts = 1; };
 
 struct Arena {
     cbkv_config cfg{};
@@ -168,6 +181,6 @@ void build_decode_plan(const Arena& a, int64_t window, int32_t n_ctas, const Dec
 void build_chunk_plan(const Arena& a, int32_t cols_per_item, ChunkPlan* plan);
 // Work list of the tcgen05 chunk kernel: one item per (sequence, kv head, tile of
 // `tokens_per_tile` new tokens); `cols_per_item` records tokens_per_tile.
-void build_chunk_tile_plan(const Arena& a, int32_t tokens_per_tile, ChunkPlan* plan);
+void build_chunk_tile_plan(const Arena& a, int32_t tokens_per_tile, ChunkPlan* plan, const TileCut& cut = TileCut());
 
 }  // namespace cbkv

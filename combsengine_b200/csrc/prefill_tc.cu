@@ -12,16 +12,17 @@
 //   warp 0        TMA producer: one 32-row box per (page, 64-column block) brings K and V of a
 //                 page in the arena's 8-row interleave; 8 pages per tile, two stages
 //   warp 1        one thread issues tcgen05.mma: S = Q K^T (two S buffers), O += P V
-//   warps 2..5    softmax: one TMEM lane (row) per thread, P written to shared memory
-//                 in the K-major swizzled layout, O rescaled in TMEM when a row max moves
+//   warps 2..9    softmax: two threads per TMEM lane (row), one for each half of a tile's keys; P goes back to
+//                 tensor memory over its S columns (16-bit pairs) and is the A operand of P V; O rescaled in
+//                 TMEM when a row max moves
 //
 // KV tiles hold KT tokens: 128 for head_dim 64 and 128; 64 for head_dim 256, where a 128-token tile of K
 // and V (128 KB) would not leave room for two stages next to the Q tile (S = Q K^T is then 128 x 64 and
 // O += P V one 128 x 256 MMA per 16 keys).
 //
 // Tensor memory: S0 [0,KT), S1 [128,128+KT), O [256, 256 + D) -> 512 columns allocated.
-// Shared memory: Q and P tiles of 128 rows stored as 64-column blocks of 128 rows x 128 bytes
-// (128-byte swizzle); two K/V stages, each D/64 blocks of 8 pages x 32 rows x 128 bytes in
+// Shared memory: the Q tile of 128 rows stored as 64-column blocks of 128 rows x 128 bytes
+// (128-byte swizzle); two K/V stages, each D/64 blocks of KT/16 pages x 32 rows x 128 bytes in
 // the arena's row order [K 0-7][V 0-7][K 8-15][V 8-15], so K and V are both 8-row groups
 // 2048 bytes apart (V starts 1024 bytes in).
 #include <cuda_bf16.h>
@@ -136,26 +137,6 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
         : "memory");
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
-// 128 consecutive columns of this thread's lane: four 32-column loads in flight, one wait
-__device__ __forceinline__ void tmem_ld128(uint32_t taddr, uint32_t (&r)[128]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%128];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47,%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%129];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%64,%65,%66,%67,%68,%69,%70,%71,%72,%73,%74,%75,%76,%77,%78,%79,%80,%81,%82,%83,%84,%85,%86,%87,%88,%89,%90,%91,%92,%93,%94,%95}, [%130];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%96,%97,%98,%99,%100,%101,%102,%103,%104,%105,%106,%107,%108,%109,%110,%111,%112,%113,%114,%115,%116,%117,%118,%119,%120,%121,%122,%123,%124,%125,%126,%127}, [%131];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]), "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]), "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]), "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63]), "=r"(r[64]), "=r"(r[65]), "=r"(r[66]), "=r"(r[67]), "=r"(r[68]), "=r"(r[69]), "=r"(r[70]), "=r"(r[71]), "=r"(r[72]), "=r"(r[73]), "=r"(r[74]), "=r"(r[75]), "=r"(r[76]), "=r"(r[77]), "=r"(r[78]), "=r"(r[79]), "=r"(r[80]), "=r"(r[81]), "=r"(r[82]), "=r"(r[83]), "=r"(r[84]), "=r"(r[85]), "=r"(r[86]), "=r"(r[87]), "=r"(r[88]), "=r"(r[89]), "=r"(r[90]), "=r"(r[91]), "=r"(r[92]), "=r"(r[93]), "=r"(r[94]), "=r"(r[95]), "=r"(r[96]), "=r"(r[97]), "=r"(r[98]), "=r"(r[99]), "=r"(r[100]), "=r"(r[101]), "=r"(r[102]), "=r"(r[103]), "=r"(r[104]), "=r"(r[105]), "=r"(r[106]), "=r"(r[107]), "=r"(r[108]), "=r"(r[109]), "=r"(r[110]), "=r"(r[111]), "=r"(r[112]), "=r"(r[113]), "=r"(r[114]), "=r"(r[115]), "=r"(r[116]), "=r"(r[117]), "=r"(r[118]), "=r"(r[119]), "=r"(r[120]), "=r"(r[121]), "=r"(r[122]), "=r"(r[123]), "=r"(r[124]), "=r"(r[125]), "=r"(r[126]), "=r"(r[127])
-        : "r"(taddr), "r"(taddr + 32), "r"(taddr + 64), "r"(taddr + 96) : "memory");
-}
-__device__ __forceinline__ void tmem_st128(uint32_t taddr, const uint32_t (&r)[128]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32,%33,%34,%35};\n\t"
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%1], {%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47,%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63,%64,%65,%66,%67};\n\t"
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%2], {%68,%69,%70,%71,%72,%73,%74,%75,%76,%77,%78,%79,%80,%81,%82,%83,%84,%85,%86,%87,%88,%89,%90,%91,%92,%93,%94,%95,%96,%97,%98,%99};\n\t"
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%3], {%100,%101,%102,%103,%104,%105,%106,%107,%108,%109,%110,%111,%112,%113,%114,%115,%116,%117,%118,%119,%120,%121,%122,%123,%124,%125,%126,%127,%128,%129,%130,%131};\n\t"
-        "tcgen05.wait::st.sync.aligned;"
-        :: "r"(taddr), "r"(taddr + 32), "r"(taddr + 64), "r"(taddr + 96), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]), "r"(r[32]), "r"(r[33]), "r"(r[34]), "r"(r[35]), "r"(r[36]), "r"(r[37]), "r"(r[38]), "r"(r[39]), "r"(r[40]), "r"(r[41]), "r"(r[42]), "r"(r[43]), "r"(r[44]), "r"(r[45]), "r"(r[46]), "r"(r[47]), "r"(r[48]), "r"(r[49]), "r"(r[50]), "r"(r[51]), "r"(r[52]), "r"(r[53]), "r"(r[54]), "r"(r[55]), "r"(r[56]), "r"(r[57]), "r"(r[58]), "r"(r[59]), "r"(r[60]), "r"(r[61]), "r"(r[62]), "r"(r[63]), "r"(r[64]), "r"(r[65]), "r"(r[66]), "r"(r[67]), "r"(r[68]), "r"(r[69]), "r"(r[70]), "r"(r[71]), "r"(r[72]), "r"(r[73]), "r"(r[74]), "r"(r[75]), "r"(r[76]), "r"(r[77]), "r"(r[78]), "r"(r[79]), "r"(r[80]), "r"(r[81]), "r"(r[82]), "r"(r[83]), "r"(r[84]), "r"(r[85]), "r"(r[86]), "r"(r[87]), "r"(r[88]), "r"(r[89]), "r"(r[90]), "r"(r[91]), "r"(r[92]), "r"(r[93]), "r"(r[94]), "r"(r[95]), "r"(r[96]), "r"(r[97]), "r"(r[98]), "r"(r[99]), "r"(r[100]), "r"(r[101]), "r"(r[102]), "r"(r[103]), "r"(r[104]), "r"(r[105]), "r"(r[106]), "r"(r[107]), "r"(r[108]), "r"(r[109]), "r"(r[110]), "r"(r[111]), "r"(r[112]), "r"(r[113]), "r"(r[114]), "r"(r[115]), "r"(r[116]), "r"(r[117]), "r"(r[118]), "r"(r[119]), "r"(r[120]), "r"(r[121]), "r"(r[122]), "r"(r[123]), "r"(r[124]), "r"(r[125]), "r"(r[126]), "r"(r[127]) : "memory");
-}
 __device__ __forceinline__ float ex2_approx(float x) {  // one MUFU op; -inf -> 0
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -183,7 +164,7 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 #define TC_DUMP(...) do { } while (0)
 #endif
 
-constexpr int kThreads = 192;
+constexpr int kThreads = 320;
 constexpr int kTmemCols = 512;
 constexpr int kPageCap = 2560;   // block-table entries staged in shared memory (40960 tokens); longer ranges read the rest from global memory
 
@@ -192,20 +173,35 @@ struct TcKeys { static constexpr int value = D == 256 ? 64 : 128; };  // tokens 
 
 template <int D>
 constexpr int tc_smem_bytes() {
-    // Q tile of 128 rows x D, two stages of K and V tiles of KT tokens x D, P tile of 128 rows x KT keys, barriers
-    // and the staged block table; at least 120 KB so that two CTAs never share an SM (each allocates all 512
+    // Q tile of 128 rows x D, two stages of K and V tiles of KT tokens x D, barriers, the staged block table and the
+    // half-row exchange; at least 120 KB so that two CTAs never share an SM (each allocates all 512
     // tensor-memory columns)
-    constexpr int need = 128 * D * 2 + 2 * 2 * TcKeys<D>::value * D * 2 + 128 * TcKeys<D>::value * 2 + 256 + kPageCap * 4;
+    constexpr int need = 128 * D * 2 + 2 * 2 * TcKeys<D>::value * D * 2 + 256 + kPageCap * 4 + 2 * 128 * 2 * 4 + 64;
     return need < 120 * 1024 ? 120 * 1024 : need;
 }
 
-// KT consecutive columns of this thread's lane
-template <int KT>
-__device__ __forceinline__ void tmem_ld_row(uint32_t taddr, uint32_t (&r)[KT]) {
-    if constexpr (KT == 128) {
-        tmem_ld128(taddr, r);
+// The CTA's work: one TileItem, and what follows from it (both kernels; X counts the item's query tiles).
+struct CtaWork {
+    SeqMeta sm;
+    int seq, h, qt, t0, t1, part, parts, slot_base, cut;
+};
+__device__ __forceinline__ CtaWork load_work(const ChunkArgs& a) {
+    const int4* p = reinterpret_cast<const int4*>(a.tiles + blockIdx.x);
+    const int4 x = __ldg(p), y = __ldg(p + 1);
+    CtaWork w;
+    w.seq = x.x; w.h = x.y; w.qt = x.z; w.t0 = x.w;
+    w.t1 = y.x; w.part = y.y & 0xffff; w.parts = y.y >> 16; w.slot_base = y.z; w.cut = y.w;
+    w.sm = a.step.seq_meta[w.seq];
+    return w;
+}
+
+// N consecutive columns of this thread's lane
+template <int N>
+__device__ __forceinline__ void tmem_ld_row(uint32_t taddr, uint32_t (&r)[N]) {
+    if constexpr (N == 32) {
+        tmem_ld32(taddr, r);
     } else {
-        static_assert(KT == 64, "KV tiles of 64 or 128 tokens");
+        static_assert(N == 64, "half a KV tile: 32 or 64 tokens");
         uint32_t lo[32], hi[32];
         tmem_ld32(taddr, lo);
         tmem_ld32(taddr + 32, hi);
@@ -213,62 +209,160 @@ __device__ __forceinline__ void tmem_ld_row(uint32_t taddr, uint32_t (&r)[KT]) {
         for (int e = 0; e < 32; e++) { r[e] = lo[e]; r[32 + e] = hi[e]; }
     }
 }
+// 16 packed columns of this thread's lane (the caller waits)
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+          "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
+// A operand from tensor memory
+__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+// 32 columns of one output row
+template <bool BF16>
+__device__ __forceinline__ void store_row32(uint16_t* dst, const float (&v)[32], float inv) {
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        uint4 w;
+        w.x = pack2<BF16>(v[u * 8 + 0] * inv, v[u * 8 + 1] * inv);
+        w.y = pack2<BF16>(v[u * 8 + 2] * inv, v[u * 8 + 3] * inv);
+        w.z = pack2<BF16>(v[u * 8 + 4] * inv, v[u * 8 + 5] * inv);
+        w.w = pack2<BF16>(v[u * 8 + 6] * inv, v[u * 8 + 7] * inv);
+        *reinterpret_cast<uint4*>(dst + u * 8) = w;
+    }
+}
+
+// ---- items cut along K/V.  A slice's rows go to memory un-normalised, with each row's (reference exponent, sum);
+// only the rows that exist are written, packed (row = q head * valid tokens + token), the row being the fast index:
+// a warp's accesses are contiguous, and a few tokens' rows cost a few KB, not the whole tile.
+template <int D>
+__device__ __forceinline__ float4* slice_rows(const ChunkArgs& a, int slot, int n_x, int X) {
+    return reinterpret_cast<float4*>(a.split_o) + ((size_t)slot * n_x + X) * (D / 4) * 128;
+}
+// Adds the slices of query tile X up: `rows` packed rows of `nv` tokens per q head, first token r0x.  Every thread of
+// `threads` takes (row, 8 columns) items; the loads of four slices travel together, so an item costs one round trip to
+// L2 per four slices however few rows there are.
+template <int D, bool BF16>
+__device__ __forceinline__ void merge_slices(const ChunkArgs& a, const CtaWork& wk, int n_x, int X, int nv, int r0x, int r, int threads) {
+    const int rows = a.geo.n_rep * nv, n_rep = a.geo.n_rep;
+    for (int idx = r; idx < rows * (D / 8); idx += threads) {
+        const int c8 = idx / rows, row = idx - c8 * rows;
+        float M = -INFINITY, L = 0.f;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+#pragma unroll 1
+        for (int p0 = 0; p0 < wk.parts; p0 += 4) {
+            float2 ml[4];
+            float4 u[4], v[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const bool ok = p0 + q < wk.parts;
+                const int slot = wk.slot_base + p0 + (ok ? q : 0);
+                ml[q] = __ldcg(a.split_ml + ((size_t)slot * n_x + X) * 128 + row);
+                const float4* src = slice_rows<D>(a, slot, n_x, X) + row;
+                u[q] = __ldcg(src + (size_t)(2 * c8) * 128);
+                v[q] = __ldcg(src + (size_t)(2 * c8 + 1) * 128);
+                if (!ok) ml[q] = make_float2(-INFINITY, 0.f);
+            }
+            float Mn = M;
+#pragma unroll
+            for (int q = 0; q < 4; q++) Mn = fmaxf(Mn, ml[q].x);
+            const float so = M == -INFINITY ? 0.f : exp2f(M - Mn);
+            x.x *= so; x.y *= so; x.z *= so; x.w *= so; y.x *= so; y.y *= so; y.z *= so; y.w *= so; L *= so;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                if (ml[q].x == -INFINITY) continue;  // keys this row does not see
+                const float f = exp2f(ml[q].x - Mn);
+                x.x += f * u[q].x; x.y += f * u[q].y; x.z += f * u[q].z; x.w += f * u[q].w;
+                y.x += f * v[q].x; y.y += f * v[q].y; y.z += f * v[q].z; y.w += f * v[q].w;
+                L += f * ml[q].y;
+            }
+            M = Mn;
+        }
+        const float inv = 1.f / L;
+        uint4 w;
+        w.x = pack2<BF16>(x.x * inv, x.y * inv); w.y = pack2<BF16>(x.z * inv, x.w * inv);
+        w.z = pack2<BF16>(y.x * inv, y.y * inv); w.w = pack2<BF16>(y.z * inv, y.w * inv);
+        const int rep = row / nv, tok = r0x + row - rep * nv;
+        uint16_t* orow = reinterpret_cast<uint16_t*>(a.out) + ((size_t)wk.sm.tok_off * a.geo.n_q + (size_t)(wk.h * n_rep + rep) * wk.sm.snew + tok) * D;
+        *reinterpret_cast<uint4*>(orow + c8 * 8) = w;
+    }
+}
+// The CTA's slices are written: draw the item's ticket.  True in every one of the `threads` calling threads (named
+// barrier `bar`, thread `first` among them) when it was the last one.  No CTA waits for another.
+__device__ __forceinline__ bool last_slice(const ChunkArgs& a, const CtaWork& wk, int bar, int threads, bool first, int* s_ticket) {
+    __threadfence();
+    bar_sync(bar, threads);
+    if (first) {
+        const int tk = atomicAdd(a.split_counter + wk.cut, 1);
+        if (tk == wk.parts - 1) a.split_counter[wk.cut] = 0;  // ready for the next launch
+        *s_ticket = tk;
+        __threadfence();
+    }
+    bar_sync(bar, threads);
+    return *s_ticket == wk.parts - 1;
+}
 
 }  // namespace
 
 template <int D, bool BF16>
-__global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmap32, const ChunkArgs a) {
-    constexpr uint32_t TILE = 128u * D * 2u;   // one operand tile (Q, K or V)
-    constexpr uint32_t BLK = 128u * 128u;      // one 64-element column block of a tile: 128 rows x 128 bytes
+__global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constant__ CUtensorMap tmap32, const ChunkArgs a) {
+    constexpr uint32_t TILE = 128u * D * 2u;   // the Q tile
+    constexpr uint32_t BLK = 128u * 128u;      // one 64-element column block of it: 128 rows x 128 bytes
     constexpr int XB = D / 64;                 // column blocks per row
     extern __shared__ __align__(1024) uint8_t smem[];
-    constexpr int KT = TcKeys<D>::value;           // tokens per KV tile
+    constexpr int KT = TcKeys<D>::value;       // tokens per KV tile
+    constexpr int HK = KT / 2;                 // keys of a softmax thread
     constexpr int PPT = KT / 16;               // pages per KV tile
     constexpr uint32_t BLKKV = PPT * 4096u;    // one 64-column block of a K/V stage: PPT pages x 32 rows x 128 bytes
     constexpr uint32_t STAGE = 2u * KT * D * 2u;  // K and V of KT tokens
     uint8_t* sQ = smem;
     uint8_t* sKV = sQ + TILE;           // 2 stages
-    uint8_t* sP = sKV + 2 * STAGE;      // 128 rows x KT keys
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sP + 128 * KT * 2);
-    // barriers: kv_full[2], kv_empty[2], s_full[2], p_full, o_done
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + 2 * STAGE);
+    // barriers: kv_full[2], kv_empty[2], s_full[2], p_full[2], o_done
     const uint32_t b_kv_full = smem_u32(bars + 0), b_kv_empty = smem_u32(bars + 2), b_s_full = smem_u32(bars + 4);
-    const uint32_t b_p_full = smem_u32(bars + 6), b_o_done = smem_u32(bars + 7);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
-    volatile int* failed = reinterpret_cast<volatile int*>(bars + 9);
+    const uint32_t b_p_full = smem_u32(bars + 6), b_o_done = smem_u32(bars + 8);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
+    volatile int* failed = reinterpret_cast<volatile int*>(bars + 11);
+    int* s_ticket = reinterpret_cast<int*>(bars + 12);
     int* s_pages = reinterpret_cast<int*>(bars + 16);   // [kPageCap] physical pages of the KV range
+    float* s_xch = reinterpret_cast<float*>(s_pages + kPageCap);  // [2 buffers][128 rows][2 halves]
+    int* s_pair = reinterpret_cast<int*>(s_xch + 2 * 128 * 2);    // [4] a wait of this pair of warps ran out
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if ((smem_u32(smem) & 1023u) != 0) {
         if (tid == 0) atomicOr(a.status, ST_SMEM_ALIGN);
         return;
     }
-    // ---- which (sequence, kv head, query tile)
-    const int item = blockIdx.x;
-    int lo = 0, hi = a.step.n_seqs - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (a.item_begin[mid] <= item) lo = mid; else hi = mid - 1;
-    }
-    const SeqMeta sm = a.step.seq_meta[lo];
-    const int Hkv = a.geo.n_kv, n_rep = a.geo.n_rep, RS = a.rep_slots, TPT = 128 / RS;
-    const int n_qt = (sm.snew + TPT - 1) / TPT;
-    const int local = item - a.item_begin[lo];
-    const int h = local / n_qt, qt = local - h * n_qt;
-    const int r0 = qt * TPT;                               // first new token of the tile
-    const int r_last = min(r0 + TPT, sm.snew) - 1;
-    const int q_min = sm.pos + r0, q_max = sm.pos + r_last;
+    // ---- which (sequence, kv head, query tile), which slice of its K/V tiles
+    const CtaWork wk = load_work(a);
+    const SeqMeta sm = wk.sm;
+    const int Hkv = a.geo.n_kv, n_rep = a.geo.n_rep, RS = a.rep_slots, TPT = 128 / RS, h = wk.h;
+    const int r0 = wk.qt * TPT;                            // first new token of the tile
+    const int nv = min(TPT, sm.snew - r0);                 // tokens of it
+    const int q_min = sm.pos + r0, q_max = q_min + nv - 1;
     const int lo_key = a.window > 0 ? max(0, q_min - a.window + 1) : 0;
-    const int p_lo = lo_key >> 4, p_hi = q_max >> 4;
-    const int n_tiles = (p_hi - p_lo + 1 + PPT - 1) / PPT;
+    const int p_lo = (lo_key >> 4) + wk.t0 * PPT, p_hi = min(q_max >> 4, (lo_key >> 4) + wk.t1 * PPT - 1);
+    const int n_tiles = wk.t1 - wk.t0;
     const int k0 = p_lo * 16;                               // absolute position of key 0 of tile 0
 
     if (tid == 0) {
-        for (int i = 0; i < 2; i++) { mbar_init(b_kv_full + i * 8, 1); mbar_init(b_kv_empty + i * 8, 1); mbar_init(b_s_full + i * 8, 1); }
-        mbar_init(b_p_full, 128);
+        for (int i = 0; i < 2; i++) {
+            mbar_init(b_kv_full + i * 8, 1); mbar_init(b_kv_empty + i * 8, 1); mbar_init(b_s_full + i * 8, 1);
+            mbar_init(b_p_full + i * 8, 256);
+        }
         mbar_init(b_o_done, 1);
         *failed = 0;
+        for (int i = 0; i < 4; i++) s_pair[i] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap32) : "memory");
     }
     if (warp == 0) {  // tensor memory for this CTA
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
@@ -280,10 +374,10 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
         const uint16_t* qbase = reinterpret_cast<const uint16_t*>(a.q) + (size_t)sm.tok_off * a.geo.n_q * D;
         for (int c = tid; c < 128 * (D / 8); c += kThreads) {
             const int m = c / (D / 8), j = c - m * (D / 8);   // row, 16-byte piece
-            const int rep = m / TPT, r = r0 + (m - rep * TPT);
+            const int rep = m / TPT, i = m - rep * TPT;
             uint4 val = make_uint4(0, 0, 0, 0);
-            if (rep < n_rep && r < sm.snew)
-                val = *reinterpret_cast<const uint4*>(qbase + ((size_t)(h * n_rep + rep) * sm.snew + r) * D + j * 8);
+            if (rep < n_rep && i < nv)
+                val = *reinterpret_cast<const uint4*>(qbase + ((size_t)(h * n_rep + rep) * sm.snew + r0 + i) * D + j * 8);
             const uint32_t off = (j >> 3) * BLK + m * 128u + (((j & 7) ^ (m & 7)) << 4);
             *reinterpret_cast<uint4*>(sQ + off) = val;
         }
@@ -298,8 +392,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
         // The block-table entries of the whole KV range were staged in shared memory by all
-        // threads (below the Q load); every lane issues one box of a tile: lane = page * (2 XB) +
-        // column block * 2 + (K or V).
+        // threads (below the Q load); every lane issues boxes of a tile: one per (page, column block).
         bool ok = true;
         long long tprev = TC_NOW(), c_wait = 0, c_issue = 0;
 #pragma unroll 1
@@ -333,7 +426,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
             // descriptors differ only in the start address field (bits 0-13, address >> 4)
             // K: 8-row groups 2048 bytes apart; V: the same groups 1024 bytes further, 64-wide d blocks BLKKV apart
             const uint64_t dq = smem_desc(smem_u32(sQ), 16, 1024), dk = smem_desc(smem_u32(sKV), 16, 2048);
-            const uint64_t dp = smem_desc(smem_u32(sP), 16, 1024), dv = smem_desc(smem_u32(sKV) + 1024, BLKKV, 2048);
+            const uint64_t dv = smem_desc(smem_u32(sKV) + 1024, BLKKV, 2048);
             auto issue_qk = [&](int j) {
                 const uint64_t kst = (uint64_t)(((j & 1) * STAGE) >> 4);
 #pragma unroll
@@ -350,6 +443,8 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
             if (ok) { tc_fence_after(); issue_qk(0); }
             for (int j = 0; ok && j < n_tiles; j++) {
                 if (j + 1 < n_tiles) {
+                    // scores of the next tile first: they are computed while this tile's softmax runs.  They go to
+                    // the other S buffer, whose P the previous P V (issued before) was the last to read.
                     TC_ACC(c_iss);
                     ok = mbar_wait_bounded(b_kv_full + ((j + 1) & 1) * 8, ((j + 1) >> 1) & 1);
                     TC_ACC(c_wkv);
@@ -358,18 +453,15 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
                     issue_qk(j + 1);
                 }
                 TC_ACC(c_iss);
-                ok = mbar_wait_bounded(b_p_full, j & 1) && !*failed;
+                ok = mbar_wait_bounded(b_p_full + (j & 1) * 8, (j >> 1) & 1) && !*failed;
                 TC_ACC(c_wp);
                 if (!ok) break;
                 tc_fence_after();
                 const int st = j & 1;
                 const uint64_t vst = (uint64_t)((st * STAGE) >> 4);
 #pragma unroll
-                for (int ks = 0; ks < PPT; ks++) {  // 16 keys per step = one page
-                    // P: K-major, keys 16 ks.. inside key block ks / 4; V: MN-major, one page (4096 bytes) per step
-                    umma(tO, dp + (uint64_t)(((ks >> 2) * BLK + (ks & 3) * 32) >> 4), dv + vst + (uint64_t)((ks * 4096) >> 4), id_pv,
-                         (j > 0 || ks > 0));
-                }
+                for (int ks = 0; ks < PPT; ks++)  // 16 keys per step = one page; P: 8 packed columns, V: MN-major, 4096 bytes per step
+                    umma_ts(tO, tS0 + st * 128 + ks * 8, dv + vst + (uint64_t)((ks * 4096) >> 4), id_pv, (j > 0 || ks > 0));
                 umma_commit(b_kv_empty + st * 8);
                 umma_commit(b_o_done);
             }
@@ -377,103 +469,103 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
             TC_DUMP(a.dbg_buf[(size_t)blockIdx.x * 16 + 2] = c_wkv; a.dbg_buf[(size_t)blockIdx.x * 16 + 3] = c_wp; a.dbg_buf[(size_t)blockIdx.x * 16 + 4] = c_iss;);
         }
     } else {
-        // ------------------------------------------------------------ softmax + epilogue, one row per thread
+        // ------------------------------------------------------------ softmax + epilogue: two threads per row
+        // The warps come in pairs that may touch the same quarter of the tensor-memory lanes; H = 0 takes the first
+        // half of a tile's keys and of the O columns, H = 1 the second.
+        const int H = (warp - 2) >> 2;
         const int lane_base = (warp & 3) * 32;             // the TMEM lanes this warp may touch
         const int m = lane_base + lane;                    // row of the tile
-        const int rep = m / TPT, r = r0 + (m - rep * TPT);
-        const bool row_ok = rep < n_rep && r < sm.snew;
-        const int q_pos = sm.pos + min(r, sm.snew - 1);    // rows past the data mimic the last token
+        const int rep = m / TPT, i = m - rep * TPT;
+        const bool row_ok = rep < n_rep && i < nv;
+        const int q_pos = q_min + min(i, nv - 1);          // rows past the data mimic the last token
         const uint32_t lane_addr = (uint32_t)lane_base << 16;
+        const int pair_bar = 1 + (warp & 3);
+        // A named barrier has no time limit, so the two warps of a pair must leave the loop in the same
+        // iteration: whichever sees a wait run out says so here before the pair's barrier, both read it after.
+        volatile int* pair_failed = s_pair + (warp & 3);
         // Exponents are taken against a reference maximum that is only moved when a row's maximum
         // exceeds it by more than 8 (a factor 256): probabilities then stay below 256, exact enough in
         // f16/bf16 with f32 sums, and O needs rescaling only on those rare moves.
-        float m_ref = -INFINITY, l_run = 0.f;
+        float m_ref = -INFINITY, l_run = 0.f;              // l_run: this half's share of the row sum
         bool ok = true;
         long long tprev = TC_NOW(), c_ws = 0, c_ld = 0, c_exp = 0, c_wo = 0, c_st = 0;
         const long long tstart = tprev;
 #pragma unroll 1
         for (int j = 0; j < n_tiles; j++) {
             ok = mbar_wait_bounded(b_s_full + (j & 1) * 8, (j >> 1) & 1) && !*failed;
-            ok = __all_sync(0xffffffffu, ok);  // the tensor-memory accesses below need the whole warp
+            ok = __all_sync(0xffffffffu, ok);
             TC_ACC(c_ws);
-            if (!ok) break;
+            if (!ok && lane == 0) *pair_failed = 1;  // the loads below then read stale columns: harmless, nothing is kept
             tc_fence_after();
             const uint32_t tS = tS0 + (j & 1) * 128 + lane_addr;
-            const int kbase = k0 + j * KT;
-            const bool need_mask = (kbase + KT - 1 > q_min) || (a.window > 0 && kbase + a.window <= q_max);
-            uint32_t sv[KT];
-            tmem_ld_row<KT>(tS, sv);
-            TC_ACC(c_ld);
-            float mx = -INFINITY;
+            const int kbase = k0 + j * KT + H * HK;
+            const bool need_mask = (kbase + HK - 1 > q_min) || (a.window > 0 && kbase + a.window <= q_max);
+            uint32_t sv[HK];
+            tmem_ld_row<HK>(tS + H * HK, sv);
             if (need_mask) {
 #pragma unroll
-                for (int e = 0; e < KT; e++) {
+                for (int e = 0; e < HK; e++) {
                     const int kp = kbase + e;
                     if (!(kp <= q_pos && (a.window <= 0 || kp + a.window > q_pos))) sv[e] = 0xff800000u;  // -inf
                 }
             }
+            float mx;
             {
                 float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
 #pragma unroll
-                for (int e = 0; e < KT; e += 4) {
+                for (int e = 0; e < HK; e += 4) {
                     m0 = fmaxf(m0, __uint_as_float(sv[e])); m1 = fmaxf(m1, __uint_as_float(sv[e + 1]));
                     m2 = fmaxf(m2, __uint_as_float(sv[e + 2])); m3 = fmaxf(m3, __uint_as_float(sv[e + 3]));
                 }
                 mx = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
             }
-            mx *= a.scale_log2;  // scale > 0: the maximum commutes with the scaling
+            float* xrow = s_xch + ((j & 1) * 128 + m) * 2;
+            xrow[H] = mx;
+            bar_sync(pair_bar, 64);  // also: both warps have their S columns in registers, so P may overwrite them
+            mx = fmaxf(mx, xrow[H ^ 1]) * a.scale_log2;  // scale > 0: the maximum commutes with the scaling
+            if (*pair_failed) { ok = false; break; }     // both warps of the pair, in the same iteration
+            TC_ACC(c_ld);
             float alpha = 1.f;
-            if (mx > m_ref + 8.f || m_ref == -INFINITY) {
-                const float m_new = mx;
-                alpha = (m_ref == -INFINITY) ? 0.f : exp2f(m_ref - m_new);
-                m_ref = m_new;
+            if (mx > m_ref + 8.f || m_ref == -INFINITY) {  // both halves see the same mx: the same decision
+                alpha = (m_ref == -INFINITY) ? 0.f : exp2f(m_ref - mx);
+                m_ref = mx;
             }
             const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
             float sum = 0.f, sum2 = 0.f;
-            uint32_t pk[KT / 2];
 #pragma unroll
-            for (int e = 0; e < KT; e += 2) {
+            for (int e = 0; e < HK; e += 2) {
                 const float p0 = ex2_approx(fmaf(__uint_as_float(sv[e]), a.scale_log2, -m_use));
                 const float p1 = ex2_approx(fmaf(__uint_as_float(sv[e + 1]), a.scale_log2, -m_use));
                 if (e & 2) sum2 += p0 + p1; else sum += p0 + p1;  // two chains
-                pk[e >> 1] = pack2<BF16>(p0, p1);
+                sv[e >> 1] = pack2<BF16>(p0, p1);  // P pair e/2 reuses a register whose score is already consumed
             }
+#pragma unroll
+            for (int c = 0; c < HK / 32; c++) tmem_st16(tS + H * (HK / 2) + c * 16, sv + c * 16);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             l_run = l_run * alpha + (sum + sum2);
             TC_ACC(c_exp);
-            // the previous P V must be finished before P is overwritten and O rescaled
-            if (j > 0) {
-                ok = mbar_wait_bounded(b_o_done, (j - 1) & 1) && !*failed;
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                tc_fence_after();
-            }
-            TC_ACC(c_wo);
-#pragma unroll
-            for (int u = 0; u < KT / 8; u++) {  // 16-byte pieces of 8 keys, K-major swizzled
-                const uint32_t off = (u >> 3) * BLK + m * 128u + (((u & 7) ^ (m & 7)) << 4);
-                *reinterpret_cast<uint4*>(sP + off) = make_uint4(pk[u * 4], pk[u * 4 + 1], pk[u * 4 + 2], pk[u * 4 + 3]);
-            }
+            // O may be rescaled once the previous P V is complete.  (S being full says that of the one before it
+            // only, so this wait is at most one phase ahead of the barrier.)
             if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-                if constexpr (D == 128) {
-                    uint32_t ov[128];
-                    tmem_ld128(tO + lane_addr, ov);
-#pragma unroll
-                    for (int e = 0; e < 128; e++) ov[e] = __float_as_uint(__uint_as_float(ov[e]) * alpha);
-                    tmem_st128(tO + lane_addr, ov);
+                bool done = mbar_wait_bounded(b_o_done, (j - 1) & 1) && !*failed;
+                done = __all_sync(0xffffffffu, done);
+                TC_ACC(c_wo);
+                if (!done) {
+                    if (lane == 0) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
                 } else {
+                    tc_fence_after();
 #pragma unroll 1
-                    for (int c = 0; c < D / 32; c++) {
+                    for (int c = 0; c < D / 64; c++) {
                         uint32_t v[32];
-                        tmem_ld32(tO + lane_addr + c * 32, v);
+                        tmem_ld32(tO + lane_addr + H * (D / 2) + c * 32, v);
 #pragma unroll
                         for (int e = 0; e < 32; e++) v[e] = __float_as_uint(__uint_as_float(v[e]) * alpha);
-                        tmem_st32(tO + lane_addr + c * 32, v);
+                        tmem_st32(tO + lane_addr + H * (D / 2) + c * 32, v);
                     }
                 }
             }
-            fence_proxy_async();   // P for the async proxy
             tc_fence_before();     // the tensor-memory traffic above is ordered before the hand-over
-            mbar_arrive(b_p_full);
+            mbar_arrive(b_p_full + (j & 1) * 8);
             TC_ACC(c_st);
         }
         TC_DUMP(if (tid == 64) {
@@ -481,33 +573,53 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
             b[5] = c_ws; b[6] = c_ld; b[7] = c_exp; b[8] = c_wo; b[9] = c_st; b[10] = TC_NOW() - tstart;
         });
         (void)tstart; (void)c_wo;
-        // ---- epilogue: O / l -> out
+        // ---- epilogue: O / l -> out, or a slice's partial rows
         if (ok) ok = mbar_wait_bounded(b_o_done, (n_tiles - 1) & 1) && !*failed;
         ok = __all_sync(0xffffffffu, ok);
-        if (ok) {
-            tc_fence_after();
-            const float inv = 1.f / l_run;
-            uint16_t* orow = reinterpret_cast<uint16_t*>(a.out) +
-                             ((size_t)sm.tok_off * a.geo.n_q + (size_t)(h * n_rep + (row_ok ? rep : 0)) * sm.snew + (row_ok ? r : 0)) * D;
-#pragma unroll 1
-            for (int c = 0; c < D / 32; c++) {
-                uint32_t v[32];
-                tmem_ld32(tO + lane_addr + c * 32, v);
-                if (row_ok) {
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        uint4 w;
-                        w.x = pack2<BF16>(__uint_as_float(v[u * 8 + 0]) * inv, __uint_as_float(v[u * 8 + 1]) * inv);
-                        w.y = pack2<BF16>(__uint_as_float(v[u * 8 + 2]) * inv, __uint_as_float(v[u * 8 + 3]) * inv);
-                        w.z = pack2<BF16>(__uint_as_float(v[u * 8 + 4]) * inv, __uint_as_float(v[u * 8 + 5]) * inv);
-                        w.w = pack2<BF16>(__uint_as_float(v[u * 8 + 6]) * inv, __uint_as_float(v[u * 8 + 7]) * inv);
-                        *reinterpret_cast<uint4*>(orow + c * 32 + u * 8) = w;
-                    }
-                }
-            }
-        } else if (lane == 0) {
+        float* xrow = s_xch + ((n_tiles & 1) * 128 + m) * 2;
+        xrow[H] = l_run;
+        bar_sync(pair_bar, 64);
+        const float l_row = l_run + xrow[H ^ 1];
+        if (!ok && lane == 0) {
             *failed = 1;
             atomicOr(a.status, ST_WAIT_TIMEOUT);
+        }
+        tc_fence_after();
+        if (wk.parts == 1) {
+            if (ok) {
+                const float inv = 1.f / l_row;
+                uint16_t* orow = reinterpret_cast<uint16_t*>(a.out) +
+                                 ((size_t)sm.tok_off * a.geo.n_q + (size_t)(h * n_rep + (row_ok ? rep : 0)) * sm.snew + (row_ok ? r0 + i : 0)) * D;
+#pragma unroll 1
+                for (int c = H * (D / 64); c < (H + 1) * (D / 64); c++) {
+                    uint32_t v[32];
+                    tmem_ld32(tO + lane_addr + c * 32, v);
+                    float f[32];
+#pragma unroll
+                    for (int e = 0; e < 32; e++) f[e] = __uint_as_float(v[e]);
+                    if (row_ok) store_row32<BF16>(orow + c * 32, f, inv);
+                }
+            }
+        } else {
+            const int slot = wk.slot_base + wk.part, prow = rep * nv + i;
+            if (ok) {
+                float4* rows = slice_rows<D>(a, slot, 1, 0) + prow;
+#pragma unroll 1
+                for (int c = H * (D / 64); c < (H + 1) * (D / 64); c++) {
+                    uint32_t v[32];
+                    tmem_ld32(tO + lane_addr + c * 32, v);
+                    if (row_ok) {
+#pragma unroll
+                        for (int u = 0; u < 8; u++)
+                            rows[(size_t)(c * 8 + u) * 128] = make_float4(__uint_as_float(v[u * 4]), __uint_as_float(v[u * 4 + 1]),
+                                                                          __uint_as_float(v[u * 4 + 2]), __uint_as_float(v[u * 4 + 3]));
+                    }
+                }
+                if (H == 0 && row_ok) a.split_ml[(size_t)slot * 128 + prow] = make_float2(m_ref, l_row);
+            }
+            // every softmax warp passes the barriers whatever happened to its waits
+            if (last_slice(a, wk, 9, 256, tid == 64, s_ticket) && !*failed)
+                merge_slices<D, BF16>(a, wk, 1, 0, nv, r0, tid - 64, 256);
         }
     }
     // ---- wind down: everybody meets, then the allocating warp frees the tensor memory
@@ -520,9 +632,9 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
 }
 
 template <int D, bool BF16>
-static cudaError_t launch_tc(const CUtensorMap& map, const CUtensorMap& map32, const ChunkArgs& a, cudaStream_t st) {
+static cudaError_t launch_tc(const CUtensorMap& map32, const ChunkArgs& a, cudaStream_t st) {
     if (a.n_items <= 0) return cudaSuccess;
-    chunk_tc_kernel<D, BF16><<<a.n_items, kThreads, tc_smem_bytes<D>(), st>>>(map, map32, a);
+    chunk_tc_kernel<D, BF16><<<a.n_items, kThreads, tc_smem_bytes<D>(), st>>>(map32, a);
     return cudaGetLastError();
 }
 
@@ -550,14 +662,6 @@ template <int D>
 constexpr int tc2_smem_bytes() {
     return 2 * 128 * D * 2 /* Q_A, Q_B */ + 2 * 2 * 128 * D * 2 /* two K/V stages */ + 256 + kPageCap * 4 +
            2 * 2 * 128 * 2 * 4 /* half-row maxima of both tiles, double-buffered */ + 64 /* the pairs' failure flags */;
-}
-
-__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
 // Q8: the layer holds int8 records (kernels.hpp, qrec_*) and the kernel converts them itself
@@ -623,32 +727,18 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         if (tid == 0) atomicOr(a.status, ST_SMEM_ALIGN);
         return;
     }
-    // CTAs past split_first share items: `parts` of them per item, each with a slice of the item's K/V tiles
-    const int parts = (a.split_parts > 1 && (int)blockIdx.x >= a.split_first) ? a.split_parts : 1;
-    const int item = parts > 1 ? a.split_first + ((int)blockIdx.x - a.split_first) / parts : (int)blockIdx.x;
-    const int part = parts > 1 ? ((int)blockIdx.x - a.split_first) % parts : 0;
-    int lo = 0, hi = a.step.n_seqs - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (a.item_begin[mid] <= item) lo = mid; else hi = mid - 1;
-    }
-    const SeqMeta sm = a.step.seq_meta[lo];
-    const int Hkv = a.geo.n_kv, n_rep = a.geo.n_rep, RS = a.rep_slots, TPT = 128 / RS;
-    const int n_qt = (sm.snew + 2 * TPT - 1) / (2 * TPT);        // pairs of tiles
-    const int local = item - a.item_begin[lo];
-    const int h = local / n_qt, qt = local - h * n_qt;
-    const int r0 = qt * 2 * TPT;                                  // first new token of tile A
+    // ---- which (sequence, kv head, pair of query tiles), which slice of its K/V tiles
+    const CtaWork wk = load_work(a);
+    const SeqMeta sm = wk.sm;
+    const int Hkv = a.geo.n_kv, n_rep = a.geo.n_rep, RS = a.rep_slots, TPT = 128 / RS, h = wk.h;
+    const int r0 = wk.qt * 2 * TPT;                               // first new token of tile A
     const int q_first = sm.pos + r0, q_last = sm.pos + min(r0 + 2 * TPT, sm.snew) - 1;
+    // With no more tokens than one tile holds (verifying a draft, the decoding sequences of a mixed step), tile B is
+    // left out altogether: the chain of one tile is then shorter than the time its K/V takes to arrive.
+    const bool two = sm.snew - r0 > TPT;
     const int lo_key = a.window > 0 ? max(0, q_first - a.window + 1) : 0;
-    int p_lo = lo_key >> 4, p_hi = q_last >> 4;
-    int n_tiles = (p_hi - p_lo + 1 + 7) >> 3;
-    if (parts > 1) {  // this CTA's slice of the tiles (possibly empty: it then hands over rows with sum 0)
-        const int per = (n_tiles + parts - 1) / parts;
-        const int t0 = min(n_tiles, part * per), t1 = min(n_tiles, t0 + per);
-        if (t1 < n_tiles) p_hi = p_lo + 8 * t1 - 1;  // inner slices end on a tile boundary: every page is real
-        p_lo += 8 * t0;
-        n_tiles = t1 - t0;
-    }
+    const int p_lo = (lo_key >> 4) + 8 * wk.t0, p_hi = min(q_last >> 4, (lo_key >> 4) + 8 * wk.t1 - 1);
+    const int n_tiles = wk.t1 - wk.t0;
     const int k0 = p_lo * 16;
 
     if (tid == 0) {
@@ -674,7 +764,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     // ---- Q tiles: row m of tile X is q head (m / TPT) at token r0 + X TPT + m % TPT
     {
         const uint16_t* qbase = reinterpret_cast<const uint16_t*>(a.q) + (size_t)sm.tok_off * a.geo.n_q * D;
-        for (int c = tid; c < 256 * (D / 8); c += (int)blockDim.x) {
+        for (int c = tid; c < (two ? 256 : 128) * (D / 8); c += (int)blockDim.x) {
             const int mm = c / (D / 8), j = c - mm * (D / 8);
             const int X = mm >> 7, m = mm & 127;
             const int rep = m / TPT, r = r0 + X * TPT + (m - rep * TPT);
@@ -846,7 +936,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                     umma(tmem + X * 128, dq + qst + qoff, dk + kst + koff, id_qk, ks > 0);
                 }
                 umma_commit(b_s_full + X * 8);
-                if (Q8 && X == 1) umma_commit(b_kv_empty + (j & 1) * 8);  // both tiles' scores of this K buffer have been issued
+                if (Q8 && X == (two ? 1 : 0)) umma_commit(b_kv_empty + (j & 1) * 8);  // all scores of this K buffer have been issued
             };
             auto issue_pv = [&](int X, int j) {
                 const uint64_t vst = Q8 ? 0ull : (uint64_t)(((j & 1) * STAGE) >> 4);
@@ -856,8 +946,8 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                 umma_commit(b_o_done + X * 8);
             };
             long long tprev = TC_NOW(), c_wkv = 0, c_wp = 0, c_iss = 0, c_pv = 0;
-            bool ok = n_tiles == 0 || mbar_wait_bounded(b_kv_full, 0);  // an empty slice of a cut item: nothing to issue
-            if (ok && n_tiles > 0) { tc_fence_after(); issue_qk(0, 0); issue_qk(1, 0); }
+            bool ok = mbar_wait_bounded(b_kv_full, 0);
+            if (ok) { tc_fence_after(); issue_qk(0, 0); if (two) issue_qk(1, 0); }
             for (int j = 0; ok && j < n_tiles; j++) {
                 TC_ACC(c_iss);
                 ok = mbar_wait_bounded(b_p_full, j & 1) && !*failed;
@@ -867,6 +957,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                 tc_fence_after();
                 issue_pv(0, j);
                 TC_ACC(c_pv);
+                if (!two && !Q8) umma_commit(b_kv_empty + (j & 1) * 8);
                 if (j + 1 < n_tiles) {
                     ok = mbar_wait_bounded(b_kv_full + ((j + 1) & 1) * 8, ((j + 1) >> 1) & 1);
                     TC_ACC(c_wkv);
@@ -875,22 +966,24 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                     issue_qk(0, j + 1);
                 }
                 TC_ACC(c_iss);
-                ok = mbar_wait_bounded(b_p_full + 8, j & 1) && !*failed;
-                TC_ACC(c_wp);
-                if (!ok) break;
-                tc_fence_after();
-                issue_pv(1, j);
-                TC_ACC(c_pv);
+                if (two) {
+                    ok = mbar_wait_bounded(b_p_full + 8, j & 1) && !*failed;
+                    TC_ACC(c_wp);
+                    if (!ok) break;
+                    tc_fence_after();
+                    issue_pv(1, j);
+                    TC_ACC(c_pv);
+                }
                 // every read of this stage (int8 layer: of the V buffer) has been issued before
-                umma_commit(Q8 ? b_v_empty : b_kv_empty + (j & 1) * 8);
-                if (j + 1 < n_tiles) issue_qk(1, j + 1);
+                if (two || Q8) umma_commit(Q8 ? b_v_empty : b_kv_empty + (j & 1) * 8);
+                if (two && j + 1 < n_tiles) issue_qk(1, j + 1);
             }
             if (!ok) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
             (void)c_pv;
             TC_DUMP(a.dbg_buf[(size_t)blockIdx.x * 16 + 2] = c_wkv; a.dbg_buf[(size_t)blockIdx.x * 16 + 3] = c_wp; a.dbg_buf[(size_t)blockIdx.x * 16 + 4] = c_iss;
                     a.dbg_buf[(size_t)blockIdx.x * 16 + 11] = c_pv;);
         }
-    } else if (warp >= 2 && warp < 18) {
+    } else if (warp >= 2 && warp < (two ? 18 : 10)) {
         // ------------------------------------------------------------ softmax + epilogue of tile X, half H of the keys
         const int X = (warp - 2) >> 3, H = ((warp - 2) >> 2) & 1;
         const int lane_base = (warp & 3) * 32;  // the quarter of the tensor-memory lanes this warp may touch
@@ -963,13 +1056,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                 sv[e >> 1] = pack2<BF16>(p0, p1);  // P pair e/2 reuses a register whose score is already consumed
             }
 #pragma unroll
-            for (int c = 0; c < 2; c++) {  // keys 64 H .. 64 H + 63 are packed columns 32 H .. 32 H + 31 of P
-                asm volatile(
-                    "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-                    ::"r"(tS + H * 32 + c * 16), "r"(sv[c * 16 + 0]), "r"(sv[c * 16 + 1]), "r"(sv[c * 16 + 2]), "r"(sv[c * 16 + 3]), "r"(sv[c * 16 + 4]),
-                      "r"(sv[c * 16 + 5]), "r"(sv[c * 16 + 6]), "r"(sv[c * 16 + 7]), "r"(sv[c * 16 + 8]), "r"(sv[c * 16 + 9]), "r"(sv[c * 16 + 10]),
-                      "r"(sv[c * 16 + 11]), "r"(sv[c * 16 + 12]), "r"(sv[c * 16 + 13]), "r"(sv[c * 16 + 14]), "r"(sv[c * 16 + 15]) : "memory");
-            }
+            for (int c = 0; c < 2; c++) tmem_st16(tS + H * 32 + c * 16, sv + c * 16);  // keys 64 H .. 64 H + 63 are packed columns 32 H .. 32 H + 31 of P
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             l_run = l_run * alpha + (sum + sum2);
             TC_ACC(c_exp);
@@ -996,7 +1083,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         });
         const long long t_loop_end = TC_NOW();
         (void)tstart; (void)c_wo; (void)t_loop_end;
-        if (ok && n_tiles > 0) ok = mbar_wait_bounded(b_o_done + X * 8, (n_tiles - 1) & 1) && !*failed;
+        if (ok) ok = mbar_wait_bounded(b_o_done + X * 8, (n_tiles - 1) & 1) && !*failed;
         ok = __all_sync(0xffffffffu, ok);
         // the row sum is the two halves' sums (exchanged whether or not the wait succeeded: the pair must
         // meet at its barrier the same number of times)
@@ -1010,18 +1097,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         }
         uint16_t* orow = reinterpret_cast<uint16_t*>(a.out) +
                          ((size_t)sm.tok_off * a.geo.n_q + (size_t)(h * n_rep + (row_ok ? rep : 0)) * sm.snew + (row_ok ? r : 0)) * D;
-        auto store_row = [&](int c, const float (&v)[32], float inv) {  // 32 output columns from c * 32
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                uint4 w;
-                w.x = pack2<BF16>(v[u * 8 + 0] * inv, v[u * 8 + 1] * inv);
-                w.y = pack2<BF16>(v[u * 8 + 2] * inv, v[u * 8 + 3] * inv);
-                w.z = pack2<BF16>(v[u * 8 + 4] * inv, v[u * 8 + 5] * inv);
-                w.w = pack2<BF16>(v[u * 8 + 6] * inv, v[u * 8 + 7] * inv);
-                *reinterpret_cast<uint4*>(orow + c * 32 + u * 8) = w;
-            }
-        };
-        if (parts == 1) {
+        if (wk.parts == 1) {
             if (ok) {
                 tc_fence_after();
                 const float inv = 1.f / l_row;
@@ -1032,72 +1108,34 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                     float f[32];
 #pragma unroll
                     for (int e = 0; e < 32; e++) f[e] = __uint_as_float(v[e]);
-                    if (row_ok) store_row(c, f, inv);
+                    if (row_ok) store_row32<BF16>(orow + c * 32, f, inv);
                 }
             }
         } else {
             // ---- a slice of a cut item: un-normalised rows and their (reference exponent, sum) go to memory, the
             // CTA draws a ticket, and the CTA that draws the item's last one adds the slices up.  No CTA waits
             // for another; every softmax warp passes both barriers whatever happened to its waits.
-            const int cut = item - a.split_first;
-            // rows are the fast index of the partial rows in memory (split_o as float4 [slice][tile][32 column
-            // groups][128 rows]): a warp's 32 rows make one contiguous 512-byte access
-            const size_t mine = ((size_t)(cut * parts + part) * 2 + X) * 128 + m;
-            float4* my_o = reinterpret_cast<float4*>(a.split_o) + ((size_t)(cut * parts + part) * 2 + X) * 32 * 128 + m;
+            const int slot = wk.slot_base + wk.part;
+            const int nv = min(TPT, sm.snew - r0 - X * TPT), prow = rep * nv + (m - rep * TPT);
             if (ok) {
-                if (n_tiles > 0) {
-                    tc_fence_after();
+                tc_fence_after();
+                float4* rows = slice_rows<D>(a, slot, 2, X) + prow;
 #pragma unroll 1
-                    for (int c = 2 * H; c < 2 * H + 2; c++) {
-                        uint32_t v[32];
-                        tmem_ld32(tO + c * 32, v);
+                for (int c = 2 * H; c < 2 * H + 2; c++) {
+                    uint32_t v[32];
+                    tmem_ld32(tO + c * 32, v);
+                    if (row_ok) {
 #pragma unroll
                         for (int u = 0; u < 8; u++)
-                            my_o[(size_t)(c * 8 + u) * 128] = make_float4(__uint_as_float(v[u * 4]), __uint_as_float(v[u * 4 + 1]),
+                            rows[(size_t)(c * 8 + u) * 128] = make_float4(__uint_as_float(v[u * 4]), __uint_as_float(v[u * 4 + 1]),
                                                                           __uint_as_float(v[u * 4 + 2]), __uint_as_float(v[u * 4 + 3]));
                     }
                 }
-                if (H == 0) a.split_ml[mine] = make_float2(n_tiles > 0 ? m_ref : -INFINITY, n_tiles > 0 ? l_row : 0.f);
+                if (H == 0 && row_ok) a.split_ml[((size_t)slot * 2 + X) * 128 + prow] = make_float2(m_ref, l_row);
             }
-            __threadfence();
-            asm volatile("bar.sync 9, 512;" ::: "memory");
             int* s_ticket = reinterpret_cast<int*>(const_cast<int*>(failed)) + 1;
-            if (tid == 64) {
-                const int tk = atomicAdd(a.split_counter + cut, 1);
-                if (tk == parts - 1) a.split_counter[cut] = 0;  // ready for the next launch
-                *s_ticket = tk;
-            }
-            asm volatile("bar.sync 9, 512;" ::: "memory");
-            if (*s_ticket == parts - 1 && ok && !*failed && row_ok) {
-                __threadfence();
-                const size_t base = ((size_t)cut * parts * 2 + X) * 128 + m;  // slice p: + p * 256
-                float mx = -INFINITY;
-                for (int p = 0; p < parts; p++) mx = fmaxf(mx, __ldcg(&a.split_ml[base + (size_t)p * 256].x));
-                float wsum = 0.f;
-                for (int p = 0; p < parts; p++) {
-                    const float2 ml = __ldcg(&a.split_ml[base + (size_t)p * 256]);
-                    if (ml.x != -INFINITY) wsum += ml.y * exp2f(ml.x - mx);
-                }
-                const float inv = 1.f / wsum;
-#pragma unroll 1
-                for (int c = 2 * H; c < 2 * H + 2; c++) {
-                    float acc[32];
-#pragma unroll
-                    for (int e = 0; e < 32; e++) acc[e] = 0.f;
-                    for (int p = 0; p < parts; p++) {
-                        const float mp = __ldcg(&a.split_ml[base + (size_t)p * 256].x);
-                        if (mp == -INFINITY) continue;  // an empty slice, or rows it never saw: its rows were not written
-                        const float w = exp2f(mp - mx);
-                        const float4* src = reinterpret_cast<const float4*>(a.split_o) + ((size_t)(cut * parts + p) * 2 + X) * 32 * 128 + m;
-#pragma unroll
-                        for (int u = 0; u < 8; u++) {
-                            const float4 t = __ldcg(src + (size_t)(c * 8 + u) * 128);
-                            acc[u * 4] += w * t.x; acc[u * 4 + 1] += w * t.y; acc[u * 4 + 2] += w * t.z; acc[u * 4 + 3] += w * t.w;
-                        }
-                    }
-                    store_row(c, acc, inv);
-                }
-            }
+            if (last_slice(a, wk, 9, two ? 512 : 256, tid == 64, s_ticket) && !*failed)
+                merge_slices<D, BF16>(a, wk, 2, X, nv, r0 + X * TPT, (tid - 64) & 255, 256);
         }
         TC_DUMP(if (tid == 64 && !Q8) { a.dbg_buf[(size_t)blockIdx.x * 16 + 14] = TC_NOW() - t_loop_end; });
     }
@@ -1112,7 +1150,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
 template <bool BF16>
 static cudaError_t launch_tc2(const CUtensorMap& map32, const CUtensorMap& map_sc, const ChunkArgs& a, cudaStream_t st) {
     if (a.n_items <= 0) return cudaSuccess;
-    const int grid = a.split_parts > 1 ? a.split_first + (a.n_items - a.split_first) * a.split_parts : a.n_items;
+    const int grid = a.n_items;
     if (a.q8_arena) chunk_tc2_kernel<128, BF16, true><<<grid, kThreads2Q8, tc2_smem_bytes_q8<128>(), st>>>(map32, map_sc, a);
     else chunk_tc2_kernel<128, BF16, false><<<grid, kThreads2, tc2_smem_bytes<128>(), st>>>(map32, map_sc, a);
     return cudaGetLastError();
@@ -1143,12 +1181,12 @@ cudaError_t chunk_tc_init() {
     return cudaSuccess;
 }
 
-// `map` must be the 16-row box view of the layer (one K or V tile of a page per box).
-cudaError_t launch_chunk_tc(const CUtensorMap& map, const CUtensorMap& map32, const ChunkArgs& a, bool bf16, cudaStream_t st) {
+// `map32`: the layer's 32-row box view (K and V of a page per box).
+cudaError_t launch_chunk_tc(const CUtensorMap& map32, const ChunkArgs& a, bool bf16, cudaStream_t st) {
     switch (a.geo.d) {
-        case 64: return bf16 ? launch_tc<64, true>(map, map32, a, st) : launch_tc<64, false>(map, map32, a, st);
-        case 128: return bf16 ? launch_tc<128, true>(map, map32, a, st) : launch_tc<128, false>(map, map32, a, st);
-        case 256: return bf16 ? launch_tc<256, true>(map, map32, a, st) : launch_tc<256, false>(map, map32, a, st);
+        case 64: return bf16 ? launch_tc<64, true>(map32, a, st) : launch_tc<64, false>(map32, a, st);
+        case 128: return bf16 ? launch_tc<128, true>(map32, a, st) : launch_tc<128, false>(map32, a, st);
+        case 256: return bf16 ? launch_tc<256, true>(map32, a, st) : launch_tc<256, false>(map32, a, st);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -313,7 +313,7 @@ class KVArena:
         check(self._lib.cbkv_set_host_route(self._h, 1 if direct else 0))
 
     def set_chunk_split(self, max_parts: int) -> None:
-        """Two-tile chunk kernel: most K/V slices per item of a launch's last, mostly empty wave (1 = never cut)."""
+        """tcgen05 chunk kernels: most K/V slices an item may be cut into (1 = never cut)."""
         check(self._lib.cbkv_set_chunk_split(self._h, max_parts))
 
     def set_chunk_kernel(self, mode: int) -> None:
@@ -346,6 +346,18 @@ class KVArena:
         items = a[6 + (n_segs + 1) * 8:].reshape(n_items, 4)
         return {"n_ctas": n_ctas, "n_items": n_items, "n_segs": n_segs, "n_units": n_units, "n_parts": n_parts,
                 "levels": levels, "segs": segs, "items": items}
+
+    def debug_tile_plan(self, window: int, tokens_per_item: int, tile_tokens: int, kv_tile: int = 128, sm_count: int = 148,
+                        max_parts: int = 64) -> dict:
+        """The work list of a tcgen05 chunk launch for the step in flight (host only): counts and `tiles` [n_ctas, 8]
+        in launch order (see include/combs_kv.h for the columns)."""
+        cap = 1 << 20
+        buf = (C.c_int32 * cap)()
+        n = self._lib.cbkv_debug_tile_plan(self._h, window, tokens_per_item, tile_tokens, kv_tile, sm_count, max_parts, buf, cap)
+        if n < 0 or n > cap:
+            raise CbkvError(-6, "no step in flight or plan too large")
+        a = np.frombuffer(buf, dtype=np.int32, count=n).copy()
+        return {"n_ctas": int(a[0]), "n_slots": int(a[1]), "n_cut": int(a[2]), "tiles": a[3:].reshape(-1, 8)}
 
 
 def static_status(stream: Optional[torch.cuda.Stream] = None) -> int:

@@ -336,13 +336,13 @@ int32_t cbkv_set_decode_tuning(cbkv_arena* arena, int32_t ctas_per_sm, int32_t s
  * flag, 0 = `stream` waits for the input copies' event before every kernel (what other steps use). */
 int32_t cbkv_set_host_route(cbkv_arena* arena, int32_t direct);
 
-/* Two-tile tcgen05 chunk kernel: when the last wave of a launch (one CTA per SM at a time) would fill at
- * most half of the SMs, its items are cut along K/V into up to `max_parts` CTAs each, whose partial rows
- * the last finisher adds up.  1 = never cut; default 4. */
+/* tcgen05 chunk kernels: when a launch has too few items for the chip (one CTA per SM at a time), or its last
+ * wave would leave most SMs idle, items are cut along K/V into up to `max_parts` CTAs each, whose partial
+ * rows the last finisher adds up.  1 = never cut; by default as many as a model of the launch finds worth it. */
 int32_t cbkv_set_chunk_split(cbkv_arena* arena, int32_t max_parts);
 
 /* Which kernel runs a step that is not pure decode: 0 = the library chooses (tcgen05
- * tiles once the step has at least 64 new tokens), 1 = the mma.sync kernel, 2 = the
+ * tiles; mma.sync for scales that are not positive), 1 = the mma.sync kernel, 2 = the
  * tcgen05/TMEM kernel with one 128-row query tile per CTA (head_dim 64, 128 or 256), 3 = the
  * tcgen05/TMEM kernel with two query tiles per CTA and P in tensor memory (head_dim 128).
  * Over int8 layers these kernels read a float copy of the step's pages made per layer and
@@ -369,6 +369,14 @@ int32_t cbkv_debug_raise(int32_t kind);
  * Returns the number of words, or -1 without a step. */
 int64_t cbkv_debug_decode_plan(cbkv_arena* arena, int64_t window, int32_t n_ctas, int32_t tail_pct, int32_t min_item,
                                int32_t* out, int64_t cap);
+
+/* The work list of a tcgen05 chunk launch for the step in flight, cut for `sm_count` SMs (0 = no cuts) into
+ * at most `max_parts` K/V slices per item, flattened into `out`: [n_ctas, n_slots, n_cut, one record of 8
+ * ints per CTA in launch order: sequence, kv head, block of tokens_per_item query tokens, first K/V tile,
+ * end tile, part | parts << 16, first slot of the item or -1, ticket or -1].  tile_tokens: query tokens per
+ * 128-row tile, kv_tile: tokens per K/V tile.  Returns the number of words, or -1 without a step. */
+int64_t cbkv_debug_tile_plan(cbkv_arena* arena, int64_t window, int32_t tokens_per_item, int32_t tile_tokens, int32_t kv_tile,
+                             int32_t sm_count, int32_t max_parts, int32_t* out, int64_t cap);
 
 /* Tuning (no reference counterpart): the share of a CTA's range that is cut into dynamically
  * claimed tail items (percent), the smallest item (pages; 0 = no tail, a static equal split) and

@@ -299,3 +299,47 @@ def test_empty_step_changes_nothing():
     free = a.num_free_pages()
     a.begin_step_host_only([], [])
     assert s.seq_len() == 20 and s.pages_used() == 2 and a.num_free_pages() == free
+
+
+@pytest.mark.parametrize("lens,new,window,tokens,tile,kv_tile,sms,max_parts", [
+    ([33], [2], 0, 32, 16, 128, 148, 64), ([1], [1], 0, 32, 16, 128, 148, 64), ([32000], [5], 0, 32, 16, 128, 148, 64),
+    ([600, 6000, 128, 2500], [5] * 4, 0, 32, 16, 128, 148, 64), ([0, 4000, 127, 129], [512, 1, 1, 1], 0, 32, 16, 128, 148, 64),
+    ([4608] * 2, [512] * 2, 0, 64, 32, 128, 148, 4), ([7000] * 8, [512] * 8, 0, 64, 32, 128, 148, 64),
+    ([4500, 900], [512, 17], 1024, 64, 64, 64, 148, 64), ([4500, 900], [512, 17], 1024, 64, 64, 64, 148, 1),
+    ([40000], [1000], 17, 64, 64, 64, 3, 64), ([5000] * 3, [300, 1, 1], 0, 128, 64, 128, 0, 64)])
+def test_tile_plan_covers_every_kv_tile_once(lens, new, window, tokens, tile, kv_tile, sms, max_parts):
+    # every (sequence, kv head, block of query tokens) exactly once, its slices gapless, in order and not empty, its
+    # slots and its ticket its own
+    a = KVArena(1, 28, 4, 128, 45000, 16, 20000)
+    seqs = [a.new_seq() for _ in lens]
+    for s_, n in zip(seqs, lens):
+        if n:
+            a.begin_step_host_only([s_], [n])
+    a.begin_step_host_only(seqs, new)
+    pl = a.debug_tile_plan(window, tokens, tile, kv_tile, sms, max_parts)
+    want = {}
+    for b, (pos, n) in enumerate(zip(lens, new)):
+        for qt in range(-(-n // tokens)):
+            first, last = pos + qt * tokens, pos + min((qt + 1) * tokens, n) - 1
+            pages = last // 16 - (max(0, first - window + 1) if window else 0) // 16 + 1
+            for h in range(4):
+                want[b, h, qt] = -(-pages * 16 // kv_tile)
+    got, slots, tickets = {}, set(), set()
+    for b, h, qt, t0, t1, pn, base, cut in pl["tiles"].tolist():
+        part, parts = pn & 0xffff, pn >> 16
+        assert t1 > t0 and 1 <= parts <= max(1, max_parts)
+        got.setdefault((b, h, qt), []).append((part, t0, t1))
+        if parts == 1:
+            assert base == cut == -1
+        else:
+            assert 0 <= base + part < pl["n_slots"] and base + part not in slots and 0 <= cut < pl["n_cut"]
+            slots.add(base + part)
+            tickets.add((cut, b, h, qt))
+    assert len(tickets) == len({t[0] for t in tickets}) == pl["n_cut"] and len(slots) == pl["n_slots"]
+    assert set(got) == set(want)
+    for key, sl in got.items():
+        sl.sort()
+        assert [p for p, _, _ in sl] == list(range(len(sl)))
+        assert sl[0][1] == 0 and sl[-1][2] == want[key] and all(x[2] == y[1] for x, y in zip(sl, sl[1:]))
+    if max_parts == 1 or sms == 0:
+        assert pl["n_cut"] == 0
