@@ -66,6 +66,7 @@ EncodeTiledFn encode_fn() {
 }
 
 constexpr int kSlots = 4;
+constexpr int kUncutUnits = 40;  // see get_decode_plan
 
 struct StepSlot {
     uint8_t* host = nullptr;  // pinned
@@ -402,6 +403,13 @@ int32_t get_decode_plan(Arena* a, int64_t window, bool quant, cudaStream_t st, D
     build_decode_plan(*a, window, max_ctas, d->split, &pd.host);
     {
         int want = std::max(1, (pd.host.n_units + dc.consumers - 1) / dc.consumers);
+        // A few short segments of one length (one sequence's first hundreds of tokens) are not cut at all: a CTA per
+        // segment streams its pages in the time that a cut would spend on tickets and the merge.
+        const int per = pd.host.n_segs > 0 ? pd.host.n_units / pd.host.n_segs : 0;
+        bool equal = pd.host.n_segs > 0 && pd.host.n_segs <= max_ctas && per <= kUncutUnits;
+        for (int i = 0; equal && i < pd.host.n_segs; i++)
+            equal = pd.host.segs[(size_t)i + 1].unit_begin - pd.host.segs[(size_t)i].unit_begin == per;
+        if (equal) want = std::min(want, pd.host.n_segs);
         if (want < pd.host.n_ctas) build_decode_plan(*a, window, want, d->split, &pd.host);
     }
     // segment and item records in one upload

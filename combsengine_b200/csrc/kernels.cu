@@ -27,6 +27,7 @@
 #include <algorithm>
 
 #include "kernels.hpp"
+#include "pdl.cuh"
 #include "q8_unpack.cuh"
 
 namespace cbkv {
@@ -465,6 +466,8 @@ __device__ __forceinline__ void issue_tile(const CUtensorMap* map, uint32_t stag
 // ------------------------------------------------------------------ append
 template <typename T>
 __global__ void append_kernel(const AppendArgs a) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int D8 = a.geo.d / 8;
     const int64_t total = (int64_t)a.step.n_tokens * a.geo.n_kv * 2 * D8;
     for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (int64_t)gridDim.x * blockDim.x) {
@@ -567,8 +570,6 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void consumer_sync(int nthreads) {
     asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
 }
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ int4 lds128(uint32_t addr) {
     int4 v;
     asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
@@ -1531,8 +1532,7 @@ cudaError_t launch_append(const AppendArgs& a, bool bf16, cudaStream_t st) {
     int64_t total = (int64_t)a.step.n_tokens * a.geo.n_kv * 2 * (a.geo.d / 8);
     int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 8);
     if (blocks <= 0) return cudaSuccess;
-    append_kernel<uint16_t><<<blocks, 256, 0, st>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(append_kernel<uint16_t>, blocks, 256, 0, st, a);
 }
 
 template <int D, int C, bool BF16, bool Q8>

@@ -15,6 +15,7 @@
 #include <algorithm>
 
 #include "kernels.hpp"
+#include "pdl.cuh"
 #include "q8_unpack.cuh"
 
 namespace cbkv {
@@ -40,6 +41,8 @@ __global__ void __launch_bounds__(256) append_quant_kernel(const AppendArgs a) {
     const int64_t kv_rows = (int64_t)a.step.n_tokens * Hkv;
     uint8_t* arena = reinterpret_cast<uint8_t*>(a.arena);
     const size_t rec = qrec_bytes(P, d);
+    pdl_wait();
+    pdl_launch_dependents();
     for (int64_t R = warp0; R < 2 * kv_rows; R += nwarps) {
         const int is_v = R >= kv_rows;
         const int64_t row = is_v ? R - kv_rows : R;
@@ -117,6 +120,8 @@ __global__ void __launch_bounds__(256) dequant_pages_kernel(const int32_t* table
     const int lane = threadIdx.x & 31;
     const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    pdl_wait();
+    pdl_launch_dependents();
     const int D = geo.d, P = geo.page_size, Hkv = geo.n_kv, G = D / 32;
     const size_t rec = qrec_bytes(P, D);
     const int k_chunks = P * D / 16, sw = qrec_swizzled(D) ? 1 : 0;
@@ -245,9 +250,7 @@ cudaError_t launch_append_quant(const AppendArgs& a, bool bf16, cudaStream_t st)
     const int64_t rows = 2 * (int64_t)a.step.n_tokens * a.geo.n_kv;
     if (rows <= 0) return cudaSuccess;
     const int blocks = (int)std::min<int64_t>((rows + 7) / 8, 148 * 8);
-    if (bf16) append_quant_kernel<true><<<blocks, 256, 0, st>>>(a);
-    else append_quant_kernel<false><<<blocks, 256, 0, st>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(bf16 ? append_quant_kernel<true> : append_quant_kernel<false>, blocks, 256, 0, st, a);
 }
 
 cudaError_t launch_dequant_pages(const int32_t* tables, int n_entries, const GeomDev& geo, const void* arena, void* scratch,
@@ -255,9 +258,8 @@ cudaError_t launch_dequant_pages(const int32_t* tables, int n_entries, const Geo
     const int64_t items = (int64_t)n_entries * geo.n_kv;
     if (items <= 0) return cudaSuccess;
     const int blocks = (int)std::min<int64_t>((items + 7) / 8, 148 * 8);
-    if (bf16) dequant_pages_kernel<true><<<blocks, 256, 0, st>>>(tables, n_entries, geo, reinterpret_cast<const uint8_t*>(arena), reinterpret_cast<uint16_t*>(scratch), status);
-    else dequant_pages_kernel<false><<<blocks, 256, 0, st>>>(tables, n_entries, geo, reinterpret_cast<const uint8_t*>(arena), reinterpret_cast<uint16_t*>(scratch), status);
-    return cudaGetLastError();
+    return launch_pdl(bf16 ? dequant_pages_kernel<true> : dequant_pages_kernel<false>, blocks, 256, 0, st, tables, n_entries, geo,
+                      reinterpret_cast<const uint8_t*>(arena), reinterpret_cast<uint16_t*>(scratch), status);
 }
 
 cudaError_t launch_generic_quant(const GenericArgs& a, bool bf16, cudaStream_t st) {

@@ -31,6 +31,7 @@
 #include <algorithm>
 
 #include "kernels.hpp"
+#include "pdl.cuh"
 #include "q8_unpack.cuh"
 
 namespace cbkv {
@@ -369,6 +370,10 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     for (int i = tid; i <= p_hi - p_lo && i < kPageCap; i += kThreads) s_pages[i] = a.step.tables[sm.tbl_off + p_lo + i];
+    // q, the pages and the partial-result buffers belong to earlier launches until here; everything above (barriers,
+    // tensor memory, the work record and the block table, which came with the step's upload) runs under their tail
+    pdl_wait();
+    pdl_launch_dependents();
     // ---- Q tile: rows m = rep * TPT + i, K-major swizzled blocks; rows past the data are zero
     {
         const uint16_t* qbase = reinterpret_cast<const uint16_t*>(a.q) + (size_t)sm.tok_off * a.geo.n_q * D;
@@ -634,8 +639,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
 template <int D, bool BF16>
 static cudaError_t launch_tc(const CUtensorMap& map32, const ChunkArgs& a, cudaStream_t st) {
     if (a.n_items <= 0) return cudaSuccess;
-    chunk_tc_kernel<D, BF16><<<a.n_items, kThreads, tc_smem_bytes<D>(), st>>>(map32, a);
-    return cudaGetLastError();
+    return launch_pdl(chunk_tc_kernel<D, BF16>, a.n_items, kThreads, tc_smem_bytes<D>(), st, map32, a);
 }
 
 
@@ -761,6 +765,10 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     for (int i = tid; i <= p_hi - p_lo && i < kPageCap; i += (int)blockDim.x) s_pages[i] = a.step.tables[sm.tbl_off + p_lo + i];
+    // q, the pages and the partial-result buffers belong to earlier launches until here; everything above (barriers,
+    // tensor memory, the work record and the block table, which came with the step's upload) runs under their tail
+    pdl_wait();
+    pdl_launch_dependents();
     // ---- Q tiles: row m of tile X is q head (m / TPT) at token r0 + X TPT + m % TPT
     {
         const uint16_t* qbase = reinterpret_cast<const uint16_t*>(a.q) + (size_t)sm.tok_off * a.geo.n_q * D;
@@ -1150,10 +1158,8 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
 template <bool BF16>
 static cudaError_t launch_tc2(const CUtensorMap& map32, const CUtensorMap& map_sc, const ChunkArgs& a, cudaStream_t st) {
     if (a.n_items <= 0) return cudaSuccess;
-    const int grid = a.n_items;
-    if (a.q8_arena) chunk_tc2_kernel<128, BF16, true><<<grid, kThreads2Q8, tc2_smem_bytes_q8<128>(), st>>>(map32, map_sc, a);
-    else chunk_tc2_kernel<128, BF16, false><<<grid, kThreads2, tc2_smem_bytes<128>(), st>>>(map32, map_sc, a);
-    return cudaGetLastError();
+    if (a.q8_arena) return launch_pdl(chunk_tc2_kernel<128, BF16, true>, a.n_items, kThreads2Q8, tc2_smem_bytes_q8<128>(), st, map32, map_sc, a);
+    return launch_pdl(chunk_tc2_kernel<128, BF16, false>, a.n_items, kThreads2, tc2_smem_bytes<128>(), st, map32, map_sc, a);
 }
 
 bool chunk_tc2_supported(int d) { return d == 128; }

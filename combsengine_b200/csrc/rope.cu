@@ -24,6 +24,7 @@
 #include <cmath>
 
 #include "kernels.hpp"
+#include "pdl.cuh"
 
 namespace cbkv {
 
@@ -163,6 +164,8 @@ __global__ void __launch_bounds__(256) rope_append_kernel(const RopeArgs a) {
     const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int d = a.geo.d, half = d >> 1, chunks = half >> 1;  // a chunk = 2 elements = 4 bytes
+    pdl_wait();
+    pdl_launch_dependents();
     const int64_t q_rows = (int64_t)a.step.n_tokens * a.geo.n_q, kv_rows = (int64_t)a.step.n_tokens * a.geo.n_kv;
     const int64_t total = q_rows + (a.k_out ? 1 : 2) * kv_rows;
     for (int64_t R = warp0; R < total; R += nwarps) {
@@ -251,6 +254,8 @@ __global__ void __launch_bounds__(256) rope_append_vec_kernel(const RopeArgs a) 
         for (int i = threadIdx.x; i < n_seqs; i += blockDim.x) s_tok[i] = a.step.seq_meta[i].tok_off;
         __syncthreads();
     }
+    pdl_wait();  // the sequence records above came with the step's upload, which no kernel overlaps
+    pdl_launch_dependents();
     const int lane = threadIdx.x & 31, t = lane % T, sub = lane / T;
     constexpr int RPW = 32 / T;  // rows per warp per round
     // row counts fit 32 bits (the launcher checks)
@@ -342,15 +347,14 @@ static cudaError_t launch_rope_t(const RopeArgs& a, int64_t rows, cudaStream_t s
     auto grid = [&](int per_block) { return (int)std::min<int64_t>((rows + per_block - 1) / per_block, 148 * 8); };
     const bool vec = rows < ((int64_t)1 << 31) - 64;  // the vector kernels count rows in 32 bits
     switch (vec ? a.geo.d : 0) {
-        case 16: rope_append_vec_kernel<BF16, 1><<<grid(8 * rpw), 256, 0, st>>>(a); break;
-        case 32: rope_append_vec_kernel<BF16, 2><<<grid(8 * rpw), 256, 0, st>>>(a); break;
-        case 64: rope_append_vec_kernel<BF16, 4><<<grid(8 * rpw), 256, 0, st>>>(a); break;
-        case 128: rope_append_vec_kernel<BF16, 8><<<grid(8 * rpw), 256, 0, st>>>(a); break;
-        case 256: rope_append_vec_kernel<BF16, 16><<<grid(8 * rpw), 256, 0, st>>>(a); break;
-        case 512: rope_append_vec_kernel<BF16, 32><<<grid(8 * rpw), 256, 0, st>>>(a); break;
-        default: rope_append_kernel<BF16><<<grid(8), 256, 0, st>>>(a); break;  // one warp per row
+        case 16: return launch_pdl(rope_append_vec_kernel<BF16, 1>, grid(8 * rpw), 256, 0, st, a);
+        case 32: return launch_pdl(rope_append_vec_kernel<BF16, 2>, grid(8 * rpw), 256, 0, st, a);
+        case 64: return launch_pdl(rope_append_vec_kernel<BF16, 4>, grid(8 * rpw), 256, 0, st, a);
+        case 128: return launch_pdl(rope_append_vec_kernel<BF16, 8>, grid(8 * rpw), 256, 0, st, a);
+        case 256: return launch_pdl(rope_append_vec_kernel<BF16, 16>, grid(8 * rpw), 256, 0, st, a);
+        case 512: return launch_pdl(rope_append_vec_kernel<BF16, 32>, grid(8 * rpw), 256, 0, st, a);
+        default: return launch_pdl(rope_append_kernel<BF16>, grid(8), 256, 0, st, a);  // one warp per row
     }
-    return cudaGetLastError();
 }
 
 cudaError_t launch_rope_append(const RopeArgs& a, bool bf16, cudaStream_t st) {
