@@ -290,8 +290,17 @@ int32_t alloc_float_layer(Arena* a, LayerArena* Lp, cudaStream_t st) {
         bool bf16 = a->cfg.dtype == CBKV_BF16;
         int32_t rc = encode_map(&L.map_kv, bf16, L.base, rows, a->cfg.head_dim, 32);
         if (rc) return rc;
-        rc = encode_map(&L.map_k16, bf16, L.base, rows, a->cfg.head_dim, 16);
-        if (rc) return rc;
+        if (a->cfg.head_dim % 64 == 0) {
+            const cuuint64_t D = (cuuint64_t)a->cfg.head_dim;
+            cuuint64_t dims[5] = {64, 8, D / 64, 2, rows / 16};
+            cuuint64_t strides[4] = {D * 2, 128, 8 * D * 2, 16 * D * 2};
+            cuuint32_t box[5] = {64, 8, (cuuint32_t)(D / 64), 1, 2};
+            cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+            CUresult r = encode_fn()(&L.map_page, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, L.base, dims,
+                                     strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+            if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled (pages) failed: " + std::to_string((int)r)); return CBKV_ERR_CUDA; }
+        }
     }
     return CBKV_OK;
 }
@@ -688,8 +697,8 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
 #endif
         ProfScope ps(d, st);
         { int32_t frc = flush_uploads(d, st); if (frc) return frc; }
-        if (use_tc2) CU_TRY(q8_direct ? launch_chunk_tc2(L.map_k16, L.map_sc, args, bf16, st) : launch_chunk_tc2(KV->map_kv, KV->map_kv, args, bf16, st));
-        else CU_TRY(launch_chunk_tc(KV->map_kv, args, bf16, st));
+        if (use_tc2) CU_TRY(q8_direct ? launch_chunk_tc2(L.map_k16, L.map_sc, args, bf16, st) : launch_chunk_tc2(KV->map_page, KV->map_page, args, bf16, st));
+        else CU_TRY(launch_chunk_tc(KV->map_page, args, bf16, st));
         g_launches++;
         d->last_kv_writer = -1;
         return CBKV_OK;

@@ -64,8 +64,9 @@ struct LayerArena {
     bool quant = false;  // base holds quantised records
     CUtensorMap map_kv;  // 2-D view [rows = pages*n_kv*32][d], box 32 rows x 64 elems, 128B swizzle;
                          // quantised: bytes in 128-byte rows, one box = one record
-    CUtensorMap map_k16; // same view, box 16 rows x 64 elems (one K or one V tile);
-                         // quantised, head_dim 128: box = the 16 rows of a record's K values or of its V values
+    CUtensorMap map_page; // float layers: {64 elems, 8 rows, d/64 column blocks, K or V, 8-token groups}, box = K or V of
+                         // one page of one kv head, as [group][column block][8 rows of 128 bytes], 128B swizzle
+    CUtensorMap map_k16; // quantised, head_dim 128: box = the 16 rows of a record's K values or of its V values
     CUtensorMap map_sc;  // quantised, head_dim 128: box = one row, a record's K scales or its V scales
 };
 
@@ -204,14 +205,14 @@ cudaError_t launch_rope_append(const RopeArgs& a, bool bf16, cudaStream_t st);
 // host side of the rotary tables (rope.cu): frequencies, then [max_position][head_dim] f32 tables
 int32_t rope_inv_freq(const cbkv_rope_config& c, std::vector<double>* inv, double* mscale);
 void rope_tables(const cbkv_rope_config& c, const std::vector<double>& inv, double mscale, float* cos_out, float* sin_out);
-// tcgen05 chunk kernel (prefill_tc.cu): head_dim 64, 128 or 256; `map32` is the layer's map_kv
+// tcgen05 chunk kernel (prefill_tc.cu): head_dim 64, 128 or 256; `map` is the layer's map_page
 bool chunk_tc_supported(int d);
 cudaError_t chunk_tc_init();
-cudaError_t launch_chunk_tc(const CUtensorMap& map32, const ChunkArgs& a, bool bf16, cudaStream_t st);
+cudaError_t launch_chunk_tc(const CUtensorMap& map, const ChunkArgs& a, bool bf16, cudaStream_t st);
 // two query tiles per CTA, P in tensor memory (head_dim 128)
 bool chunk_tc2_supported(int d);
-// int8 layer (a.q8_arena non-null): `map32` = the layer's map_k16, `map_sc` = its map_sc; float layer: map_sc is not used
-cudaError_t launch_chunk_tc2(const CUtensorMap& map32, const CUtensorMap& map_sc, const ChunkArgs& a, bool bf16, cudaStream_t st);
+// float layer: `map` = the layer's map_page, map_sc is not used; int8 layer (a.q8_arena non-null): its map_k16 and map_sc
+cudaError_t launch_chunk_tc2(const CUtensorMap& map, const CUtensorMap& map_sc, const ChunkArgs& a, bool bf16, cudaStream_t st);
 cudaError_t kernels_init();  // raises the dynamic shared memory limits once per process
 
 }  // namespace cbkv

@@ -9,9 +9,9 @@
 // the tile's i-th token (TPT = 128 / RS tokens, RS = n_rep rounded up to a power of
 // two), so the K/V tiles are shared by the whole q-head group.
 //
-//   warp 0        TMA producer: one 32-row box per (page, 64-column block) brings K and V of a
-//                 page in the arena's 8-row interleave; 8 pages per tile, two stages
-//   warp 1        one thread issues tcgen05.mma: S = Q K^T (two S buffers), O += P V
+//   warp 0        TMA producer: one copy per page and operand
+//   warp 1        one thread issues tcgen05.mma: S = Q K^T (two S buffers), O += P V, whichever
+//                 has its operands first
 //   warps 2..9    softmax: two threads per TMEM lane (row), one for each half of a tile's keys; P goes back to
 //                 tensor memory over its S columns (16-bit pairs) and is the A operand of P V; O rescaled in
 //                 TMEM when a row max moves
@@ -22,9 +22,9 @@
 //
 // Tensor memory: S0 [0,KT), S1 [128,128+KT), O [256, 256 + D) -> 512 columns allocated.
 // Shared memory: the Q tile of 128 rows stored as 64-column blocks of 128 rows x 128 bytes
-// (128-byte swizzle); two K/V stages, each D/64 blocks of KT/16 pages x 32 rows x 128 bytes in
-// the arena's row order [K 0-7][V 0-7][K 8-15][V 8-15], so K and V are both 8-row groups
-// 2048 bytes apart (V starts 1024 bytes in).
+// (128-byte swizzle); two K and two V buffers, [page][8-token group][column block][8 rows x 128 bytes]:
+// the five-dimensional view of a layer (LayerArena::map_page) takes K or V of a page out of the arena's
+// [K 0-7][V 0-7][K 8-15][V 8-15] order in one copy.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -78,6 +78,22 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
         ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+// K or V of one page of one kv head (LayerArena::map_page): all its column blocks in one copy
+__device__ __forceinline__ void tma_load_page(uint32_t dst, const CUtensorMap* map, int is_v, int row16, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %2, %2, %3, %4}], [%5];"
+        ::"r"(dst), "l"(map), "r"(0), "r"(is_v), "r"(row16), "r"(bar) : "memory");
+}
+// Non-blocking look at a barrier phase.
+__device__ __forceinline__ uint32_t mbar_test_wait(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok;
 }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -174,7 +190,7 @@ struct TcKeys { static constexpr int value = D == 256 ? 64 : 128; };  // tokens 
 
 template <int D>
 constexpr int tc_smem_bytes() {
-    // Q tile of 128 rows x D, two stages of K and V tiles of KT tokens x D, barriers, the staged block table and the
+    // Q tile of 128 rows x D, two K and two V tiles of KT tokens x D, barriers, the staged block table and the
     // half-row exchange; at least 120 KB so that two CTAs never share an SM (each allocates all 512
     // tensor-memory columns)
     constexpr int need = 128 * D * 2 + 2 * 2 * TcKeys<D>::value * D * 2 + 256 + kPageCap * 4 + 2 * 128 * 2 * 4 + 64;
@@ -322,17 +338,18 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
     constexpr int KT = TcKeys<D>::value;       // tokens per KV tile
     constexpr int HK = KT / 2;                 // keys of a softmax thread
     constexpr int PPT = KT / 16;               // pages per KV tile
-    constexpr uint32_t BLKKV = PPT * 4096u;    // one 64-column block of a K/V stage: PPT pages x 32 rows x 128 bytes
-    constexpr uint32_t STAGE = 2u * KT * D * 2u;  // K and V of KT tokens
+    constexpr uint32_t KVB = (uint32_t)KT * D * 2u;  // K or V of KT tokens: [page][8-token group][column block][8 rows of 128 bytes]
+    constexpr uint32_t PGB = 16u * D * 2u;           // one page of it
     uint8_t* sQ = smem;
-    uint8_t* sKV = sQ + TILE;           // 2 stages
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + 2 * STAGE);
-    // barriers: kv_full[2], kv_empty[2], s_full[2], p_full[2], o_done
-    const uint32_t b_kv_full = smem_u32(bars + 0), b_kv_empty = smem_u32(bars + 2), b_s_full = smem_u32(bars + 4);
-    const uint32_t b_p_full = smem_u32(bars + 6), b_o_done = smem_u32(bars + 8);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
-    volatile int* failed = reinterpret_cast<volatile int*>(bars + 11);
-    int* s_ticket = reinterpret_cast<int*>(bars + 12);
+    uint8_t* sK = sQ + TILE;            // 2 K buffers, 2 V buffers: K is free again once its scores are computed
+    uint8_t* sV = sK + 2 * KVB;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sV + 2 * KVB);
+    // barriers: k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_full[2], o_done
+    const uint32_t b_k_full = smem_u32(bars + 0), b_k_empty = smem_u32(bars + 2), b_v_full = smem_u32(bars + 4), b_v_empty = smem_u32(bars + 6);
+    const uint32_t b_s_full = smem_u32(bars + 8), b_p_full = smem_u32(bars + 10), b_o_done = smem_u32(bars + 12);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
+    volatile int* failed = reinterpret_cast<volatile int*>(bars + 14);
+    int* s_ticket = reinterpret_cast<int*>(bars + 15);
     int* s_pages = reinterpret_cast<int*>(bars + 16);   // [kPageCap] physical pages of the KV range
     float* s_xch = reinterpret_cast<float*>(s_pages + kPageCap);  // [2 buffers][128 rows][2 halves]
     int* s_pair = reinterpret_cast<int*>(s_xch + 2 * 128 * 2);    // [4] a wait of this pair of warps ran out
@@ -356,7 +373,8 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
 
     if (tid == 0) {
         for (int i = 0; i < 2; i++) {
-            mbar_init(b_kv_full + i * 8, 1); mbar_init(b_kv_empty + i * 8, 1); mbar_init(b_s_full + i * 8, 1);
+            mbar_init(b_k_full + i * 8, 1); mbar_init(b_k_empty + i * 8, 1); mbar_init(b_v_full + i * 8, 1); mbar_init(b_v_empty + i * 8, 1);
+            mbar_init(b_s_full + i * 8, 1);
             mbar_init(b_p_full + i * 8, 256);
         }
         mbar_init(b_o_done, 1);
@@ -370,14 +388,17 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     for (int i = tid; i <= p_hi - p_lo && i < kPageCap; i += kThreads) s_pages[i] = a.step.tables[sm.tbl_off + p_lo + i];
+    tc_fence_before();
+    __syncthreads();  // barriers and block table are ready: the producer starts while the other warps bring Q
+    tc_fence_after();
     // q, the pages and the partial-result buffers belong to earlier launches until here; everything above (barriers,
     // tensor memory, the work record and the block table, which came with the step's upload) runs under their tail
     pdl_wait();
     pdl_launch_dependents();
-    // ---- Q tile: rows m = rep * TPT + i, K-major swizzled blocks; rows past the data are zero
-    {
+    // ---- Q tile (every warp but the producer): rows m = rep * TPT + i, K-major swizzled blocks; rows past the data are zero
+    if (warp != 0) {
         const uint16_t* qbase = reinterpret_cast<const uint16_t*>(a.q) + (size_t)sm.tok_off * a.geo.n_q * D;
-        for (int c = tid; c < 128 * (D / 8); c += kThreads) {
+        for (int c = tid - 32; c < 128 * (D / 8); c += kThreads - 32) {
             const int m = c / (D / 8), j = c - m * (D / 8);   // row, 16-byte piece
             const int rep = m / TPT, i = m - rep * TPT;
             uint4 val = make_uint4(0, 0, 0, 0);
@@ -386,41 +407,43 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
             const uint32_t off = (j >> 3) * BLK + m * 128u + (((j & 7) ^ (m & 7)) << 4);
             *reinterpret_cast<uint4*>(sQ + off) = val;
         }
+        fence_proxy_async();   // Q was written through the generic proxy, the MMA reads it through the async proxy
+        bar_sync(10, kThreads - 32);
     }
-    fence_proxy_async();   // Q was written through the generic proxy, the MMA reads it through the async proxy
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const uint32_t tS0 = tmem, tO = tmem + 256;
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        // The block-table entries of the whole KV range were staged in shared memory by all
-        // threads (below the Q load); every lane issues boxes of a tile: one per (page, column block).
+        // The block-table entries of the whole KV range were staged in shared memory by all threads; one copy per
+        // page brings its K, another its V, each issued by the page's lane.
         bool ok = true;
         long long tprev = TC_NOW(), c_wait = 0, c_issue = 0;
 #pragma unroll 1
         for (int j = 0; j < n_tiles && ok; j++) {
             const int st = j & 1;
-            if (lane == 0) {
-                if (j >= 2 && !mbar_wait_bounded(b_kv_empty + st * 8, ((j >> 1) - 1) & 1)) ok = false;
-                TC_ACC(c_wait);
-                if (*failed) ok = false;
-                if (ok) mbar_expect_tx(b_kv_full + st * 8, STAGE);
-                else { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
-            }
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-            if (!ok) break;
-            for (int bx = lane; bx < PPT * XB; bx += 32) {
-                const int pg = bx / XB, x = bx - pg * XB;
-                // pages past the last visible one repeat it: finite data that the causal mask hides
-                const int idx = min(j * PPT + pg, p_hi - p_lo);
-                int phys = idx < kPageCap ? s_pages[idx] : a.step.tables[sm.tbl_off + p_lo + idx];
+            // pages past the last visible one repeat it: finite data that the causal mask hides
+            int phys = 0;
+            if (lane < PPT) {
+                const int idx = min(j * PPT + lane, p_hi - p_lo);
+                phys = idx < kPageCap ? s_pages[idx] : a.step.tables[sm.tbl_off + p_lo + idx];
                 if (phys < 0 || phys >= a.geo.num_pages) { atomicOr(a.status, ST_BAD_PAGE); phys = 0; }
-                tma_load_2d(smem_u32(sKV + st * STAGE + x * BLKKV + pg * 4096), &tmap32, x * 64, (phys * Hkv + h) * 32, b_kv_full + st * 8);
             }
-            if (lane == 0) TC_ACC(c_issue);
+#pragma unroll
+            for (int is_v = 0; is_v < 2 && ok; is_v++) {
+                const uint32_t full = (is_v ? b_v_full : b_k_full) + st * 8, empty = (is_v ? b_v_empty : b_k_empty) + st * 8;
+                if (lane == 0) {
+                    if (j >= 2 && !mbar_wait_bounded(empty, ((j >> 1) - 1) & 1)) ok = false;
+                    TC_ACC(c_wait);
+                    if (*failed) ok = false;
+                    if (ok) mbar_expect_tx(full, KVB);
+                    else { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
+                }
+                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                if (ok && lane < PPT)
+                    tma_load_page(smem_u32((is_v ? sV : sK) + st * KVB + lane * PGB), &tmap32, is_v, (phys * Hkv + h) * 2, full);
+                if (lane == 0) TC_ACC(c_issue);
+            }
         }
         TC_DUMP(if (lane == 0) { a.dbg_buf[(size_t)blockIdx.x * 16 + 0] = c_wait; a.dbg_buf[(size_t)blockIdx.x * 16 + 1] = c_issue; a.dbg_buf[(size_t)blockIdx.x * 16 + 15] = n_tiles; });
     } else if (warp == 1) {
@@ -428,47 +451,59 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
         if (lane == 0) {
             const uint32_t id_qk = instr_desc(BF16, 128, KT, false);
             const uint32_t id_pv = instr_desc(BF16, 128, D, true);
-            // descriptors differ only in the start address field (bits 0-13, address >> 4)
-            // K: 8-row groups 2048 bytes apart; V: the same groups 1024 bytes further, 64-wide d blocks BLKKV apart
-            const uint64_t dq = smem_desc(smem_u32(sQ), 16, 1024), dk = smem_desc(smem_u32(sKV), 16, 2048);
-            const uint64_t dv = smem_desc(smem_u32(sKV) + 1024, BLKKV, 2048);
+            // descriptors differ only in the start address field (bits 0-13, address >> 4); 8-token groups of K and V
+            // are XB * 1024 bytes apart, 64-wide column blocks 1024
+            const uint64_t dq = smem_desc(smem_u32(sQ), 16, 1024), dk = smem_desc(smem_u32(sK), 16, XB * 1024);
+            const uint64_t dv = smem_desc(smem_u32(sV), 1024, XB * 1024);
             auto issue_qk = [&](int j) {
-                const uint64_t kst = (uint64_t)(((j & 1) * STAGE) >> 4);
+                const uint64_t kst = (uint64_t)(((j & 1) * KVB) >> 4);
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ks++) {
                     // 16 elements = 32 bytes inside the swizzled row, four steps per 64-column block
                     const uint64_t qoff = (uint64_t)(((ks >> 2) * BLK + (ks & 3) * 32) >> 4);
-                    const uint64_t koff = (uint64_t)(((ks >> 2) * BLKKV + (ks & 3) * 32) >> 4);
+                    const uint64_t koff = (uint64_t)(((ks >> 2) * 1024 + (ks & 3) * 32) >> 4);
                     umma(tS0 + (j & 1) * 128, dq + qoff, dk + kst + koff, id_qk, ks > 0);
                 }
                 umma_commit(b_s_full + (j & 1) * 8);
+                umma_commit(b_k_empty + (j & 1) * 8);
             };
             long long tprev = TC_NOW(), c_wkv = 0, c_wp = 0, c_iss = 0;
-            bool ok = mbar_wait_bounded(b_kv_full, 0);
-            if (ok) { tc_fence_after(); issue_qk(0); }
+            bool ok = true;
+            int next_qk = 0;  // scores issued so far
+#pragma unroll 1
             for (int j = 0; ok && j < n_tiles; j++) {
-                if (j + 1 < n_tiles) {
-                    // scores of the next tile first: they are computed while this tile's softmax runs.  They go to
-                    // the other S buffer, whose P the previous P V (issued before) was the last to read.
-                    TC_ACC(c_iss);
-                    ok = mbar_wait_bounded(b_kv_full + ((j + 1) & 1) * 8, ((j + 1) >> 1) & 1);
-                    TC_ACC(c_wkv);
-                    if (!ok) break;
-                    tc_fence_after();
-                    issue_qk(j + 1);
+                // Until this tile's P is there: the scores of the next tile as soon as its K has landed.  They go to the
+                // other S buffer, whose P the previous P V (issued before) was the last to read.  Neither waits for the
+                // other: a P V held up by a K that is still on its way would hold up the V buffer it frees.
+                uint64_t t0 = 0;
+                for (int n = 0;; n++) {
+                    if (next_qk <= j + 1 && next_qk < n_tiles && mbar_test_wait(b_k_full + (next_qk & 1) * 8, (next_qk >> 1) & 1)) {
+                        TC_ACC(c_wkv);
+                        tc_fence_after();
+                        issue_qk(next_qk++);
+                        TC_ACC(c_iss);
+                    }
+                    if (next_qk > j && mbar_test_wait(b_p_full + (j & 1) * 8, (j >> 1) & 1)) break;
+                    if ((n & 63) == 63) {
+                        if (*failed) ok = false;
+                        if (t0 == 0) t0 = global_ns();
+                        else if (global_ns() - t0 > 200000000ull) ok = false;
+                        if (!ok) break;
+                    }
                 }
-                TC_ACC(c_iss);
-                ok = mbar_wait_bounded(b_p_full + (j & 1) * 8, (j >> 1) & 1) && !*failed;
                 TC_ACC(c_wp);
+                if (ok) ok = mbar_wait_bounded(b_v_full + (j & 1) * 8, (j >> 1) & 1) && !*failed;
+                TC_ACC(c_wkv);
                 if (!ok) break;
                 tc_fence_after();
                 const int st = j & 1;
-                const uint64_t vst = (uint64_t)((st * STAGE) >> 4);
+                const uint64_t vst = (uint64_t)((st * KVB) >> 4);
 #pragma unroll
-                for (int ks = 0; ks < PPT; ks++)  // 16 keys per step = one page; P: 8 packed columns, V: MN-major, 4096 bytes per step
-                    umma_ts(tO, tS0 + st * 128 + ks * 8, dv + vst + (uint64_t)((ks * 4096) >> 4), id_pv, (j > 0 || ks > 0));
-                umma_commit(b_kv_empty + st * 8);
+                for (int ks = 0; ks < PPT; ks++)  // 16 keys per step = one page; P: 8 packed columns, V: MN-major
+                    umma_ts(tO, tS0 + st * 128 + ks * 8, dv + vst + (uint64_t)((ks * PGB) >> 4), id_pv, (j > 0 || ks > 0));
+                umma_commit(b_v_empty + st * 8);
                 umma_commit(b_o_done);
+                TC_ACC(c_iss);
             }
             if (!ok) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
             TC_DUMP(a.dbg_buf[(size_t)blockIdx.x * 16 + 2] = c_wkv; a.dbg_buf[(size_t)blockIdx.x * 16 + 3] = c_wp; a.dbg_buf[(size_t)blockIdx.x * 16 + 4] = c_iss;);
@@ -549,8 +584,8 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             l_run = l_run * alpha + (sum + sum2);
             TC_ACC(c_exp);
-            // O may be rescaled once the previous P V is complete.  (S being full says that of the one before it
-            // only, so this wait is at most one phase ahead of the barrier.)
+            // O may be rescaled once the previous P V is complete.  (S being full says that at least of the one
+            // before it, so this wait is at most one phase ahead of the barrier.)
             if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
                 bool done = mbar_wait_bounded(b_o_done, (j - 1) & 1) && !*failed;
                 done = __all_sync(0xffffffffu, done);
@@ -696,15 +731,15 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     constexpr uint32_t TILE = 128u * D * 2u;   // one Q tile
     constexpr uint32_t BLK = 128u * 128u;      // 64-column block of a Q tile
     constexpr int XB = D / 64;
-    constexpr uint32_t BLKKV = 8u * 4096u;     // 64-column block of a K/V stage
-    constexpr uint32_t STAGE = 2u * TILE;
+    constexpr uint32_t STAGE = 2u * TILE;      // a K and a V buffer
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sQ = smem;                 // Q_A then Q_B
-    uint8_t* sKV = sQ + 2 * TILE;       // 2 stages
+    uint8_t* sKV = sQ + 2 * TILE;       // float layer: 2 K buffers, 2 V buffers of 32 KB, [page][8-token group][column block][8 rows of 128 bytes]
     uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + 2 * STAGE);
     // barriers: kv_full[2], kv_empty[2], s_full[A,B], p_full[A,B], o_done[A,B]
     const uint32_t b_kv_full = smem_u32(bars + 0), b_kv_empty = smem_u32(bars + 2), b_s_full = smem_u32(bars + 4);
     const uint32_t b_p_full = smem_u32(bars + 6), b_o_done = smem_u32(bars + 8);
+    const uint32_t b_vf2 = smem_u32(bars + 12), b_ve2 = smem_u32(bars + 14);  // float layer: v_full[2], v_empty[2]; kv_full / kv_empty are K's
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
     volatile int* failed = reinterpret_cast<volatile int*>(bars + 11);
     int* s_pages = reinterpret_cast<int*>(bars + 16);
@@ -721,7 +756,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     uint8_t* sRawV0 = sRawK + kRawK * HALF;
     uint8_t* sRawV1 = reinterpret_cast<uint8_t*>(s_xch + 2 * 2 * 128 * 2) + 128;  // 128-byte aligned, as every slot is
     const uint32_t b_q8 = smem_u32(sRawV1 + (kRawV - kRawVInStage) * HALF);
-    const uint32_t b_v_full = b_q8, b_v_empty = b_q8 + 8, b_rawk = b_q8 + 16, b_rawv = b_rawk + kRawK * 8;
+    const uint32_t b_v_full = Q8 ? b_q8 : b_vf2, b_v_empty = Q8 ? b_q8 + 8 : b_ve2, b_rawk = b_q8 + 16, b_rawv = b_rawk + kRawK * 8;
     (void)sRawK; (void)sRawV0; (void)sRawV1; (void)b_v_full; (void)b_v_empty; (void)b_rawk; (void)b_rawv; (void)REC;
 
     const long long t_entry = TC_NOW();
@@ -750,8 +785,8 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
             mbar_init(b_kv_full + i * 8, 1); mbar_init(b_kv_empty + i * 8, 1); mbar_init(b_s_full + i * 8, 1);
             mbar_init(b_p_full + i * 8, 256); mbar_init(b_o_done + i * 8, 1);
         }
-        if constexpr (Q8) {  // kv_full / kv_empty above are K's here
-            mbar_init(b_v_full, 1); mbar_init(b_v_empty, 1);
+        for (int i = 0; i < (Q8 ? 1 : 2); i++) { mbar_init(b_v_full + i * 8, 1); mbar_init(b_v_empty + i * 8, 1); }
+        if constexpr (Q8) {
             for (int i = 0; i < kRawK + kRawV; i++) mbar_init(b_rawk + i * 8, 1);
         }
         *failed = 0;
@@ -765,14 +800,18 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     for (int i = tid; i <= p_hi - p_lo && i < kPageCap; i += (int)blockDim.x) s_pages[i] = a.step.tables[sm.tbl_off + p_lo + i];
+    tc_fence_before();
+    __syncthreads();  // barriers and block table are ready: the producer starts while the other warps bring Q
+    tc_fence_after();
     // q, the pages and the partial-result buffers belong to earlier launches until here; everything above (barriers,
     // tensor memory, the work record and the block table, which came with the step's upload) runs under their tail
     pdl_wait();
     pdl_launch_dependents();
-    // ---- Q tiles: row m of tile X is q head (m / TPT) at token r0 + X TPT + m % TPT
-    {
+    // ---- Q tiles (every warp but the float layer's producer): row m of tile X is q head (m / TPT) at token r0 + X TPT + m % TPT
+    if (Q8 || warp != 0) {
+        const int first = Q8 ? 0 : 32, n_thr = (int)blockDim.x - first;
         const uint16_t* qbase = reinterpret_cast<const uint16_t*>(a.q) + (size_t)sm.tok_off * a.geo.n_q * D;
-        for (int c = tid; c < (two ? 256 : 128) * (D / 8); c += (int)blockDim.x) {
+        for (int c = tid - first; c < (two ? 256 : 128) * (D / 8); c += n_thr) {
             const int mm = c / (D / 8), j = c - mm * (D / 8);
             const int X = mm >> 7, m = mm & 127;
             const int rep = m / TPT, r = r0 + X * TPT + (m - rep * TPT);
@@ -782,11 +821,9 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
             const uint32_t off = X * TILE + (j >> 3) * BLK + m * 128u + (((j & 7) ^ (m & 7)) << 4);
             *reinterpret_cast<uint4*>(sQ + off) = val;
         }
+        fence_proxy_async();
+        bar_sync(10, n_thr);
     }
-    fence_proxy_async();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
     if (Q8 && warp >= 18) {
@@ -900,29 +937,33 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         TC_DUMP(if (tid == 18 * 32) { unsigned long long* b = a.dbg_buf + (size_t)blockIdx.x * 16; b[0] = c_wait; b[1] = c_issue + c_conv + c_meet; b[12] = c_conv; b[13] = c_meet; b[14] = c_issue; b[15] = n_tiles; });
         (void)c_wait; (void)c_issue; (void)c_conv; (void)c_meet; (void)tprev;
     } else if (!Q8 && warp == 0) {
-        // ------------------------------------------------------------ TMA producer
+        // ------------------------------------------------------------ TMA producer: one copy per page and operand
         bool ok = true;
         long long tprev = TC_NOW(), c_wait = 0, c_issue = 0;
 #pragma unroll 1
         for (int j = 0; j < n_tiles && ok; j++) {
             const int st = j & 1;
-            if (lane == 0) {
-                if (j >= 2 && !mbar_wait_bounded(b_kv_empty + st * 8, ((j >> 1) - 1) & 1)) ok = false;
-                TC_ACC(c_wait);
-                if (*failed) ok = false;
-                if (ok) mbar_expect_tx(b_kv_full + st * 8, STAGE);
-                else { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
-            }
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-            if (!ok) break;
-            for (int bx = lane; bx < 8 * XB; bx += 32) {
-                const int pg = bx / XB, x = bx - pg * XB;
-                const int idx = min(j * 8 + pg, p_hi - p_lo);  // pages past the end repeat the last one (masked)
-                int phys = idx < kPageCap ? s_pages[idx] : a.step.tables[sm.tbl_off + p_lo + idx];
+            int phys = 0;
+            if (lane < 8) {
+                const int idx = min(j * 8 + lane, p_hi - p_lo);  // pages past the end repeat the last one (masked)
+                phys = idx < kPageCap ? s_pages[idx] : a.step.tables[sm.tbl_off + p_lo + idx];
                 if (phys < 0 || phys >= a.geo.num_pages) { atomicOr(a.status, ST_BAD_PAGE); phys = 0; }
-                tma_load_2d(smem_u32(sKV + st * STAGE + x * BLKKV + pg * 4096), &tmap32, x * 64, (phys * Hkv + h) * 32, b_kv_full + st * 8);
             }
-            if (lane == 0) TC_ACC(c_issue);
+#pragma unroll
+            for (int is_v = 0; is_v < 2 && ok; is_v++) {
+                const uint32_t full = (is_v ? b_v_full : b_kv_full) + st * 8, empty = (is_v ? b_v_empty : b_kv_empty) + st * 8;
+                if (lane == 0) {
+                    if (j >= 2 && !mbar_wait_bounded(empty, ((j >> 1) - 1) & 1)) ok = false;
+                    TC_ACC(c_wait);
+                    if (*failed) ok = false;
+                    if (ok) mbar_expect_tx(full, TILE);
+                    else { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
+                }
+                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                if (ok && lane < 8)
+                    tma_load_page(smem_u32(sKV + (2 * is_v + st) * TILE + lane * (16 * D * 2)), &tmap32, is_v, (phys * Hkv + h) * 2, full);
+                if (lane == 0) TC_ACC(c_issue);
+            }
         }
         TC_DUMP(if (lane == 0) { a.dbg_buf[(size_t)blockIdx.x * 16 + 0] = c_wait; a.dbg_buf[(size_t)blockIdx.x * 16 + 1] = c_issue; a.dbg_buf[(size_t)blockIdx.x * 16 + 15] = n_tiles; });
     } else if (warp == 1) {
@@ -930,11 +971,12 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         if (lane == 0) {
             const uint32_t id_qk = instr_desc(BF16, 128, 128, false);
             const uint32_t id_pv = instr_desc(BF16, 128, D, true);
-            // float layer: a stage holds pages as they lie in device memory (K and V rows of a page interleaved in
-            // groups of eight); int8 layer: the loader warps lay K and V out separately (see the shared memory map)
-            constexpr uint32_t KBUF = Q8 ? QBUF : STAGE, KBLK = Q8 ? QBLK : BLKKV, GRP = Q8 ? 1024u : 2048u, VPAGE = Q8 ? 2048u : 4096u;
+            // 64-wide column blocks, 8-token groups and pages of a K or V buffer (see the shared memory map)
+            constexpr uint32_t KBUF = Q8 ? QBUF : TILE, KBLK = Q8 ? QBLK : 1024u, GRP = Q8 ? 1024u : XB * 1024u, VPAGE = Q8 ? 2048u : 2 * XB * 1024u;
             const uint64_t dq = smem_desc(smem_u32(sQ), 16, 1024), dk = smem_desc(smem_u32(sKV), 16, GRP);
-            const uint64_t dv = smem_desc(smem_u32(sKV) + (Q8 ? 2 * QBUF : 1024u), KBLK, GRP);
+            const uint64_t dv = smem_desc(smem_u32(sKV) + 2 * KBUF, KBLK, GRP);
+            auto v_bar = [&](uint32_t b, int j) { return b + (Q8 ? 0u : (uint32_t)(j & 1) * 8); };  // int8 layers have one V buffer
+            auto v_par = [&](int j) { return (uint32_t)(Q8 ? j & 1 : (j >> 1) & 1); };
             auto issue_qk = [&](int X, int j) {
                 const uint64_t kst = (uint64_t)(((j & 1) * KBUF) >> 4), qst = (uint64_t)((X * TILE) >> 4);
 #pragma unroll
@@ -944,10 +986,10 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                     umma(tmem + X * 128, dq + qst + qoff, dk + kst + koff, id_qk, ks > 0);
                 }
                 umma_commit(b_s_full + X * 8);
-                if (Q8 && X == (two ? 1 : 0)) umma_commit(b_kv_empty + (j & 1) * 8);  // all scores of this K buffer have been issued
+                if (X == (two ? 1 : 0)) umma_commit(b_kv_empty + (j & 1) * 8);  // all scores of this K buffer have been issued
             };
             auto issue_pv = [&](int X, int j) {
-                const uint64_t vst = Q8 ? 0ull : (uint64_t)(((j & 1) * STAGE) >> 4);
+                const uint64_t vst = Q8 ? 0ull : (uint64_t)(((j & 1) * KBUF) >> 4);
 #pragma unroll
                 for (int ks = 0; ks < 8; ks++)  // 16 keys = one page per step; P: 8 packed columns per step
                     umma_ts(tmem + 256 + X * 128, tmem + X * 128 + ks * 8, dv + vst + (uint64_t)((ks * VPAGE) >> 4), id_pv, (j > 0 || ks > 0));
@@ -960,12 +1002,12 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                 TC_ACC(c_iss);
                 ok = mbar_wait_bounded(b_p_full, j & 1) && !*failed;
                 TC_ACC(c_wp);
-                if (Q8 && ok) { ok = mbar_wait_bounded(b_v_full, j & 1); TC_ACC(c_wkv); }
+                if (ok) { ok = mbar_wait_bounded(v_bar(b_v_full, j), v_par(j)); TC_ACC(c_wkv); }
                 if (!ok) break;
                 tc_fence_after();
                 issue_pv(0, j);
                 TC_ACC(c_pv);
-                if (!two && !Q8) umma_commit(b_kv_empty + (j & 1) * 8);
+                if (!two) umma_commit(v_bar(b_v_empty, j));
                 if (j + 1 < n_tiles) {
                     ok = mbar_wait_bounded(b_kv_full + ((j + 1) & 1) * 8, ((j + 1) >> 1) & 1);
                     TC_ACC(c_wkv);
@@ -982,8 +1024,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                     issue_pv(1, j);
                     TC_ACC(c_pv);
                 }
-                // every read of this stage (int8 layer: of the V buffer) has been issued before
-                if (two || Q8) umma_commit(Q8 ? b_v_empty : b_kv_empty + (j & 1) * 8);
+                if (two) umma_commit(v_bar(b_v_empty, j));  // every read of this V buffer has been issued before
                 if (two && j + 1 < n_tiles) issue_qk(1, j + 1);
             }
             if (!ok) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
