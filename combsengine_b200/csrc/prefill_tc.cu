@@ -20,9 +20,8 @@
 // and V (128 KB) would not leave room for two stages next to the Q tile (S = Q K^T is then 128 x 64 and
 // O += P V one 128 x 256 MMA per 16 keys).
 //
-// Tensor memory: S0 [0,KT), S1 [128,128+KT), O [256, 256 + D) -> 512 columns allocated.
-// Shared memory: the Q tile of 128 rows stored as 64-column blocks of 128 rows x 128 bytes
-// (128-byte swizzle); two K and two V buffers, [page][8-token group][column block][8 rows x 128 bytes]:
+// Tensor memory: S0 [0,KT), S1 [KT, 2 KT), Q [2 KT, 2 KT + D / 2) packed, O [512 - D, 512) -> 512 columns allocated.
+// Shared memory: kTcBufs K and V buffers each, [page][8-token group][column block][8 rows x 128 bytes]:
 // the five-dimensional view of a layer (LayerArena::map_page) takes K or V of a page out of the arena's
 // [K 0-7][V 0-7][K 8-15][V 8-15] order in one copy.
 #include <cuda_bf16.h>
@@ -185,15 +184,16 @@ constexpr int kThreads = 320;
 constexpr int kTmemCols = 512;
 constexpr int kPageCap = 2560;   // block-table entries staged in shared memory (40960 tokens); longer ranges read the rest from global memory
 
+constexpr int kTcBufs = 3;       // K buffers and V buffers of the one-tile kernel
+
 template <int D>
 struct TcKeys { static constexpr int value = D == 256 ? 64 : 128; };  // tokens per KV tile
 
 template <int D>
 constexpr int tc_smem_bytes() {
-    // Q tile of 128 rows x D, two K and two V tiles of KT tokens x D, barriers, the staged block table and the
-    // half-row exchange; at least 120 KB so that two CTAs never share an SM (each allocates all 512
-    // tensor-memory columns)
-    constexpr int need = 128 * D * 2 + 2 * 2 * TcKeys<D>::value * D * 2 + 256 + kPageCap * 4 + 2 * 128 * 2 * 4 + 64;
+    // K and V buffers of KT tokens x D, barriers, the staged block table and the half-row exchange; at least 120 KB
+    // so that two CTAs never share an SM (each allocates all 512 tensor-memory columns)
+    constexpr int need = 2 * kTcBufs * TcKeys<D>::value * D * 2 + 256 + kPageCap * 4 + 2 * 128 * 2 * 4 + 64;
     return need < 120 * 1024 ? 120 * 1024 : need;
 }
 
@@ -331,8 +331,6 @@ __device__ __forceinline__ bool last_slice(const ChunkArgs& a, const CtaWork& wk
 
 template <int D, bool BF16>
 __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constant__ CUtensorMap tmap32, const ChunkArgs a) {
-    constexpr uint32_t TILE = 128u * D * 2u;   // the Q tile
-    constexpr uint32_t BLK = 128u * 128u;      // one 64-element column block of it: 128 rows x 128 bytes
     constexpr int XB = D / 64;                 // column blocks per row
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int KT = TcKeys<D>::value;       // tokens per KV tile
@@ -340,17 +338,17 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
     constexpr int PPT = KT / 16;               // pages per KV tile
     constexpr uint32_t KVB = (uint32_t)KT * D * 2u;  // K or V of KT tokens: [page][8-token group][column block][8 rows of 128 bytes]
     constexpr uint32_t PGB = 16u * D * 2u;           // one page of it
-    uint8_t* sQ = smem;
-    uint8_t* sK = sQ + TILE;            // 2 K buffers, 2 V buffers: K is free again once its scores are computed
-    uint8_t* sV = sK + 2 * KVB;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sV + 2 * KVB);
-    // barriers: k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_full[2], o_done
-    const uint32_t b_k_full = smem_u32(bars + 0), b_k_empty = smem_u32(bars + 2), b_v_full = smem_u32(bars + 4), b_v_empty = smem_u32(bars + 6);
-    const uint32_t b_s_full = smem_u32(bars + 8), b_p_full = smem_u32(bars + 10), b_o_done = smem_u32(bars + 12);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
-    volatile int* failed = reinterpret_cast<volatile int*>(bars + 14);
-    int* s_ticket = reinterpret_cast<int*>(bars + 15);
-    int* s_pages = reinterpret_cast<int*>(bars + 16);   // [kPageCap] physical pages of the KV range
+    constexpr int NB = kTcBufs;
+    uint8_t* sK = smem;                 // NB K buffers, NB V buffers: K is free again once its scores are computed
+    uint8_t* sV = sK + NB * KVB;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sV + NB * KVB);
+    const uint32_t b_k_full = smem_u32(bars + 0), b_k_empty = smem_u32(bars + NB), b_v_full = smem_u32(bars + 2 * NB), b_v_empty = smem_u32(bars + 3 * NB);
+    const uint32_t b_s_full = smem_u32(bars + 4 * NB), b_p_full = smem_u32(bars + 4 * NB + 2), b_o_done = smem_u32(bars + 4 * NB + 4);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4 * NB + 5);
+    volatile int* failed = reinterpret_cast<volatile int*>(bars + 4 * NB + 6);
+    int* s_ticket = reinterpret_cast<int*>(bars + 4 * NB + 7);
+    static_assert(4 * NB + 8 <= 32, "barriers");
+    int* s_pages = reinterpret_cast<int*>(bars + 32);   // [kPageCap] physical pages of the KV range
     float* s_xch = reinterpret_cast<float*>(s_pages + kPageCap);  // [2 buffers][128 rows][2 halves]
     int* s_pair = reinterpret_cast<int*>(s_xch + 2 * 128 * 2);    // [4] a wait of this pair of warps ran out
 
@@ -372,11 +370,10 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
     const int k0 = p_lo * 16;                               // absolute position of key 0 of tile 0
 
     if (tid == 0) {
-        for (int i = 0; i < 2; i++) {
+        for (int i = 0; i < NB; i++) {
             mbar_init(b_k_full + i * 8, 1); mbar_init(b_k_empty + i * 8, 1); mbar_init(b_v_full + i * 8, 1); mbar_init(b_v_empty + i * 8, 1);
-            mbar_init(b_s_full + i * 8, 1);
-            mbar_init(b_p_full + i * 8, 256);
         }
+        for (int i = 0; i < 2; i++) { mbar_init(b_s_full + i * 8, 1); mbar_init(b_p_full + i * 8, 256); }
         mbar_init(b_o_done, 1);
         *failed = 0;
         for (int i = 0; i < 4; i++) s_pair[i] = 0;
@@ -395,23 +392,32 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
     // tensor memory, the work record and the block table, which came with the step's upload) runs under their tail
     pdl_wait();
     pdl_launch_dependents();
-    // ---- Q tile (every warp but the producer): rows m = rep * TPT + i, K-major swizzled blocks; rows past the data are zero
-    if (warp != 0) {
-        const uint16_t* qbase = reinterpret_cast<const uint16_t*>(a.q) + (size_t)sm.tok_off * a.geo.n_q * D;
-        for (int c = tid - 32; c < 128 * (D / 8); c += kThreads - 32) {
-            const int m = c / (D / 8), j = c - m * (D / 8);   // row, 16-byte piece
-            const int rep = m / TPT, i = m - rep * TPT;
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if (rep < n_rep && i < nv)
-                val = *reinterpret_cast<const uint4*>(qbase + ((size_t)(h * n_rep + rep) * sm.snew + r0 + i) * D + j * 8);
-            const uint32_t off = (j >> 3) * BLK + m * 128u + (((j & 7) ^ (m & 7)) << 4);
-            *reinterpret_cast<uint4*>(sQ + off) = val;
-        }
-        fence_proxy_async();   // Q was written through the generic proxy, the MMA reads it through the async proxy
-        bar_sync(10, kThreads - 32);
-    }
     const uint32_t tmem = *tmem_slot;
-    const uint32_t tS0 = tmem, tO = tmem + 256;
+    const uint32_t tS0 = tmem, tQ = tmem + 2 * KT, tO = tmem + 512 - D;
+    static_assert(2 * KT + D / 2 + D <= 512, "tensor memory");
+    // ---- Q goes to tensor memory (the A operand of S, packed pairs like P): from shared memory the 128-row A and the
+    // K tile together would need more than the 128 bytes a cycle that it delivers.  Row m = rep * TPT + i; each of a
+    // row's two softmax threads brings half of it; rows past the data are zero.
+    if (warp >= 2) {
+        const int m = (warp & 3) * 32 + lane, H = (warp - 2) >> 2, rep = m / TPT, i = m - rep * TPT;
+        const bool row_ok = rep < n_rep && i < nv;
+        const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(a.q) + (size_t)sm.tok_off * a.geo.n_q * D +
+                                                          ((size_t)(h * n_rep + (row_ok ? rep : 0)) * sm.snew + r0 + (row_ok ? i : 0)) * D + H * (D / 2));
+#pragma unroll
+        for (int c = 0; c < D / 64; c++) {  // 32 elements: 16 packed columns
+            uint32_t w[16];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const uint4 v = row_ok ? src[c * 4 + u] : make_uint4(0, 0, 0, 0);
+                w[u * 4] = v.x; w[u * 4 + 1] = v.y; w[u * 4 + 2] = v.z; w[u * 4 + 3] = v.w;
+            }
+            tmem_st16(tQ + ((uint32_t)(warp & 3) << 21) + H * (D / 4) + c * 16, w);
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        tc_fence_before();
+    }
+    if (warp >= 1) bar_sync(10, kThreads - 32);  // every warp but the producer
+    tc_fence_after();
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
@@ -421,7 +427,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
         long long tprev = TC_NOW(), c_wait = 0, c_issue = 0;
 #pragma unroll 1
         for (int j = 0; j < n_tiles && ok; j++) {
-            const int st = j & 1;
+            const int st = j % NB;
             // pages past the last visible one repeat it: finite data that the causal mask hides
             int phys = 0;
             if (lane < PPT) {
@@ -433,7 +439,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
             for (int is_v = 0; is_v < 2 && ok; is_v++) {
                 const uint32_t full = (is_v ? b_v_full : b_k_full) + st * 8, empty = (is_v ? b_v_empty : b_k_empty) + st * 8;
                 if (lane == 0) {
-                    if (j >= 2 && !mbar_wait_bounded(empty, ((j >> 1) - 1) & 1)) ok = false;
+                    if (j >= NB && !mbar_wait_bounded(empty, (j / NB - 1) & 1)) ok = false;
                     TC_ACC(c_wait);
                     if (*failed) ok = false;
                     if (ok) mbar_expect_tx(full, KVB);
@@ -453,19 +459,14 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
             const uint32_t id_pv = instr_desc(BF16, 128, D, true);
             // descriptors differ only in the start address field (bits 0-13, address >> 4); 8-token groups of K and V
             // are XB * 1024 bytes apart, 64-wide column blocks 1024
-            const uint64_t dq = smem_desc(smem_u32(sQ), 16, 1024), dk = smem_desc(smem_u32(sK), 16, XB * 1024);
-            const uint64_t dv = smem_desc(smem_u32(sV), 1024, XB * 1024);
+            const uint64_t dk = smem_desc(smem_u32(sK), 16, XB * 1024), dv = smem_desc(smem_u32(sV), 1024, XB * 1024);
             auto issue_qk = [&](int j) {
-                const uint64_t kst = (uint64_t)(((j & 1) * KVB) >> 4);
+                const uint64_t kst = (uint64_t)((uint32_t)(j % NB) * KVB >> 4);
 #pragma unroll
-                for (int ks = 0; ks < D / 16; ks++) {
-                    // 16 elements = 32 bytes inside the swizzled row, four steps per 64-column block
-                    const uint64_t qoff = (uint64_t)(((ks >> 2) * BLK + (ks & 3) * 32) >> 4);
-                    const uint64_t koff = (uint64_t)(((ks >> 2) * 1024 + (ks & 3) * 32) >> 4);
-                    umma(tS0 + (j & 1) * 128, dq + qoff, dk + kst + koff, id_qk, ks > 0);
-                }
+                for (int ks = 0; ks < D / 16; ks++)  // 16 elements = 32 bytes inside the swizzled row, four steps per 64-column block
+                    umma_ts(tS0 + (j & 1) * KT, tQ + ks * 8, dk + kst + (uint64_t)(((ks >> 2) * 1024 + (ks & 3) * 32) >> 4), id_qk, ks > 0);
                 umma_commit(b_s_full + (j & 1) * 8);
-                umma_commit(b_k_empty + (j & 1) * 8);
+                umma_commit(b_k_empty + (j % NB) * 8);
             };
             long long tprev = TC_NOW(), c_wkv = 0, c_wp = 0, c_iss = 0;
             bool ok = true;
@@ -477,7 +478,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
                 // other: a P V held up by a K that is still on its way would hold up the V buffer it frees.
                 uint64_t t0 = 0;
                 for (int n = 0;; n++) {
-                    if (next_qk <= j + 1 && next_qk < n_tiles && mbar_test_wait(b_k_full + (next_qk & 1) * 8, (next_qk >> 1) & 1)) {
+                    if (next_qk <= j + 1 && next_qk < n_tiles && mbar_test_wait(b_k_full + (next_qk % NB) * 8, (next_qk / NB) & 1)) {
                         TC_ACC(c_wkv);
                         tc_fence_after();
                         issue_qk(next_qk++);
@@ -492,15 +493,15 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
                     }
                 }
                 TC_ACC(c_wp);
-                if (ok) ok = mbar_wait_bounded(b_v_full + (j & 1) * 8, (j >> 1) & 1) && !*failed;
+                if (ok) ok = mbar_wait_bounded(b_v_full + (j % NB) * 8, (j / NB) & 1) && !*failed;
                 TC_ACC(c_wkv);
                 if (!ok) break;
                 tc_fence_after();
-                const int st = j & 1;
+                const int st = j % NB;
                 const uint64_t vst = (uint64_t)((st * KVB) >> 4);
 #pragma unroll
                 for (int ks = 0; ks < PPT; ks++)  // 16 keys per step = one page; P: 8 packed columns, V: MN-major
-                    umma_ts(tO, tS0 + st * 128 + ks * 8, dv + vst + (uint64_t)((ks * PGB) >> 4), id_pv, (j > 0 || ks > 0));
+                    umma_ts(tO, tS0 + (j & 1) * KT + ks * 8, dv + vst + (uint64_t)((ks * PGB) >> 4), id_pv, (j > 0 || ks > 0));
                 umma_commit(b_v_empty + st * 8);
                 umma_commit(b_o_done);
                 TC_ACC(c_iss);
@@ -537,7 +538,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
             TC_ACC(c_ws);
             if (!ok && lane == 0) *pair_failed = 1;  // the loads below then read stale columns: harmless, nothing is kept
             tc_fence_after();
-            const uint32_t tS = tS0 + (j & 1) * 128 + lane_addr;
+            const uint32_t tS = tS0 + (j & 1) * KT + lane_addr;
             const int kbase = k0 + j * KT + H * HK;
             const bool need_mask = (kbase + HK - 1 > q_min) || (a.window > 0 && kbase + a.window <= q_max);
             uint32_t sv[HK];
