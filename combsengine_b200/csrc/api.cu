@@ -111,7 +111,6 @@ struct DeviceState {
     int chunk_mode = 0;       // cbkv_set_chunk_kernel: 0 = choose, 1 = mma.sync, 2 = tcgen05 one tile, 3 = two tiles, 4 = two tiles, int8 records converted in the kernel
     struct TilePlanDev { ChunkPlan host; const TileItem* tiles = nullptr; };
     std::map<std::pair<int64_t, int>, TilePlanDev> tile_plans;  // of the step, by (window, tokens per work item)
-    std::map<int64_t, bool> two_tiles;                          // of the step, by window: which kernel (two_tiles_pay)
     float* part_o = nullptr;
     float* part_ml = nullptr;
     size_t part_cap = 0;
@@ -371,7 +370,6 @@ int32_t upload_step(Arena* a, cudaStream_t st) {
     d->chunk_plan_ok = false;
     d->chunk_item_begin = nullptr;
     d->tile_plans.clear();
-    d->two_tiles.clear();
     d->step = StepDev{};
     d->last_kv_writer = -1;  // the upload is a full stream dependency
     d->unit_rows_used = 0;
@@ -531,47 +529,15 @@ bool ensure_split(Arena* a, size_t slots, size_t cuts, cudaStream_t st) {
     return true;
 }
 
-// Times of the two tcgen05 chunk kernels for the launch model (per-role cycle counters and launches of known shape at
-// 1.9 GHz): head_dim 128, two query tiles 2.45 us per 128-token K/V tile and 1.75 us with the second one empty, one
-// query tile 1.28 us; head_dim 256, one tile, 1.3 us per 64 tokens.
-TileCut tile_cut(const Arena* a, int64_t window, bool two_tiles) {
-    const DeviceState* d = static_cast<const DeviceState*>(a->dev);
-    TileCut c;
-    c.window = window; c.tile_tokens = 128 / rep_slots_of(a->n_rep()); c.sm_count = d->sm_count; c.max_parts = d->chunk_split;
-    if (two_tiles) { c.cta_us = 7.f; c.tile_us = 2.45f; c.half_us = 1.75f; }
-    else if (a->cfg.head_dim == 256) { c.kv_tile = 64; }
-    else { c.tile_us = c.half_us = 1.28f; }
-    return c;
-}
-
-// head_dim 128 has two kernels.  Two query tiles per CTA cost less per row (half the K/V traffic), one makes twice as
-// many, shorter CTAs and leaves no half of a CTA empty: 8 prompts of 8192 tokens 11.46 against 11.96 ms (two layers),
-// but one prompt of 4096 0.88 against 0.68, verification steps 1.63 against 1.34 and mixed steps 5.28 against 4.17 ms.
-// The launch model decides, once per step and window.
-bool two_tiles_pay(Arena* a, int64_t window) {
+// Work list of a tcgen05 chunk launch: tokens_per_item new tokens per item in tiles of tile_tokens, K/V tiles of
+// kv_tile tokens.  Built once per step and window; the partial-result buffers grow with it.
+int32_t get_tile_plan(Arena* a, int64_t window, int tokens_per_item, int tile_tokens, int kv_tile, cudaStream_t st, DeviceState::TilePlanDev** out) {
     DeviceState* d = dev_of(a);
-    auto it = d->two_tiles.find(window);
-    if (it != d->two_tiles.end()) return it->second;
-    ChunkPlan one, two;
-    const TileCut c1 = tile_cut(a, window, false), c2 = tile_cut(a, window, true);
-    build_chunk_tile_plan(*a, c1.tile_tokens, &one, c1);
-    build_chunk_tile_plan(*a, 2 * c2.tile_tokens, &two, c2);
-    // no estimate: more CTAs than the model is run over, where the cost per row decides
-    const bool pay = one.est_us == 0.f || (two.est_us > 0.f && two.est_us < one.est_us);
-    d->two_tiles.emplace(window, pay);
-    return pay;
-}
-
-// Work list of a tcgen05 chunk launch, built once per step, window and kernel.
-int32_t get_tile_plan(Arena* a, int64_t window, bool two_tiles, cudaStream_t st, DeviceState::TilePlanDev** out) {
-    DeviceState* d = dev_of(a);
-    const TileCut cut0 = tile_cut(a, window, two_tiles);
-    const int tokens_per_item = (two_tiles ? 2 : 1) * cut0.tile_tokens;
     const auto key = std::make_pair(window, tokens_per_item);
     auto it = d->tile_plans.find(key);
     if (it != d->tile_plans.end()) { *out = &it->second; return CBKV_OK; }
     DeviceState::TilePlanDev pd;
-    TileCut cut = cut0;
+    TileCut cut{window, kv_tile, tile_tokens, d->sm_count, d->chunk_split};
     build_chunk_tile_plan(*a, tokens_per_item, &pd.host, cut);
     if (!ensure_split(a, (size_t)pd.host.n_slots, (size_t)pd.host.n_cut, st)) {
         cut.max_parts = 1;
@@ -642,7 +608,7 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
     // (their softmax takes row maxima before scaling, which needs a positive scale)
     const bool tc_able = d->fast && d->tc_ok && scale > 0 && !a->step_is_decode;
     const bool use_tc2 = tc_able && chunk_tc2_supported(a->cfg.head_dim) &&
-                         (d->chunk_mode == 3 || d->chunk_mode == 4 || (d->chunk_mode == 0 && two_tiles_pay(a, w)));
+                         (d->chunk_mode == 3 || d->chunk_mode == 4 || d->chunk_mode == 0);
     const bool use_tc = tc_able && !use_tc2 && (d->chunk_mode == 2 || d->chunk_mode == 0);
     // int8 pages: decode steps stream the records through the decode kernel; the chunk kernels read a float
     // copy made per layer and step (mode 4: the two-tile kernel converts the records itself, slower so far);
@@ -712,13 +678,14 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
         return CBKV_OK;
     }
     if (use_tc || use_tc2) {
+        const int tile_tokens = 128 / rep_slots_of(a->n_rep());
         DeviceState::TilePlanDev* pd = nullptr;
-        int32_t rc = get_tile_plan(a, w, use_tc2, st, &pd);
+        int32_t rc = get_tile_plan(a, w, (use_tc2 ? 2 : 1) * tile_tokens, tile_tokens, !use_tc2 && a->cfg.head_dim == 256 ? 64 : 128, st, &pd);
         if (rc) return rc;
         ChunkArgs args{};
         args.step = d->step; args.geo = geom(a); args.tiles = pd->tiles; args.n_items = (int32_t)pd->host.tiles.size();
         args.q = q; args.out = out; args.status = d->status; args.window = (int32_t)w; args.scale_log2 = scale_log2;
-        args.rep_slots = rep_slots_of(a->n_rep());
+        args.rep_slots = 128 / tile_tokens;
         args.q8_arena = q8_direct ? L.base : nullptr;
         args.split_o = d->split_o; args.split_ml = d->split_ml; args.split_counter = d->split_counter;
 #ifdef CBKV_MEASURE
@@ -1590,7 +1557,6 @@ int32_t cbkv_set_chunk_split(cbkv_arena* arena, int32_t max_parts) {
     if (rc) return rc;
     dev_of(a)->chunk_split = max_parts;
     dev_of(a)->tile_plans.clear();
-    dev_of(a)->two_tiles.clear();
     return CBKV_OK;
     });
 }

@@ -330,12 +330,13 @@ void build_chunk_plan(const Arena& a, int32_t cols_per_item, ChunkPlan* pl) {
 
 namespace {
 
-// Launch model of the tcgen05 chunk kernels, in microseconds.  Besides TileCut's times: a slice writes its rows
-// (128 rows x d x 4 bytes per query tile, about 90 KB/us), and the CTA that merges reads them all back (about
-// 45 KB/us, and 1.5 us for the ticket and the first round trip).
-constexpr float kWriteKBus = 90.f, kMergeKBus = 45.f, kMergeUs = 1.5f;
+// Launch model of the tcgen05 chunk kernels, in units of one K/V tile of a full item: a CTA costs kCtaCost
+// besides its tiles (tensor-memory allocation, first loads, epilogue), a K/V tile of an item that fills one of
+// its two query tiles kHalfTile, a slice kSliceCost more (its partial rows), and the merge at the end
+// kMergeCost for each slice of the full 256 rows.
+constexpr float kCtaCost = 3.f, kHalfTile = 0.7f, kSliceCost = 0.7f, kMergeCost = 0.7f;
 
-struct TileWork { int32_t seq, h, qt, n_tiles; float per_tile, kb; };  // an uncut item: its K/V tiles, us for each, size of its rows
+struct TileWork { int32_t seq, h, qt, n_tiles; float per_tile, rows; };  // an uncut item
 
 // End of the last CTA when `sm_count` SMs take the CTAs in launch order.
 float launch_end(const std::vector<float>& cost, int sm_count, std::vector<float>* heap) {
@@ -381,8 +382,8 @@ void build_chunk_tile_plan(const Arena& a, int32_t tokens_per_tile, ChunkPlan* p
             const int64_t q_first = m.pos + r0, q_last = q_first + toks - 1;
             const int64_t lo_key = cut.window > 0 ? std::max<int64_t>(0, q_first - cut.window + 1) : 0;
             const int32_t pages = (int32_t)((q_last >> 4) - (lo_key >> 4) + 1), ppt = cut.kv_tile / 16;
-            TileWork w{b, 0, qt, (pages + ppt - 1) / ppt, toks > tile_tokens || tile_tokens == tokens_per_tile ? cut.tile_us : cut.half_us,
-                       (float)toks * (float)a.n_rep() * (float)a.cfg.head_dim * 4e-3f};
+            TileWork w{b, 0, qt, (pages + ppt - 1) / ppt, toks > tile_tokens ? 1.f : kHalfTile, (float)toks / (float)tokens_per_tile};
+            if (tile_tokens == tokens_per_tile) w.per_tile = 1.f;  // one query tile per CTA
             g.cost = std::max(g.cost, w.per_tile * w.n_tiles);
             work.push_back(w);
         }
@@ -416,7 +417,7 @@ void build_chunk_tile_plan(const Arena& a, int32_t tokens_per_tile, ChunkPlan* p
                     if (p > 1) {
                         base[(size_t)qt] = slots; id[(size_t)qt] = cuts;
                         slots += p; cuts++;
-                        merge = std::max(merge, kMergeUs + (float)p * w.kb / kMergeKBus);
+                        merge = std::max(merge, kMergeCost * (0.5f + (float)p * w.rows));
                     }
                 }
                 for (int p = 0; p < most; p++)
@@ -426,7 +427,7 @@ void build_chunk_tile_plan(const Arena& a, int32_t tokens_per_tile, ChunkPlan* p
                         const TileWork& w = work[(size_t)(g.first + qt)];
                         const int per = (w.n_tiles + np - 1) / np, t0 = p * per, t1 = std::min(w.n_tiles, t0 + per);
                         if (out) out->push_back({g.seq, h, qt, t0, t1, p | (np << 16), base[(size_t)qt], id[(size_t)qt]});
-                        else cost.push_back(cut.cta_us + w.per_tile * (float)(t1 - t0) + (np > 1 ? w.kb / kWriteKBus : 0.f));
+                        else cost.push_back(kCtaCost + w.per_tile * (float)(t1 - t0) + (np > 1 ? kSliceCost : 0.f));
                     }
             }
         }
@@ -434,7 +435,6 @@ void build_chunk_tile_plan(const Arena& a, int32_t tokens_per_tile, ChunkPlan* p
         return out ? 0.f : launch_end(cost, cut.sm_count, &heap) + merge;
     };
 
-    pl->est_us = 0.f;
     float limit = 0.f;
     int64_t rem = 0;
     int rem_parts = 1;
@@ -449,15 +449,14 @@ void build_chunk_tile_plan(const Arena& a, int32_t tokens_per_tile, ChunkPlan* p
         double total = 0.;
         float longest = 0.f;
         for (const TileWork& w : work) { total += (double)w.per_tile * w.n_tiles; longest = std::max(longest, w.per_tile * w.n_tiles); }
-        const float even = (float)(total * a.cfg.n_kv_heads / cut.sm_count);  // us of tiles per SM
+        const float even = (float)(total * a.cfg.n_kv_heads / cut.sm_count);  // tiles per SM
         if (items <= 4 * cut.sm_count)
             for (float f : {1.3f, 1.f, 0.75f, 0.5f, 0.35f}) {
-                const float lim = std::max(cut.tile_us, even * f);
+                const float lim = std::max(1.f, even * f);
                 if (lim >= longest) continue;
                 const float e = emit(lim, 0, 1, nullptr, nullptr, nullptr);
                 if (e < best) { best = e; limit = lim; rem = 0; rem_parts = 1; }
             }
-        pl->est_us = best;
     }
     emit(limit, rem, rem_parts, &pl->tiles, &pl->n_slots, &pl->n_cut);
 }

@@ -125,7 +125,6 @@ struct ChunkPlan {
     std::vector<int32_t> item_begin;  // n_seqs + 1
     std::vector<struct TileItem> tiles;  // tcgen05 kernels: one record per CTA, in launch order
     int32_t n_slots = 0, n_cut = 0;      // partial-result slots and tickets that the cut items take
-    float est_us = 0.f;                  // what the launch model expects (0 without cuts to choose from)
 };
 
 // One CTA of a tcgen05 chunk launch: K/V tiles [t0, t1) of one (sequence, kv head, block of query tokens).  An
@@ -136,14 +135,8 @@ struct TileItem {  // 32 bytes, read by the kernels as two 16-byte words
     int32_t t1, part_nparts /* part | nparts << 16 */, slot_base, cut;
 };
 // How a tcgen05 chunk launch may be cut: `window` of the layer, tokens per K/V tile, query tokens per 128-row
-// tile, SMs (one CTA each at a time; 0 = never cut), most slices per item; and the kernel's measured times in
-// microseconds: a CTA without its tiles (tensor-memory allocation, first loads, epilogue), a K/V tile of a full
-// item, one of an item that leaves the second query tile empty.
-struct TileCut {
-    int64_t window = 0;
-    int32_t kv_tile = 128, tile_tokens = 0, sm_count = 0, max_parts = 1;
-    float cta_us = 5.f, tile_us = 1.3f, half_us = 1.3f;
-};
+// tile, SMs (one CTA each at a time; 0 = never cut), most slices per item.
+struct TileCut { int64_t window = 0; int32_t kv_tile = 128, tile_tokens = 0, sm_count = 0, max_parts = 1; };
 
 struct Arena {
     cbkv_config cfg{};

@@ -265,66 +265,51 @@ __device__ __forceinline__ float4* slice_rows(const ChunkArgs& a, int slot, int 
     return reinterpret_cast<float4*>(a.split_o) + ((size_t)slot * n_x + X) * (D / 4) * 128;
 }
 // Adds the slices of query tile X up: `rows` packed rows of `nv` tokens per q head, first token r0x.  Every thread of
-// `threads` takes (row, 8 columns) items, two at a time and two slices at a time: eight 16-byte loads in flight that
-// are all needed, also when an item was cut in two.
+// `threads` takes (row, 8 columns) items; the loads of four slices travel together, so an item costs one round trip to
+// L2 per four slices however few rows there are.
 template <int D, bool BF16>
 __device__ __forceinline__ void merge_slices(const ChunkArgs& a, const CtaWork& wk, int n_x, int X, int nv, int r0x, int r, int threads) {
-    const int rows = a.geo.n_rep * nv, n_rep = a.geo.n_rep, n = rows * (D / 8);
-    for (int idx = r; idx < n; idx += 2 * threads) {
-        int row[2], c8[2];
-        float M[2], L[2];
-        float4 x[2], y[2];
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-            const int id = min(idx + e * threads, n - 1);
-            c8[e] = id / rows; row[e] = id - c8[e] * rows;
-            M[e] = -INFINITY; L[e] = 0.f;
-            x[e] = y[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+    const int rows = a.geo.n_rep * nv, n_rep = a.geo.n_rep;
+    for (int idx = r; idx < rows * (D / 8); idx += threads) {
+        const int c8 = idx / rows, row = idx - c8 * rows;
+        float M = -INFINITY, L = 0.f;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
 #pragma unroll 1
-        for (int p0 = 0; p0 < wk.parts; p0 += 2) {
-            float2 ml[2][2];
-            float4 u[2][2], v[2][2];
+        for (int p0 = 0; p0 < wk.parts; p0 += 4) {
+            float2 ml[4];
+            float4 u[4], v[4];
 #pragma unroll
-            for (int e = 0; e < 2; e++)
-#pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    const bool ok = p0 + q < wk.parts;
-                    const int slot = wk.slot_base + p0 + (ok ? q : 0);
-                    ml[e][q] = __ldcg(a.split_ml + ((size_t)slot * n_x + X) * 128 + row[e]);
-                    const float4* src = slice_rows<D>(a, slot, n_x, X) + row[e];
-                    u[e][q] = __ldcg(src + (size_t)(2 * c8[e]) * 128);
-                    v[e][q] = __ldcg(src + (size_t)(2 * c8[e] + 1) * 128);
-                    if (!ok) ml[e][q] = make_float2(-INFINITY, 0.f);
-                }
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const float Mn = fmaxf(M[e], fmaxf(ml[e][0].x, ml[e][1].x));
-                const float so = M[e] == -INFINITY ? 0.f : exp2f(M[e] - Mn);
-                x[e].x *= so; x[e].y *= so; x[e].z *= so; x[e].w *= so; y[e].x *= so; y[e].y *= so; y[e].z *= so; y[e].w *= so;
-                L[e] *= so;
-#pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    if (ml[e][q].x == -INFINITY) continue;  // keys this row does not see
-                    const float f = exp2f(ml[e][q].x - Mn);
-                    x[e].x += f * u[e][q].x; x[e].y += f * u[e][q].y; x[e].z += f * u[e][q].z; x[e].w += f * u[e][q].w;
-                    y[e].x += f * v[e][q].x; y[e].y += f * v[e][q].y; y[e].z += f * v[e][q].z; y[e].w += f * v[e][q].w;
-                    L[e] += f * ml[e][q].y;
-                }
-                M[e] = Mn;
+            for (int q = 0; q < 4; q++) {
+                const bool ok = p0 + q < wk.parts;
+                const int slot = wk.slot_base + p0 + (ok ? q : 0);
+                ml[q] = __ldcg(a.split_ml + ((size_t)slot * n_x + X) * 128 + row);
+                const float4* src = slice_rows<D>(a, slot, n_x, X) + row;
+                u[q] = __ldcg(src + (size_t)(2 * c8) * 128);
+                v[q] = __ldcg(src + (size_t)(2 * c8 + 1) * 128);
+                if (!ok) ml[q] = make_float2(-INFINITY, 0.f);
             }
-        }
+            float Mn = M;
 #pragma unroll
-        for (int e = 0; e < 2; e++) {
-            if (idx + e * threads >= n) break;
-            const float inv = 1.f / L[e];
-            uint4 w;
-            w.x = pack2<BF16>(x[e].x * inv, x[e].y * inv); w.y = pack2<BF16>(x[e].z * inv, x[e].w * inv);
-            w.z = pack2<BF16>(y[e].x * inv, y[e].y * inv); w.w = pack2<BF16>(y[e].z * inv, y[e].w * inv);
-            const int rep = row[e] / nv, tok = r0x + row[e] - rep * nv;
-            uint16_t* orow = reinterpret_cast<uint16_t*>(a.out) + ((size_t)wk.sm.tok_off * a.geo.n_q + (size_t)(wk.h * n_rep + rep) * wk.sm.snew + tok) * D;
-            *reinterpret_cast<uint4*>(orow + c8[e] * 8) = w;
+            for (int q = 0; q < 4; q++) Mn = fmaxf(Mn, ml[q].x);
+            const float so = M == -INFINITY ? 0.f : exp2f(M - Mn);
+            x.x *= so; x.y *= so; x.z *= so; x.w *= so; y.x *= so; y.y *= so; y.z *= so; y.w *= so; L *= so;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                if (ml[q].x == -INFINITY) continue;  // keys this row does not see
+                const float f = exp2f(ml[q].x - Mn);
+                x.x += f * u[q].x; x.y += f * u[q].y; x.z += f * u[q].z; x.w += f * u[q].w;
+                y.x += f * v[q].x; y.y += f * v[q].y; y.z += f * v[q].z; y.w += f * v[q].w;
+                L += f * ml[q].y;
+            }
+            M = Mn;
         }
+        const float inv = 1.f / L;
+        uint4 w;
+        w.x = pack2<BF16>(x.x * inv, x.y * inv); w.y = pack2<BF16>(x.z * inv, x.w * inv);
+        w.z = pack2<BF16>(y.x * inv, y.y * inv); w.w = pack2<BF16>(y.z * inv, y.w * inv);
+        const int rep = row / nv, tok = r0x + row - rep * nv;
+        uint16_t* orow = reinterpret_cast<uint16_t*>(a.out) + ((size_t)wk.sm.tok_off * a.geo.n_q + (size_t)(wk.h * n_rep + rep) * wk.sm.snew + tok) * D;
+        *reinterpret_cast<uint4*>(orow + c8 * 8) = w;
     }
 }
 // The CTA's slices are written: draw the item's ticket.  True in every one of the `threads` calling threads (named
