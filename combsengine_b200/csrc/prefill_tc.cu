@@ -585,8 +585,9 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             l_run = l_run * alpha + (sum + sum2);
             TC_ACC(c_exp);
-            // O may be rescaled once the previous P V is complete.  (S being full says that at least of the one
-            // before it, so this wait is at most one phase ahead of the barrier.)
+            // O may be rescaled once the previous P V is complete.  A parity wait cannot tell a phase from the one two
+            // before it, so it holds only where the phase before the awaited one is known to be complete.  Here: the
+            // scores of tile j were issued after P V of tile j - 2, so S being full says that phase j - 2 is.
             if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
                 bool done = mbar_wait_bounded(b_o_done, (j - 1) & 1) && !*failed;
                 done = __all_sync(0xffffffffu, done);
@@ -614,7 +615,10 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
             b[5] = c_ws; b[6] = c_ld; b[7] = c_exp; b[8] = c_wo; b[9] = c_st; b[10] = TC_NOW() - tstart;
         });
         (void)tstart; (void)c_wo;
-        // ---- epilogue: O / l -> out, or a slice's partial rows
+        // ---- epilogue: O / l -> out, or a slice's partial rows.  The last scores say that P V of tile n - 3 is complete
+        // and no more, so phase n - 2 is waited for before n - 1: asked for n - 1 alone, a barrier still in phase n - 2
+        // would answer with phase n - 3, of the same parity (with n = 2, with none at all).
+        if (ok && n_tiles > 1) ok = mbar_wait_bounded(b_o_done, (n_tiles - 2) & 1);
         if (ok) ok = mbar_wait_bounded(b_o_done, (n_tiles - 1) & 1) && !*failed;
         ok = __all_sync(0xffffffffu, ok);
         float* xrow = s_xch + ((n_tiles & 1) * 128 + m) * 2;
@@ -1133,6 +1137,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         });
         const long long t_loop_end = TC_NOW();
         (void)tstart; (void)c_wo; (void)t_loop_end;
+        // (this tile's last scores were issued after its P V of tile n - 2: the wait is one phase ahead, see chunk_tc_kernel)
         if (ok) ok = mbar_wait_bounded(b_o_done + X * 8, (n_tiles - 1) & 1) && !*failed;
         ok = __all_sync(0xffffffffu, ok);
         // the row sum is the two halves' sums (exchanged whether or not the wait succeeded: the pair must

@@ -1,0 +1,77 @@
+"""Chunk steps on the tcgen05 kernels against the oracle (needs a B200): steps of a few tokens and mixed steps at every
+head_dim that the kernels take, items of one K/V tile and of many, cut along K/V and whole, with and without windows."""
+import numpy as np
+import pytest
+import torch
+
+from kvcase import Pair, assert_attention_close
+
+pytestmark = pytest.mark.gpu
+
+REPEATS = 40
+
+
+def _inputs(p, pos, new, grow):
+    """q, k, v of one layer, packed.  `grow`: K rows lengthen with their position and every query points along them, so a
+    row's maximum rises by more than a factor 2^8 from one K/V tile to the next and O is rescaled; otherwise that is rare."""
+    q, k, v = ([p.rand(h, n) for n in new] for h in (p.n_q, p.n_kv, p.n_kv))
+    if grow:
+        for i, (p0, n) in enumerate(zip(pos, new)):
+            t = np.arange(p0, p0 + n, dtype=np.float32)[None, :, None] / 64
+            k[i] = (0.1 * k[i].astype(np.float32) + t * 4 / np.sqrt(p.d)).astype(np.float16)
+            q[i] = (0.1 * q[i].astype(np.float32) + 1).astype(np.float16)
+    return [np.concatenate([x.reshape(-1) for x in xs]) for xs in (q, k, v)]
+
+
+def _fill(p, pair, n, layers, grow):
+    """n cached tokens, appended without attention."""
+    p.g.begin_step([pair[0]], [n])
+    p.o.batch_begin([pair[1]], [n])
+    for l in layers:
+        _, k, v = _inputs(p, [0], [n], grow)
+        p.g.append(l, torch.from_numpy(k).cuda(), torch.from_numpy(v).cuda())
+        pair[1].append_only(l, k.reshape(p.n_kv, n, p.d), v.reshape(p.n_kv, n, p.d), 0)
+
+
+def _step(p, pairs, new, layers, grow, repeats=REPEATS):
+    """One step against the oracle, then rolled back and run again: every run has to give the same bits."""
+    gs, os_ = [s[0] for s in pairs], [s[1] for s in pairs]
+    pos, scale = [s.seq_len() for s in gs], p.d ** -0.5
+    data = {l: _inputs(p, pos, new, grow) for l in layers}
+    dev = {l: [torch.from_numpy(x).cuda() for x in data[l]] for l in layers}
+    outs = []
+    for r in range(repeats):
+        p.g.begin_step(gs, new)
+        outs.append([p.g.attention(l, *dev[l], scale) for l in layers])
+        if r + 1 < repeats:
+            for s, n in zip(gs, new):
+                s.popn(n)
+    assert p.g.device_status() == 0
+    p.o.batch_begin(os_, new)
+    for i, l in enumerate(layers):
+        ref = p.o.batch_layer(os_, new, l, *data[l], p.n_q, scale, None)
+        assert_attention_close(outs[0][i].cpu().numpy(), ref, f"layer {l} contexts {pos} new {new}")
+        for r in range(1, repeats):
+            assert torch.equal(outs[r][i], outs[0][i]), f"layer {l} contexts {pos} new {new}: run {r} differs"
+
+
+KERNELS = [(9, 3, 64, 0), (28, 4, 128, 2), (28, 4, 128, 3), (8, 4, 256, 0)]  # q heads, kv heads, head_dim, chunk kernel
+
+
+@pytest.mark.parametrize("grow", [False, True])
+@pytest.mark.parametrize("n_q,n_kv,d,kernel", KERNELS)
+def test_few_and_mixed_tokens_over_items_of_one_to_many_kv_tiles(n_q, n_kv, d, kernel, grow):
+    # A layer with a window next to a global one.  K/V tiles hold 64 or 128 tokens: the contexts give items of 1, 2, 3, 4
+    # and more tiles; alone, a long one is cut into short slices, in a batch into longer ones.
+    p = Pair(2, n_q, n_kv, d, 8192, num_pages=1400, windows=[300, None], seed=d + kernel, shuffle_free_list=True,
+             popn_refuses=False, chunk_kernel=kernel)
+    for ctx in (1, 60, 126, 250, 380, 500, 2050):
+        s = p.new_seq()
+        _fill(p, s, ctx, [0, 1], grow)
+        _step(p, [s], [5 if ctx % 4 else 2], [0, 1], grow)
+    long = p.new_seq()
+    _fill(p, long, 6100, [0, 1], grow)
+    _step(p, [long], [9], [0, 1], grow)
+    everyone = p.seqs
+    _step(p, everyone, [5] * len(everyone), [0, 1], grow)
+    _step(p, everyone, [1, 2, 3, 1, 140, 9, 1, 130], [0, 1], grow)  # two prompts' chunks among others' few tokens
