@@ -126,7 +126,7 @@ struct DeviceState {
     float* split_o = nullptr;
     float2* split_ml = nullptr;
     int32_t* split_counter = nullptr;
-    size_t split_cap = 0, split_cut_cap = 0;  // slots the buffers hold, counters
+    size_t split_cuts = 0;             // counters
     int last_kv_writer = -1;  // layer whose pages the most recent launch wrote (-1: none since the last upload)
     // host-buffer entry point staging
     uint8_t* io = nullptr;
@@ -376,7 +376,7 @@ int32_t upload_step(Arena* a, cudaStream_t st) {
     // tickets and claim counters start every step at zero, whatever an earlier launch that gave up left behind:
     // the decode kernels' by the step's first unit-table kernel (get_decode_plan), the chunk kernel's here
     d->zero_pending = true;
-    if (d->split_counter && !a->step_is_decode) CU_TRY(cudaMemsetAsync(d->split_counter, 0, d->split_cut_cap * sizeof(int32_t), st));
+    if (d->split_counter && !a->step_is_decode) CU_TRY(cudaMemsetAsync(d->split_counter, 0, d->split_cuts * sizeof(int32_t), st));
     if (a->step_meta.empty()) {  // an empty step: nothing to upload, nothing will launch
         d->uploaded_step = a->step_id;
         return CBKV_OK;
@@ -499,38 +499,36 @@ int rep_slots_of(int n_rep) {
     return rs;
 }
 
-// Room for the partial results of a chunk launch's cut items.  False (nothing is cut then) when there is no memory
-// for it, or when the buffers would have to move while the stream is being captured.
-bool ensure_split(Arena* a, size_t slots, size_t cuts, cudaStream_t st) {
+// Room for the partial results of any chunk launch's cut items (kSplitSlotsPerSm): allocated once, by the arena's first
+// plan with a cut, and kept, because plans of other windows of the step are launched again.  False (nothing is cut
+// then) when there is no memory for it, or when it would have to be allocated while the stream is being captured.
+bool ensure_split(Arena* a, cudaStream_t st) {
     DeviceState* d = dev_of(a);
-    if (slots <= d->split_cap && cuts <= d->split_cut_cap) return true;
+    if (d->split_o) return true;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) { cudaGetLastError(); return false; }
-    if (cudaStreamSynchronize(st) != cudaSuccess) return false;  // the launch that follows reports it
-    if (d->split_o) cudaFree(d->split_o);
-    if (d->split_ml) cudaFree(d->split_ml);
-    if (d->split_counter) cudaFree(d->split_counter);
-    d->split_o = nullptr; d->split_ml = nullptr; d->split_counter = nullptr;
-    d->split_cap = d->split_cut_cap = 0;
-    const size_t ncap = std::max(slots + slots / 4, (size_t)d->sm_count), ccap = std::max(2 * cuts, (size_t)d->sm_count);
+    const size_t slots = (size_t)kSplitSlotsPerSm * (size_t)d->sm_count, cuts = slots / 2;  // a cut has two slices or more
     const size_t rows = chunk_tc2_supported(a->cfg.head_dim) ? 256 : 128;  // of a slot, whichever kernel comes later
-    if (cudaMalloc(&d->split_o, ncap * rows * a->cfg.head_dim * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&d->split_ml, ncap * rows * sizeof(float2)) != cudaSuccess ||
-        cudaMalloc(&d->split_counter, ccap * sizeof(int32_t)) != cudaSuccess ||
-        cudaMemsetAsync(d->split_counter, 0, ccap * sizeof(int32_t), st) != cudaSuccess) {
+    float* o = nullptr;
+    float2* ml = nullptr;
+    int32_t* counter = nullptr;
+    if (cudaMalloc(&o, slots * rows * a->cfg.head_dim * sizeof(float)) != cudaSuccess ||
+        cudaMalloc(&ml, slots * rows * sizeof(float2)) != cudaSuccess ||
+        cudaMalloc(&counter, cuts * sizeof(int32_t)) != cudaSuccess ||
+        cudaMemsetAsync(counter, 0, cuts * sizeof(int32_t), st) != cudaSuccess) {
         cudaGetLastError();
-        if (d->split_o) cudaFree(d->split_o);
-        if (d->split_ml) cudaFree(d->split_ml);
-        if (d->split_counter) cudaFree(d->split_counter);
-        d->split_o = nullptr; d->split_ml = nullptr; d->split_counter = nullptr;
+        if (o) cudaFree(o);
+        if (ml) cudaFree(ml);
+        if (counter) cudaFree(counter);
         return false;
     }
-    d->split_cap = ncap; d->split_cut_cap = ccap;
+    d->split_o = o; d->split_ml = ml; d->split_counter = counter;
+    d->split_cuts = cuts;
     return true;
 }
 
 // Work list of a tcgen05 chunk launch: tokens_per_item new tokens per item in tiles of tile_tokens, K/V tiles of
-// kv_tile tokens.  Built once per step and window; the partial-result buffers grow with it.
+// kv_tile tokens.  Built once per step and window.
 int32_t get_tile_plan(Arena* a, int64_t window, int tokens_per_item, int tile_tokens, int kv_tile, cudaStream_t st, DeviceState::TilePlanDev** out) {
     DeviceState* d = dev_of(a);
     const auto key = std::make_pair(window, tokens_per_item);
@@ -539,7 +537,7 @@ int32_t get_tile_plan(Arena* a, int64_t window, int tokens_per_item, int tile_to
     DeviceState::TilePlanDev pd;
     TileCut cut{window, kv_tile, tile_tokens, d->sm_count, d->chunk_split};
     build_chunk_tile_plan(*a, tokens_per_item, &pd.host, cut);
-    if (!ensure_split(a, (size_t)pd.host.n_slots, (size_t)pd.host.n_cut, st)) {
+    if (pd.host.n_cut > 0 && !ensure_split(a, st)) {
         cut.max_parts = 1;
         build_chunk_tile_plan(*a, tokens_per_item, &pd.host, cut);
     }

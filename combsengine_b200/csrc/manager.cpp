@@ -2,6 +2,7 @@
 #include "manager.hpp"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <functional>
@@ -432,7 +433,8 @@ void build_chunk_tile_plan(const Arena& a, int32_t tokens_per_tile, ChunkPlan* p
             }
         }
         if (n_slots) { *n_slots = slots; *n_cut = cuts; }
-        return out ? 0.f : launch_end(cost, cut.sm_count, &heap) + merge;
+        if (out) return 0.f;
+        return slots > kSplitSlotsPerSm * cut.sm_count ? INFINITY : launch_end(cost, cut.sm_count, &heap) + merge;
     };
 
     float limit = 0.f;

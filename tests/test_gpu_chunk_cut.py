@@ -75,3 +75,39 @@ def test_few_and_mixed_tokens_over_items_of_one_to_many_kv_tiles(n_q, n_kv, d, k
     everyone = p.seqs
     _step(p, everyone, [5] * len(everyone), [0, 1], grow)
     _step(p, everyone, [1, 2, 3, 1, 140, 9, 1, 130], [0, 1], grow)  # two prompts' chunks among others' few tokens
+
+
+@pytest.mark.parametrize("order", [(0, 1), (1, 0)])
+def test_cut_plans_of_two_windows_share_a_step(order):
+    # 58 sequences of very different lengths: the layer with a window is cut into fewer slices of more items than the
+    # global one, and each is launched again after the other.  Reference: the same step with nothing cut.
+    from combsengine_b200 import KVArena
+    ctx, new = [30000] * 15 + [1100] * 26 + [120] * 17, 5
+    n_q, n_kv, d = 8, 4, 256
+    g = KVArena(2, n_q, n_kv, d, 30016, 16, sum(c // 16 + 2 for c in ctx), [1024, None], sliding_popn_refuses=False)
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    rand = lambda n: torch.randn(n, generator=gen, device="cuda", dtype=torch.float16)
+    seqs = [g.new_seq() for _ in ctx]
+    for s, c in zip(seqs, ctx):
+        g.begin_step([s], [c])
+        for l in range(2):
+            g.append(l, rand(c * n_kv * d), rand(c * n_kv * d))
+    q = [rand(len(ctx) * new * n_q * d) for _ in range(2)]
+    kv = [[rand(len(ctx) * new * n_kv * d) for _ in range(2)] for _ in range(2)]
+    outs = {}
+    for parts in (64, 1):
+        g.begin_step(seqs, [new] * len(ctx))
+        if parts == 1:
+            g.set_chunk_split(1)
+        else:
+            plans = [g.debug_tile_plan(w, 64, 64, 64) for w in (1024, 0)]
+            assert plans[0]["n_cut"] > 148 > plans[1]["n_cut"] > 0 and plans[1]["n_slots"] > plans[0]["n_slots"] * 5 // 4
+        for l in order:
+            g.append(l, *kv[l])
+        outs[parts] = [g.paged_attention(l, q[l], d ** -0.5) for l in order + order]
+        assert g.device_status() == 0
+        for s in seqs:
+            s.popn(new)
+    for cut, whole in zip(outs[64], outs[1]):
+        assert_attention_close(cut.cpu().numpy(), whole.cpu().numpy(), f"order {order}")
+    assert all(torch.equal(outs[64][i], outs[64][i + 2]) for i in range(2))

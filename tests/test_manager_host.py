@@ -343,3 +343,19 @@ def test_tile_plan_covers_every_kv_tile_once(lens, new, window, tokens, tile, kv
         assert sl[0][1] == 0 and sl[-1][2] == want[key] and all(x[2] == y[1] for x, y in zip(sl, sl[1:]))
     if max_parts == 1 or sms == 0:
         assert pl["n_cut"] == 0
+
+
+@pytest.mark.parametrize("sms", [2, 7, 148])
+def test_tile_plans_never_need_more_slots_than_the_buffers_have(sms):
+    # the partial-result buffers are allocated once, for 4 slices per SM and half as many cut items
+    a = KVArena(1, 28, 4, 128, 45000, 16, 60000)
+    seqs = [a.new_seq() for _ in range(40)]
+    for i, s_ in enumerate(seqs):
+        a.begin_step_host_only([s_], [100 + 23 * i * i])
+    for n in (1, 2, 9, 40):
+        for new in ([5] * n, [1] * (n - 1) + [700]):
+            a.begin_step_host_only(seqs[40 - n:], new)
+            for window in (0, 1024):
+                for tokens, tile, kv_tile in ((32, 16, 128), (16, 16, 128), (64, 64, 64)):
+                    pl = a.debug_tile_plan(window, tokens, tile, kv_tile, sms)
+                    assert pl["n_slots"] <= 4 * sms and pl["n_cut"] <= 2 * sms
