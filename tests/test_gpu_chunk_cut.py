@@ -111,3 +111,33 @@ def test_cut_plans_of_two_windows_share_a_step(order):
     for cut, whole in zip(outs[64], outs[1]):
         assert_attention_close(cut.cpu().numpy(), whole.cpu().numpy(), f"order {order}")
     assert all(torch.equal(outs[64][i], outs[64][i + 2]) for i in range(2))
+
+
+def _arena_with_context(d, ctx, seed=3, layers=1):
+    from combsengine_b200 import KVArena
+    g = KVArena(layers, 8, 2, d, 2048, 16, 400, sliding_popn_refuses=False)
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    rand = lambda n: torch.randn(n, generator=gen, device="cuda", dtype=torch.float16)
+    s = g.new_seq()
+    g.begin_step([s], [ctx])
+    for l in range(layers):
+        g.append(l, rand(ctx * 2 * d), rand(ctx * 2 * d))
+    return g, s, rand
+
+
+@pytest.mark.parametrize("d", [64, 128, 256])
+@pytest.mark.parametrize("new", [5, 200])
+def test_queries_and_outputs_at_any_element_address(d, new):
+    # the tensor-core kernels move 16 bytes at a time; q at a multiple of 4 bytes and out at any element take the other one
+    g, s, rand = _arena_with_context(d, 700)
+    q, k, v = (rand(new * h * d) for h in (8, 2, 2))
+    outs = []
+    for q_off, out_off in ((0, 0), (2, 0), (0, 1), (6, 3)):
+        qv = torch.empty(q.numel() + 8, dtype=q.dtype, device="cuda")[q_off:q_off + q.numel()].copy_(q)
+        out = torch.zeros(q.numel() + 8, dtype=q.dtype, device="cuda")[out_off:out_off + q.numel()]
+        g.begin_step([s], [new])
+        outs.append(g.attention(0, qv, k, v, d ** -0.5, out=out).cpu().numpy())
+        assert g.device_status() == 0
+        s.popn(new)
+    for o in outs[1:]:
+        assert_attention_close(o, outs[0])
