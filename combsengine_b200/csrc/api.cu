@@ -603,10 +603,10 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
     const float scale_log2 = (float)(scale * 1.4426950408889634);
     // tensor-core chunk kernels, whatever the number of new tokens: a few tokens leave most of a tile's rows empty,
     // but their items are cut along K/V until the chip is full, so the step runs at the rate its K/V arrives
-    // (their softmax takes row maxima before scaling, which needs a positive scale; they read q and write out 16 bytes
+    // (their softmax masks and takes row maxima before scaling, which needs a scale whose 32-bit value is positive; they read q and write out 16 bytes
     // at a time, the mma.sync kernel takes any address that fits its elements)
     const bool aligned16 = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-    const bool tc_able = d->fast && d->tc_ok && scale > 0 && aligned16 && !a->step_is_decode;
+    const bool tc_able = d->fast && d->tc_ok && scale_log2 > 0.f && aligned16 && !a->step_is_decode;
     const bool use_tc2 = tc_able && chunk_tc2_supported(a->cfg.head_dim) &&
                          (d->chunk_mode == 3 || d->chunk_mode == 4 || d->chunk_mode == 0);
     const bool use_tc = tc_able && !use_tc2 && (d->chunk_mode == 2 || d->chunk_mode == 0);

@@ -141,3 +141,13 @@ def test_queries_and_outputs_at_any_element_address(d, new):
         s.popn(new)
     for o in outs[1:]:
         assert_attention_close(o, outs[0])
+
+
+@pytest.mark.parametrize("d", [64, 128, 256])
+def test_scale_that_vanishes_in_32_bits(d):
+    # every visible key gets the same weight; masked scores stay masked
+    p = Pair(1, 8, 2, d, 512, seed=d)
+    s = p.new_seq()
+    p.step([s], [70], scale=1e-50)
+    p.step([s], [5], scale=1e-50)
+    p.step([s], [5], scale=1e-44)
