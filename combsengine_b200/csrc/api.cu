@@ -67,6 +67,7 @@ EncodeTiledFn encode_fn() {
 
 constexpr int kSlots = 4;
 constexpr int kUncutUnits = 40;  // see get_decode_plan
+constexpr int kMaxChunkSplit = 64;
 
 struct StepSlot {
     uint8_t* host = nullptr;  // pinned
@@ -122,7 +123,7 @@ struct DeviceState {
     bool host_direct = true;  // cbkv_set_host_route
     bool zero_pending = false; // the step's first unit-table kernel still has to zero the decode kernels' counters
     // tcgen05 chunk kernels: partial results of items cut along K/V (ChunkArgs::split_*)
-    int chunk_split = 64;              // most slices per item, 1 = never cut (cbkv_set_chunk_split)
+    int chunk_split = kMaxChunkSplit;  // most slices per item, 1 = never cut (cbkv_set_chunk_split)
     float* split_o = nullptr;
     float2* split_ml = nullptr;
     int32_t* split_counter = nullptr;
@@ -1552,7 +1553,7 @@ int32_t cbkv_set_host_route(cbkv_arena* arena, int32_t direct) {
 int32_t cbkv_set_chunk_split(cbkv_arena* arena, int32_t max_parts) {
     return fenced([&]() -> int32_t {
     Arena* a = reinterpret_cast<Arena*>(arena);
-    if (!a || max_parts < 1 || max_parts > 8) { set_error("bad argument"); return CBKV_ERR_ARG; }
+    if (!a || max_parts < 1 || max_parts > kMaxChunkSplit) { set_error("bad argument"); return CBKV_ERR_ARG; }
     int32_t rc = ensure_device(a);
     if (rc) return rc;
     dev_of(a)->chunk_split = max_parts;

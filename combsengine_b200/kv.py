@@ -313,7 +313,7 @@ class KVArena:
         check(self._lib.cbkv_set_host_route(self._h, 1 if direct else 0))
 
     def set_chunk_split(self, max_parts: int) -> None:
-        """tcgen05 chunk kernels: most K/V slices an item may be cut into (1 = never cut)."""
+        """tcgen05 chunk kernels: most K/V slices an item may be cut into, 1..64 (1 = never cut; default 64)."""
         check(self._lib.cbkv_set_chunk_split(self._h, max_parts))
 
     def set_chunk_kernel(self, mode: int) -> None:

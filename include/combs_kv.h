@@ -338,7 +338,8 @@ int32_t cbkv_set_host_route(cbkv_arena* arena, int32_t direct);
 
 /* tcgen05 chunk kernels: when a launch has too few items for the chip (one CTA per SM at a time), or its last
  * wave would leave most SMs idle, items are cut along K/V into up to `max_parts` CTAs each, whose partial
- * rows the last finisher adds up.  1 = never cut; by default as many as a model of the launch finds worth it. */
+ * rows the last finisher adds up, when a model of the launch finds it worth it.  1 = never cut; up to 64,
+ * the default. */
 int32_t cbkv_set_chunk_split(cbkv_arena* arena, int32_t max_parts);
 
 /* Which kernel runs a step that is not pure decode: 0 = the library chooses (tcgen05

@@ -151,3 +151,22 @@ def test_scale_that_vanishes_in_32_bits(d):
     p.step([s], [70], scale=1e-50)
     p.step([s], [5], scale=1e-50)
     p.step([s], [5], scale=1e-44)
+
+
+def test_the_cut_can_be_set_back_to_its_default():
+    from combsengine_b200 import CbkvError
+    g, s, rand = _arena_with_context(128, 1500)
+    q, k, v = (rand(5 * h * 128) for h in (8, 2, 2))
+    outs = []
+    for parts in (None, 1, 8, 64):
+        if parts:
+            g.set_chunk_split(parts)
+        g.begin_step([s], [5])
+        outs.append(g.attention(0, q, k, v, 0.1))
+        s.popn(5)
+    assert torch.equal(outs[0], outs[3])  # the same slices, summed in the same order
+    for o in outs[1:3]:
+        assert_attention_close(o.cpu().numpy(), outs[0].cpu().numpy())
+    for bad in (0, 65):
+        with pytest.raises(CbkvError):
+            g.set_chunk_split(bad)
