@@ -584,9 +584,9 @@ int32_t run_append(Arena* a, int layer, const void* k, const void* v, cudaStream
     AppendArgs args{d->step, geom(a), k, v, d->layers[(size_t)layer].base, d->status};
     if (d->layers[(size_t)layer].quant) {
         args.geo.tiled = 0;
-        CU_TRY(launch_append_quant(args, a->cfg.dtype == CBKV_BF16, st));
+        CU_TRY(launch_append_quant(args, a->cfg.dtype == CBKV_BF16, d->pdl, st));
     } else {
-        CU_TRY(launch_append(args, a->cfg.dtype == CBKV_BF16, st));
+        CU_TRY(launch_append(args, a->cfg.dtype == CBKV_BF16, d->pdl, st));
     }
     g_launches++;
     d->last_kv_writer = layer;
@@ -625,7 +625,7 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
         }
         GeomDev g = geom(a);
         { int32_t frc = flush_uploads(d, st); if (frc) return frc; }
-        CU_TRY(launch_dequant_pages(d->step.tables, (int)a->step_tables.size(), g, L.base, d->qscratch.base, d->status, bf16, st));
+        CU_TRY(launch_dequant_pages(d->step.tables, (int)a->step_tables.size(), g, L.base, d->qscratch.base, d->status, bf16, d->pdl, st));
         g_launches++;
         KV = &d->qscratch;
     } else if (L.quant && !q8_direct && !(d->fast && a->step_is_decode && !(debug_flags() & 16))) {
@@ -698,8 +698,8 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
 #endif
         ProfScope ps(d, st);
         { int32_t frc = flush_uploads(d, st); if (frc) return frc; }
-        if (use_tc2) CU_TRY(q8_direct ? launch_chunk_tc2(L.map_k16, L.map_sc, args, bf16, st) : launch_chunk_tc2(KV->map_page, KV->map_page, args, bf16, st));
-        else CU_TRY(launch_chunk_tc(KV->map_page, args, bf16, st));
+        if (use_tc2) CU_TRY(q8_direct ? launch_chunk_tc2(L.map_k16, L.map_sc, args, bf16, d->pdl, st) : launch_chunk_tc2(KV->map_page, KV->map_page, args, bf16, d->pdl, st));
+        else CU_TRY(launch_chunk_tc(KV->map_page, args, bf16, d->pdl, st));
         g_launches++;
         d->last_kv_writer = -1;
         return CBKV_OK;
@@ -993,7 +993,7 @@ static int32_t run_rope_append(Arena* a, int layer, const Rope* r, const cbkv_qk
     args.gemma = norm ? norm->gemma : 0;
     args.status = d->status;
     { int32_t frc = flush_uploads(d, st); if (frc) return frc; }
-    CU_TRY(launch_rope_append(args, a->cfg.dtype == CBKV_BF16, st));
+    CU_TRY(launch_rope_append(args, a->cfg.dtype == CBKV_BF16, d->pdl, st));
     g_launches++;
     if (!k_out) d->last_kv_writer = layer;
     return CBKV_OK;

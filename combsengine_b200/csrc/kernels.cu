@@ -1527,12 +1527,12 @@ cudaError_t kernels_init() {
     return cudaSuccess;
 }
 
-cudaError_t launch_append(const AppendArgs& a, bool bf16, cudaStream_t st) {
+cudaError_t launch_append(const AppendArgs& a, bool bf16, bool overlap, cudaStream_t st) {
     (void)bf16;  // a bit copy: the element type does not matter
     int64_t total = (int64_t)a.step.n_tokens * a.geo.n_kv * 2 * (a.geo.d / 8);
     int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 8);
     if (blocks <= 0) return cudaSuccess;
-    return launch_pdl(append_kernel<uint16_t>, blocks, 256, 0, st, a);
+    return launch_pdl(overlap, append_kernel<uint16_t>, blocks, 256, 0, st, a);
 }
 
 template <int D, int C, bool BF16, bool Q8>

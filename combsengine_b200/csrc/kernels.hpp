@@ -186,7 +186,8 @@ DecodeConfig decode_config(int d, int n_rep, int ctas_per_sm, int stages, int co
 struct ChunkConfig { int warps, stages, smem_bytes, cols_per_item; };
 ChunkConfig chunk_config(int d);
 
-cudaError_t launch_append(const AppendArgs& a, bool bf16, cudaStream_t st);
+// overlap: the launch may start under its predecessor's tail (pdl.cuh)
+cudaError_t launch_append(const AppendArgs& a, bool bf16, bool overlap, cudaStream_t st);
 cudaError_t launch_decode(const CUtensorMap& map, const DecodeArgs& a, int n_ctas, int consumers, int smem_bytes, bool pdl, bool bf16, cudaStream_t st,
                           bool q8 = false);  // q8: the layer holds int8 records, `map` is the byte view with one record per box
 cudaError_t launch_chunk(const CUtensorMap& map, const ChunkArgs& a, bool bf16, cudaStream_t st);
@@ -197,22 +198,22 @@ cudaError_t launch_resolve_units(const SegInfo* segs, int n_segs, const int32_t*
                                  int32_t* unit_row, int n_units, int32_t* status, cudaStream_t st,
                                  int32_t* zero_a = nullptr, int n_a = 0, int32_t* zero_b = nullptr, int n_b = 0);
 cudaError_t launch_init_quant(void* arena, size_t n_records, int page_size, int d, cudaStream_t st);
-cudaError_t launch_append_quant(const AppendArgs& a, bool bf16, cudaStream_t st);
+cudaError_t launch_append_quant(const AppendArgs& a, bool bf16, bool overlap, cudaStream_t st);
 cudaError_t launch_dequant_pages(const int32_t* tables, int n_entries, const GeomDev& geo, const void* arena, void* scratch,
-                                 int32_t* status, bool bf16, cudaStream_t st);
+                                 int32_t* status, bool bf16, bool overlap, cudaStream_t st);
 cudaError_t launch_generic_quant(const GenericArgs& a, bool bf16, cudaStream_t st);
-cudaError_t launch_rope_append(const RopeArgs& a, bool bf16, cudaStream_t st);
+cudaError_t launch_rope_append(const RopeArgs& a, bool bf16, bool overlap, cudaStream_t st);
 // host side of the rotary tables (rope.cu): frequencies, then [max_position][head_dim] f32 tables
 int32_t rope_inv_freq(const cbkv_rope_config& c, std::vector<double>* inv, double* mscale);
 void rope_tables(const cbkv_rope_config& c, const std::vector<double>& inv, double mscale, float* cos_out, float* sin_out);
 // tcgen05 chunk kernel (prefill_tc.cu): head_dim 64, 128 or 256; `map` is the layer's map_page
 bool chunk_tc_supported(int d);
 cudaError_t chunk_tc_init();
-cudaError_t launch_chunk_tc(const CUtensorMap& map, const ChunkArgs& a, bool bf16, cudaStream_t st);
+cudaError_t launch_chunk_tc(const CUtensorMap& map, const ChunkArgs& a, bool bf16, bool overlap, cudaStream_t st);
 // two query tiles per CTA, P in tensor memory (head_dim 128)
 bool chunk_tc2_supported(int d);
 // float layer: `map` = the layer's map_page, map_sc is not used; int8 layer (a.q8_arena non-null): its map_k16 and map_sc
-cudaError_t launch_chunk_tc2(const CUtensorMap& map, const CUtensorMap& map_sc, const ChunkArgs& a, bool bf16, cudaStream_t st);
+cudaError_t launch_chunk_tc2(const CUtensorMap& map, const CUtensorMap& map_sc, const ChunkArgs& a, bool bf16, bool overlap, cudaStream_t st);
 cudaError_t kernels_init();  // raises the dynamic shared memory limits once per process
 
 }  // namespace cbkv

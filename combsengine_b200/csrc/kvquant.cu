@@ -246,19 +246,19 @@ cudaError_t launch_init_quant(void* arena, size_t n_records, int page_size, int 
     return cudaGetLastError();
 }
 
-cudaError_t launch_append_quant(const AppendArgs& a, bool bf16, cudaStream_t st) {
+cudaError_t launch_append_quant(const AppendArgs& a, bool bf16, bool overlap, cudaStream_t st) {
     const int64_t rows = 2 * (int64_t)a.step.n_tokens * a.geo.n_kv;
     if (rows <= 0) return cudaSuccess;
     const int blocks = (int)std::min<int64_t>((rows + 7) / 8, 148 * 8);
-    return launch_pdl(bf16 ? append_quant_kernel<true> : append_quant_kernel<false>, blocks, 256, 0, st, a);
+    return launch_pdl(overlap, bf16 ? append_quant_kernel<true> : append_quant_kernel<false>, blocks, 256, 0, st, a);
 }
 
 cudaError_t launch_dequant_pages(const int32_t* tables, int n_entries, const GeomDev& geo, const void* arena, void* scratch,
-                                 int32_t* status, bool bf16, cudaStream_t st) {
+                                 int32_t* status, bool bf16, bool overlap, cudaStream_t st) {
     const int64_t items = (int64_t)n_entries * geo.n_kv;
     if (items <= 0) return cudaSuccess;
     const int blocks = (int)std::min<int64_t>((items + 7) / 8, 148 * 8);
-    return launch_pdl(bf16 ? dequant_pages_kernel<true> : dequant_pages_kernel<false>, blocks, 256, 0, st, tables, n_entries, geo,
+    return launch_pdl(overlap, bf16 ? dequant_pages_kernel<true> : dequant_pages_kernel<false>, blocks, 256, 0, st, tables, n_entries, geo,
                       reinterpret_cast<const uint8_t*>(arena), reinterpret_cast<uint16_t*>(scratch), status);
 }
 

@@ -677,9 +677,9 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
 }
 
 template <int D, bool BF16>
-static cudaError_t launch_tc(const CUtensorMap& map32, const ChunkArgs& a, cudaStream_t st) {
+static cudaError_t launch_tc(const CUtensorMap& map32, const ChunkArgs& a, bool overlap, cudaStream_t st) {
     if (a.n_items <= 0) return cudaSuccess;
-    return launch_pdl(chunk_tc_kernel<D, BF16>, a.n_items, kThreads, tc_smem_bytes<D>(), st, map32, a);
+    return launch_pdl(overlap, chunk_tc_kernel<D, BF16>, a.n_items, kThreads, tc_smem_bytes<D>(), st, map32, a);
 }
 
 
@@ -1203,18 +1203,18 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
 }
 
 template <bool BF16>
-static cudaError_t launch_tc2(const CUtensorMap& map32, const CUtensorMap& map_sc, const ChunkArgs& a, cudaStream_t st) {
+static cudaError_t launch_tc2(const CUtensorMap& map32, const CUtensorMap& map_sc, const ChunkArgs& a, bool overlap, cudaStream_t st) {
     if (a.n_items <= 0) return cudaSuccess;
-    if (a.q8_arena) return launch_pdl(chunk_tc2_kernel<128, BF16, true>, a.n_items, kThreads2Q8, tc2_smem_bytes_q8<128>(), st, map32, map_sc, a);
-    return launch_pdl(chunk_tc2_kernel<128, BF16, false>, a.n_items, kThreads2, tc2_smem_bytes<128>(), st, map32, map_sc, a);
+    if (a.q8_arena) return launch_pdl(overlap, chunk_tc2_kernel<128, BF16, true>, a.n_items, kThreads2Q8, tc2_smem_bytes_q8<128>(), st, map32, map_sc, a);
+    return launch_pdl(overlap, chunk_tc2_kernel<128, BF16, false>, a.n_items, kThreads2, tc2_smem_bytes<128>(), st, map32, map_sc, a);
 }
 
 bool chunk_tc2_supported(int d) { return d == 128; }
 
 // Two query tiles per CTA (head_dim 128): the work list has one item per pair of tiles.
-cudaError_t launch_chunk_tc2(const CUtensorMap& map32, const CUtensorMap& map_sc, const ChunkArgs& a, bool bf16, cudaStream_t st) {
+cudaError_t launch_chunk_tc2(const CUtensorMap& map32, const CUtensorMap& map_sc, const ChunkArgs& a, bool bf16, bool overlap, cudaStream_t st) {
     if (a.geo.d != 128) return cudaErrorInvalidValue;
-    return bf16 ? launch_tc2<true>(map32, map_sc, a, st) : launch_tc2<false>(map32, map_sc, a, st);
+    return bf16 ? launch_tc2<true>(map32, map_sc, a, overlap, st) : launch_tc2<false>(map32, map_sc, a, overlap, st);
 }
 
 bool chunk_tc_supported(int d) { return d == 64 || d == 128 || d == 256; }
@@ -1235,11 +1235,11 @@ cudaError_t chunk_tc_init() {
 }
 
 // `map32`: the layer's 32-row box view (K and V of a page per box).
-cudaError_t launch_chunk_tc(const CUtensorMap& map32, const ChunkArgs& a, bool bf16, cudaStream_t st) {
+cudaError_t launch_chunk_tc(const CUtensorMap& map32, const ChunkArgs& a, bool bf16, bool overlap, cudaStream_t st) {
     switch (a.geo.d) {
-        case 64: return bf16 ? launch_tc<64, true>(map32, a, st) : launch_tc<64, false>(map32, a, st);
-        case 128: return bf16 ? launch_tc<128, true>(map32, a, st) : launch_tc<128, false>(map32, a, st);
-        case 256: return bf16 ? launch_tc<256, true>(map32, a, st) : launch_tc<256, false>(map32, a, st);
+        case 64: return bf16 ? launch_tc<64, true>(map32, a, overlap, st) : launch_tc<64, false>(map32, a, overlap, st);
+        case 128: return bf16 ? launch_tc<128, true>(map32, a, overlap, st) : launch_tc<128, false>(map32, a, overlap, st);
+        case 256: return bf16 ? launch_tc<256, true>(map32, a, overlap, st) : launch_tc<256, false>(map32, a, overlap, st);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -341,26 +341,26 @@ __global__ void __launch_bounds__(256) rope_append_vec_kernel(const RopeArgs a) 
 }
 
 template <bool BF16>
-static cudaError_t launch_rope_t(const RopeArgs& a, int64_t rows, cudaStream_t st) {
+static cudaError_t launch_rope_t(const RopeArgs& a, int64_t rows, bool overlap, cudaStream_t st) {
     const int t = a.geo.d / 16;
     const int rpw = t ? 32 / t : 0;
     auto grid = [&](int per_block) { return (int)std::min<int64_t>((rows + per_block - 1) / per_block, 148 * 8); };
     const bool vec = rows < ((int64_t)1 << 31) - 64;  // the vector kernels count rows in 32 bits
     switch (vec ? a.geo.d : 0) {
-        case 16: return launch_pdl(rope_append_vec_kernel<BF16, 1>, grid(8 * rpw), 256, 0, st, a);
-        case 32: return launch_pdl(rope_append_vec_kernel<BF16, 2>, grid(8 * rpw), 256, 0, st, a);
-        case 64: return launch_pdl(rope_append_vec_kernel<BF16, 4>, grid(8 * rpw), 256, 0, st, a);
-        case 128: return launch_pdl(rope_append_vec_kernel<BF16, 8>, grid(8 * rpw), 256, 0, st, a);
-        case 256: return launch_pdl(rope_append_vec_kernel<BF16, 16>, grid(8 * rpw), 256, 0, st, a);
-        case 512: return launch_pdl(rope_append_vec_kernel<BF16, 32>, grid(8 * rpw), 256, 0, st, a);
-        default: return launch_pdl(rope_append_kernel<BF16>, grid(8), 256, 0, st, a);  // one warp per row
+        case 16: return launch_pdl(overlap, rope_append_vec_kernel<BF16, 1>, grid(8 * rpw), 256, 0, st, a);
+        case 32: return launch_pdl(overlap, rope_append_vec_kernel<BF16, 2>, grid(8 * rpw), 256, 0, st, a);
+        case 64: return launch_pdl(overlap, rope_append_vec_kernel<BF16, 4>, grid(8 * rpw), 256, 0, st, a);
+        case 128: return launch_pdl(overlap, rope_append_vec_kernel<BF16, 8>, grid(8 * rpw), 256, 0, st, a);
+        case 256: return launch_pdl(overlap, rope_append_vec_kernel<BF16, 16>, grid(8 * rpw), 256, 0, st, a);
+        case 512: return launch_pdl(overlap, rope_append_vec_kernel<BF16, 32>, grid(8 * rpw), 256, 0, st, a);
+        default: return launch_pdl(overlap, rope_append_kernel<BF16>, grid(8), 256, 0, st, a);  // one warp per row
     }
 }
 
-cudaError_t launch_rope_append(const RopeArgs& a, bool bf16, cudaStream_t st) {
+cudaError_t launch_rope_append(const RopeArgs& a, bool bf16, bool overlap, cudaStream_t st) {
     const int64_t rows = (int64_t)a.step.n_tokens * (a.geo.n_q + (a.k_out ? 1 : 2) * a.geo.n_kv);
     if (rows <= 0) return cudaSuccess;
-    return bf16 ? launch_rope_t<true>(a, rows, st) : launch_rope_t<false>(a, rows, st);
+    return bf16 ? launch_rope_t<true>(a, rows, overlap, st) : launch_rope_t<false>(a, rows, overlap, st);
 }
 
 }  // namespace cbkv

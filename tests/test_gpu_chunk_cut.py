@@ -170,3 +170,40 @@ def test_the_cut_can_be_set_back_to_its_default():
     for bad in (0, 65):
         with pytest.raises(CbkvError):
             g.set_chunk_split(bad)
+
+
+@pytest.mark.parametrize("overlap", [True, False])
+@pytest.mark.parametrize("d,int8", [(64, False), (128, False), (128, True)])
+def test_overlap_switch_covers_every_launch_of_a_chunk_step(d, int8, overlap):
+    # captured into a graph that is not run: launches that may overlap are joined by programmatic edges
+    import ctypes as C
+    from combsengine_b200 import KVArena, RotaryEmbedding, attention_rope
+    rt = C.CDLL("libcudart.so.12")
+    g = KVArena(1, 8, 2, d, 256, 16, 40, quantize_kv=int8)
+    g.set_decode_tuning(overlap_launches=overlap)
+    rope = RotaryEmbedding(g, 10000.0, 256)
+    s = g.new_seq()
+    q, k, v = (torch.randn(70 * h * d, device="cuda").half() for h in (8, 2, 2))
+    out = torch.empty_like(q)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    g.begin_step([s], [70], stream=stream)
+
+    def calls():
+        g.attention(0, q, k, v, 0.1, out=out, stream=stream)
+        attention_rope(g, 0, rope, q, k, v, 0.1, out=out, stream=stream)
+
+    calls()  # uploads, plans and workspaces are in place after this
+    st, graph, n = C.c_void_p(stream.cuda_stream), C.c_void_p(), C.c_size_t()
+    assert rt.cudaStreamBeginCapture(st, 2) == 0  # relaxed
+    calls()
+    assert rt.cudaStreamEndCapture(st, C.byref(graph)) == 0
+    assert rt.cudaGraphGetEdges_v2(graph, None, None, None, C.byref(n)) == 0
+    ends, data = [(C.c_void_p * n.value)() for _ in range(2)], (C.c_ubyte * 8 * n.value)()  # from port, to port, type, padding
+    assert rt.cudaGraphGetEdges_v2(graph, *ends, data, C.byref(n)) == 0
+    assert n.value == (6 if int8 else 3)
+    assert [e[2] for e in data] == [1 if overlap else 0] * n.value
+    assert rt.cudaGraphDestroy(graph) == 0
+    torch.cuda.synchronize()
+    assert g.device_status() == 0
+    rope.close()
