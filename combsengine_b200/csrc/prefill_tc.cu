@@ -689,7 +689,7 @@ static cudaError_t launch_tc(const CUtensorMap& map32, const ChunkArgs& a, bool 
 // memory (it overwrites the first 64 columns of its S tile as packed 16-bit pairs and is the
 // A operand of the P V product), so no shared memory is spent on P.
 //
-//   warp 0        TMA producer (as above)
+//   warp 0        TMA producer: K and V of a tile in one stage, a box of both per page and 64 columns
 //   warp 1        MMA issuer:  QK_A, QK_B, then per K/V tile  PV_A, QK_A', PV_B, QK_B'
 //   warps 2..9    softmax of tile A        warps 10..17  softmax of tile B
 //
@@ -698,6 +698,11 @@ static cudaError_t launch_tc(const CUtensorMap& map32, const ChunkArgs& a, bool 
 // may touch the same quarter of the tensor-memory lanes; one takes keys 0-63 of the tile, the other keys
 // 64-127 (and, when the row maximum moves, the matching half of the O columns).  They exchange their half-row
 // maxima through shared memory once per tile and their half-row sums once at the end.
+//
+// K and V in buffers of their own, as in the kernel above, with the producer started before Q is in place, gain
+// nothing here, where two tiles of work per load hide its wait, and cost another barrier per tile: 8 prompts of 8192
+// tokens over four layers 23.9 ms against 23.5, 6 ragged prompts over int8 pages 4.46 against 4.38, verification of
+// 16 drafts 3.06 against 3.02.
 //
 // Tensor memory: S_A [0,128), S_B [128,256), O_A [256,384), O_B [384,512).
 constexpr int kThreads2 = 576;
@@ -736,15 +741,15 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     constexpr uint32_t TILE = 128u * D * 2u;   // one Q tile
     constexpr uint32_t BLK = 128u * 128u;      // 64-column block of a Q tile
     constexpr int XB = D / 64;
-    constexpr uint32_t STAGE = 2u * TILE;      // a K and a V buffer
+    constexpr uint32_t BLKKV = 8u * 4096u;     // 64-column block of a K/V stage
+    constexpr uint32_t STAGE = 2u * TILE;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sQ = smem;                 // Q_A then Q_B
-    uint8_t* sKV = sQ + 2 * TILE;       // float layer: 2 K buffers, 2 V buffers of 32 KB, [page][8-token group][column block][8 rows of 128 bytes]
+    uint8_t* sKV = sQ + 2 * TILE;       // 2 stages
     uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + 2 * STAGE);
     // barriers: kv_full[2], kv_empty[2], s_full[A,B], p_full[A,B], o_done[A,B]
     const uint32_t b_kv_full = smem_u32(bars + 0), b_kv_empty = smem_u32(bars + 2), b_s_full = smem_u32(bars + 4);
     const uint32_t b_p_full = smem_u32(bars + 6), b_o_done = smem_u32(bars + 8);
-    const uint32_t b_vf2 = smem_u32(bars + 12), b_ve2 = smem_u32(bars + 14);  // float layer: v_full[2], v_empty[2]; kv_full / kv_empty are K's
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
     volatile int* failed = reinterpret_cast<volatile int*>(bars + 11);
     int* s_pages = reinterpret_cast<int*>(bars + 16);
@@ -761,7 +766,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     uint8_t* sRawV0 = sRawK + kRawK * HALF;
     uint8_t* sRawV1 = reinterpret_cast<uint8_t*>(s_xch + 2 * 2 * 128 * 2) + 128;  // 128-byte aligned, as every slot is
     const uint32_t b_q8 = smem_u32(sRawV1 + (kRawV - kRawVInStage) * HALF);
-    const uint32_t b_v_full = Q8 ? b_q8 : b_vf2, b_v_empty = Q8 ? b_q8 + 8 : b_ve2, b_rawk = b_q8 + 16, b_rawv = b_rawk + kRawK * 8;
+    const uint32_t b_v_full = b_q8, b_v_empty = b_q8 + 8, b_rawk = b_q8 + 16, b_rawv = b_rawk + kRawK * 8;
     (void)sRawK; (void)sRawV0; (void)sRawV1; (void)b_v_full; (void)b_v_empty; (void)b_rawk; (void)b_rawv; (void)REC;
 
     const long long t_entry = TC_NOW();
@@ -790,8 +795,8 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
             mbar_init(b_kv_full + i * 8, 1); mbar_init(b_kv_empty + i * 8, 1); mbar_init(b_s_full + i * 8, 1);
             mbar_init(b_p_full + i * 8, 256); mbar_init(b_o_done + i * 8, 1);
         }
-        for (int i = 0; i < (Q8 ? 1 : 2); i++) { mbar_init(b_v_full + i * 8, 1); mbar_init(b_v_empty + i * 8, 1); }
-        if constexpr (Q8) {
+        if constexpr (Q8) {  // kv_full / kv_empty above are K's here
+            mbar_init(b_v_full, 1); mbar_init(b_v_empty, 1);
             for (int i = 0; i < kRawK + kRawV; i++) mbar_init(b_rawk + i * 8, 1);
         }
         *failed = 0;
@@ -805,18 +810,14 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     for (int i = tid; i <= p_hi - p_lo && i < kPageCap; i += (int)blockDim.x) s_pages[i] = a.step.tables[sm.tbl_off + p_lo + i];
-    tc_fence_before();
-    __syncthreads();  // barriers and block table are ready: the producer starts while the other warps bring Q
-    tc_fence_after();
     // q, the pages and the partial-result buffers belong to earlier launches until here; everything above (barriers,
     // tensor memory, the work record and the block table, which came with the step's upload) runs under their tail
     pdl_wait();
     pdl_launch_dependents();
-    // ---- Q tiles (every warp but the float layer's producer): row m of tile X is q head (m / TPT) at token r0 + X TPT + m % TPT
-    if (Q8 || warp != 0) {
-        const int first = Q8 ? 0 : 32, n_thr = (int)blockDim.x - first;
+    // ---- Q tiles: row m of tile X is q head (m / TPT) at token r0 + X TPT + m % TPT
+    {
         const uint16_t* qbase = reinterpret_cast<const uint16_t*>(a.q) + (size_t)sm.tok_off * a.geo.n_q * D;
-        for (int c = tid - first; c < (two ? 256 : 128) * (D / 8); c += n_thr) {
+        for (int c = tid; c < (two ? 256 : 128) * (D / 8); c += (int)blockDim.x) {
             const int mm = c / (D / 8), j = c - mm * (D / 8);
             const int X = mm >> 7, m = mm & 127;
             const int rep = m / TPT, r = r0 + X * TPT + (m - rep * TPT);
@@ -826,9 +827,11 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
             const uint32_t off = X * TILE + (j >> 3) * BLK + m * 128u + (((j & 7) ^ (m & 7)) << 4);
             *reinterpret_cast<uint4*>(sQ + off) = val;
         }
-        fence_proxy_async();
-        bar_sync(10, n_thr);
     }
+    fence_proxy_async();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
     if (Q8 && warp >= 18) {
@@ -942,33 +945,29 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         TC_DUMP(if (tid == 18 * 32) { unsigned long long* b = a.dbg_buf + (size_t)blockIdx.x * 16; b[0] = c_wait; b[1] = c_issue + c_conv + c_meet; b[12] = c_conv; b[13] = c_meet; b[14] = c_issue; b[15] = n_tiles; });
         (void)c_wait; (void)c_issue; (void)c_conv; (void)c_meet; (void)tprev;
     } else if (!Q8 && warp == 0) {
-        // ------------------------------------------------------------ TMA producer: one copy per page and operand
+        // ------------------------------------------------------------ TMA producer
         bool ok = true;
         long long tprev = TC_NOW(), c_wait = 0, c_issue = 0;
 #pragma unroll 1
         for (int j = 0; j < n_tiles && ok; j++) {
             const int st = j & 1;
-            int phys = 0;
-            if (lane < 8) {
-                const int idx = min(j * 8 + lane, p_hi - p_lo);  // pages past the end repeat the last one (masked)
-                phys = idx < kPageCap ? s_pages[idx] : a.step.tables[sm.tbl_off + p_lo + idx];
+            if (lane == 0) {
+                if (j >= 2 && !mbar_wait_bounded(b_kv_empty + st * 8, ((j >> 1) - 1) & 1)) ok = false;
+                TC_ACC(c_wait);
+                if (*failed) ok = false;
+                if (ok) mbar_expect_tx(b_kv_full + st * 8, STAGE);
+                else { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
+            }
+            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+            if (!ok) break;
+            for (int bx = lane; bx < 8 * XB; bx += 32) {
+                const int pg = bx / XB, x = bx - pg * XB;
+                const int idx = min(j * 8 + pg, p_hi - p_lo);  // pages past the end repeat the last one (masked)
+                int phys = idx < kPageCap ? s_pages[idx] : a.step.tables[sm.tbl_off + p_lo + idx];
                 if (phys < 0 || phys >= a.geo.num_pages) { atomicOr(a.status, ST_BAD_PAGE); phys = 0; }
+                tma_load_2d(smem_u32(sKV + st * STAGE + x * BLKKV + pg * 4096), &tmap32, x * 64, (phys * Hkv + h) * 32, b_kv_full + st * 8);
             }
-#pragma unroll
-            for (int is_v = 0; is_v < 2 && ok; is_v++) {
-                const uint32_t full = (is_v ? b_v_full : b_kv_full) + st * 8, empty = (is_v ? b_v_empty : b_kv_empty) + st * 8;
-                if (lane == 0) {
-                    if (j >= 2 && !mbar_wait_bounded(empty, ((j >> 1) - 1) & 1)) ok = false;
-                    TC_ACC(c_wait);
-                    if (*failed) ok = false;
-                    if (ok) mbar_expect_tx(full, TILE);
-                    else { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
-                }
-                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-                if (ok && lane < 8)
-                    tma_load_page(smem_u32(sKV + (2 * is_v + st) * TILE + lane * (16 * D * 2)), &tmap32, is_v, (phys * Hkv + h) * 2, full);
-                if (lane == 0) TC_ACC(c_issue);
-            }
+            if (lane == 0) TC_ACC(c_issue);
         }
         TC_DUMP(if (lane == 0) { a.dbg_buf[(size_t)blockIdx.x * 16 + 0] = c_wait; a.dbg_buf[(size_t)blockIdx.x * 16 + 1] = c_issue; a.dbg_buf[(size_t)blockIdx.x * 16 + 15] = n_tiles; });
     } else if (warp == 1) {
@@ -976,12 +975,11 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         if (lane == 0) {
             const uint32_t id_qk = instr_desc(BF16, 128, 128, false);
             const uint32_t id_pv = instr_desc(BF16, 128, D, true);
-            // 64-wide column blocks, 8-token groups and pages of a K or V buffer (see the shared memory map)
-            constexpr uint32_t KBUF = Q8 ? QBUF : TILE, KBLK = Q8 ? QBLK : 1024u, GRP = Q8 ? 1024u : XB * 1024u, VPAGE = Q8 ? 2048u : 2 * XB * 1024u;
+            // float layer: a stage holds pages as they lie in device memory (K and V rows of a page interleaved in
+            // groups of eight); int8 layer: the loader warps lay K and V out separately (see the shared memory map)
+            constexpr uint32_t KBUF = Q8 ? QBUF : STAGE, KBLK = Q8 ? QBLK : BLKKV, GRP = Q8 ? 1024u : 2048u, VPAGE = Q8 ? 2048u : 4096u;
             const uint64_t dq = smem_desc(smem_u32(sQ), 16, 1024), dk = smem_desc(smem_u32(sKV), 16, GRP);
-            const uint64_t dv = smem_desc(smem_u32(sKV) + 2 * KBUF, KBLK, GRP);
-            auto v_bar = [&](uint32_t b, int j) { return b + (Q8 ? 0u : (uint32_t)(j & 1) * 8); };  // int8 layers have one V buffer
-            auto v_par = [&](int j) { return (uint32_t)(Q8 ? j & 1 : (j >> 1) & 1); };
+            const uint64_t dv = smem_desc(smem_u32(sKV) + (Q8 ? 2 * QBUF : 1024u), KBLK, GRP);
             auto issue_qk = [&](int X, int j) {
                 const uint64_t kst = (uint64_t)(((j & 1) * KBUF) >> 4), qst = (uint64_t)((X * TILE) >> 4);
 #pragma unroll
@@ -991,10 +989,10 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                     umma(tmem + X * 128, dq + qst + qoff, dk + kst + koff, id_qk, ks > 0);
                 }
                 umma_commit(b_s_full + X * 8);
-                if (X == (two ? 1 : 0)) umma_commit(b_kv_empty + (j & 1) * 8);  // all scores of this K buffer have been issued
+                if (Q8 && X == (two ? 1 : 0)) umma_commit(b_kv_empty + (j & 1) * 8);  // all scores of this K buffer have been issued
             };
             auto issue_pv = [&](int X, int j) {
-                const uint64_t vst = Q8 ? 0ull : (uint64_t)(((j & 1) * KBUF) >> 4);
+                const uint64_t vst = Q8 ? 0ull : (uint64_t)(((j & 1) * STAGE) >> 4);
 #pragma unroll
                 for (int ks = 0; ks < 8; ks++)  // 16 keys = one page per step; P: 8 packed columns per step
                     umma_ts(tmem + 256 + X * 128, tmem + X * 128 + ks * 8, dv + vst + (uint64_t)((ks * VPAGE) >> 4), id_pv, (j > 0 || ks > 0));
@@ -1007,12 +1005,12 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                 TC_ACC(c_iss);
                 ok = mbar_wait_bounded(b_p_full, j & 1) && !*failed;
                 TC_ACC(c_wp);
-                if (ok) { ok = mbar_wait_bounded(v_bar(b_v_full, j), v_par(j)); TC_ACC(c_wkv); }
+                if (Q8 && ok) { ok = mbar_wait_bounded(b_v_full, j & 1); TC_ACC(c_wkv); }
                 if (!ok) break;
                 tc_fence_after();
                 issue_pv(0, j);
                 TC_ACC(c_pv);
-                if (!two) umma_commit(v_bar(b_v_empty, j));
+                if (!two && !Q8) umma_commit(b_kv_empty + (j & 1) * 8);
                 if (j + 1 < n_tiles) {
                     ok = mbar_wait_bounded(b_kv_full + ((j + 1) & 1) * 8, ((j + 1) >> 1) & 1);
                     TC_ACC(c_wkv);
@@ -1029,7 +1027,8 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                     issue_pv(1, j);
                     TC_ACC(c_pv);
                 }
-                if (two) umma_commit(v_bar(b_v_empty, j));  // every read of this V buffer has been issued before
+                // every read of this stage (int8 layer: of the V buffer) has been issued before
+                if (two || Q8) umma_commit(Q8 ? b_v_empty : b_kv_empty + (j & 1) * 8);
                 if (two && j + 1 < n_tiles) issue_qk(1, j + 1);
             }
             if (!ok) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
