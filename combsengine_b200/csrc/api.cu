@@ -110,7 +110,7 @@ struct DeviceState {
     const int32_t* chunk_item_begin = nullptr;
     bool tc_ok = false;       // the tcgen05 chunk kernel covers this geometry
     int chunk_mode = 0;       // cbkv_set_chunk_kernel: 0 = choose, 1 = mma.sync, 2 = tcgen05 one tile, 3 = two tiles, 4 = two tiles, int8 records converted in the kernel
-    struct TilePlanDev { ChunkPlan host; const TileItem* tiles = nullptr; };
+    struct TilePlanDev { ChunkPlan host; const TileItem* tiles = nullptr; bool mma = false; /* the mma.sync kernel is expected to be faster */ };
     std::map<std::pair<int64_t, int>, TilePlanDev> tile_plans;  // of the step, by (window, tokens per work item)
     float* part_o = nullptr;
     float* part_ml = nullptr;
@@ -538,14 +538,22 @@ int32_t get_tile_plan(Arena* a, int64_t window, int tokens_per_item, int tile_to
     DeviceState::TilePlanDev pd;
     TileCut cut{window, kv_tile, tile_tokens, d->sm_count, d->chunk_split};
     build_chunk_tile_plan(*a, tokens_per_item, &pd.host, cut);
-    if (pd.host.n_cut > 0 && !ensure_split(a, st)) {
-        cut.max_parts = 1;
-        build_chunk_tile_plan(*a, tokens_per_item, &pd.host, cut);
+    // One tcgen05 CTA per SM at a time costs more to start than a few pages take the mma.sync kernel, of which eight
+    // warps (items) share an SM: steps with more (sequence, kv head) pairs than SMs over short contexts, and prompts of
+    // some tens of tokens.  64 sequences x 2 tokens after 33 (8 kv heads, head_dim 128): 12.7 against 28.7 us, after
+    // 600: 45 against 65; 32 x 2 after 600: 43 against 34; a 40-token prompt (4 kv heads) 10.3 against 13.0.
+    pd.mma = chunk_mma_launch_us(*a, window, chunk_config(a->cfg.head_dim).cols_per_item, d->sm_count) <
+             chunk_tile_launch_us(*a, pd.host, cut);
+    if (!(pd.mma && d->chunk_mode == 0)) {
+        if (pd.host.n_cut > 0 && !ensure_split(a, st)) {
+            cut.max_parts = 1;
+            build_chunk_tile_plan(*a, tokens_per_item, &pd.host, cut);
+        }
+        const void* p = nullptr;
+        int32_t rc = slot_upload(d, pd.host.tiles.data(), pd.host.tiles.size() * sizeof(TileItem), st, &p);
+        if (rc) return rc;
+        pd.tiles = (const TileItem*)p;
     }
-    const void* p = nullptr;
-    int32_t rc = slot_upload(d, pd.host.tiles.data(), pd.host.tiles.size() * sizeof(TileItem), st, &p);
-    if (rc) return rc;
-    pd.tiles = (const TileItem*)p;
     auto ins = d->tile_plans.emplace(key, std::move(pd));
     *out = &ins.first->second;
     return CBKV_OK;
@@ -603,14 +611,20 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
     LayerArena& L = d->layers[(size_t)layer];
     const float scale_log2 = (float)(scale * 1.4426950408889634);
     // tensor-core chunk kernels, whatever the number of new tokens: a few tokens leave most of a tile's rows empty,
-    // but their items are cut along K/V until the chip is full, so the step runs at the rate its K/V arrives
-    // (their softmax masks and takes row maxima before scaling, which needs a scale whose 32-bit value is positive; they read q and write out 16 bytes
-    // at a time, the mma.sync kernel takes any address that fits its elements)
+    // but their items are cut along K/V until the chip is full, so the step runs at the rate its K/V arrives; the
+    // mma.sync kernel where that is expected to be faster (get_tile_plan), and where they cannot go
+    // (their softmax masks and takes row maxima before scaling, which needs a scale whose 32-bit value is positive; they read q
+    // and write out 16 bytes at a time, the mma.sync kernel takes any address that fits its elements)
     const bool aligned16 = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-    const bool tc_able = d->fast && d->tc_ok && scale_log2 > 0.f && aligned16 && !a->step_is_decode;
-    const bool use_tc2 = tc_able && chunk_tc2_supported(a->cfg.head_dim) &&
-                         (d->chunk_mode == 3 || d->chunk_mode == 4 || d->chunk_mode == 0);
-    const bool use_tc = tc_able && !use_tc2 && (d->chunk_mode == 2 || d->chunk_mode == 0);
+    bool use_tc = d->fast && d->tc_ok && scale_log2 > 0.f && aligned16 && !a->step_is_decode && d->chunk_mode != 1;
+    const bool use_tc2 = use_tc && chunk_tc2_supported(a->cfg.head_dim) && d->chunk_mode != 2;
+    const int tile_tokens = 128 / rep_slots_of(a->n_rep());
+    DeviceState::TilePlanDev* tp = nullptr;
+    if (use_tc) {
+        int32_t rc = get_tile_plan(a, w, (use_tc2 ? 2 : 1) * tile_tokens, tile_tokens, !use_tc2 && a->cfg.head_dim == 256 ? 64 : 128, st, &tp);
+        if (rc) return rc;
+        if (tp->mma && d->chunk_mode == 0) use_tc = false;
+    }
     // int8 pages: decode steps stream the records through the decode kernel; the chunk kernels read a float
     // copy made per layer and step (mode 4: the two-tile kernel converts the records itself, slower so far);
     // shapes outside the fast path de-quantise on the fly in the generic kernel
@@ -678,13 +692,9 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
         d->last_kv_writer = k_fused ? layer : -1;
         return CBKV_OK;
     }
-    if (use_tc || use_tc2) {
-        const int tile_tokens = 128 / rep_slots_of(a->n_rep());
-        DeviceState::TilePlanDev* pd = nullptr;
-        int32_t rc = get_tile_plan(a, w, (use_tc2 ? 2 : 1) * tile_tokens, tile_tokens, !use_tc2 && a->cfg.head_dim == 256 ? 64 : 128, st, &pd);
-        if (rc) return rc;
+    if (use_tc) {
         ChunkArgs args{};
-        args.step = d->step; args.geo = geom(a); args.tiles = pd->tiles; args.n_items = (int32_t)pd->host.tiles.size();
+        args.step = d->step; args.geo = geom(a); args.tiles = tp->tiles; args.n_items = (int32_t)tp->host.tiles.size();
         args.q = q; args.out = out; args.status = d->status; args.window = (int32_t)w; args.scale_log2 = scale_log2;
         args.rep_slots = 128 / tile_tokens;
         args.q8_arena = q8_direct ? L.base : nullptr;
@@ -1573,6 +1583,7 @@ int32_t cbkv_set_chunk_kernel(cbkv_arena* arena, int32_t mode) {
     }
     if (mode == 2 && !dev_of(a)->tc_ok) { set_error("the tensor-core chunk kernel covers head_dim 64, 128 and 256 with 16-token pages only"); return CBKV_ERR_ARG; }
     dev_of(a)->chunk_mode = mode;
+    dev_of(a)->tile_plans.clear();
     return CBKV_OK;
     });
 }

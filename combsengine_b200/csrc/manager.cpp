@@ -463,4 +463,47 @@ void build_chunk_tile_plan(const Arena& a, int32_t tokens_per_tile, ChunkPlan* p
     emit(limit, rem, rem_parts, &pl->tiles, &pl->n_slots, &pl->n_cut);
 }
 
+namespace {
+
+// Measured per head_dim over batches of 1 to 64 sequences with 33 to 2000 cached tokens (GQA groups of 2 to 7, f16):
+// a tcgen05 launch takes fixed_us, then per wave of one CTA per SM cta_us + tile_us for each K/V tile (head_dim 128:
+// [0] with one query tile, [1] with both); the mma.sync kernel, one warp per item over all its pages, mma_us + page_us
+// for each page of the longest item, `warps` of them per SM at a time; with more items than that, kMmaRounds times as
+// much per round.
+struct ChunkTimes { float cta_us[2], tile_us[2], mma_us, page_us; int32_t warps; };
+constexpr float kChunkFixedUs = 1.7f, kMmaRounds = 1.5f;
+ChunkTimes chunk_times(int32_t d) {
+    switch (d) {
+        case 64: return {{5.f, 5.f}, {1.f, 1.f}, 11.f, 1.04f, 12};
+        case 128: return {{5.8f, 10.f}, {2.1f, 2.45f}, 8.f, 0.84f, 8};
+        default: return {{6.f, 6.f}, {1.3f, 1.3f}, 7.5f, 0.88f, 4};  // 256
+    }
+}
+
+}  // namespace
+
+float chunk_tile_launch_us(const Arena& a, const ChunkPlan& pl, const TileCut& cut) {
+    const ChunkTimes t = chunk_times(a.cfg.head_dim);
+    std::vector<float> cost, heap;
+    cost.reserve(pl.tiles.size());
+    for (const TileItem& w : pl.tiles) {
+        const int both = a.step_meta[(size_t)w.seq].snew - w.qt * pl.cols_per_item > cut.tile_tokens ? 1 : 0;
+        cost.push_back(t.cta_us[both] + t.tile_us[both] * (float)(w.t1 - w.t0));
+    }
+    return kChunkFixedUs + launch_end(cost, cut.sm_count, &heap);
+}
+
+float chunk_mma_launch_us(const Arena& a, int64_t window, int32_t cols_per_item, int32_t sm_count) {
+    const ChunkTimes t = chunk_times(a.cfg.head_dim);
+    int64_t items = 0, longest = 0;
+    for (const SeqMeta& m : a.step_meta) {
+        if (m.snew == 0) continue;
+        const int64_t lo_key = window > 0 ? std::max<int64_t>(0, (int64_t)m.pos - window + 1) : 0;
+        items += (int64_t)a.cfg.n_kv_heads * (((int64_t)m.snew * a.n_rep() + cols_per_item - 1) / cols_per_item);
+        longest = std::max<int64_t>(longest, (((int64_t)m.pos + m.snew - 1) >> 4) - (lo_key >> 4) + 1);
+    }
+    const int64_t at_once = (int64_t)sm_count * t.warps, rounds = (items + at_once - 1) / at_once;
+    return t.mma_us + t.page_us * (float)longest * (rounds > 1 ? kMmaRounds * (float)rounds : 1.f);
+}
+
 }  // namespace cbkv

@@ -187,4 +187,9 @@ void build_chunk_plan(const Arena& a, int32_t cols_per_item, ChunkPlan* plan);
 // `tokens_per_tile` new tokens); `cols_per_item` records tokens_per_tile.
 void build_chunk_tile_plan(const Arena& a, int32_t tokens_per_tile, ChunkPlan* plan, const TileCut& cut = TileCut());
 
+// Expected times of a chunk step's launch (append included), in microseconds: of the tcgen05 kernel that runs `plan`
+// (made by build_chunk_tile_plan with `cut`), and of the mma.sync kernel.
+float chunk_tile_launch_us(const Arena& a, const ChunkPlan& plan, const TileCut& cut);
+float chunk_mma_launch_us(const Arena& a, int64_t window, int32_t cols_per_item, int32_t sm_count);
+
 }  // namespace cbkv

@@ -343,7 +343,8 @@ int32_t cbkv_set_host_route(cbkv_arena* arena, int32_t direct);
 int32_t cbkv_set_chunk_split(cbkv_arena* arena, int32_t max_parts);
 
 /* Which kernel runs a step that is not pure decode: 0 = the library chooses (tcgen05
- * tiles; mma.sync for scales that are not positive), 1 = the mma.sync kernel, 2 = the
+ * tiles; mma.sync where many short sequences or a short prompt make that faster, for
+ * scales that are not positive and for q or out off a 16-byte boundary), 1 = the mma.sync kernel, 2 = the
  * tcgen05/TMEM kernel with one 128-row query tile per CTA (head_dim 64, 128 or 256), 3 = the
  * tcgen05/TMEM kernel with two query tiles per CTA and P in tensor memory (head_dim 128).
  * Over int8 layers these kernels read a float copy of the step's pages made per layer and

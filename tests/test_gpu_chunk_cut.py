@@ -181,6 +181,7 @@ def test_overlap_switch_covers_every_launch_of_a_chunk_step(d, int8, overlap):
     rt = C.CDLL("libcudart.so.12")
     g = KVArena(1, 8, 2, d, 256, 16, 40, quantize_kv=int8)
     g.set_decode_tuning(overlap_launches=overlap)
+    g.set_chunk_kernel(3 if d == 128 else 2)  # the mma.sync kernel is never launched early
     rope = RotaryEmbedding(g, 10000.0, 256)
     s = g.new_seq()
     q, k, v = (torch.randn(70 * h * d, device="cuda").half() for h in (8, 2, 2))
@@ -207,3 +208,30 @@ def test_overlap_switch_covers_every_launch_of_a_chunk_step(d, int8, overlap):
     torch.cuda.synchronize()
     assert g.device_status() == 0
     rope.close()
+
+
+@pytest.mark.parametrize("n_q,n_kv,d,tcgen05,n_seqs,ctx,new,mma", [
+    (32, 8, 128, 3, 64, 33, 2, True), (32, 8, 128, 3, 18, 33, 2, False), (32, 8, 128, 3, 64, 600, 2, True), (32, 8, 128, 3, 32, 600, 2, False),
+    (28, 4, 128, 3, 1, 1, 40, True), (28, 4, 128, 3, 1, 400, 40, False), (8, 4, 256, 2, 64, 33, 5, True), (8, 4, 256, 2, 64, 900, 5, False),
+    (9, 3, 64, 2, 64, 33, 5, False)])
+def test_many_short_sequences_take_the_mma_kernel(n_q, n_kv, d, tcgen05, n_seqs, ctx, new, mma):
+    # on either side of the line the output is, bit for bit, that of the kernel which the rule names
+    from combsengine_b200 import KVArena
+    g = KVArena(1, n_q, n_kv, d, 1024, 16, n_seqs * 64, sliding_popn_refuses=False)
+    gen = torch.Generator(device="cuda").manual_seed(d)
+    rand = lambda n: torch.randn(n, generator=gen, device="cuda", dtype=torch.float16)
+    seqs = [g.new_seq() for _ in range(n_seqs)]
+    g.begin_step(seqs, [ctx] * n_seqs)
+    g.append(0, rand(n_seqs * ctx * n_kv * d), rand(n_seqs * ctx * n_kv * d))
+    q, k, v = (rand(n_seqs * new * h * d) for h in (n_q, n_kv, n_kv))
+    outs = {}
+    for kernel in (0, 1, tcgen05):
+        g.set_chunk_kernel(kernel)
+        g.begin_step(seqs, [new] * n_seqs)
+        outs[kernel] = g.attention(0, q, k, v, d ** -0.5)
+        assert g.device_status() == 0
+        for s in seqs:
+            s.popn(new)
+    assert not torch.equal(outs[1], outs[tcgen05])
+    assert torch.equal(outs[0], outs[1 if mma else tcgen05])
+    assert_attention_close(outs[0].cpu().numpy(), outs[tcgen05 if mma else 1].cpu().numpy())
