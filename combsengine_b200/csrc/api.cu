@@ -66,7 +66,6 @@ EncodeTiledFn encode_fn() {
 }
 
 constexpr int kSlots = 4;
-constexpr int kUncutUnits = 40;  // see get_decode_plan
 constexpr int kMaxChunkSplit = 64;
 
 struct StepSlot {
@@ -413,10 +412,18 @@ int32_t get_decode_plan(Arena* a, int64_t window, bool quant, cudaStream_t st, D
     build_decode_plan(*a, window, max_ctas, d->split, &pd.host);
     {
         int want = std::max(1, (pd.host.n_units + dc.consumers - 1) / dc.consumers);
-        // A few short segments of one length (one sequence's first hundreds of tokens) are not cut at all: a CTA per
-        // segment streams its pages in the time that a cut would spend on tickets and the merge.
+        // Short segments of one length (one sequence's first hundreds of tokens), no more than CTAs, are not cut: a CTA
+        // per segment streams its pages in the time that a cut spends on tickets and the merge.  Measured cut / uncut,
+        // us per launch, 1 to 16 sequences:
+        //   float, head_dim 64:   16 pages 7.9 / 5.1,  40 pages 7.9 / 7.0,   96 pages 7.0 / 10.7
+        //   float, head_dim 128:  16 pages 9.3 / 5.8,  40 pages 9.2 / 8.0,   96 pages 7.9 / 13.4
+        //   float, head_dim 256:  16 pages 11.4 / 7.1, 24 pages 7.5 / 9.4,   40 pages 10.9 / 12.8
+        //   int8,  head_dim 128:  8 pages 7.1 / 6.1,   16 pages 7.3 / 7.5,   40 pages 8.2 / 11.5
+        //   int8,  head_dim 256:  16 pages 12.7 / 10.2, 24 pages 9.7 / 12.5, 40 pages 13.0 / 14.5
+        // Batches of unequal lengths keep the even split: the launch would last as long as the longest segment.
+        const int uncut_pages = !quant && a->cfg.head_dim <= 128 ? 40 : 16;
         const int per = pd.host.n_segs > 0 ? pd.host.n_units / pd.host.n_segs : 0;
-        bool equal = pd.host.n_segs > 0 && pd.host.n_segs <= max_ctas && per <= kUncutUnits;
+        bool equal = pd.host.n_segs > 0 && pd.host.n_segs <= max_ctas && per <= uncut_pages;
         for (int i = 0; equal && i < pd.host.n_segs; i++)
             equal = pd.host.segs[(size_t)i + 1].unit_begin - pd.host.segs[(size_t)i].unit_begin == per;
         if (equal) want = std::min(want, pd.host.n_segs);

@@ -235,3 +235,29 @@ def test_many_short_sequences_take_the_mma_kernel(n_q, n_kv, d, tcgen05, n_seqs,
     assert not torch.equal(outs[1], outs[tcgen05])
     assert torch.equal(outs[0], outs[1 if mma else tcgen05])
     assert_attention_close(outs[0].cpu().numpy(), outs[tcgen05 if mma else 1].cpu().numpy())
+
+
+@pytest.mark.parametrize("n_q,n_kv,d,int8,pages,uncut", [
+    (9, 3, 64, False, 40, True), (9, 3, 64, False, 41, False), (32, 8, 128, False, 40, True), (32, 8, 128, False, 41, False),
+    (8, 4, 256, False, 16, True), (8, 4, 256, False, 24, False), (32, 8, 128, True, 16, True), (32, 8, 128, True, 24, False)])
+def test_short_decode_is_cut_where_that_is_faster(n_q, n_kv, d, int8, pages, uncut):
+    # one CTA per (sequence, kv head), asked for by the CTA limit, gives the same bits as the default where nothing is cut
+    from combsengine_b200 import KVArena
+    g = KVArena(1, n_q, n_kv, d, 1024, 16, 128, quantize_kv=int8)
+    gen = torch.Generator(device="cuda").manual_seed(d)
+    rand = lambda n: torch.randn(n, generator=gen, device="cuda", dtype=torch.float16)
+    seqs = [g.new_seq() for _ in range(2)]
+    n = 16 * pages - 3
+    g.begin_step(seqs, [n] * 2)
+    g.append(0, rand(2 * n * n_kv * d), rand(2 * n * n_kv * d))
+    q, k, v = (rand(2 * h * d) for h in (n_q, n_kv, n_kv))
+    outs = []
+    for max_ctas in (0, 2 * n_kv):
+        g.set_decode_tuning(max_ctas=max_ctas)
+        g.begin_step(seqs, [1] * 2)
+        outs.append(g.attention(0, q, k, v, d ** -0.5))
+        for s in seqs:
+            s.popn(1)
+    assert g.device_status() == 0
+    assert torch.equal(outs[0], outs[1]) == uncut
+    assert_attention_close(outs[0].cpu().numpy(), outs[1].cpu().numpy())
