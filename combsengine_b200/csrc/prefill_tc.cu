@@ -16,9 +16,9 @@
 //                 tensor memory over its S columns (16-bit pairs) and is the A operand of P V; O rescaled in
 //                 TMEM when a row max moves
 //
-// KV tiles hold KT tokens: 128 for head_dim 64 and 128; 64 for head_dim 256, where a 128-token tile of K
-// and V (128 KB) would not leave room for two stages next to the Q tile (S = Q K^T is then 128 x 64 and
-// O += P V one 128 x 256 MMA per 16 keys).
+// KV tiles hold KT tokens: 128 for head_dim 64 and 128; 64 for head_dim 256, where two S buffers of 128 columns, Q
+// (128) and O (256) would be more than the 512 columns of tensor memory, and three K and three V buffers of 64 KB more
+// than shared memory (S = Q K^T is then 128 x 64 and O += P V one 128 x 256 MMA per 16 keys).
 //
 // Tensor memory: S0 [0,KT), S1 [KT, 2 KT), Q [2 KT, 2 KT + D / 2) packed, O [512 - D, 512) -> 512 columns allocated.
 // Shared memory: kTcBufs K and V buffers each, [page][8-token group][column block][8 rows x 128 bytes]:
@@ -330,7 +330,7 @@ __device__ __forceinline__ bool last_slice(const ChunkArgs& a, const CtaWork& wk
 }  // namespace
 
 template <int D, bool BF16>
-__global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constant__ CUtensorMap tmap32, const ChunkArgs a) {
+__global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constant__ CUtensorMap tmap, const ChunkArgs a) {
     constexpr int XB = D / 64;                 // column blocks per row
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int KT = TcKeys<D>::value;       // tokens per KV tile
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
         *failed = 0;
         for (int i = 0; i < 4; i++) s_pair[i] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap32) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap) : "memory");
     }
     if (warp == 0) {  // tensor memory for this CTA
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
                 }
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
                 if (ok && lane < PPT)
-                    tma_load_page(smem_u32((is_v ? sV : sK) + st * KVB + lane * PGB), &tmap32, is_v, (phys * Hkv + h) * 2, full);
+                    tma_load_page(smem_u32((is_v ? sV : sK) + st * KVB + lane * PGB), &tmap, is_v, (phys * Hkv + h) * 2, full);
                 if (lane == 0) TC_ACC(c_issue);
             }
         }
@@ -677,9 +677,9 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
 }
 
 template <int D, bool BF16>
-static cudaError_t launch_tc(const CUtensorMap& map32, const ChunkArgs& a, bool overlap, cudaStream_t st) {
+static cudaError_t launch_tc(const CUtensorMap& map, const ChunkArgs& a, bool overlap, cudaStream_t st) {
     if (a.n_items <= 0) return cudaSuccess;
-    return launch_pdl(overlap, chunk_tc_kernel<D, BF16>, a.n_items, kThreads, tc_smem_bytes<D>(), st, map32, a);
+    return launch_pdl(overlap, chunk_tc_kernel<D, BF16>, a.n_items, kThreads, tc_smem_bytes<D>(), st, map, a);
 }
 
 
@@ -1233,12 +1233,12 @@ cudaError_t chunk_tc_init() {
     return cudaSuccess;
 }
 
-// `map32`: the layer's 32-row box view (K and V of a page per box).
-cudaError_t launch_chunk_tc(const CUtensorMap& map32, const ChunkArgs& a, bool bf16, bool overlap, cudaStream_t st) {
+// `map`: the layer's map_page (K or V of a page per copy).
+cudaError_t launch_chunk_tc(const CUtensorMap& map, const ChunkArgs& a, bool bf16, bool overlap, cudaStream_t st) {
     switch (a.geo.d) {
-        case 64: return bf16 ? launch_tc<64, true>(map32, a, overlap, st) : launch_tc<64, false>(map32, a, overlap, st);
-        case 128: return bf16 ? launch_tc<128, true>(map32, a, overlap, st) : launch_tc<128, false>(map32, a, overlap, st);
-        case 256: return bf16 ? launch_tc<256, true>(map32, a, overlap, st) : launch_tc<256, false>(map32, a, overlap, st);
+        case 64: return bf16 ? launch_tc<64, true>(map, a, overlap, st) : launch_tc<64, false>(map, a, overlap, st);
+        case 128: return bf16 ? launch_tc<128, true>(map, a, overlap, st) : launch_tc<128, false>(map, a, overlap, st);
+        case 256: return bf16 ? launch_tc<256, true>(map, a, overlap, st) : launch_tc<256, false>(map, a, overlap, st);
         default: return cudaErrorInvalidValue;
     }
 }
