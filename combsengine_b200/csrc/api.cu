@@ -608,9 +608,10 @@ int32_t run_append(Arena* a, int layer, const void* k, const void* v, cudaStream
     return CBKV_OK;
 }
 
-// k, v non-null on a decode step => the append rides inside the decode kernel.
+// k, v non-null on a decode step => the append rides inside the decode kernel; rope.table non-null there => the norm and
+// rotation of q and k as well.
 int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, const void* v_fused, void* out,
-                      double scale, int64_t window, cudaStream_t st) {
+                      double scale, int64_t window, cudaStream_t st, const RopeDev& rope = RopeDev{}) {
     DeviceState* d = dev_of(a);
     const bool bf16 = a->cfg.dtype == CBKV_BF16;
     const int64_t w = a->layer_window(layer, window);
@@ -667,7 +668,7 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
         args.segs = pd->segs; args.items = pd->items; args.unit_row = d->unit_rows + pd->unit_row_off;
         args.n_segs = pd->host.n_segs; args.n_items = pd->host.n_items; args.n_ctas = pd->host.n_ctas;
         args.n_units = pd->host.n_units; args.tail_pct = pd->host.levels > 1 ? d->split.tail_pct : 0;
-        args.q = q; args.out = out; args.k_new = k_fused; args.v_new = v_fused; args.arena = L.base;
+        args.q = q; args.out = out; args.k_new = k_fused; args.v_new = v_fused; args.arena = L.base; args.rope = rope;
         args.part_o = d->part_o; args.part_ml = d->part_ml; args.seg_counter = d->seg_counter; args.status = d->status;
         args.work_counters = d->work_counters; args.work_slot = (int32_t)(d->launch_seq++ & 3u);
         args.window = (int32_t)w; args.scale_log2 = scale_log2;
@@ -987,11 +988,8 @@ int32_t cbkv_rope_destroy(cbkv_rope* rope) {
     });
 }
 
-// k_out non-null: rotated k goes to that dense buffer and nothing is written to pages (int8 layers,
-// whose append quantises afterwards).
-static int32_t run_rope_append(Arena* a, int layer, const Rope* r, const cbkv_qk_norm* norm, const void* q, const void* k,
-                               const void* v, void* q_out, void* k_out, cudaStream_t st) {
-    DeviceState* d = dev_of(a);
+// The tables and weights as the kernels take them; refuses a step past the table.
+static int32_t rope_dev(Arena* a, const Rope* r, const cbkv_qk_norm* norm, RopeDev* out) {
     if (r->arena != a) { set_error("rope tables belong to another arena"); return CBKV_ERR_ARG; }
     for (const SeqMeta& m : a->step_meta)
         if ((int64_t)m.pos + m.snew > r->max_position) {
@@ -999,15 +997,21 @@ static int32_t run_rope_append(Arena* a, int layer, const Rope* r, const cbkv_qk
                       std::to_string(r->max_position));
             return CBKV_ERR_ARG;
         }
+    out->table = r->table; out->max_position = r->max_position;
+    if (norm) { out->q_weight = norm->q_weight; out->k_weight = norm->k_weight; out->eps = (float)norm->eps; out->gemma = norm->gemma; }
+    return CBKV_OK;
+}
+
+// k_out non-null: rotated k goes to that dense buffer and nothing is written to pages (int8 layers,
+// whose append quantises afterwards).
+static int32_t run_rope_append(Arena* a, int layer, const Rope* r, const cbkv_qk_norm* norm, const void* q, const void* k,
+                               const void* v, void* q_out, void* k_out, cudaStream_t st) {
+    DeviceState* d = dev_of(a);
     RopeArgs args{};
+    if (int32_t rc = rope_dev(a, r, norm, &args.rope)) return rc;
     args.step = d->step; args.geo = geom(a);
     args.q = q; args.k = k; args.v = v; args.q_out = q_out; args.k_out = k_out;
     args.arena = d->layers[(size_t)layer].base;
-    args.table = r->table; args.max_position = r->max_position;
-    args.q_weight = norm ? norm->q_weight : nullptr;
-    args.k_weight = norm ? norm->k_weight : nullptr;
-    args.eps = norm ? (float)norm->eps : 0.f;
-    args.gemma = norm ? norm->gemma : 0;
     args.status = d->status;
     { int32_t frc = flush_uploads(d, st); if (frc) return frc; }
     CU_TRY(launch_rope_append(args, a->cfg.dtype == CBKV_BF16, d->pdl, st));
@@ -1066,9 +1070,17 @@ int32_t cbkv_attention_rope(cbkv_arena* arena, int32_t layer, const cbkv_rope* r
     DeviceState* d = dev_of(a);
     CU_TRY(cudaSetDevice(d->device));
     if ((rc = materialize(a, layer, st))) return rc;
+    const bool quant = d->layers[(size_t)layer].quant;
+    const DecodeConfig dc = decode_config(a->cfg.head_dim, a->n_rep(), d->decode_ctas_per_sm, d->decode_stages, d->decode_consumers, quant);
+    if (d->fast && a->step_is_decode && decode_rotates(a->cfg.head_dim, dc.consumers, quant) && !(quant && (debug_flags() & 16))) {
+        // norm, rotation and append ride inside the decode kernel: one launch instead of two, and its pages are on their
+        // way before the previous layer's launch has ended
+        RopeDev rd;
+        if ((rc = rope_dev(a, reinterpret_cast<const Rope*>(rope), norm, &rd))) return rc;
+        return run_attention(a, layer, q, k, v, out, scale, window, st, rd);
+    }
     const size_t qb = ((size_t)a->step_tokens * a->cfg.n_q_heads * a->cfg.head_dim * 2 + 255) & ~(size_t)255;
     const size_t kb = ((size_t)a->step_tokens * a->cfg.n_kv_heads * a->cfg.head_dim * 2 + 255) & ~(size_t)255;
-    const bool quant = d->layers[(size_t)layer].quant;
     if ((rc = rope_scratch(a, st, qb + (quant ? kb : 0)))) return rc;
     if (quant) {  // int8 pages: rotate q and k to scratch; the append (fused into the decode kernel when it can be) quantises
         uint8_t* krot = d->qrot + qb;

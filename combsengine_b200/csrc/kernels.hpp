@@ -82,6 +82,16 @@ struct GeomDev {
     int32_t tiled;  // 1: rows of a (page, kv head) in the 8-row K/V interleave (see page_row)
 };
 
+// Rotary table and QK norm weights of a layer, for kernels that apply them on the way (rope.cu).
+struct RopeDev {
+    const void* table = nullptr;     // per position head_dim/2 cosines, then head_dim/2 sines, in the storage type; null: q and k come rotated
+    int64_t max_position = 0;
+    const void* q_weight = nullptr;  // head_dim elements each, null without a norm
+    const void* k_weight = nullptr;
+    float eps = 0.f;
+    int32_t gemma = 0;
+};
+
 struct DecodeArgs {
     GeomDev geo;
     const SegInfo* segs;        // n_segs + 1 records (manager.hpp)
@@ -94,6 +104,7 @@ struct DecodeArgs {
     const void* k_new;  // non-null: write the step's new row into its page and attend it (fused append)
     const void* v_new;
     void* arena;        // this layer's pages (for the fused append's global write)
+    RopeDev rope;       // table non-null: q and k_new are normed and rotated here
     float* part_o;      // [n_parts][8][d] partial numerators
     float* part_ml;     // [n_parts][8][2] running max (log2 domain) and denominator
     int32_t* seg_counter;    // per segment: tickets of the parts that are done (0 between launches)
@@ -160,8 +171,7 @@ struct GenericArgs {
     float scale;
 };
 
-// Rotate-and-append (rope.cu).  `table` holds, per position, head_dim/2 cosines then head_dim/2 sines in
-// the storage type; q_weight / k_weight (head_dim elements, storage type) are null without QK norm.
+// Rotate-and-append (rope.cu).
 struct RopeArgs {
     StepDev step;
     GeomDev geo;
@@ -171,18 +181,15 @@ struct RopeArgs {
     void* q_out;
     void* k_out;   // non-null: rotated k goes here (dense, same layout as k) and v is left alone; `arena` is unused
     void* arena;
-    const void* table;
-    int64_t max_position;
-    const void* q_weight;
-    const void* k_weight;
-    float eps;
-    int32_t gemma;
+    RopeDev rope;
     int32_t* status;
 };
 
 // Decode kernel configuration for a head_dim (0 warps = not supported by the fast path).
 struct DecodeConfig { int consumers, stages, smem_bytes, ctas_per_sm, comb_cols, comb_bufs; };
 DecodeConfig decode_config(int d, int n_rep, int ctas_per_sm, int stages, int consumers, bool q8 = false);
+// Whether the variant that norms and rotates exists (with the default number of consumer warps).
+bool decode_rotates(int d, int consumers, bool q8);
 struct ChunkConfig { int warps, stages, smem_bytes, cols_per_item; };
 ChunkConfig chunk_config(int d);
 

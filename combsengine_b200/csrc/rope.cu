@@ -25,6 +25,7 @@
 
 #include "kernels.hpp"
 #include "pdl.cuh"
+#include "rope.cuh"
 
 namespace cbkv {
 
@@ -93,56 +94,6 @@ void rope_tables(const cbkv_rope_config& c, const std::vector<double>& inv, doub
 }
 
 // ------------------------------------------------------------------ device
-// Two storage-type elements in one 32-bit word, with the non-fusing 2-wide instructions:
-// each product and each sum is rounded on its own, never contracted into a multiply-add.
-template <bool BF16> struct Pack;
-template <> struct Pack<false> {
-    using V2 = __half2;
-    static __device__ __forceinline__ float2 up(uint32_t v) { return __half22float2(*reinterpret_cast<__half2*>(&v)); }
-    static __device__ __forceinline__ float rt(float f) { return __half2float(__float2half_rn(f)); }
-    static __device__ __forceinline__ uint32_t down(float a, float b) {
-        __half2 h = __floats2half2_rn(a, b);
-        return *reinterpret_cast<uint32_t*>(&h);
-    }
-};
-template <> struct Pack<true> {
-    using V2 = __nv_bfloat162;
-    static __device__ __forceinline__ float2 up(uint32_t v) { return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&v)); }
-    static __device__ __forceinline__ float rt(float f) { return __bfloat162float(__float2bfloat16_rn(f)); }
-    static __device__ __forceinline__ uint32_t down(float a, float b) {
-        __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-        return *reinterpret_cast<uint32_t*>(&h);
-    }
-};
-
-// rope.rs:196-201 on two (i, i+half) pairs: out[i] = x1*cos + (-x2)*sin, out[i+half] = x2*cos + x1*sin.
-template <bool BF16>
-__device__ __forceinline__ void rotate2(uint32_t& x1, uint32_t& x2, uint32_t c, uint32_t s) {
-    using V2 = typename Pack<BF16>::V2;
-    const V2 a = *reinterpret_cast<V2*>(&x1), b = *reinterpret_cast<V2*>(&x2);
-    const V2 cc = *reinterpret_cast<V2*>(&c), ss = *reinterpret_cast<V2*>(&s);
-    V2 o1 = __hadd2_rn(__hmul2_rn(a, cc), __hmul2_rn(__hneg2(b), ss));
-    V2 o2 = __hadd2_rn(__hmul2_rn(b, cc), __hmul2_rn(a, ss));
-    x1 = *reinterpret_cast<uint32_t*>(&o1);
-    x2 = *reinterpret_cast<uint32_t*>(&o2);
-}
-
-// y = x * inv_rms * w in f32, rounded once (norm.rs:27-28); gemma: w + 1 formed in the storage type.
-template <bool BF16>
-__device__ __forceinline__ uint32_t norm2(uint32_t x, uint32_t w, float inv_rms, bool gemma) {
-    using P = Pack<BF16>;
-    const float2 u = P::up(x);
-    float2 wf = P::up(w);
-    if (gemma) { wf.x = P::rt(__fadd_rn(wf.x, 1.f)); wf.y = P::rt(__fadd_rn(wf.y, 1.f)); }
-    return P::down(__fmul_rn(__fmul_rn(u.x, inv_rms), wf.x), __fmul_rn(__fmul_rn(u.y, inv_rms), wf.y));
-}
-
-template <bool BF16>
-__device__ __forceinline__ float sumsq2(uint32_t x) {
-    const float2 u = Pack<BF16>::up(x);
-    return __fadd_rn(__fmul_rn(u.x, u.x), __fmul_rn(u.y, u.y));
-}
-
 // Which sequence a packed row belongs to: the last one whose first row is <= row.
 __device__ __forceinline__ int seq_of_row(const StepDev& s, int64_t row, int heads) {
     int lo = 0, hi = s.n_seqs - 1;
@@ -196,8 +147,8 @@ __global__ void __launch_bounds__(256) rope_append_kernel(const RopeArgs a) {
             continue;
         }
         uint32_t x1[ROPE_MAX_IT], x2[ROPE_MAX_IT], cw[ROPE_MAX_IT], sw[ROPE_MAX_IT];
-        const int tpos = min(gpos, (int)a.max_position - 1);  // the host refuses a step past the table
-        const uint32_t* trow = reinterpret_cast<const uint32_t*>(a.table) + (int64_t)tpos * half;  // 2 * chunks words
+        const int tpos = min(gpos, (int)a.rope.max_position - 1);  // the host refuses a step past the table
+        const uint32_t* trow = reinterpret_cast<const uint32_t*>(a.rope.table) + (int64_t)tpos * half;  // 2 * chunks words
 #pragma unroll
         for (int it = 0; it < ROPE_MAX_IT; it++) {
             const int c = lane + it * 32;
@@ -208,7 +159,7 @@ __global__ void __launch_bounds__(256) rope_append_kernel(const RopeArgs a) {
                 sw[it] = trow[chunks + c];
             }
         }
-        const void* wv = kind == 0 ? a.q_weight : a.k_weight;
+        const void* wv = kind == 0 ? a.rope.q_weight : a.rope.k_weight;
         if (wv) {  // mean(x^2) over head_dim, norm.rs:22-23
             float ss = 0.f;
 #pragma unroll
@@ -216,14 +167,14 @@ __global__ void __launch_bounds__(256) rope_append_kernel(const RopeArgs a) {
                 if (lane + it * 32 < chunks) ss = __fadd_rn(ss, __fadd_rn(sumsq2<BF16>(x1[it]), sumsq2<BF16>(x2[it])));
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) ss = __fadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, o));
-            const float inv_rms = __frcp_rn(__fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)d), a.eps)));
+            const float inv_rms = inv_rms_of(ss, d, a.rope.eps);
             const uint32_t* w32 = reinterpret_cast<const uint32_t*>(wv);
 #pragma unroll
             for (int it = 0; it < ROPE_MAX_IT; it++) {
                 const int c = lane + it * 32;
                 if (c < chunks) {
-                    x1[it] = norm2<BF16>(x1[it], w32[c], inv_rms, a.gemma != 0);
-                    x2[it] = norm2<BF16>(x2[it], w32[chunks + c], inv_rms, a.gemma != 0);
+                    x1[it] = norm2<BF16>(x1[it], w32[c], inv_rms, a.rope.gemma != 0);
+                    x2[it] = norm2<BF16>(x2[it], w32[chunks + c], inv_rms, a.rope.gemma != 0);
                 }
             }
         }
@@ -289,8 +240,8 @@ __global__ void __launch_bounds__(256) rope_append_vec_kernel(const RopeArgs a) 
         const int gpos = sm.pos + (int)r;
         uint4 tc = make_uint4(0, 0, 0, 0), ts = tc;
         if (kind != 2) {
-            const int tpos = min(gpos, (int)a.max_position - 1);
-            const uint4* trow = reinterpret_cast<const uint4*>(a.table) + (size_t)tpos * (2 * T);
+            const int tpos = min(gpos, (int)a.rope.max_position - 1);
+            const uint4* trow = reinterpret_cast<const uint4*>(a.rope.table) + (size_t)tpos * (2 * T);
             tc = trow[t]; ts = trow[T + t];
         }
         uint4* dst;
@@ -308,7 +259,7 @@ __global__ void __launch_bounds__(256) rope_append_vec_kernel(const RopeArgs a) 
             dst = reinterpret_cast<uint4*>(a.arena) + drow * (2 * T);
         }
         uint32_t A[4] = {xa.x, xa.y, xa.z, xa.w}, B[4] = {xb.x, xb.y, xb.z, xb.w};
-        const void* wv = kind == 0 ? a.q_weight : (kind == 1 ? a.k_weight : nullptr);
+        const void* wv = kind == 0 ? a.rope.q_weight : (kind == 1 ? a.rope.k_weight : nullptr);
         if (wv) {
             float ss = 0.f;
 #pragma unroll
@@ -318,14 +269,14 @@ __global__ void __launch_bounds__(256) rope_append_vec_kernel(const RopeArgs a) 
             const unsigned grp = T == 32 ? 0xffffffffu : (((1u << T) - 1u) << (sub * T));
 #pragma unroll
             for (int o = T / 2; o > 0; o >>= 1) ss = __fadd_rn(ss, __shfl_xor_sync(grp, ss, o));
-            const float inv_rms = __frcp_rn(__fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)a.geo.d), a.eps)));
+            const float inv_rms = inv_rms_of(ss, a.geo.d, a.rope.eps);
             const uint4* w4 = reinterpret_cast<const uint4*>(wv);
             const uint4 wa = w4[t], wb = w4[T + t];
             const uint32_t WA[4] = {wa.x, wa.y, wa.z, wa.w}, WB[4] = {wb.x, wb.y, wb.z, wb.w};
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                A[j] = norm2<BF16>(A[j], WA[j], inv_rms, a.gemma != 0);
-                B[j] = norm2<BF16>(B[j], WB[j], inv_rms, a.gemma != 0);
+                A[j] = norm2<BF16>(A[j], WA[j], inv_rms, a.rope.gemma != 0);
+                B[j] = norm2<BF16>(B[j], WB[j], inv_rms, a.rope.gemma != 0);
             }
         }
         if (kind != 2) {
