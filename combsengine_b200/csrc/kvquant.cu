@@ -97,6 +97,122 @@ __global__ void __launch_bounds__(256) append_quant_kernel(const AppendArgs a) {
     }
 }
 
+// 16 consecutive values of a row (half a group): bytes q + 128, four to a word, and the group's scale, which the lane next
+// door has the other half of.
+template <bool BF16>
+__device__ __forceinline__ float quantise16(const uint4& x0, const uint4& x1, uint32_t (&bytes)[4]) {
+    const uint32_t w[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+    float v[16], amax = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        v[2 * i] = q_up<BF16>((uint16_t)(w[i] & 0xffff));
+        v[2 * i + 1] = q_up<BF16>((uint16_t)(w[i] >> 16));
+        amax = fmaxf(amax, fmaxf(fabsf(v[2 * i]), fabsf(v[2 * i + 1])));
+    }
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    const float scale = fmaxf(__fdiv_rn(amax, 127.0f), 1e-8f);        // kv.rs:296-301
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        bytes[i] = 0;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            float q = roundf(__fdiv_rn(v[4 * i + j], scale));         // kv.rs:302-305
+            q = fminf(fmaxf(q, -127.f), 127.f);
+            bytes[i] |= (uint32_t)((int)q + 128) << (8 * j);
+        }
+    }
+    return scale;
+}
+
+// The same for 16-token pages and head_dim 64, 128 or 256: T = d / 16 lanes share a row, each takes 16 consecutive values,
+// and V goes two tokens at a time, because the bytes of a pair of tokens alternate in a record: 32 contiguous bytes per
+// lane, and one word for the pair's two scales, instead of single bytes.  A pair with only one token in this step (a
+// sequence's first or last) leaves the other's bytes alone.
+template <bool BF16, int T>
+__global__ void __launch_bounds__(256) append_quant_vec_kernel(const AppendArgs a) {
+    constexpr int D = T * 16, P = 16, RPW = 32 / T;
+    constexpr int SEQ_SMEM = 1024;
+    __shared__ int s_tok[SEQ_SMEM];
+    const int n_seqs = a.step.n_seqs, Hkv = a.geo.n_kv;
+    const bool in_smem = n_seqs <= SEQ_SMEM;
+    if (in_smem) {  // the sequence records came with the step's upload, which no kernel overlaps
+        for (int i = threadIdx.x; i < n_seqs; i += blockDim.x) s_tok[i] = a.step.seq_meta[i].tok_off;
+        __syncthreads();
+    }
+    pdl_wait();
+    pdl_launch_dependents();
+    const int lane = threadIdx.x & 31, t = lane % T, sub = lane / T;
+    const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    // K rows first, then slots for V pairs: n / 2 + 1 or one more per (sequence, kv head), so that a sequence's first
+    // slot follows from the tokens before it; a slot past the sequence's last pair has nothing to do
+    const int64_t k_rows = (int64_t)a.step.n_tokens * Hkv, v_slots = ((int64_t)a.step.n_tokens / 2 + n_seqs) * Hkv;
+    const int64_t k_rounds = (k_rows + RPW - 1) / RPW, rounds = k_rounds + (v_slots + RPW - 1) / RPW;
+    uint8_t* arena = reinterpret_cast<uint8_t*>(a.arena);
+    const size_t rec = qrec_bytes(P, D);
+    auto tok_off = [&](int b) { return in_smem ? s_tok[b] : a.step.seq_meta[b].tok_off; };
+    for (int64_t R = warp0; R < rounds; R += nwarps) {
+        const bool is_v = R >= k_rounds;  // the same for the whole warp
+        const int64_t idx = (is_v ? R - k_rounds : R) * RPW + sub;
+        bool live = idx < (is_v ? v_slots : k_rows);
+        auto first = [&](int b) { return is_v ? ((int64_t)tok_off(b) / 2 + b) * Hkv : (int64_t)tok_off(b) * Hkv; };
+        int lo = 0, hi = n_seqs - 1;  // the last sequence whose first row (slot) is <= idx
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (first(mid) <= idx) lo = mid; else hi = mid - 1;
+        }
+        const SeqMeta sm = a.step.seq_meta[lo];
+        const int local = (int)(idx - first(lo));
+        const int per = is_v ? (sm.tok_off + sm.snew) / 2 - sm.tok_off / 2 + 1 : sm.snew;  // rows or slots per kv head
+        const int h = per > 0 ? local / per : 0;
+        int r = local - h * per;                                         // K: the token
+        if (is_v) r = 2 * (sm.pos / 2 + r) - sm.pos;                     // V: the pair's first token, -1 when that one is cached already
+        const bool has0 = r >= 0 && r < sm.snew, has1 = is_v && r + 1 < sm.snew;
+        live = live && h < Hkv && (has0 || has1);
+        const int gpos = sm.pos + r;                                     // kv.rs:749
+        int phys = live ? a.step.tables[sm.tbl_off + gpos / P] : 0;      // kv.rs:752
+        if (live && (phys < 0 || phys >= a.geo.num_pages)) { if (t == 0) atomicOr(a.status, ST_BAD_PAGE); live = false; }
+        const int slot = gpos & (P - 1);                                 // kv.rs:750
+        const size_t row = (size_t)sm.tok_off * Hkv + (size_t)h * sm.snew;
+        const uint4* src = reinterpret_cast<const uint4*>(is_v ? a.v : a.k) + (int64_t)(row * (2 * T)) + (int64_t)r * (2 * T) + 2 * t;
+        const uint4 zero = make_uint4(0, 0, 0, 0);
+        uint4 x0 = zero, x1 = zero, y0 = zero, y1 = zero;
+        if (live && has0) { x0 = src[0]; x1 = src[1]; }
+        if (live && has1) { y0 = src[2 * T]; y1 = src[2 * T + 1]; }
+        uint32_t bx[4], by[4];
+        const float sx = quantise16<BF16>(x0, x1, bx);
+        uint8_t* recp = arena + ((size_t)(live ? phys : 0) * Hkv + (live ? h : 0)) * rec;
+        const int j0 = 16 * t, grp = j0 >> 5;
+        if (!is_v) {
+            if (live) {
+                *reinterpret_cast<uint4*>(recp + qrec_value_off(0, slot, j0, P, D)) = make_uint4(bx[0], bx[1], bx[2], bx[3]);
+                if ((t & 1) == 0) *reinterpret_cast<uint16_t*>(recp + qrec_scale_off(0, slot, grp, P, D)) = q_down<BF16>(sx);
+            }
+            continue;
+        }
+        const float sy = quantise16<BF16>(y0, y1, by);
+        if (!live) continue;
+        if (has0 && has1) {
+            uint32_t o[8];  // byte 2 i of the first token's value, 2 i + 1 of the second's
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                o[2 * i] = __byte_perm(bx[i], by[i], 0x5140);
+                o[2 * i + 1] = __byte_perm(bx[i], by[i], 0x7362);
+            }
+            uint4* dst = reinterpret_cast<uint4*>(recp + qrec_value_off(1, slot, j0, P, D));
+            dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+            dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+            if ((t & 1) == 0)
+                *reinterpret_cast<uint32_t*>(recp + qrec_scale_off(1, slot, grp, P, D)) = (uint32_t)q_down<BF16>(sx) | ((uint32_t)q_down<BF16>(sy) << 16);
+        } else {
+            const int s1 = has0 ? slot : slot + 1;  // r = -1: the pair's second token, in the same page
+#pragma unroll
+            for (int i = 0; i < 16; i++)
+                recp[qrec_value_off(1, s1, j0 + i, P, D)] = (uint8_t)((has0 ? bx[i >> 2] : by[i >> 2]) >> (8 * (i & 3)));
+            if ((t & 1) == 0) *reinterpret_cast<uint16_t*>(recp + qrec_scale_off(1, s1, grp, P, D)) = q_down<BF16>(has0 ? sx : sy);
+        }
+    }
+}
+
 // A fresh quantised arena reads as the reference's zero-filled one (kv.rs:699-705): packed words 0
 // mean q = -128 in lanes 0-2 and q = 0 in lane 3, i.e. record bytes 0, 0, 0, 0x80; scales 0.
 __global__ void init_quant_kernel(uint8_t* arena, size_t n_records, int P, int d) {
@@ -249,6 +365,16 @@ cudaError_t launch_init_quant(void* arena, size_t n_records, int page_size, int 
 cudaError_t launch_append_quant(const AppendArgs& a, bool bf16, bool overlap, cudaStream_t st) {
     const int64_t rows = 2 * (int64_t)a.step.n_tokens * a.geo.n_kv;
     if (rows <= 0) return cudaSuccess;
+    if (a.geo.page_size == 16 && (a.geo.d == 64 || a.geo.d == 128 || a.geo.d == 256)) {
+        const int rpw = 512 / a.geo.d;  // rows or pairs of a warp
+        const int64_t warps = (rows / 2 + rpw - 1) / rpw + ((a.step.n_tokens / 2 + a.step.n_seqs) * (int64_t)a.geo.n_kv + rpw - 1) / rpw;
+        const int blocks = (int)std::min<int64_t>((warps + 7) / 8, 148 * 8);
+        switch (a.geo.d) {
+            case 64: return launch_pdl(overlap, bf16 ? append_quant_vec_kernel<true, 4> : append_quant_vec_kernel<false, 4>, blocks, 256, 0, st, a);
+            case 128: return launch_pdl(overlap, bf16 ? append_quant_vec_kernel<true, 8> : append_quant_vec_kernel<false, 8>, blocks, 256, 0, st, a);
+            default: return launch_pdl(overlap, bf16 ? append_quant_vec_kernel<true, 16> : append_quant_vec_kernel<false, 16>, blocks, 256, 0, st, a);
+        }
+    }
     const int blocks = (int)std::min<int64_t>((rows + 7) / 8, 148 * 8);
     return launch_pdl(overlap, bf16 ? append_quant_kernel<true> : append_quant_kernel<false>, blocks, 256, 0, st, a);
 }
