@@ -4,6 +4,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -15,6 +16,10 @@ NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-shared", "-cudart", "static", "-ldl",
 ]
+
+
+PYCALL = os.path.join(HERE, "_pycall.so")  # the Python mirror's hot calls (csrc/pycall.cpp)
+PYCALL_SOURCE = os.path.join(CSRC, "pycall.cpp")
 
 
 def _nvcc() -> str:
@@ -36,6 +41,7 @@ def build(force: bool = False, verbose: bool = False, measure: bool = False) -> 
     """The product library, or (measure=True) the measurement flavour: the same sources with
     -DCBKV_MEASURE, which adds timers and phase switches the product build does not contain."""
     lib = LIB_MEASURE if measure else LIB
+    build_pycall(force)
     if not force and not needs_build(lib):
         return lib
     cmd = [_nvcc(), *NVCC_FLAGS, *( ["-DCBKV_MEASURE"] if measure else []), "-ccbin", "/usr/bin/g++",
@@ -48,6 +54,20 @@ def build(force: bool = False, verbose: bool = False, measure: bool = False) -> 
     if verbose:
         sys.stderr.write(r.stderr)
     return lib
+
+
+def build_pycall(force: bool = False) -> str:
+    if not force and os.path.exists(PYCALL) and os.path.getmtime(PYCALL) >= os.path.getmtime(PYCALL_SOURCE):
+        return PYCALL
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cmd = ["/usr/bin/g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-w", "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(root, "include"),
+           "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"), "-I/usr/local/cuda/include", PYCALL_SOURCE,
+           "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-o", PYCALL]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed:\n" + r.stdout + r.stderr)
+    return PYCALL
 
 
 if __name__ == "__main__":

@@ -134,6 +134,24 @@ def load() -> C.CDLL:
     return lib
 
 
+_native = None
+
+
+def native():
+    """csrc/pycall.cpp, bound to the loaded library: the calls a layer or a step makes, without ctypes."""
+    global _native
+    if _native is None:
+        import torch  # noqa: F401  (its libraries have to be there first)
+        if not os.path.exists(os.path.join(HERE, "_pycall.so")):
+            raise ImportError("_pycall.so is missing: build it with `python -m combsengine_b200._build`")
+        from . import _pycall
+        lib = load()
+        _pycall.bind(*(C.cast(getattr(lib, f), C.c_void_p).value
+                       for f in ("cbkv_attention", "cbkv_attention_rope", "cbkv_begin_step", "cbkv_popn")))
+        _native = _pycall
+    return _native
+
+
 class CbkvError(RuntimeError):
     """A non-zero return code of the C ABI, with the library's message."""
 

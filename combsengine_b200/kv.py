@@ -93,6 +93,10 @@ class PagedSeq:
 
     def popn(self, n: int) -> int:
         """kv.rs:807-835: tokens actually dropped; 0 = refused."""
+        r = self.arena._native.popn(self._h, n)
+        if type(r) is tuple:
+            check(r[0])
+            return r[1]
         popped = C.c_int64(0)
         check(self.arena._lib.cbkv_popn(self._h, n, C.byref(popped)))
         return popped.value
@@ -126,6 +130,7 @@ class KVArena:
                  dtype: torch.dtype = torch.float16, device: int = 0, sliding_popn_refuses: bool = True,
                  quantize_kv: bool = False):
         self._lib = _lib.load()
+        self._native = _lib.native()
         if windows is not None and len(windows) != num_layers:
             raise CbkvError(-4, "one window entry per layer")  # kv.rs:513
         if dtype not in _DTYPES:
@@ -146,6 +151,7 @@ class KVArena:
         self._seqs: set[PagedSeq] = set()
         self.num_layers, self.n_q_heads, self.n_kv_heads, self.head_dim = num_layers, n_q_heads, n_kv_heads, head_dim
         self.page_size, self.dtype, self.device = page_size, dtype, device
+        self._bf16 = _DTYPES[dtype]
         self.max_seq_len = max_seq_len
         self.num_pages = num_pages if num_pages > 0 else -(-max_seq_len // page_size)
         self.step_tokens = 0
@@ -184,6 +190,11 @@ class KVArena:
 
     def begin_step(self, seqs: Sequence[PagedSeq], new_tokens: Sequence[int], pos: Optional[Sequence[int]] = None,
                    stream: Optional[torch.cuda.Stream] = None) -> None:
+        r = self._native.begin_step(self._h, seqs, new_tokens, pos, stream)
+        if type(r) is tuple:
+            check(r[0])
+            self.step_tokens = r[1]
+            return
         n, hs, nt, ps = self._step_args(seqs, new_tokens, pos)
         check(self._lib.cbkv_begin_step(self._h, hs, nt, ps, n, _stream_ptr(stream)))
         self.step_tokens = int(sum(int(x) for x in new_tokens))
@@ -204,6 +215,12 @@ class KVArena:
                   window: Optional[int] = None, out: Optional[torch.Tensor] = None,
                   stream: Optional[torch.cuda.Stream] = None) -> torch.Tensor:
         """attention_opts for every sequence of the step: append + attention (kv.rs:655-791)."""
+        t = self.step_tokens * self.head_dim
+        r = self._native.attention(self._h, layer, q, k, v, out, scale, window, stream, self._bf16, t * self.n_q_heads, t * self.n_kv_heads)
+        if type(r) is not int:
+            return r
+        if r != self._native.SLOW:
+            check(r)
         self._chk(q, self.n_q_heads, "q"); self._chk(k, self.n_kv_heads, "k"); self._chk(v, self.n_kv_heads, "v")
         if out is None:
             out = torch.empty_like(q)
@@ -438,7 +455,7 @@ class PagedKVCache:
             self.arena.begin_step([self.seq], [seq], [pos])
         elif pos + seq != self.seq.seq_len():
             raise CbkvError(-1, "paged cache expects dense contiguous appends (pos == seq_len)")
-        return self.arena.attention(layer, q.contiguous(), k.contiguous(), v.contiguous(), scale, window).view(q.shape)
+        return self.arena.attention(layer, q.contiguous(), k.contiguous(), v.contiguous(), scale, window)
 
     def seq_len(self) -> int:
         return self.seq.seq_len()

@@ -137,10 +137,17 @@ def attention_rope(arena: KVArena, layer: int, rope: RotaryEmbedding, q: torch.T
                    scale: float, window: Optional[int] = None, norm: Optional[QKNorm] = None,
                    out: Optional[torch.Tensor] = None, stream=None) -> torch.Tensor:
     """llama.rs:275-289 for one layer: QK norm, rotation, append, attention."""
+    ns = norm._struct(arena) if norm is not None else None
+    native, t = arena._native, arena.step_tokens * arena.head_dim
+    r = native.attention_rope(arena._h, layer, rope._h, 0 if ns is None else C.addressof(ns), q, k, v, out, scale, window, stream,
+                              arena._bf16, t * arena.n_q_heads, t * arena.n_kv_heads)
+    if type(r) is not int:
+        return r
+    if r != native.SLOW:
+        check(r)
     arena._chk(q, arena.n_q_heads, "q"); arena._chk(k, arena.n_kv_heads, "k"); arena._chk(v, arena.n_kv_heads, "v")
     if out is None:
         out = torch.empty_like(q)
-    ns = norm._struct(arena) if norm is not None else None
     check(arena._lib.cbkv_attention_rope(arena._h, layer, rope._h, C.byref(ns) if ns is not None else None, q.data_ptr(),
                                          k.data_ptr(), v.data_ptr(), out.data_ptr(), float(scale),
                                          0 if window is None else int(window), _stream_ptr(stream)))
