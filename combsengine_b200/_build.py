@@ -10,8 +10,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libcombskv.so")
 LIB_MEASURE = os.path.join(HERE, "libcombskv_measure.so")  # -DCBKV_MEASURE: per-role timers, switches read from CBKV_DEBUG
-SOURCES = ["manager.cpp", "sessions.cpp", "kernels.cu", "prefill_tc.cu", "rope.cu", "kvquant.cu", "api.cu", "noalloc.cu"]
-HEADERS = ["manager.hpp", "kernels.hpp", "pdl.cuh", "tile.cuh", "rope.cuh", "q8_unpack.cuh", os.path.join("..", "..", "include", "combs_kv.h")]
+SOURCES = ["manager.cpp", "sessions.cpp", "kernels.cu", "prefill_tc.cu", "chunk_pair.cu", "rope.cu", "kvquant.cu", "api.cu", "noalloc.cu"]
+HEADERS = ["manager.hpp", "kernels.hpp", "pdl.cuh", "tile.cuh", "tc.cuh", "rope.cuh", "q8_unpack.cuh", os.path.join("..", "..", "include", "combs_kv.h")]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-shared", "-cudart", "static", "-ldl",

@@ -108,8 +108,15 @@ struct DeviceState {
     ChunkPlan chunk_host;
     const int32_t* chunk_item_begin = nullptr;
     bool tc_ok = false;       // the tcgen05 chunk kernel covers this geometry
-    int chunk_mode = 0;       // cbkv_set_chunk_kernel: 0 = choose, 1 = mma.sync, 2 = tcgen05 one tile, 3 = two tiles, 4 = two tiles, int8 records converted in the kernel
-    struct TilePlanDev { ChunkPlan host; const TileItem* tiles = nullptr; bool mma = false; /* the mma.sync kernel is expected to be faster */ };
+    // cbkv_set_chunk_kernel: 0 = choose between 1 and the tcgen05 kernels 2 and 3, 1 = mma.sync, 2 = tcgen05 one tile, 3 = two
+    // tiles, 4 = two tiles, int8 records converted in the kernel, 5 = as 0, and pairs of SMs
+    int chunk_mode = 5;
+    bool chunk_chooses() const { return chunk_mode == 0 || chunk_mode == 5; }
+    struct TilePlanDev {
+        ChunkPlan host;
+        const TileItem* tiles = nullptr;
+        bool mma = false, pair = false;  // the mma.sync kernel, pairs of SMs are expected to be faster
+    };
     std::map<std::pair<int64_t, int>, TilePlanDev> tile_plans;  // of the step, by (window, tokens per work item)
     float* part_o = nullptr;
     float* part_ml = nullptr;
@@ -201,6 +208,7 @@ int32_t ensure_device(Arena* a) {
         if (chunk_tc_supported(D)) {
             ke = chunk_tc_init();
             if (ke != cudaSuccess) { delete d; set_error(std::string("chunk_tc_init: ") + cudaGetErrorString(ke)); return CBKV_ERR_CUDA; }
+            if (chunk_pair_supported(D) && (ke = chunk_pair_init()) != cudaSuccess) { delete d; set_error(std::string("chunk_pair_init: ") + cudaGetErrorString(ke)); return CBKV_ERR_CUDA; }
             d->tc_ok = true;
         }
     }
@@ -299,6 +307,12 @@ int32_t alloc_float_layer(Arena* a, LayerArena* Lp, cudaStream_t st) {
             CUresult r = encode_fn()(&L.map_page, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, L.base, dims,
                                      strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+            if (r == CUDA_SUCCESS && D >= 128) {
+                box[2] = (cuuint32_t)(D / 128);
+                r = encode_fn()(&L.map_vhalf, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, L.base, dims,
+                                strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+            }
             if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled (pages) failed: " + std::to_string((int)r)); return CBKV_ERR_CUDA; }
         }
     }
@@ -545,16 +559,32 @@ int32_t get_tile_plan(Arena* a, int64_t window, int tokens_per_item, int tile_to
     DeviceState::TilePlanDev pd;
     TileCut cut{window, kv_tile, tile_tokens, d->sm_count, d->chunk_split};
     build_chunk_tile_plan(*a, tokens_per_item, &pd.host, cut);
+    float us = chunk_tile_launch_us(*a, pd.host, cut);
     // One tcgen05 CTA per SM at a time costs more to start than a few pages take the mma.sync kernel, of which eight
     // warps (items) share an SM: steps with more (sequence, kv head) pairs than SMs over short contexts, and prompts of
     // some tens of tokens.  64 sequences x 2 tokens after 33 (8 kv heads, head_dim 128): 12.7 against 28.7 us, after
     // 600: 45 against 65; 32 x 2 after 600: 43 against 34; a 40-token prompt (4 kv heads) 10.3 against 13.0.
-    pd.mma = chunk_mma_launch_us(*a, window, chunk_config(a->cfg.head_dim).cols_per_item, d->sm_count) <
-             chunk_tile_launch_us(*a, pd.host, cut);
-    if (!(pd.mma && d->chunk_mode == 0)) {
+    const float mma_us = chunk_mma_launch_us(*a, window, chunk_config(a->cfg.head_dim).cols_per_item, d->sm_count);
+    // Pairs of SMs take a query tile per CTA: at head_dim 128 a launch that leaves SMs idle ends sooner (a prompt of 512
+    // after 512, 8 kv heads: 19.5 against 31.0 us; four of them after 1024: 92 against 73), at head_dim 256 every launch
+    // of more than some tens of tokens does (8 prompts of 512 after 7680: 236 against 338; one after 512: 24 against 49).
+    if (d->chunk_mode == 5 && chunk_pair_supported(a->cfg.head_dim)) {
+        const TileCut pc{window, 128, 2 * tile_tokens, d->sm_count / 2, d->chunk_split, true};
+        ChunkPlan pairs;
+        build_chunk_tile_plan(*a, 2 * tile_tokens, &pairs, pc);
+        const float pair_us = chunk_tile_launch_us(*a, pairs, pc);
+        if (pair_us < us) {
+            pd.pair = true;
+            pd.host = std::move(pairs);
+            cut = pc;
+            us = pair_us;
+        }
+    }
+    pd.mma = mma_us < us;
+    if (!(pd.mma && d->chunk_chooses())) {
         if (pd.host.n_cut > 0 && !ensure_split(a, st)) {
             cut.max_parts = 1;
-            build_chunk_tile_plan(*a, tokens_per_item, &pd.host, cut);
+            build_chunk_tile_plan(*a, pd.pair ? 2 * tile_tokens : tokens_per_item, &pd.host, cut);
         }
         const void* p = nullptr;
         int32_t rc = slot_upload(d, pd.host.tiles.data(), pd.host.tiles.size() * sizeof(TileItem), st, &p);
@@ -631,7 +661,7 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
     if (use_tc) {
         int32_t rc = get_tile_plan(a, w, (use_tc2 ? 2 : 1) * tile_tokens, tile_tokens, !use_tc2 && a->cfg.head_dim == 256 ? 64 : 128, st, &tp);
         if (rc) return rc;
-        if (tp->mma && d->chunk_mode == 0) use_tc = false;
+        if (tp->mma && d->chunk_chooses()) use_tc = false;
     }
     // int8 pages: decode steps stream the records through the decode kernel; the chunk kernels read a float
     // copy made per layer and step (mode 4: the two-tile kernel converts the records itself, slower so far);
@@ -716,7 +746,8 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
 #endif
         ProfScope ps(d, st);
         { int32_t frc = flush_uploads(d, st); if (frc) return frc; }
-        if (use_tc2) CU_TRY(q8_direct ? launch_chunk_tc2(L.map_k16, L.map_sc, args, bf16, d->pdl, st) : launch_chunk_tc2(KV->map_kv, KV->map_kv, args, bf16, d->pdl, st));
+        if (tp->pair) CU_TRY(launch_chunk_pair(KV->map_page, KV->map_vhalf, args, bf16, d->pdl, st));
+        else if (use_tc2) CU_TRY(q8_direct ? launch_chunk_tc2(L.map_k16, L.map_sc, args, bf16, d->pdl, st) : launch_chunk_tc2(KV->map_kv, KV->map_kv, args, bf16, d->pdl, st));
         else CU_TRY(launch_chunk_tc(KV->map_page, args, bf16, d->pdl, st));
         g_launches++;
         d->last_kv_writer = -1;
@@ -1594,10 +1625,10 @@ int32_t cbkv_set_chunk_split(cbkv_arena* arena, int32_t max_parts) {
 int32_t cbkv_set_chunk_kernel(cbkv_arena* arena, int32_t mode) {
     return fenced([&]() -> int32_t {
     Arena* a = reinterpret_cast<Arena*>(arena);
-    if (!a || mode < 0 || mode > 4) { set_error("bad argument"); return CBKV_ERR_ARG; }
+    if (!a || mode < 0 || mode > 5) { set_error("bad argument"); return CBKV_ERR_ARG; }
     int32_t rc = ensure_device(a);
     if (rc) return rc;
-    if (mode >= 3 && !(dev_of(a)->tc_ok && chunk_tc2_supported(a->cfg.head_dim))) {
+    if ((mode == 3 || mode == 4) && !(dev_of(a)->tc_ok && chunk_tc2_supported(a->cfg.head_dim))) {
         set_error("the two-tile tensor-core chunk kernel covers head_dim 128 with 16-token pages only"); return CBKV_ERR_ARG;
     }
     if (mode == 2 && !dev_of(a)->tc_ok) { set_error("the tensor-core chunk kernel covers head_dim 64, 128 and 256 with 16-token pages only"); return CBKV_ERR_ARG; }

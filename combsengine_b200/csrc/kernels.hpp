@@ -66,6 +66,7 @@ struct LayerArena {
                          // quantised: bytes in 128-byte rows, one box = one record
     CUtensorMap map_page; // float layers: {64 elems, 8 rows, d/64 column blocks, K or V, 8-token groups}, box = K or V of
                          // one page of one kv head, as [group][column block][8 rows of 128 bytes], 128B swizzle
+    CUtensorMap map_vhalf; // the same with half of the column blocks in the box (head_dim 128 and 256)
     CUtensorMap map_k16; // quantised, head_dim 128: box = the 16 rows of a record's K values or of its V values
     CUtensorMap map_sc;  // quantised, head_dim 128: box = one row, a record's K scales or its V scales
 };
@@ -221,6 +222,11 @@ cudaError_t launch_chunk_tc(const CUtensorMap& map, const ChunkArgs& a, bool bf1
 bool chunk_tc2_supported(int d);
 // float layer: `map` = the layer's map_kv, map_sc is not used; int8 layer (a.q8_arena non-null): its map_k16 and map_sc
 cudaError_t launch_chunk_tc2(const CUtensorMap& map, const CUtensorMap& map_sc, const ChunkArgs& a, bool bf16, bool overlap, cudaStream_t st);
+// pairs of SMs (chunk_pair.cu): head_dim 128 or 256; map_k = the layer's map_page, map_v its map_vhalf; one work item per
+// two query tiles
+bool chunk_pair_supported(int d);
+cudaError_t chunk_pair_init();
+cudaError_t launch_chunk_pair(const CUtensorMap& map_k, const CUtensorMap& map_v, const ChunkArgs& a, bool bf16, bool overlap, cudaStream_t st);
 cudaError_t kernels_init();  // raises the dynamic shared memory limits once per process
 
 }  // namespace cbkv

@@ -336,6 +336,7 @@ namespace {
 // its two query tiles kHalfTile, a slice kSliceCost more (its partial rows), and the merge at the end
 // kMergeCost for each slice of the full 256 rows.
 constexpr float kCtaCost = 3.f, kHalfTile = 0.7f, kSliceCost = 0.7f, kMergeCost = 0.7f;
+constexpr float kPairCtaCost = 5.f, kPairSliceCost = 1.f, kPairMergeCost = 1.f;  // the same for pairs of CTAs, whose K/V tiles are shorter
 
 struct TileWork { int32_t seq, h, qt, n_tiles; float per_tile, rows; };  // an uncut item
 
@@ -363,6 +364,7 @@ float launch_end(const std::vector<float>& cost, int sm_count, std::vector<float
 void build_chunk_tile_plan(const Arena& a, int32_t tokens_per_tile, ChunkPlan* pl, const TileCut& cut) {
     const int n = (int)a.step_meta.size();
     const int tile_tokens = cut.tile_tokens > 0 ? cut.tile_tokens : tokens_per_tile;
+    const float cta_cost = cut.pair ? kPairCtaCost : kCtaCost, slice_cost = cut.pair ? kPairSliceCost : kSliceCost, merge_cost = cut.pair ? kPairMergeCost : kMergeCost;
     pl->cols_per_item = tokens_per_tile;
     pl->item_begin.assign((size_t)n + 1, 0);
     pl->tiles.clear();
@@ -418,7 +420,7 @@ void build_chunk_tile_plan(const Arena& a, int32_t tokens_per_tile, ChunkPlan* p
                     if (p > 1) {
                         base[(size_t)qt] = slots; id[(size_t)qt] = cuts;
                         slots += p; cuts++;
-                        merge = std::max(merge, kMergeCost * (0.5f + (float)p * w.rows));
+                        merge = std::max(merge, merge_cost * (0.5f + (float)p * w.rows));
                     }
                 }
                 for (int p = 0; p < most; p++)
@@ -428,7 +430,7 @@ void build_chunk_tile_plan(const Arena& a, int32_t tokens_per_tile, ChunkPlan* p
                         const TileWork& w = work[(size_t)(g.first + qt)];
                         const int per = (w.n_tiles + np - 1) / np, t0 = p * per, t1 = std::min(w.n_tiles, t0 + per);
                         if (out) out->push_back({g.seq, h, qt, t0, t1, p | (np << 16), base[(size_t)qt], id[(size_t)qt]});
-                        else cost.push_back(kCtaCost + w.per_tile * (float)(t1 - t0) + (np > 1 ? kSliceCost : 0.f));
+                        else cost.push_back(cta_cost + w.per_tile * (float)(t1 - t0) + (np > 1 ? slice_cost : 0.f));
                     }
             }
         }
@@ -469,14 +471,15 @@ namespace {
 // a tcgen05 launch takes fixed_us, then per wave of one CTA per SM cta_us + tile_us for each K/V tile (head_dim 128:
 // [0] with one query tile, [1] with both); the mma.sync kernel, one warp per item over all its pages, mma_us + page_us
 // for each page of the longest item, `warps` of them per SM at a time; with more items than that, kMmaRounds times as
-// much per round.
-struct ChunkTimes { float cta_us[2], tile_us[2], mma_us, page_us; int32_t warps; };
+// much per round.  Pairs of CTAs (prompts of 40 to 512 tokens, 1 to 8 of them, up to 7680 cached tokens): pair_cta_us and
+// pair_tile_us per wave of one pair per two SMs.
+struct ChunkTimes { float cta_us[2], tile_us[2], mma_us, page_us; int32_t warps; float pair_cta_us, pair_tile_us; };
 constexpr float kChunkFixedUs = 1.7f, kMmaRounds = 1.5f;
 ChunkTimes chunk_times(int32_t d) {
     switch (d) {
-        case 64: return {{5.f, 5.f}, {1.f, 1.f}, 11.f, 1.04f, 12};
-        case 128: return {{5.8f, 10.f}, {2.1f, 2.45f}, 8.f, 0.84f, 8};
-        default: return {{6.f, 6.f}, {1.3f, 1.3f}, 7.5f, 0.88f, 4};  // 256
+        case 64: return {{5.f, 5.f}, {1.f, 1.f}, 11.f, 1.04f, 12, 0.f, 0.f};
+        case 128: return {{5.8f, 10.f}, {2.1f, 2.45f}, 8.f, 0.84f, 8, 9.f, 1.25f};
+        default: return {{6.f, 6.f}, {1.3f, 1.3f}, 7.5f, 0.88f, 4, 9.f, 1.9f};  // 256
     }
 }
 
@@ -488,7 +491,8 @@ float chunk_tile_launch_us(const Arena& a, const ChunkPlan& pl, const TileCut& c
     cost.reserve(pl.tiles.size());
     for (const TileItem& w : pl.tiles) {
         const int both = a.step_meta[(size_t)w.seq].snew - w.qt * pl.cols_per_item > cut.tile_tokens ? 1 : 0;
-        cost.push_back(t.cta_us[both] + t.tile_us[both] * (float)(w.t1 - w.t0));
+        if (cut.pair) cost.push_back(t.pair_cta_us + t.pair_tile_us * (float)(w.t1 - w.t0));
+        else cost.push_back(t.cta_us[both] + t.tile_us[both] * (float)(w.t1 - w.t0));
     }
     return kChunkFixedUs + launch_end(cost, cut.sm_count, &heap);
 }

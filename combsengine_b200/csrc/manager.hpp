@@ -135,8 +135,9 @@ struct TileItem {  // 32 bytes, read by the kernels as two 16-byte words
     int32_t t1, part_nparts /* part | nparts << 16 */, slot_base, cut;
 };
 // How a tcgen05 chunk launch may be cut: `window` of the layer, tokens per K/V tile, query tokens per 128-row
-// tile, SMs (one CTA each at a time; 0 = never cut), most slices per item.
-struct TileCut { int64_t window = 0; int32_t kv_tile = 128, tile_tokens = 0, sm_count = 0, max_parts = 1; };
+// tile, SMs (one CTA each at a time; 0 = never cut), most slices per item; pair: an item is a pair of CTAs with a query
+// tile each, `sm_count` counts pairs of SMs.
+struct TileCut { int64_t window = 0; int32_t kv_tile = 128, tile_tokens = 0, sm_count = 0, max_parts = 1; bool pair = false; };
 // No launch is cut into more slices than this many per SM, so that the partial-result buffers have one size (at 148
 // SMs, head_dim 128 or 256: 592 slots, 78 MB) and never have to grow under a plan that is already made.  The launch
 // model asked for at most 3.9 per SM over 2800 steps of 1 to 128 sequences.

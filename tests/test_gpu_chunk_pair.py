@@ -1,0 +1,58 @@
+"""Prompts' chunks on pairs of SMs (the library's choice for launches that they shorten), against the oracle (needs a B200)."""
+import pytest
+import torch
+
+from kvcase import Pair
+from test_gpu_chunk_cut import _fill, _step
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("grow", [False, True])
+@pytest.mark.parametrize("n_q,n_kv,d", [(28, 4, 128), (32, 8, 128), (8, 8, 128), (8, 4, 256), (8, 1, 256)])
+def test_chunks_on_pairs_of_sms(n_q, n_kv, d, grow):
+    # tokens per query tile: 16 to 128; chunks that fill one tile, two, and leave the second with none or a few; KV tiles of
+    # 64 or 128 tokens: one, two and many of them, cut and whole
+    p = Pair(2, n_q, n_kv, d, 4096, num_pages=1600, windows=[150, None], seed=d + n_q, shuffle_free_list=True, popn_refuses=False)
+    for ctx in (0, 1, 50, 130, 900, 2050):
+        s = p.new_seq()
+        if ctx:
+            _fill(p, s, ctx, [0, 1], grow)
+    for s in p.seqs:
+        _step(p, [s], [70], [0, 1], grow, repeats=5)
+        _step(p, [s], [257], [0, 1], grow, repeats=5)
+    _step(p, p.seqs, [128, 65, 80, 129, 200, 97], [0, 1], grow, repeats=20)
+    p.g.set_chunk_split(1)
+    _step(p, p.seqs, [128, 65, 80, 129, 200, 97], [0, 1], grow, repeats=5)
+
+
+def test_prompts_in_both_types_against_64_bits():
+    from combsengine_b200 import KVArena
+    for dtype in (torch.float16, torch.bfloat16):
+        for d, n_q, n_kv, new in ((128, 32, 8, 90), (128, 28, 4, 300), (256, 8, 4, 200)):
+            gen = torch.Generator(device="cuda").manual_seed(d)
+            g = KVArena(1, n_q, n_kv, d, 2048, 16, 400, dtype=dtype, sliding_popn_refuses=False)
+            rand = lambda n: torch.randn(n, generator=gen, device="cuda", dtype=dtype)
+            seqs, ctx = [g.new_seq() for _ in range(3)], [37, 500, 1203]
+            g.begin_step(seqs, ctx)
+            k0, v0 = rand(sum(ctx) * n_kv * d), rand(sum(ctx) * n_kv * d)
+            g.append(0, k0, v0)
+            q, k, v = (rand(3 * new * h * d) for h in (n_q, n_kv, n_kv))
+            g.begin_step(seqs, [new] * 3)
+            out = g.attention(0, q, k, v, d ** -0.5)
+            assert g.device_status() == 0
+            # f64 reference
+            off = ko = 0
+            for c in ctx:
+                K = torch.cat([k0.view(-1)[ko * n_kv * d:(ko + c) * n_kv * d].view(n_kv, c, d), k[off * n_kv * d:(off + new) * n_kv * d].view(n_kv, new, d)], 1).double()
+                V = torch.cat([v0.view(-1)[ko * n_kv * d:(ko + c) * n_kv * d].view(n_kv, c, d), v[off * n_kv * d:(off + new) * n_kv * d].view(n_kv, new, d)], 1).double()
+                Q = q[off * n_q * d:(off + new) * n_q * d].view(n_q, new, d).double()
+                s = Q @ K.repeat_interleave(n_q // n_kv, 0).transpose(1, 2) * d ** -0.5
+                s.masked_fill_(torch.arange(c + new, device="cuda")[None, :] > c + torch.arange(new, device="cuda")[:, None], -float("inf"))
+                ref = s.softmax(-1) @ V.repeat_interleave(n_q // n_kv, 0)
+                got = out[off * n_q * d:(off + new) * n_q * d].view(n_q, new, d).double()
+                # outputs and probabilities are rounded to 8 (bf16) or 11 bits: 2^-9 and 2^-12 relative each, as rms
+                # over many terms well below these
+                assert (got - ref).norm() / ref.norm() < (2 ** -8 if dtype == torch.bfloat16 else 2 ** -10.5)
+                off += new
+                ko += c
