@@ -334,7 +334,7 @@ class KVArena:
         check(self._lib.cbkv_set_chunk_split(self._h, max_parts))
 
     def set_chunk_kernel(self, mode: int) -> None:
-        """0 = library's choice, 1 = mma.sync chunk kernel, 2 = tcgen05/TMEM kernel (one query tile per
+        """5 (default) = library's choice among all, 0 = among 1 to 3, 1 = mma.sync chunk kernel, 2 = tcgen05/TMEM kernel (one query tile per
         CTA), 3 = tcgen05/TMEM kernel with two query tiles per CTA (head_dim 128); int8 layers are read
         through a float copy made per layer and step, except in mode 4 = as 3 with the int8 records
         converted inside the kernel (slower so far)."""

@@ -342,14 +342,15 @@ int32_t cbkv_set_host_route(cbkv_arena* arena, int32_t direct);
  * the default. */
 int32_t cbkv_set_chunk_split(cbkv_arena* arena, int32_t max_parts);
 
-/* Which kernel runs a step that is not pure decode: 0 = the library chooses (tcgen05
+/* Which kernel runs a step that is not pure decode: 0 = the library chooses among 1 to 3 (tcgen05
  * tiles; mma.sync where many short sequences or a short prompt make that faster, for
  * scales that are not positive and for q or out off a 16-byte boundary), 1 = the mma.sync kernel, 2 = the
  * tcgen05/TMEM kernel with one 128-row query tile per CTA (head_dim 64, 128 or 256), 3 = the
  * tcgen05/TMEM kernel with two query tiles per CTA and P in tensor memory (head_dim 128).
  * Over int8 layers these kernels read a float copy of the step's pages made per layer and
  * step; 4 = as 3, but the kernel fetches the int8 records and converts them itself (no
- * float copy; slower so far, kept for measurement). */
+ * float copy; slower so far, kept for measurement); 5 (the default) = as 0, and pairs of SMs
+ * (cta_group::2, head_dim 128 or 256) where the launch model expects them to be faster. */
 int32_t cbkv_set_chunk_kernel(cbkv_arena* arena, int32_t mode);
 
 /* ---- test hooks (host only, no device is touched) --------------------------- */
