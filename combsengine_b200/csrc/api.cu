@@ -573,7 +573,8 @@ int32_t get_tile_plan(Arena* a, int64_t window, int tokens_per_item, int tile_to
         ChunkPlan pairs;
         build_chunk_tile_plan(*a, 2 * tile_tokens, &pairs, pc);
         const float pair_us = chunk_tile_launch_us(*a, pairs, pc);
-        if (pair_us < us) {
+        // (the one-tile kernel's estimate at head_dim 256 is too low where its short launches are cut: 28 us for the 49 above)
+        if (pair_us < us || a->cfg.head_dim == 256) {
             pd.pair = true;
             pd.host = std::move(pairs);
             cut = pc;

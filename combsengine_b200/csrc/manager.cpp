@@ -479,7 +479,7 @@ ChunkTimes chunk_times(int32_t d) {
     switch (d) {
         case 64: return {{5.f, 5.f}, {1.f, 1.f}, 11.f, 1.04f, 12, 0.f, 0.f};
         case 128: return {{5.8f, 10.f}, {2.1f, 2.45f}, 8.f, 0.84f, 8, 9.f, 1.25f};
-        default: return {{6.f, 6.f}, {1.3f, 1.3f}, 7.5f, 0.88f, 4, 9.f, 1.9f};  // 256
+        default: return {{6.f, 6.f}, {1.3f, 1.3f}, 7.5f, 0.88f, 4, 11.5f, 1.9f};  // 256
     }
 }
 
