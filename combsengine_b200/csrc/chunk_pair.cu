@@ -43,12 +43,13 @@ constexpr int kPairBufs = 5;
 // barriers, each 8 bytes
 constexpr int kBKFull = 0, kBVFull = kBKFull + kPairBufs, kBKEmpty = kBVFull + kPairBufs, kBVEmpty = kBKEmpty + kPairBufs;
 constexpr int kBSFull = kBVEmpty + kPairBufs, kBPFull = kBSFull + 2, kBODone = kBPFull + 2, kBQFull = kBODone + 2;
+constexpr int kPairWords = 4 + 8;  // 8-byte words after the barriers: tensor memory, failed and ticket, then the 16 flags of the pairs of warps
 constexpr int kBSFree = kBQFull + 1, kBRef = kBSFree + 2 /* [2 buffers][4 quarters] */, kBCount = kBRef + 8;
 
 template <int D>
 constexpr int pair_smem_bytes() {
-    return 128 * D * 2 /* Q */ + 2 * PairBufs<D>::value * (kPairKeys / 2) * D * 2 + (kBCount + 16) * 8 + kPageCap * 4 +
-           (2 * 2 * 128 /* half-row maxima */ + 2 * 128 /* reference exponents */ + 4 * 128 /* row sums */) * 4;
+    return 128 * D * 2 /* Q */ + 2 * PairBufs<D>::value * (kPairKeys / 2) * D * 2 + (kBCount + kPairWords) * 8 + kPageCap * 4 +
+           (2 * 2 * 2 * 128 /* half-row maxima */ + 2 * 128 /* reference exponents */ + 4 * 128 /* row sums */) * 4;
 }
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -129,10 +130,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kBCount);
     volatile int* failed = reinterpret_cast<volatile int*>(bars + kBCount + 1);
     int* s_ticket = reinterpret_cast<int*>(bars + kBCount + 2);
-    int* s_pair = reinterpret_cast<int*>(bars + kBCount + 4);      // [8] a wait of this pair of warps ran out
-    int* s_pages = reinterpret_cast<int*>(bars + kBCount + 16);    // [kPageCap] physical pages of the KV range
-    float* s_xch = reinterpret_cast<float*>(s_pages + kPageCap);   // [S buffer][128 rows][2 halves]
-    float* s_ref = s_xch + 2 * 2 * 128;                            // [S buffer][128 rows]
+    int* s_pair = reinterpret_cast<int*>(bars + kBCount + 4);      // [8 pairs of warps][parity of the group's tile] a wait ran out
+    int* s_pages = reinterpret_cast<int*>(bars + kBCount + kPairWords);  // [kPageCap] physical pages of the KV range
+    float* s_xch = reinterpret_cast<float*>(s_pages + kPageCap);   // [S buffer][parity of the group's tile][128 rows][2 halves]
+    float* s_ref = s_xch + 2 * 2 * 2 * 128;                        // [S buffer][128 rows]
     float* s_sum = s_ref + 2 * 128;                                // [group][half][128 rows]
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -172,7 +173,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
         for (int i = 0; i < 2; i++) mbar_init(bar(kBSFree + i), 16);
         for (int i = 0; i < 8; i++) mbar_init(bar(kBRef + i), 1);
         *failed = 0;
-        for (int i = 0; i < 8; i++) s_pair[i] = 0;
+        for (int i = 0; i < 16; i++) s_pair[i] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_k) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_v) : "memory");
@@ -307,8 +308,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
             if (lane == 0) arrive_cluster_release(at_rank0(bar(kBQFull)));
         }
         // A named barrier has no time limit, so the two warps of a pair must leave the loop in the same
-        // iteration: whichever sees a wait run out says so here before the pair's barrier, both read it after.
-        volatile int* pair_failed = s_pair + pair_id;
+        // iteration: whichever sees a wait run out says so before the pair's barrier, both read it after.  Flags and
+        // half-row maxima have two places each, taken in turn: a warp may pass the barrier, and with P in columns of its
+        // own find its next scores there and write again, before the other has read what it wrote for this tile.  It
+        // cannot come back to the same place without the barrier in between, which the other reaches after that read.
         const uint32_t tS = tS0 + X * KT + lane_addr, tP = tP0 + X * PSTRIDE + lane_addr;
         const uint32_t p_full0 = at_rank0(bar(kBPFull + X)), s_free0 = at_rank0(bar(kBSFree + X));
         // Exponents are taken against a reference that is only moved when a row's maximum exceeds it by more than 8 (a
@@ -346,7 +349,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
                 }
                 mx = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
             }
-            float* xrow = s_xch + (X * 128 + m) * 2;
+            const int turn = (j >> 1) & 1;
+            volatile int* pair_failed = s_pair + pair_id * 2 + turn;
+            float* xrow = s_xch + ((X * 2 + turn) * 128 + m) * 2;
             xrow[H] = mx;
             // the reference that the tile before left; read before the pair's barrier, after which its place may be reused
             float m_ref = -INFINITY;
