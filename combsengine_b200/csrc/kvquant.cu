@@ -365,7 +365,9 @@ cudaError_t launch_init_quant(void* arena, size_t n_records, int page_size, int 
 cudaError_t launch_append_quant(const AppendArgs& a, bool bf16, bool overlap, cudaStream_t st) {
     const int64_t rows = 2 * (int64_t)a.step.n_tokens * a.geo.n_kv;
     if (rows <= 0) return cudaSuccess;
-    if (a.geo.page_size == 16 && (a.geo.d == 64 || a.geo.d == 128 || a.geo.d == 256)) {
+    // 16 bytes a load where k and v allow it; the kernel of one row per warp takes them at any multiple of 8
+    const bool aligned16 = ((reinterpret_cast<uintptr_t>(a.k) | reinterpret_cast<uintptr_t>(a.v)) & 15) == 0;
+    if (aligned16 && a.geo.page_size == 16 && (a.geo.d == 64 || a.geo.d == 128 || a.geo.d == 256)) {
         const int rpw = 512 / a.geo.d;  // rows or pairs of a warp
         const int64_t warps = (rows / 2 + rpw - 1) / rpw + ((a.step.n_tokens / 2 + a.step.n_seqs) * (int64_t)a.geo.n_kv + rpw - 1) / rpw;
         const int blocks = (int)std::min<int64_t>((warps + 7) / 8, 148 * 8);

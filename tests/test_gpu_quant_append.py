@@ -1,6 +1,8 @@
 """The quantising append over token pairs: sequences that start and end on either side of a pair (needs a B200)."""
 import pytest
+import torch
 
+from combsengine_b200 import KVArena
 from kvcase import Pair
 
 pytestmark = pytest.mark.gpu
@@ -18,3 +20,29 @@ def test_pages_hold_the_oracles_bytes_whatever_the_parity(d):
     p.step([seqs[3]], [29])
     p.step([seqs[0]], [1])
     p.assert_state_equal("used")
+
+
+@pytest.mark.parametrize("d", [64, 128, 256])
+@pytest.mark.parametrize("k_off,v_off", [(4, 0), (0, 4), (4, 12)])
+def test_rows_that_start_at_8_bytes_fill_the_same_pages(d, k_off, v_off):
+    # contiguous views into larger buffers, as a fused projection leaves them; one call appends, the other attends as well
+    gen = torch.Generator(device="cuda").manual_seed(d)
+    rand = lambda n: torch.randn(n, generator=gen, device="cuda", dtype=torch.float16)
+    view = lambda x, off: torch.zeros(x.numel() + 16, dtype=x.dtype, device="cuda")[off:off + x.numel()].copy_(x)
+    g = KVArena(1, 8, 2, d, 512, 16, 40, quantize_kv=True)
+    s = g.new_seq()
+    n = 37
+    q, k, v = (rand(n * h * d) for h in (8, 2, 2))
+
+    def pages(kx, vx):
+        g.begin_step([s], [n])
+        out = g.attention(0, q, kx, vx, d ** -0.5)
+        rows = [g.export_page_quant(0, int(page)) for page in s.block_table()]
+        s.popn(n)
+        return out, rows
+
+    out, rows = pages(k, v)
+    out8, rows8 = pages(view(k, k_off), view(v, v_off))
+    assert g.device_status() == 0
+    assert torch.equal(out, out8)
+    assert all((x == y).all() for a, b in zip(rows, rows8) for x, y in zip(a, b))
