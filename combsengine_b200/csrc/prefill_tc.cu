@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
     static_assert(4 * NB + 8 <= 32, "barriers");
     int* s_pages = reinterpret_cast<int*>(bars + 32);   // [kPageCap] physical pages of the KV range
     float* s_xch = reinterpret_cast<float*>(s_pages + kPageCap);  // [2 buffers][128 rows][2 halves]
-    int* s_pair = reinterpret_cast<int*>(s_xch + 2 * 128 * 2);    // [4] a wait of this pair of warps ran out
+    int* s_pair = reinterpret_cast<int*>(s_xch + 2 * 128 * 2);    // [4 pairs of warps][tile parity] a wait ran out
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if ((smem_u32(smem) & 1023u) != 0) {
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
         for (int i = 0; i < 2; i++) { mbar_init(b_s_full + i * 8, 1); mbar_init(b_p_full + i * 8, 256); }
         mbar_init(b_o_done, 1);
         *failed = 0;
-        for (int i = 0; i < 4; i++) s_pair[i] = 0;
+        for (int i = 0; i < 8; i++) s_pair[i] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap) : "memory");
     }
@@ -248,8 +248,8 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
         const uint32_t lane_addr = (uint32_t)lane_base << 16;
         const int pair_bar = 1 + (warp & 3);
         // A named barrier has no time limit, so the two warps of a pair must leave the loop in the same
-        // iteration: whichever sees a wait run out says so here before the pair's barrier, both read it after.
-        volatile int* pair_failed = s_pair + (warp & 3);
+        // iteration: whichever sees a wait run out says so before the pair's barrier, both read it after.  Two flags
+        // in turn: a warp may be at the next tile before the other has read this one's.
         // Exponents are taken against a reference maximum that is only moved when a row's maximum
         // exceeds it by more than 8 (a factor 256): probabilities then stay below 256, exact enough in
         // f16/bf16 with f32 sums, and O needs rescaling only on those rare moves.
@@ -262,6 +262,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
             ok = mbar_wait_bounded(b_s_full + (j & 1) * 8, (j >> 1) & 1) && !*failed;
             ok = __all_sync(0xffffffffu, ok);
             TC_ACC(c_ws);
+            volatile int* pair_failed = s_pair + (warp & 3) * 2 + (j & 1);
             if (!ok && lane == 0) *pair_failed = 1;  // the loads below then read stale columns: harmless, nothing is kept
             tc_fence_after();
             const uint32_t tS = tS0 + (j & 1) * KT + lane_addr;
