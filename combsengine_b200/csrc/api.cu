@@ -111,13 +111,11 @@ struct DeviceState {
     // cbkv_set_chunk_kernel: 0 = choose between 1 and the tcgen05 kernels 2 and 3, 1 = mma.sync, 2 = tcgen05 one tile, 3 = two
     // tiles, 4 = two tiles, int8 records converted in the kernel, 5 = as 0, and pairs of SMs
     int chunk_mode = 5;
-    bool chunk_chooses() const { return chunk_mode == 0 || chunk_mode == 5; }
     struct TilePlanDev {
-        ChunkPlan host;
+        ChunkLaunch launch;
         const TileItem* tiles = nullptr;
-        bool mma = false, pair = false;  // the mma.sync kernel, pairs of SMs are expected to be faster
     };
-    std::map<std::pair<int64_t, int>, TilePlanDev> tile_plans;  // of the step, by (window, tokens per work item)
+    std::map<int64_t, TilePlanDev> tile_plans;  // of the step, by window
     float* part_o = nullptr;
     float* part_ml = nullptr;
     size_t part_cap = 0;
@@ -549,50 +547,39 @@ bool ensure_split(Arena* a, cudaStream_t st) {
     return true;
 }
 
-// Work list of a tcgen05 chunk launch: tokens_per_item new tokens per item in tiles of tile_tokens, K/V tiles of
-// kv_tile tokens.  Built once per step and window.
-int32_t get_tile_plan(Arena* a, int64_t window, int tokens_per_item, int tile_tokens, int kv_tile, cudaStream_t st, DeviceState::TilePlanDev** out) {
+// Who may run a chunk step's launch over `window`, in which tiles (cbkv_set_chunk_kernel).
+ChunkChoice chunk_choice(const Arena& a, int mode, int64_t window, int sm_count, int max_parts) {
+    const int D = a.cfg.head_dim, tile_tokens = 128 / rep_slots_of(a.n_rep());
+    const bool two_tiles = chunk_tc2_supported(D) && mode != 2;
+    ChunkChoice c;
+    c.one_tokens = (two_tiles ? 2 : 1) * tile_tokens;
+    c.one = TileCut{window, !two_tiles && D == 256 ? 64 : 128, tile_tokens, sm_count, max_parts};
+    c.pairs = mode == 5 && chunk_pair_supported(D);
+    c.pair_tokens = 2 * tile_tokens;
+    c.pair = TileCut{window, 128, 2 * tile_tokens, sm_count / 2, max_parts, true};
+    if (mode == 0 || mode == 5) c.mma_cols = chunk_config(D).cols_per_item;
+    return c;
+}
+
+// Kernel and work list of a chunk launch.  Built once per step and window.
+int32_t get_tile_plan(Arena* a, int64_t window, cudaStream_t st, DeviceState::TilePlanDev** out) {
     DeviceState* d = dev_of(a);
-    const auto key = std::make_pair(window, tokens_per_item);
-    auto it = d->tile_plans.find(key);
+    auto it = d->tile_plans.find(window);
     if (it != d->tile_plans.end()) { *out = &it->second; return CBKV_OK; }
     DeviceState::TilePlanDev pd;
-    TileCut cut{window, kv_tile, tile_tokens, d->sm_count, d->chunk_split};
-    build_chunk_tile_plan(*a, tokens_per_item, &pd.host, cut);
-    float us = chunk_tile_launch_us(*a, pd.host, cut);
-    // One tcgen05 CTA per SM at a time costs more to start than a few pages take the mma.sync kernel, of which eight
-    // warps (items) share an SM: steps with more (sequence, kv head) pairs than SMs over short contexts, and prompts of
-    // some tens of tokens.  64 sequences x 2 tokens after 33 (8 kv heads, head_dim 128): 12.7 against 28.7 us, after
-    // 600: 45 against 65; 32 x 2 after 600: 43 against 34; a 40-token prompt (4 kv heads) 10.3 against 13.0.
-    const float mma_us = chunk_mma_launch_us(*a, window, chunk_config(a->cfg.head_dim).cols_per_item, d->sm_count);
-    // Pairs of SMs take a query tile per CTA: at head_dim 128 a launch that leaves SMs idle ends sooner (a prompt of 512
-    // after 512, 8 kv heads: 19.5 against 31.0 us; four of them after 1024: 92 against 73), at head_dim 256 every launch
-    // of more than some tens of tokens does (8 prompts of 512 after 7680: 236 against 338; one after 512: 24 against 49).
-    if (d->chunk_mode == 5 && chunk_pair_supported(a->cfg.head_dim)) {
-        const TileCut pc{window, 128, 2 * tile_tokens, d->sm_count / 2, d->chunk_split, true};
-        ChunkPlan pairs;
-        build_chunk_tile_plan(*a, 2 * tile_tokens, &pairs, pc);
-        const float pair_us = chunk_tile_launch_us(*a, pairs, pc);
-        // (the one-tile kernel's estimate at head_dim 256 is too low where its short launches are cut: 28 us for the 49 above)
-        if (pair_us < us || a->cfg.head_dim == 256) {
-            pd.pair = true;
-            pd.host = std::move(pairs);
-            cut = pc;
-            us = pair_us;
-        }
-    }
-    pd.mma = mma_us < us;
-    if (!(pd.mma && d->chunk_chooses())) {
-        if (pd.host.n_cut > 0 && !ensure_split(a, st)) {
-            cut.max_parts = 1;
-            build_chunk_tile_plan(*a, pd.pair ? 2 * tile_tokens : tokens_per_item, &pd.host, cut);
+    ChunkChoice c = chunk_choice(*a, d->chunk_mode, window, d->sm_count, d->chunk_split);
+    pd.launch = plan_chunk_launch(*a, c);
+    if (!pd.launch.mma) {
+        if (pd.launch.plan.n_cut > 0 && !ensure_split(a, st)) {
+            const TileCut& cut = pd.launch.pair ? c.pair : c.one;
+            build_chunk_tile_plan(*a, pd.launch.pair ? c.pair_tokens : c.one_tokens, &pd.launch.plan, TileCut{window, cut.kv_tile, cut.tile_tokens, cut.sm_count, 1, cut.pair});
         }
         const void* p = nullptr;
-        int32_t rc = slot_upload(d, pd.host.tiles.data(), pd.host.tiles.size() * sizeof(TileItem), st, &p);
+        int32_t rc = slot_upload(d, pd.launch.plan.tiles.data(), pd.launch.plan.tiles.size() * sizeof(TileItem), st, &p);
         if (rc) return rc;
         pd.tiles = (const TileItem*)p;
     }
-    auto ins = d->tile_plans.emplace(key, std::move(pd));
+    auto ins = d->tile_plans.emplace(window, std::move(pd));
     *out = &ins.first->second;
     return CBKV_OK;
 }
@@ -660,9 +647,9 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
     const int tile_tokens = 128 / rep_slots_of(a->n_rep());
     DeviceState::TilePlanDev* tp = nullptr;
     if (use_tc) {
-        int32_t rc = get_tile_plan(a, w, (use_tc2 ? 2 : 1) * tile_tokens, tile_tokens, !use_tc2 && a->cfg.head_dim == 256 ? 64 : 128, st, &tp);
+        int32_t rc = get_tile_plan(a, w, st, &tp);
         if (rc) return rc;
-        if (tp->mma && d->chunk_chooses()) use_tc = false;
+        if (tp->launch.mma) use_tc = false;
     }
     // int8 pages: decode steps stream the records through the decode kernel; the chunk kernels read a float
     // copy made per layer and step (mode 4: the two-tile kernel converts the records itself, slower so far);
@@ -733,7 +720,7 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
     }
     if (use_tc) {
         ChunkArgs args{};
-        args.step = d->step; args.geo = geom(a); args.tiles = tp->tiles; args.n_items = (int32_t)tp->host.tiles.size();
+        args.step = d->step; args.geo = geom(a); args.tiles = tp->tiles; args.n_items = (int32_t)tp->launch.plan.tiles.size();
         args.q = q; args.out = out; args.status = d->status; args.window = (int32_t)w; args.scale_log2 = scale_log2;
         args.rep_slots = 128 / tile_tokens;
         args.q8_arena = q8_direct ? L.base : nullptr;
@@ -747,7 +734,7 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
 #endif
         ProfScope ps(d, st);
         { int32_t frc = flush_uploads(d, st); if (frc) return frc; }
-        if (tp->pair) CU_TRY(launch_chunk_pair(KV->map_page, KV->map_vhalf, args, bf16, d->pdl, st));
+        if (tp->launch.pair) CU_TRY(launch_chunk_pair(KV->map_page, KV->map_vhalf, args, bf16, d->pdl, st));
         else if (use_tc2) CU_TRY(q8_direct ? launch_chunk_tc2(L.map_k16, L.map_sc, args, bf16, d->pdl, st) : launch_chunk_tc2(KV->map_kv, KV->map_kv, args, bf16, d->pdl, st));
         else CU_TRY(launch_chunk_tc(KV->map_page, args, bf16, d->pdl, st));
         g_launches++;
@@ -1674,6 +1661,24 @@ int64_t cbkv_debug_tile_plan(cbkv_arena* arena, int64_t window, int32_t tokens_p
     std::vector<int32_t> flat = {(int32_t)pl.tiles.size(), pl.n_slots, pl.n_cut};
     const int32_t* tp = reinterpret_cast<const int32_t*>(pl.tiles.data());
     flat.insert(flat.end(), tp, tp + pl.tiles.size() * 8);
+    for (int64_t i = 0; i < (int64_t)flat.size() && i < cap; i++) out[i] = flat[(size_t)i];
+    return (int64_t)flat.size();
+    });
+}
+
+// Host-only view of the choice between the chunk kernels for the step in flight (used by the CPU tests): out = [the kernel
+// as cbkv_set_chunk_kernel numbers it (2 or 3: one or two tiles, 5: pairs of SMs, 1: mma.sync), CTAs run through the launch
+// model to decide, n_ctas, n_slots, n_cut, TileItem records].
+int64_t cbkv_debug_chunk_choice(cbkv_arena* arena, int64_t window, int32_t mode, int32_t sm_count, int32_t max_parts, int32_t* out, int64_t cap) {
+    return fenced64([&]() -> int64_t {
+    Arena* a = reinterpret_cast<Arena*>(arena);
+    if (!a || a->step_meta.empty() || !out || mode < 0 || mode > 5 || mode == 1 || sm_count < 2 || max_parts < 1) return -1;
+    const ChunkChoice c = chunk_choice(*a, mode, window, sm_count, max_parts);
+    const ChunkLaunch l = plan_chunk_launch(*a, c);
+    const int32_t kernel = l.mma ? 1 : l.pair ? 5 : c.one_tokens > c.one.tile_tokens ? 3 : 2;
+    std::vector<int32_t> flat = {kernel, (int32_t)l.modelled, (int32_t)l.plan.tiles.size(), l.plan.n_slots, l.plan.n_cut};
+    const int32_t* tp = reinterpret_cast<const int32_t*>(l.plan.tiles.data());
+    flat.insert(flat.end(), tp, tp + l.plan.tiles.size() * 8);
     for (int64_t i = 0; i < (int64_t)flat.size() && i < cap; i++) out[i] = flat[(size_t)i];
     return (int64_t)flat.size();
     });

@@ -5,7 +5,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
-#include <functional>
+#include <memory>
 
 namespace cbkv {
 
@@ -338,135 +338,6 @@ namespace {
 constexpr float kCtaCost = 3.f, kHalfTile = 0.7f, kSliceCost = 0.7f, kMergeCost = 0.7f;
 constexpr float kPairCtaCost = 5.f, kPairSliceCost = 1.f, kPairMergeCost = 1.f;  // the same for pairs of CTAs, whose K/V tiles are shorter
 
-struct TileWork { int32_t seq, h, qt, n_tiles; float per_tile, rows; };  // an uncut item
-
-// End of the last CTA when `sm_count` SMs take the CTAs in launch order.
-float launch_end(const std::vector<float>& cost, int sm_count, std::vector<float>* heap) {
-    heap->assign((size_t)sm_count, 0.f);
-    float end = 0.f;
-    for (float c : cost) {
-        std::pop_heap(heap->begin(), heap->end(), std::greater<float>());
-        const float e = heap->back() + c;
-        heap->back() = e;
-        std::push_heap(heap->begin(), heap->end(), std::greater<float>());
-        end = std::max(end, e);
-    }
-    return end;
-}
-
-}  // namespace
-
-// CTAs are launched longest (sequence, kv head) first; the items of one (sequence, kv head) stay together, slice
-// by slice, because they read the same K/V.  Whether and how finely items are cut is decided by running the
-// launch model over a few candidates: no cut, the remainder of the last wave cut in equal parts (a launch of
-// several waves whose last is mostly empty), and every item longer than a limit cut into slices of at most that
-// (a launch that has too few items for the chip: a few tokens of a few sequences over long contexts).
-void build_chunk_tile_plan(const Arena& a, int32_t tokens_per_tile, ChunkPlan* pl, const TileCut& cut) {
-    const int n = (int)a.step_meta.size();
-    const int tile_tokens = cut.tile_tokens > 0 ? cut.tile_tokens : tokens_per_tile;
-    const float cta_cost = cut.pair ? kPairCtaCost : kCtaCost, slice_cost = cut.pair ? kPairSliceCost : kSliceCost, merge_cost = cut.pair ? kPairMergeCost : kMergeCost;
-    pl->cols_per_item = tokens_per_tile;
-    pl->item_begin.assign((size_t)n + 1, 0);
-    pl->tiles.clear();
-    pl->n_slots = pl->n_cut = 0;
-    int64_t items = 0;
-    struct Group { int32_t seq, first, n_qt; float cost; };
-    std::vector<TileWork> work;    // of one kv head, per sequence and block of query tokens
-    std::vector<Group> groups;
-    for (int b = 0; b < n; b++) {
-        const SeqMeta& m = a.step_meta[(size_t)b];
-        const int n_qt = (m.snew + tokens_per_tile - 1) / tokens_per_tile;
-        pl->item_begin[(size_t)b] = (int32_t)items;
-        items += (int64_t)a.cfg.n_kv_heads * n_qt;
-        if (n_qt == 0) continue;
-        Group g{b, (int32_t)work.size(), n_qt, 0.f};
-        for (int qt = 0; qt < n_qt; qt++) {
-            const int r0 = qt * tokens_per_tile, toks = std::min(tokens_per_tile, m.snew - r0);
-            const int64_t q_first = m.pos + r0, q_last = q_first + toks - 1;
-            const int64_t lo_key = cut.window > 0 ? std::max<int64_t>(0, q_first - cut.window + 1) : 0;
-            const int32_t pages = (int32_t)((q_last >> 4) - (lo_key >> 4) + 1), ppt = cut.kv_tile / 16;
-            TileWork w{b, 0, qt, (pages + ppt - 1) / ppt, toks > tile_tokens ? 1.f : kHalfTile, (float)toks / (float)tokens_per_tile};
-            if (tile_tokens == tokens_per_tile) w.per_tile = 1.f;  // one query tile per CTA
-            g.cost = std::max(g.cost, w.per_tile * w.n_tiles);
-            work.push_back(w);
-        }
-        groups.push_back(g);
-    }
-    pl->item_begin[(size_t)n] = (int32_t)items;
-    pl->n_items = (int32_t)items;
-    std::stable_sort(groups.begin(), groups.end(), [](const Group& x, const Group& y) { return x.cost > y.cost; });
-
-    // parts of an item: ceil(cost / limit), and for the last `rem` items of the launch order at least rem_parts
-    std::vector<float> cost, heap;
-    auto emit = [&](float limit, int64_t rem, int rem_parts, std::vector<TileItem>* out, int32_t* n_slots, int32_t* n_cut) -> float {
-        cost.clear();
-        int32_t slots = 0, cuts = 0;
-        float merge = 0.f;
-        int64_t at = 0;
-        std::vector<int32_t> parts, base, id;
-        for (const Group& g : groups) {
-            for (int h = 0; h < a.cfg.n_kv_heads; h++) {
-                int most = 1;
-                parts.assign((size_t)g.n_qt, 1); base.assign((size_t)g.n_qt, -1); id.assign((size_t)g.n_qt, -1);
-                for (int qt = 0; qt < g.n_qt; qt++, at++) {
-                    const TileWork& w = work[(size_t)(g.first + qt)];
-                    int p = limit > 0.f ? (int)std::min(1e6f, w.per_tile * (float)w.n_tiles / limit + 0.999f) : 1;
-                    if (at >= items - rem) p = std::max(p, rem_parts);
-                    p = std::max(1, std::min(std::min(p, cut.max_parts), w.n_tiles));
-                    const int per = (w.n_tiles + p - 1) / p;
-                    p = (w.n_tiles + per - 1) / per;  // no empty slices
-                    parts[(size_t)qt] = p;
-                    most = std::max(most, p);
-                    if (p > 1) {
-                        base[(size_t)qt] = slots; id[(size_t)qt] = cuts;
-                        slots += p; cuts++;
-                        merge = std::max(merge, merge_cost * (0.5f + (float)p * w.rows));
-                    }
-                }
-                for (int p = 0; p < most; p++)
-                    for (int qt = 0; qt < g.n_qt; qt++) {
-                        const int np = parts[(size_t)qt];
-                        if (p >= np) continue;
-                        const TileWork& w = work[(size_t)(g.first + qt)];
-                        const int per = (w.n_tiles + np - 1) / np, t0 = p * per, t1 = std::min(w.n_tiles, t0 + per);
-                        if (out) out->push_back({g.seq, h, qt, t0, t1, p | (np << 16), base[(size_t)qt], id[(size_t)qt]});
-                        else cost.push_back(cta_cost + w.per_tile * (float)(t1 - t0) + (np > 1 ? slice_cost : 0.f));
-                    }
-            }
-        }
-        if (n_slots) { *n_slots = slots; *n_cut = cuts; }
-        if (out) return 0.f;
-        return slots > kSplitSlotsPerSm * cut.sm_count ? INFINITY : launch_end(cost, cut.sm_count, &heap) + merge;
-    };
-
-    float limit = 0.f;
-    int64_t rem = 0;
-    int rem_parts = 1;
-    if (cut.sm_count > 0 && cut.max_parts > 1 && items > 0 && items <= 8192) {
-        float best = emit(0.f, 0, 1, nullptr, nullptr, nullptr);
-        const int64_t r = items % cut.sm_count;
-        if (items > cut.sm_count && r > 0)
-            for (int p = 2; p <= std::min<int64_t>(4, cut.sm_count / r); p++) {
-                const float e = emit(0.f, r, p, nullptr, nullptr, nullptr);
-                if (e < best) { best = e; rem = r; rem_parts = p; limit = 0.f; }
-            }
-        double total = 0.;
-        float longest = 0.f;
-        for (const TileWork& w : work) { total += (double)w.per_tile * w.n_tiles; longest = std::max(longest, w.per_tile * w.n_tiles); }
-        const float even = (float)(total * a.cfg.n_kv_heads / cut.sm_count);  // tiles per SM
-        if (items <= 4 * cut.sm_count)
-            for (float f : {1.3f, 1.f, 0.75f, 0.5f, 0.35f}) {
-                const float lim = std::max(1.f, even * f);
-                if (lim >= longest) continue;
-                const float e = emit(lim, 0, 1, nullptr, nullptr, nullptr);
-                if (e < best) { best = e; limit = lim; rem = 0; rem_parts = 1; }
-            }
-    }
-    emit(limit, rem, rem_parts, &pl->tiles, &pl->n_slots, &pl->n_cut);
-}
-
-namespace {
-
 // Measured per head_dim over batches of 1 to 64 sequences with 33 to 2000 cached tokens (GQA groups of 2 to 7, f16):
 // a tcgen05 launch takes fixed_us, then per wave of one CTA per SM cta_us + tile_us for each K/V tile (head_dim 128:
 // [0] with one query tile, [1] with both); the mma.sync kernel, one warp per item over all its pages, mma_us + page_us
@@ -483,18 +354,253 @@ ChunkTimes chunk_times(int32_t d) {
     }
 }
 
+// SMs that take CTAs in launch order, each the next one that is free: a heap of the times at which they are, padded so that
+// every inner node has two children and the way down has no branch but its end.
+class Sms {
+public:
+    void start(int n) {
+        n_ = (size_t)n;
+        taken_ = 0;
+        end_ = 0.f;
+        free_at_.clear();
+    }
+    void run(float us) {
+        if (taken_ < n_) {  // an idle SM
+            free_at_.push_back(us);
+            end_ = std::max(end_, us);
+            if (++taken_ == n_) {
+                std::make_heap(free_at_.begin(), free_at_.end(), [](float x, float y) { return x > y; });
+                free_at_.resize(2 * n_ + 1, INFINITY);
+            }
+            return;
+        }
+        float* f = free_at_.data();
+        const float t = f[0] + us;
+        end_ = std::max(end_, t);
+        size_t i = 0;
+        while (i < n_) {
+            const size_t c = 2 * i + 1 + (f[2 * i + 2] < f[2 * i + 1] ? 1 : 0);
+            if (!(f[c] < t)) break;
+            f[i] = f[c];
+            i = c;
+        }
+        f[i] = t;
+    }
+    float end() const { return end_; }
+
+private:
+    std::vector<float> free_at_;
+    size_t n_ = 0, taken_ = 0;
+    float end_ = 0.f;
+};
+
+// CTAs are launched longest (sequence, kv head) first; the items of one (sequence, kv head) stay together, slice
+// by slice, because they read the same K/V.  Whether and how finely items are cut is decided by running the
+// launch model over a few candidates: no cut, the remainder of the last wave cut in equal parts (a launch of
+// several waves whose last is mostly empty), and every item longer than a limit cut into slices of at most that
+// (a launch that has too few items for the chip: a few tokens of a few sequences over long contexts).
+//
+// This runs on the host in front of a step's first chunk launch, once per window, so what it costs is seen by steps of
+// few layers: the kv heads of a sequence share everything but their place in the order, and a candidate whose work
+// divided evenly would already end later than the best so far is not run through the model.
+class TilePlanner {
+public:
+    TilePlanner(const Arena& a, int32_t tokens_per_tile, const TileCut& cut)
+        : a_(a), cut_(cut), tokens_(tokens_per_tile), tile_tokens_(cut.tile_tokens > 0 ? cut.tile_tokens : tokens_per_tile) {
+        const int n = (int)a.step_meta.size();
+        item_begin_.assign((size_t)n + 1, 0);
+        for (int b = 0; b < n; b++) {
+            const SeqMeta& m = a.step_meta[(size_t)b];
+            const int n_qt = (m.snew + tokens_ - 1) / tokens_;
+            item_begin_[(size_t)b] = (int32_t)items_;
+            items_ += (int64_t)a.cfg.n_kv_heads * n_qt;
+            if (n_qt == 0) continue;
+            Group g{b, (int32_t)work_.size(), n_qt, 0.f};
+            for (int qt = 0; qt < n_qt; qt++) {
+                const int r0 = qt * tokens_, toks = std::min(tokens_, m.snew - r0);
+                const int64_t q_first = m.pos + r0, q_last = q_first + toks - 1;
+                const int64_t lo_key = cut.window > 0 ? std::max<int64_t>(0, q_first - cut.window + 1) : 0;
+                const int32_t pages = (int32_t)((q_last >> 4) - (lo_key >> 4) + 1), ppt = cut.kv_tile / 16;
+                const bool both = toks > tile_tokens_;
+                // one query tile per CTA: the same for every item
+                Work w{(pages + ppt - 1) / ppt, both || tile_tokens_ == tokens_ ? 1.f : kHalfTile, (float)toks / (float)tokens_, both ? 1 : 0};
+                g.cost = std::max(g.cost, w.per_tile * w.n_tiles);
+                work_.push_back(w);
+            }
+            groups_.push_back(g);
+        }
+        item_begin_[(size_t)n] = (int32_t)items_;
+        std::stable_sort(groups_.begin(), groups_.end(), [](const Group& x, const Group& y) { return x.cost > y.cost; });
+    }
+
+    // How the items are cut: the candidate that ends first.
+    void choose() {
+        how_ = How{};
+        if (!(cut_.sm_count > 0 && cut_.max_parts > 1 && items_ > 0 && items_ <= 8192)) return;
+        float best = end_of(How{}, INFINITY);
+        auto consider = [&](const How& how) {
+            const float e = end_of(how, best);
+            if (e < best) { best = e; how_ = how; }
+        };
+        const int64_t r = items_ % cut_.sm_count;
+        if (items_ > cut_.sm_count && r > 0)
+            for (int p = 2; p <= std::min<int64_t>(4, cut_.sm_count / r); p++) consider(How{0.f, r, p});
+        if (items_ > 4 * cut_.sm_count) return;
+        double total = 0.;
+        float longest = 0.f;
+        for (const Work& w : work_) { total += (double)w.per_tile * w.n_tiles; longest = std::max(longest, w.per_tile * (float)w.n_tiles); }
+        const float even = (float)(total * a_.cfg.n_kv_heads / cut_.sm_count);  // tiles per SM
+        for (float f : {1.3f, 1.f, 0.75f, 0.5f, 0.35f}) {
+            const float lim = std::max(1.f, even * f);
+            if (lim < longest) consider(How{lim, 0, 1});
+        }
+    }
+
+    // Expected time of the launch in microseconds, and what it cannot be below however its items are cut.
+    float launch_us() {
+        const ChunkTimes t = chunk_times(a_.cfg.head_dim);
+        sms_.start(cut_.sm_count);
+        each_cta(how_, [&](const Work& w, int, int, int, int tiles, int, int) { sms_.run(cta_us(t, w, tiles)); modelled_++; });
+        return kChunkFixedUs + sms_.end();
+    }
+    float least_us() const {
+        const ChunkTimes t = chunk_times(a_.cfg.head_dim);
+        double total = 0.;
+        float shortest = INFINITY;
+        for (const Work& w : work_) { total += cta_us(t, w, w.n_tiles); shortest = std::min(shortest, cta_us(t, w, 1)); }
+        return work_.empty() ? 0.f : 0.999f * (kChunkFixedUs + std::max(shortest, (float)(total * a_.cfg.n_kv_heads / cut_.sm_count)));
+    }
+
+    void emit(ChunkPlan* pl) {
+        pl->cols_per_item = tokens_;
+        pl->item_begin = item_begin_;
+        pl->n_items = (int32_t)items_;
+        pl->tiles.clear();
+        pl->n_slots = pl->n_cut = 0;
+        std::vector<int32_t> base, id;  // of the current (sequence, kv head), by block of query tokens
+        each_cta(how_, [&](const Work& w, int seq, int h, int qt, int tiles, int part, int parts) {
+            if (part == 0) {
+                base.resize(std::max(base.size(), (size_t)qt + 1)); id.resize(base.size());
+                base[(size_t)qt] = parts > 1 ? pl->n_slots : -1; id[(size_t)qt] = parts > 1 ? pl->n_cut : -1;
+                if (parts > 1) { pl->n_slots += parts; pl->n_cut++; }
+            }
+            const int t0 = part * ((w.n_tiles + parts - 1) / parts);
+            pl->tiles.push_back({seq, h, qt, t0, t0 + tiles, part | (parts << 16), base[(size_t)qt], id[(size_t)qt]});
+        });
+    }
+
+    int64_t modelled() const { return modelled_; }
+
+private:
+    struct Work { int32_t n_tiles; float per_tile, rows; int32_t both; };  // an uncut item, the same for every kv head
+    struct Group { int32_t seq, first, n_qt; float cost; };
+    // parts of an item: ceil(cost / limit), and for the last `rem` items of the launch order at least rem_parts
+    struct How { float limit = 0.f; int64_t rem = 0; int rem_parts = 1; };
+
+    float cta_us(const ChunkTimes& t, const Work& w, int tiles) const {
+        return cut_.pair ? t.pair_cta_us + t.pair_tile_us * (float)tiles : t.cta_us[w.both] + t.tile_us[w.both] * (float)tiles;
+    }
+
+    int parts_of(const Work& w, const How& how, bool tail) const {
+        int p = how.limit > 0.f ? (int)std::min(1e6f, w.per_tile * (float)w.n_tiles / how.limit + 0.999f) : 1;
+        if (tail) p = std::max(p, how.rem_parts);
+        p = std::max(1, std::min(std::min(p, cut_.max_parts), w.n_tiles));
+        const int per = (w.n_tiles + p - 1) / p;
+        return (w.n_tiles + per - 1) / per;  // no empty slices
+    }
+
+    // f(item, sequence, kv head, block of query tokens, its K/V tiles, part, parts) of every CTA in launch order
+    template <typename F>
+    void each_cta(const How& how, F&& f) {
+        int64_t at = 0;
+        for (const Group& g : groups_) {
+            int most = 1;
+            for (int h = 0; h < a_.cfg.n_kv_heads; h++, at += g.n_qt) {
+                if (h == 0 || (how.rem > 0 && at + g.n_qt > items_ - how.rem)) {  // the heads share their cut up to the tail
+                    parts_.resize((size_t)g.n_qt);
+                    most = 1;
+                    for (int qt = 0; qt < g.n_qt; qt++)
+                        most = std::max(most, parts_[(size_t)qt] = parts_of(work_[(size_t)(g.first + qt)], how, at + qt >= items_ - how.rem));
+                }
+                for (int p = 0; p < most; p++)
+                    for (int qt = 0; qt < g.n_qt; qt++) {
+                        const int np = parts_[(size_t)qt];
+                        if (p >= np) continue;
+                        const Work& w = work_[(size_t)(g.first + qt)];
+                        const int per = (w.n_tiles + np - 1) / np;
+                        f(w, g.seq, h, qt, std::min(w.n_tiles, (p + 1) * per) - p * per, p, np);
+                    }
+            }
+        }
+    }
+
+    // When the launch ends, in the model's units, or infinity when that is not before `best` or takes too many slots.
+    float end_of(const How& how, float best) {
+        const float cta_cost = cut_.pair ? kPairCtaCost : kCtaCost, slice_cost = cut_.pair ? kPairSliceCost : kSliceCost,
+                    merge_cost = cut_.pair ? kPairMergeCost : kMergeCost;
+        float merge = 0.f, longest = 0.f;
+        int64_t slots = 0;
+        if (how.rem == 0) {  // what one kv head says about all of them
+            double total = 0.;
+            for (const Work& w : work_) {
+                const int np = parts_of(w, how, false), per = (w.n_tiles + np - 1) / np;
+                if (np > 1) { slots += np; merge = std::max(merge, merge_cost * (0.5f + (float)np * w.rows)); }
+                total += w.per_tile * (double)w.n_tiles + np * (double)(cta_cost + (np > 1 ? slice_cost : 0.f));
+                longest = std::max(longest, cta_cost + w.per_tile * (float)per + (np > 1 ? slice_cost : 0.f));
+            }
+            if (slots * a_.cfg.n_kv_heads > (int64_t)kSplitSlotsPerSm * cut_.sm_count) return INFINITY;
+            if (std::max(longest, 0.999f * (float)(total * a_.cfg.n_kv_heads / cut_.sm_count)) + merge >= best) return INFINITY;
+        }
+        sms_.start(cut_.sm_count);
+        slots = 0;
+        each_cta(how, [&](const Work& w, int, int, int, int tiles, int part, int parts) {
+            if (part == 0 && parts > 1) { slots += parts; merge = std::max(merge, merge_cost * (0.5f + (float)parts * w.rows)); }
+            sms_.run(cta_cost + w.per_tile * (float)tiles + (parts > 1 ? slice_cost : 0.f));
+            modelled_++;
+        });
+        return slots > (int64_t)kSplitSlotsPerSm * cut_.sm_count ? INFINITY : sms_.end() + merge;
+    }
+
+    const Arena& a_;
+    const TileCut cut_;
+    const int32_t tokens_, tile_tokens_;
+    int64_t items_ = 0, modelled_ = 0;
+    std::vector<int32_t> item_begin_, parts_;
+    std::vector<Work> work_;  // per sequence and block of query tokens
+    std::vector<Group> groups_;
+    How how_;
+    Sms sms_;
+};
+
 }  // namespace
 
-float chunk_tile_launch_us(const Arena& a, const ChunkPlan& pl, const TileCut& cut) {
-    const ChunkTimes t = chunk_times(a.cfg.head_dim);
-    std::vector<float> cost, heap;
-    cost.reserve(pl.tiles.size());
-    for (const TileItem& w : pl.tiles) {
-        const int both = a.step_meta[(size_t)w.seq].snew - w.qt * pl.cols_per_item > cut.tile_tokens ? 1 : 0;
-        if (cut.pair) cost.push_back(t.pair_cta_us + t.pair_tile_us * (float)(w.t1 - w.t0));
-        else cost.push_back(t.cta_us[both] + t.tile_us[both] * (float)(w.t1 - w.t0));
+void build_chunk_tile_plan(const Arena& a, int32_t tokens_per_tile, ChunkPlan* pl, const TileCut& cut) {
+    TilePlanner p(a, tokens_per_tile, cut);
+    p.choose();
+    p.emit(pl);
+}
+
+ChunkLaunch plan_chunk_launch(const Arena& a, const ChunkChoice& c) {
+    ChunkLaunch out;
+    const float mma_us = c.mma_cols > 0 ? chunk_mma_launch_us(a, c.one.window, c.mma_cols, c.one.sm_count) : INFINITY;
+    // Head_dim 256 takes pairs at every size; see chunk_times for head_dim 128.
+    const bool only_pairs = c.pairs && (c.one_tokens == 0 || a.cfg.head_dim == 256);
+    std::unique_ptr<TilePlanner> one, two;
+    float least = INFINITY;
+    if (!only_pairs) { one.reset(new TilePlanner(a, c.one_tokens, c.one)); if (c.chooses()) least = one->least_us(); }
+    if (c.pairs) { two.reset(new TilePlanner(a, c.pair_tokens, c.pair)); if (c.chooses()) least = std::min(least, two->least_us()); }
+    if (mma_us < least) { out.mma = true; return out; }  // whatever a plan would say
+    float us = INFINITY;
+    if (one) { one->choose(); if (c.chooses()) us = one->launch_us(); }
+    if (two && two->least_us() < us) {
+        two->choose();
+        const float pair_us = c.chooses() ? two->launch_us() : 0.f;
+        if (pair_us < us) { out.pair = true; us = pair_us; }
     }
-    return kChunkFixedUs + launch_end(cost, cut.sm_count, &heap);
+    out.modelled = (one ? one->modelled() : 0) + (two ? two->modelled() : 0);
+    out.mma = mma_us < us;
+    if (!out.mma) (out.pair ? two : one)->emit(&out.plan);
+    return out;
 }
 
 float chunk_mma_launch_us(const Arena& a, int64_t window, int32_t cols_per_item, int32_t sm_count) {

@@ -188,9 +188,23 @@ void build_chunk_plan(const Arena& a, int32_t cols_per_item, ChunkPlan* plan);
 // `tokens_per_tile` new tokens); `cols_per_item` records tokens_per_tile.
 void build_chunk_tile_plan(const Arena& a, int32_t tokens_per_tile, ChunkPlan* plan, const TileCut& cut = TileCut());
 
-// Expected times of a chunk step's launch (append included), in microseconds: of the tcgen05 kernel that runs `plan`
-// (made by build_chunk_tile_plan with `cut`), and of the mma.sync kernel.
-float chunk_tile_launch_us(const Arena& a, const ChunkPlan& plan, const TileCut& cut);
+// Which kernels a chunk step's launch is chosen among, and its work list when the choice is a tcgen05 kernel.
+struct ChunkChoice {
+    int32_t one_tokens = 0;   // tokens per item of the one- or two-tile kernel, 0 = not a candidate
+    TileCut one;
+    bool pairs = false;       // pairs of SMs are a candidate
+    int32_t pair_tokens = 0;
+    TileCut pair;
+    int32_t mma_cols = 0;     // columns per item of the mma.sync kernel, 0 = not a candidate
+    bool chooses() const { return mma_cols > 0 || (pairs && one_tokens > 0); }
+};
+struct ChunkLaunch {
+    bool mma = false, pair = false;
+    ChunkPlan plan;
+    int64_t modelled = 0;     // CTAs that were run through the launch model to decide: what the decision cost
+};
+ChunkLaunch plan_chunk_launch(const Arena& a, const ChunkChoice& choice);
+// Expected time of the mma.sync kernel's launch (append included), in microseconds.
 float chunk_mma_launch_us(const Arena& a, int64_t window, int32_t cols_per_item, int32_t sm_count);
 
 }  // namespace cbkv

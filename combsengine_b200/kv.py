@@ -376,6 +376,17 @@ class KVArena:
         a = np.frombuffer(buf, dtype=np.int32, count=n).copy()
         return {"n_ctas": int(a[0]), "n_slots": int(a[1]), "n_cut": int(a[2]), "tiles": a[3:].reshape(-1, 8)}
 
+    def debug_chunk_choice(self, window: int = 0, mode: int = 5, sm_count: int = 148, max_parts: int = 64) -> dict:
+        """Which chunk kernel the step in flight takes and what deciding costs (host only, see include/combs_kv.h)."""
+        cap = 1 << 20
+        buf = (C.c_int32 * cap)()
+        n = self._lib.cbkv_debug_chunk_choice(self._h, window, mode, sm_count, max_parts, buf, cap)
+        if n < 0 or n > cap:
+            raise CbkvError(-6, "no step in flight or plan too large")
+        a = np.frombuffer(buf, dtype=np.int32, count=n).copy()
+        return {"kernel": int(a[0]), "modelled": int(a[1]), "n_ctas": int(a[2]), "n_slots": int(a[3]), "n_cut": int(a[4]),
+                "tiles": a[5:].reshape(-1, 8)}
+
 
 def static_status(stream: Optional[torch.cuda.Stream] = None) -> int:
     """Status word of the last ``decode_attention_static`` call on the current device (0 = clean); waits for

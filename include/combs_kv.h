@@ -381,6 +381,13 @@ int64_t cbkv_debug_decode_plan(cbkv_arena* arena, int64_t window, int32_t n_ctas
 int64_t cbkv_debug_tile_plan(cbkv_arena* arena, int64_t window, int32_t tokens_per_item, int32_t tile_tokens, int32_t kv_tile,
                              int32_t sm_count, int32_t max_parts, int32_t* out, int64_t cap);
 
+/* The choice between the chunk kernels for the step in flight, as cbkv_set_chunk_kernel(mode) would have it
+ * made on `sm_count` SMs with at most `max_parts` slices per item: [kernel (1 = mma.sync, 2 / 3 = one / two
+ * tiles per CTA, 5 = pairs of SMs), CTAs that were run through the launch model to decide, n_ctas, n_slots,
+ * n_cut, records as above (none for mma.sync)].  Returns the number of words, or -1 without a step. */
+int64_t cbkv_debug_chunk_choice(cbkv_arena* arena, int64_t window, int32_t mode, int32_t sm_count, int32_t max_parts,
+                                int32_t* out, int64_t cap);
+
 /* Tuning (no reference counterpart): the share of a CTA's range that is cut into dynamically
  * claimed tail items (percent), the smallest item (pages; 0 = no tail, a static equal split) and
  * the number of halvings + 2.  Negative / < 2 = keep. */

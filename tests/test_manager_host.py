@@ -359,3 +359,20 @@ def test_tile_plans_never_need_more_slots_than_the_buffers_have(sms):
                 for tokens, tile, kv_tile in ((32, 16, 128), (16, 16, 128), (64, 64, 64)):
                     pl = a.debug_tile_plan(window, tokens, tile, kv_tile, sms)
                     assert pl["n_slots"] <= 4 * sms and pl["n_cut"] <= 2 * sms
+
+
+@pytest.mark.parametrize("n_q,n_kv,d,n_seqs,new,lo,hi,kernel,most", [
+    (32, 8, 128, 64, 3, 40, 100, 1, 0), (8, 4, 256, 64, 3, 100, 1000, 1, 0), (32, 8, 128, 32, 3, 100, 1000, 3, 512),
+    (28, 4, 128, 64, 5, 100, 3000, 3, 800), (32, 8, 128, 8, 5, 512, 6144, 3, 1496), (32, 8, 128, 1, 512, 512, 512, 5, 800)])
+def test_a_chunk_kernel_is_chosen_without_modelling_every_launch(n_q, n_kv, d, n_seqs, new, lo, hi, kernel, most):
+    # CTAs run through the launch model, which the host does in front of a step's first launch: none where the mma.sync
+    # kernel is below what any plan could reach, and no more than the plan of one kernel takes when every candidate of its
+    # cut is run (1536, 2084, 1816, 2088, 1496 and 1392; 1024, 1158, 1162, 1426, 928 and 848 more for pairs)
+    lens = [int(lo + (i + 1) * 0.618 % 1 * (hi - lo)) for i in range(n_seqs)]
+    a = KVArena(1, n_q, n_kv, d, 8192, 16, 16384)
+    seqs = [a.new_seq() for _ in lens]
+    a.begin_step_host_only(seqs, lens)
+    a.begin_step_host_only(seqs, [new] * n_seqs)
+    got = a.debug_chunk_choice()
+    assert got["kernel"] == kernel and got["modelled"] <= most
+    assert (got["n_ctas"] > 0) == (kernel != 1)
