@@ -18,7 +18,6 @@ NVCC_FLAGS = [
 ]
 
 
-PYCALL = os.path.join(HERE, "_pycall.so")  # the Python mirror's hot calls (csrc/pycall.cpp)
 PYCALL_SOURCE = os.path.join(CSRC, "pycall.cpp")
 
 
@@ -41,7 +40,6 @@ def build(force: bool = False, verbose: bool = False, measure: bool = False) -> 
     """The product library, or (measure=True) the measurement flavour: the same sources with
     -DCBKV_MEASURE, which adds timers and phase switches the product build does not contain."""
     lib = LIB_MEASURE if measure else LIB
-    build_pycall(force)
     if not force and not needs_build(lib):
         return lib
     cmd = [_nvcc(), *NVCC_FLAGS, *( ["-DCBKV_MEASURE"] if measure else []), "-ccbin", "/usr/bin/g++",
@@ -56,19 +54,32 @@ def build(force: bool = False, verbose: bool = False, measure: bool = False) -> 
     return lib
 
 
+def pycall_path() -> str:
+    """The Python mirror's hot calls (csrc/pycall.cpp).  The file is bound to torch's C++ and to CPython's binary interface, so
+    its name carries both versions: another torch or Python finds no file of its own instead of one that does not load."""
+    import torch
+    return os.path.join(HERE, f"_pycall.torch-{torch.__version__}{sysconfig.get_config_var('EXT_SUFFIX')}")
+
+
 def build_pycall(force: bool = False) -> str:
-    if not force and os.path.exists(PYCALL) and os.path.getmtime(PYCALL) >= os.path.getmtime(PYCALL_SOURCE):
-        return PYCALL
+    """Needs torch and Python's headers, unlike the library; without the file the same calls go through ctypes."""
+    path = pycall_path()
+    if not force and os.path.exists(path) and os.path.getmtime(path) >= os.path.getmtime(PYCALL_SOURCE):
+        return path
     import torch
     root = os.path.dirname(torch.__file__)
     cmd = ["/usr/bin/g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-w", "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(root, "include"),
            "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"), "-I/usr/local/cuda/include", PYCALL_SOURCE,
-           "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-o", PYCALL]
+           "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-o", path]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("g++ failed:\n" + r.stdout + r.stderr)
-    return PYCALL
+    return path
 
 
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="-v" in sys.argv, measure="--measure" in sys.argv))
+    try:
+        print(build_pycall(force="--force" in sys.argv))
+    except (ImportError, RuntimeError) as e:
+        print(f"not built, the Python calls go through ctypes: {e}")

@@ -6,6 +6,8 @@ machine without a B200 every compute call returns an error.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -135,22 +137,28 @@ def load() -> C.CDLL:
     return lib
 
 
-_native = None
+_native = None  # False: there is none
 
 
 def native():
-    """csrc/pycall.cpp, bound to the loaded library: the calls a layer or a step makes, without ctypes."""
+    """csrc/pycall.cpp, bound to the loaded library: the calls a layer or a step makes, without ctypes.  None where the
+    file for this torch and Python is missing: the callers go through ctypes then, slower on the host and to the same
+    kernels."""
     global _native
     if _native is None:
-        import torch  # noqa: F401  (its libraries have to be there first)
-        if not os.path.exists(os.path.join(HERE, "_pycall.so")):
-            raise ImportError("_pycall.so is missing: build it with `python -m combsengine_b200._build`")
-        from . import _pycall
-        lib = load()
-        _pycall.bind(*(C.cast(getattr(lib, f), C.c_void_p).value
+        from ._build import pycall_path  # imports torch, whose libraries have to be there first
+        path = pycall_path()
+        if not os.path.exists(path):
+            _native = False
+        else:
+            loader = importlib.machinery.ExtensionFileLoader("_pycall", path)
+            mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_pycall", loader))
+            loader.exec_module(mod)
+            lib = load()
+            mod.bind(*(C.cast(getattr(lib, f), C.c_void_p).value
                        for f in ("cbkv_attention", "cbkv_attention_rope", "cbkv_begin_step", "cbkv_popn")))
-        _native = _pycall
-    return _native
+            _native = mod
+    return _native or None
 
 
 class CbkvError(RuntimeError):

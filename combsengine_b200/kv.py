@@ -93,10 +93,11 @@ class PagedSeq:
 
     def popn(self, n: int) -> int:
         """kv.rs:807-835: tokens actually dropped; 0 = refused."""
-        r = self.arena._native.popn(self._h, n)
-        if type(r) is tuple:
-            check(r[0])
-            return r[1]
+        if self.arena._native is not None:
+            r = self.arena._native.popn(self._h, n)
+            if type(r) is tuple:
+                check(r[0])
+                return r[1]
         popped = C.c_int64(0)
         check(self.arena._lib.cbkv_popn(self._h, n, C.byref(popped)))
         return popped.value
@@ -190,11 +191,12 @@ class KVArena:
 
     def begin_step(self, seqs: Sequence[PagedSeq], new_tokens: Sequence[int], pos: Optional[Sequence[int]] = None,
                    stream: Optional[torch.cuda.Stream] = None) -> None:
-        r = self._native.begin_step(self._h, seqs, new_tokens, pos, stream)
-        if type(r) is tuple:
-            check(r[0])
-            self.step_tokens = r[1]
-            return
+        if self._native is not None:
+            r = self._native.begin_step(self._h, seqs, new_tokens, pos, stream)
+            if type(r) is tuple:
+                check(r[0])
+                self.step_tokens = r[1]
+                return
         n, hs, nt, ps = self._step_args(seqs, new_tokens, pos)
         check(self._lib.cbkv_begin_step(self._h, hs, nt, ps, n, _stream_ptr(stream)))
         self.step_tokens = int(sum(int(x) for x in new_tokens))
@@ -215,12 +217,13 @@ class KVArena:
                   window: Optional[int] = None, out: Optional[torch.Tensor] = None,
                   stream: Optional[torch.cuda.Stream] = None) -> torch.Tensor:
         """attention_opts for every sequence of the step: append + attention (kv.rs:655-791)."""
-        t = self.step_tokens * self.head_dim
-        r = self._native.attention(self._h, layer, q, k, v, out, scale, window, stream, self._bf16, t * self.n_q_heads, t * self.n_kv_heads)
-        if type(r) is not int:
-            return r
-        if r != self._native.SLOW:
-            check(r)
+        if self._native is not None:
+            t = self.step_tokens * self.head_dim
+            r = self._native.attention(self._h, layer, q, k, v, out, scale, window, stream, self._bf16, t * self.n_q_heads, t * self.n_kv_heads)
+            if type(r) is not int:
+                return r
+            if r != self._native.SLOW:
+                check(r)
         self._chk(q, self.n_q_heads, "q"); self._chk(k, self.n_kv_heads, "k"); self._chk(v, self.n_kv_heads, "v")
         if out is None:
             out = torch.empty_like(q)

@@ -139,12 +139,13 @@ def attention_rope(arena: KVArena, layer: int, rope: RotaryEmbedding, q: torch.T
     """llama.rs:275-289 for one layer: QK norm, rotation, append, attention."""
     ns = norm._struct(arena) if norm is not None else None
     native, t = arena._native, arena.step_tokens * arena.head_dim
-    r = native.attention_rope(arena._h, layer, rope._h, 0 if ns is None else C.addressof(ns), q, k, v, out, scale, window, stream,
-                              arena._bf16, t * arena.n_q_heads, t * arena.n_kv_heads)
-    if type(r) is not int:
-        return r
-    if r != native.SLOW:
-        check(r)
+    if native is not None:
+        r = native.attention_rope(arena._h, layer, rope._h, 0 if ns is None else C.addressof(ns), q, k, v, out, scale, window, stream,
+                                  arena._bf16, t * arena.n_q_heads, t * arena.n_kv_heads)
+        if type(r) is not int:
+            return r
+        if r != native.SLOW:
+            check(r)
     arena._chk(q, arena.n_q_heads, "q"); arena._chk(k, arena.n_kv_heads, "k"); arena._chk(v, arena.n_kv_heads, "v")
     if out is None:
         out = torch.empty_like(q)

@@ -20,7 +20,9 @@ def _built_oracle():
 
 @pytest.fixture(scope="session", autouse=True)
 def _built_library():
-    # a fresh checkout has no libcombskv.so (built artefacts are not tracked): compile it once, where nvcc exists
+    # a fresh checkout has neither of the two (built artefacts are not tracked): compile them once, where nvcc exists
     from combsengine_b200 import _build
     if not os.path.exists(_build.LIB):
         _build.build()
+    if not os.path.exists(_build.pycall_path()):
+        _build.build_pycall()
