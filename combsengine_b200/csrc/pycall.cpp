@@ -132,15 +132,18 @@ PyObject* begin_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     try {
         if (n != 5 || !as_ptr(a[0], &arena) || !PyList_Check(a[1]) || !PyList_Check(a[2]) || (a[3] != Py_None && !PyList_Check(a[3]))) return slow();
         const Py_ssize_t m = PyList_GET_SIZE(a[1]);
-        if (PyList_GET_SIZE(a[2]) != m || (a[3] != Py_None && PyList_GET_SIZE(a[3]) != m)) return slow();
+        auto same_length = [&] { return PyList_GET_SIZE(a[1]) == m && PyList_GET_SIZE(a[2]) == m && (a[3] == Py_None || PyList_GET_SIZE(a[3]) == m); };
+        if (!same_length()) return slow();
         std::vector<void*> seqs((size_t)m + 1);
         std::vector<int64_t> news((size_t)m + 1), pos((size_t)m + 1);
         int64_t total = 0;
         for (Py_ssize_t i = 0; i < m; i++) {
-            PyObject* h = PyObject_GetAttr(PyList_GET_ITEM(a[1], i), handle_name);
+            PyObject* s = Py_NewRef(PyList_GET_ITEM(a[1], i));
+            PyObject* h = PyObject_GetAttr(s, handle_name);  // may run Python code, and that may change the lists
             const bool ok = h && as_ptr(h, &seqs[(size_t)i]);
             Py_XDECREF(h);
-            if (!ok || PyList_GET_SIZE(a[1]) != m || !as_int(PyList_GET_ITEM(a[2], i), &news[(size_t)i])) return slow();
+            Py_DECREF(s);
+            if (!ok || !same_length() || !as_int(PyList_GET_ITEM(a[2], i), &news[(size_t)i])) return slow();
             if (a[3] != Py_None && !as_int(PyList_GET_ITEM(a[3], i), &pos[(size_t)i])) return slow();
             total += news[(size_t)i];
         }
