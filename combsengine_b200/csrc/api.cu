@@ -109,7 +109,7 @@ struct DeviceState {
     const int32_t* chunk_item_begin = nullptr;
     bool tc_ok = false;       // the tcgen05 chunk kernel covers this geometry
     // cbkv_set_chunk_kernel: 0 = choose between 1 and the tcgen05 kernels 2 and 3, 1 = mma.sync, 2 = tcgen05 one tile, 3 = two
-    // tiles, 4 = two tiles, int8 records converted in the kernel, 5 = as 0, and pairs of SMs
+    // tiles, 4 = two tiles, int8 records converted in the kernel, 5 = as 0, and pairs of SMs, 6 = pairs of SMs
     int chunk_mode = 5;
     struct TilePlanDev {
         ChunkLaunch launch;
@@ -552,9 +552,9 @@ ChunkChoice chunk_choice(const Arena& a, int mode, int64_t window, int sm_count,
     const int D = a.cfg.head_dim, tile_tokens = 128 / rep_slots_of(a.n_rep());
     const bool two_tiles = chunk_tc2_supported(D) && mode != 2;
     ChunkChoice c;
-    c.one_tokens = (two_tiles ? 2 : 1) * tile_tokens;
+    c.one_tokens = mode == 6 ? 0 : (two_tiles ? 2 : 1) * tile_tokens;
     c.one = TileCut{window, !two_tiles && D == 256 ? 64 : 128, tile_tokens, sm_count, max_parts};
-    c.pairs = mode == 5 && chunk_pair_supported(D);
+    c.pairs = (mode == 5 || mode == 6) && chunk_pair_supported(D);
     c.pair_tokens = 2 * tile_tokens;
     c.pair = TileCut{window, 128, 2 * tile_tokens, sm_count / 2, max_parts, true};
     if (mode == 0 || mode == 5) c.mma_cols = chunk_config(D).cols_per_item;
@@ -1613,11 +1613,14 @@ int32_t cbkv_set_chunk_split(cbkv_arena* arena, int32_t max_parts) {
 int32_t cbkv_set_chunk_kernel(cbkv_arena* arena, int32_t mode) {
     return fenced([&]() -> int32_t {
     Arena* a = reinterpret_cast<Arena*>(arena);
-    if (!a || mode < 0 || mode > 5) { set_error("bad argument"); return CBKV_ERR_ARG; }
+    if (!a || mode < 0 || mode > 6) { set_error("bad argument"); return CBKV_ERR_ARG; }
     int32_t rc = ensure_device(a);
     if (rc) return rc;
     if ((mode == 3 || mode == 4) && !(dev_of(a)->tc_ok && chunk_tc2_supported(a->cfg.head_dim))) {
         set_error("the two-tile tensor-core chunk kernel covers head_dim 128 with 16-token pages only"); return CBKV_ERR_ARG;
+    }
+    if (mode == 6 && !(dev_of(a)->tc_ok && chunk_pair_supported(a->cfg.head_dim))) {
+        set_error("the chunk kernel on pairs of SMs covers head_dim 128 and 256 with 16-token pages only"); return CBKV_ERR_ARG;
     }
     if (mode == 2 && !dev_of(a)->tc_ok) { set_error("the tensor-core chunk kernel covers head_dim 64, 128 and 256 with 16-token pages only"); return CBKV_ERR_ARG; }
     dev_of(a)->chunk_mode = mode;
@@ -1667,15 +1670,15 @@ int64_t cbkv_debug_tile_plan(cbkv_arena* arena, int64_t window, int32_t tokens_p
 }
 
 // Host-only view of the choice between the chunk kernels for the step in flight (used by the CPU tests): out = [the kernel
-// as cbkv_set_chunk_kernel numbers it (2 or 3: one or two tiles, 5: pairs of SMs, 1: mma.sync), CTAs run through the launch
+// as cbkv_set_chunk_kernel numbers it (2 or 3: one or two tiles, 6: pairs of SMs, 1: mma.sync), CTAs run through the launch
 // model to decide, n_ctas, n_slots, n_cut, TileItem records].
 int64_t cbkv_debug_chunk_choice(cbkv_arena* arena, int64_t window, int32_t mode, int32_t sm_count, int32_t max_parts, int32_t* out, int64_t cap) {
     return fenced64([&]() -> int64_t {
     Arena* a = reinterpret_cast<Arena*>(arena);
-    if (!a || a->step_meta.empty() || !out || mode < 0 || mode > 5 || mode == 1 || sm_count < 2 || max_parts < 1) return -1;
+    if (!a || a->step_meta.empty() || !out || mode < 0 || mode > 6 || mode == 1 || (mode == 6 && !chunk_pair_supported(a->cfg.head_dim)) || sm_count < 2 || max_parts < 1) return -1;
     const ChunkChoice c = chunk_choice(*a, mode, window, sm_count, max_parts);
     const ChunkLaunch l = plan_chunk_launch(*a, c);
-    const int32_t kernel = l.mma ? 1 : l.pair ? 5 : c.one_tokens > c.one.tile_tokens ? 3 : 2;
+    const int32_t kernel = l.mma ? 1 : l.pair ? 6 : c.one_tokens > c.one.tile_tokens ? 3 : 2;
     std::vector<int32_t> flat = {kernel, (int32_t)l.modelled, (int32_t)l.plan.tiles.size(), l.plan.n_slots, l.plan.n_cut};
     const int32_t* tp = reinterpret_cast<const int32_t*>(l.plan.tiles.data());
     flat.insert(flat.end(), tp, tp + l.plan.tiles.size() * 8);

@@ -350,7 +350,7 @@ int32_t cbkv_set_chunk_split(cbkv_arena* arena, int32_t max_parts);
  * Over int8 layers these kernels read a float copy of the step's pages made per layer and
  * step; 4 = as 3, but the kernel fetches the int8 records and converts them itself (no
  * float copy; slower so far, kept for measurement); 5 (the default) = as 0, and pairs of SMs
- * (cta_group::2, head_dim 128 or 256) where the launch model expects them to be faster. */
+ * (cta_group::2, head_dim 128 or 256) where the launch model expects them to be faster; 6 = pairs of SMs. */
 int32_t cbkv_set_chunk_kernel(cbkv_arena* arena, int32_t mode);
 
 /* ---- test hooks (host only, no device is touched) --------------------------- */
@@ -383,7 +383,7 @@ int64_t cbkv_debug_tile_plan(cbkv_arena* arena, int64_t window, int32_t tokens_p
 
 /* The choice between the chunk kernels for the step in flight, as cbkv_set_chunk_kernel(mode) would have it
  * made on `sm_count` SMs with at most `max_parts` slices per item: [kernel (1 = mma.sync, 2 / 3 = one / two
- * tiles per CTA, 5 = pairs of SMs), CTAs that were run through the launch model to decide, n_ctas, n_slots,
+ * tiles per CTA, 6 = pairs of SMs), CTAs that were run through the launch model to decide, n_ctas, n_slots,
  * n_cut, records as above (none for mma.sync)].  Returns the number of words, or -1 without a step. */
 int64_t cbkv_debug_chunk_choice(cbkv_arena* arena, int64_t window, int32_t mode, int32_t sm_count, int32_t max_parts,
                                 int32_t* out, int64_t cap);

@@ -55,7 +55,7 @@ def _step(p, pairs, new, layers, grow, repeats=REPEATS):
             assert torch.equal(outs[r][i], outs[0][i]), f"layer {l} contexts {pos} new {new}: run {r} differs"
 
 
-KERNELS = [(9, 3, 64, 0), (28, 4, 128, 2), (28, 4, 128, 3), (8, 4, 256, 0)]  # q heads, kv heads, head_dim, chunk kernel
+KERNELS = [(9, 3, 64, 0), (28, 4, 128, 2), (28, 4, 128, 3), (28, 4, 128, 5), (28, 4, 128, 6), (8, 4, 256, 0), (8, 4, 256, 5), (8, 4, 256, 6)]  # q heads, kv heads, head_dim, chunk kernel
 
 
 @pytest.mark.parametrize("grow", [False, True])

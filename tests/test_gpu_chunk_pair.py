@@ -1,4 +1,4 @@
-"""Prompts' chunks on pairs of SMs (the library's choice for launches that they shorten), against the oracle (needs a B200)."""
+"""Chunk attention on pairs of SMs, and where the library chooses it, against the oracle (needs a B200)."""
 import pytest
 import torch
 
@@ -11,9 +11,10 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("grow", [False, True])
 @pytest.mark.parametrize("n_q,n_kv,d", [(28, 4, 128), (32, 8, 128), (8, 8, 128), (8, 4, 256), (8, 1, 256)])
 def test_chunks_on_pairs_of_sms(n_q, n_kv, d, grow):
-    # tokens per query tile: 16 to 128; chunks that fill one tile, two, and leave the second with none or a few; KV tiles of
-    # 64 or 128 tokens: one, two and many of them, cut and whole
-    p = Pair(2, n_q, n_kv, d, 4096, num_pages=1600, windows=[150, None], seed=d + n_q, shuffle_free_list=True, popn_refuses=False)
+    # tokens per query tile: 16 to 128; chunks that fill one tile, two, and leave the second with none or a few; KV tiles:
+    # one, two and many of them, cut and whole
+    p = Pair(2, n_q, n_kv, d, 4096, num_pages=1600, windows=[150, None], seed=d + n_q, shuffle_free_list=True, popn_refuses=False,
+             chunk_kernel=6)
     for ctx in (0, 1, 50, 130, 900, 2050):
         s = p.new_seq()
         if ctx:
@@ -21,7 +22,9 @@ def test_chunks_on_pairs_of_sms(n_q, n_kv, d, grow):
     for s in p.seqs:
         _step(p, [s], [70], [0, 1], grow, repeats=5)
         _step(p, [s], [257], [0, 1], grow, repeats=5)
+        _step(p, [s], [5 if ctx % 4 else 1], [0, 1], grow, repeats=5)
     _step(p, p.seqs, [128, 65, 80, 129, 200, 97], [0, 1], grow, repeats=20)
+    _step(p, p.seqs, [1, 140, 2, 9, 1, 5], [0, 1], grow, repeats=20)
     p.g.set_chunk_split(1)
     _step(p, p.seqs, [128, 65, 80, 129, 200, 97], [0, 1], grow, repeats=5)
 
@@ -32,6 +35,7 @@ def test_prompts_in_both_types_against_64_bits():
         for d, n_q, n_kv, new in ((128, 32, 8, 90), (128, 28, 4, 300), (256, 8, 4, 200)):
             gen = torch.Generator(device="cuda").manual_seed(d)
             g = KVArena(1, n_q, n_kv, d, 2048, 16, 400, dtype=dtype, sliding_popn_refuses=False)
+            g.set_chunk_kernel(6)
             rand = lambda n: torch.randn(n, generator=gen, device="cuda", dtype=dtype)
             seqs, ctx = [g.new_seq() for _ in range(3)], [37, 500, 1203]
             g.begin_step(seqs, ctx)
@@ -60,13 +64,14 @@ def test_prompts_in_both_types_against_64_bits():
 
 def test_both_halves_of_a_row_see_the_same_maxima_over_many_tiles():
     # 512 tokens after 6000, nothing cut: 48 to 51 KV tiles per item, whose row maxima rise and move the reference nearly
-    # every tile.  Every run has to give the same bits, and be that of the pairs, not of the two-tile kernel.
+    # every tile.  Every run has to give the same bits.
     from combsengine_b200 import KVArena
     n_q, n_kv, d, ctx, new = 32, 8, 128, 6000, 512
     gen = torch.Generator(device="cuda").manual_seed(7)
     rand = lambda n: torch.randn(n, generator=gen, device="cuda", dtype=torch.float16)
     g = KVArena(1, n_q, n_kv, d, 8192, 16, 512, sliding_popn_refuses=False)
     g.set_chunk_split(1)
+    g.set_chunk_kernel(6)
     rise = lambda first, n: (0.1 * rand(n_kv * n * d).view(n_kv, n, d) + torch.arange(first, first + n, device="cuda")[None, :, None] / 128).half().view(-1)
     s = g.new_seq()
     g.begin_step([s], [ctx])
@@ -85,5 +90,51 @@ def test_both_halves_of_a_row_see_the_same_maxima_over_many_tiles():
     g.set_chunk_kernel(3)
     other = run()
     assert g.device_status() == 0
-    assert not torch.equal(first, other)
     assert (first.double() - other.double()).norm() <= 2 ** -9 * other.double().norm()  # P and the output rounded to 11 bits
+
+
+@pytest.mark.parametrize("n_q,n_kv,d", [(28, 4, 128), (8, 4, 256)])
+def test_int8_pages_on_pairs_of_sms(n_q, n_kv, d):
+    # the kernel reads the float copy of the step's pages, through the copy's own maps
+    p = Pair(1, n_q, n_kv, d, 2048, num_pages=400, seed=d, shuffle_free_list=True, quantize_kv=True, chunk_kernel=6)
+    seqs = [p.new_seq() for _ in range(3)]
+    p.step(seqs, [300, 17, 90])
+    p.step(seqs, [129, 5, 700])
+    p.step([seqs[1]], [40])
+    p.assert_state_equal("used")
+
+
+def test_pairs_are_refused_where_there_is_no_such_kernel():
+    from combsengine_b200 import CbkvError, KVArena
+    g = KVArena(1, 8, 2, 64, 256, 16, 16)
+    with pytest.raises(CbkvError):
+        g.set_chunk_kernel(6)
+    for bad in (-1, 7):
+        with pytest.raises(CbkvError):
+            g.set_chunk_kernel(bad)
+
+
+@pytest.mark.parametrize("n_q,n_kv,d,n_seqs,ctx,new,kernel", [
+    (32, 8, 128, 1, 512, 512, 6), (28, 4, 128, 1, 400, 40, 6), (32, 8, 128, 4, 1024, 512, 3), (28, 4, 128, 8, 2000, 5, 3), (32, 8, 128, 64, 33, 2, 1),
+    (8, 4, 256, 1, 512, 512, 6), (8, 4, 256, 64, 33, 5, 1)])
+def test_the_default_takes_pairs_where_its_model_expects_them_to_end_sooner(n_q, n_kv, d, n_seqs, ctx, new, kernel):
+    # on either side of the line the output is, bit for bit, that of the kernel which the rule names
+    from combsengine_b200 import KVArena
+    g = KVArena(1, n_q, n_kv, d, 4096, 16, n_seqs * 160, sliding_popn_refuses=False)
+    gen = torch.Generator(device="cuda").manual_seed(d)
+    rand = lambda n: torch.randn(n, generator=gen, device="cuda", dtype=torch.float16)
+    seqs = [g.new_seq() for _ in range(n_seqs)]
+    g.begin_step(seqs, [ctx] * n_seqs)
+    g.append(0, rand(n_seqs * ctx * n_kv * d), rand(n_seqs * ctx * n_kv * d))
+    q, k, v = (rand(n_seqs * new * h * d) for h in (n_q, n_kv, n_kv))
+    outs = {}
+    for mode in (5, 1, 3 if d == 128 else 2, 6):
+        g.set_chunk_kernel(mode)
+        g.begin_step(seqs, [new] * n_seqs)
+        assert mode != 5 or g.debug_chunk_choice()["kernel"] == kernel
+        outs[mode] = g.attention(0, q, k, v, d ** -0.5)
+        assert g.device_status() == 0
+        for s in seqs:
+            s.popn(new)
+    same = [mode for mode in outs if mode != 5 and torch.equal(outs[mode], outs[5])]
+    assert same == [kernel]

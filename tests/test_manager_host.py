@@ -363,7 +363,7 @@ def test_tile_plans_never_need_more_slots_than_the_buffers_have(sms):
 
 @pytest.mark.parametrize("n_q,n_kv,d,n_seqs,new,lo,hi,kernel,most", [
     (32, 8, 128, 64, 3, 40, 100, 1, 0), (8, 4, 256, 64, 3, 100, 1000, 1, 0), (32, 8, 128, 32, 3, 100, 1000, 3, 512),
-    (28, 4, 128, 64, 5, 100, 3000, 3, 800), (32, 8, 128, 8, 5, 512, 6144, 3, 1496), (32, 8, 128, 1, 512, 512, 512, 5, 800)])
+    (28, 4, 128, 64, 5, 100, 3000, 3, 800), (32, 8, 128, 8, 5, 512, 6144, 3, 1496), (32, 8, 128, 1, 512, 512, 512, 6, 800)])
 def test_a_chunk_kernel_is_chosen_without_modelling_every_launch(n_q, n_kv, d, n_seqs, new, lo, hi, kernel, most):
     # CTAs run through the launch model, which the host does in front of a step's first launch: none where the mma.sync
     # kernel is below what any plan could reach, and no more than the plan of one kernel takes when every candidate of its
@@ -376,3 +376,20 @@ def test_a_chunk_kernel_is_chosen_without_modelling_every_launch(n_q, n_kv, d, n
     got = a.debug_chunk_choice()
     assert got["kernel"] == kernel and got["modelled"] <= most
     assert (got["n_ctas"] > 0) == (kernel != 1)
+
+
+@pytest.mark.parametrize("sms", [2, 7, 148])
+@pytest.mark.parametrize("n_q,n_kv,d", [(28, 4, 128), (8, 4, 256)])
+def test_pairs_of_sms_never_need_more_slots_or_tickets_than_the_buffers_have(n_q, n_kv, d, sms):
+    # the partial-result buffers: 4 slots per SM, of 256 rows at head_dim 128 and of 128 at head_dim 256, half as many
+    # tickets; an item of a pair takes 256 rows a slot and a ticket for each of its two tiles
+    a = KVArena(1, n_q, n_kv, d, 45000, 16, 60000)
+    seqs = [a.new_seq() for _ in range(40)]
+    for i, s_ in enumerate(seqs):
+        a.begin_step_host_only([s_], [100 + 23 * i * i])
+    for n in (1, 2, 9, 40):
+        for new in ([5] * n, [1] * (n - 1) + [700], [512] * n):
+            a.begin_step_host_only(seqs[40 - n:], new)
+            for window in (0, 1024):
+                pl = a.debug_chunk_choice(window, 6, sms)
+                assert pl["kernel"] == 6 and pl["n_slots"] * (1 if d == 128 else 2) <= 4 * sms and 2 * pl["n_cut"] <= 2 * sms
