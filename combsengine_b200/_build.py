@@ -1,10 +1,10 @@
 """Builds libcombskv.so (the C-ABI library) in-tree with nvcc for sm_100a."""
 from __future__ import annotations
 
+import importlib.machinery
 import os
 import subprocess
 import sys
-import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -58,7 +58,7 @@ def pycall_path() -> str:
     """The Python mirror's hot calls (csrc/pycall.cpp).  The file is bound to torch's C++ and to CPython's binary interface, so
     its name carries both versions: another torch or Python finds no file of its own instead of one that does not load."""
     import torch
-    return os.path.join(HERE, f"_pycall.torch-{torch.__version__}{sysconfig.get_config_var('EXT_SUFFIX')}")
+    return os.path.join(HERE, f"_pycall.torch-{torch.__version__}{importlib.machinery.EXTENSION_SUFFIXES[0]}")
 
 
 def build_pycall(force: bool = False) -> str:
@@ -66,6 +66,8 @@ def build_pycall(force: bool = False) -> str:
     path = pycall_path()
     if not force and os.path.exists(path) and os.path.getmtime(path) >= os.path.getmtime(PYCALL_SOURCE):
         return path
+    import sysconfig
+
     import torch
     root = os.path.dirname(torch.__file__)
     cmd = ["/usr/bin/g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-w", "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(root, "include"),
