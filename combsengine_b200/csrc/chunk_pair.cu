@@ -198,6 +198,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
         bool ok = true;
+        int asked[2] = {0, 0};  // K and V buffers that this CTA has asked copies for
 #pragma unroll 1
         for (int j = 0; j < n_tiles && ok; j++) {
             const int st = j % NB;
@@ -219,6 +220,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
                 }
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
                 if (!ok) break;
+                asked[is_v]++;
                 const uint32_t full0 = at_rank0(full);
                 if (is_v) {
                     if (lane < PPT) load_page_pair(smem_u32(sV + st * HALF) + lane * PGV, &tmap_v, rank * XBV, 1, (phys * Hkv + h) * 2, full0);
@@ -227,9 +229,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
                 }
             }
         }
-        // Leave last: every buffer's final use is over, so no copy and no arrival is on its way to this CTA any more.
-        for (int i = max(0, n_tiles - NB) + lane; i < n_tiles && ok; i += 32)
-            if (!mbar_wait_bounded(bar(kBKEmpty + i % NB), (i / NB) & 1) || !mbar_wait_bounded(bar(kBVEmpty + i % NB), (i / NB) & 1)) ok = false;
+        // Leave last: every buffer's final use is over, so no copy and no arrival is on its way to this CTA any more.  If
+        // somebody gave up that use may never come; the wait for it is then a hundred milliseconds in which the copies land.
+#pragma unroll
+        for (int is_v = 0; is_v < 2; is_v++)
+            for (int i = max(0, asked[is_v] - NB) + lane; i < asked[is_v]; i += 32)
+                if (!mbar_wait_bounded(bar((is_v ? kBVEmpty : kBKEmpty) + i % NB), (i / NB) & 1)) ok = false;
         if (!ok) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer

@@ -150,6 +150,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
         // The block-table entries of the whole KV range were staged in shared memory by all threads; one copy per
         // page brings its K, another its V, each issued by the page's lane.
         bool ok = true;
+        int asked[2] = {0, 0};  // K and V buffers whose copies have been announced
         long long tprev = TC_NOW(), c_wait = 0, c_issue = 0;
 #pragma unroll 1
         for (int j = 0; j < n_tiles && ok; j++) {
@@ -168,7 +169,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
                     if (j >= NB && !mbar_wait_bounded(empty, (j / NB - 1) & 1)) ok = false;
                     TC_ACC(c_wait);
                     if (*failed) ok = false;
-                    if (ok) mbar_expect_tx(full, KVB);
+                    if (ok) { mbar_expect_tx(full, KVB); asked[is_v]++; }
                     else { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
                 }
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
@@ -177,6 +178,12 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
                 if (lane == 0) TC_ACC(c_issue);
             }
         }
+        // never leave with a copy in flight, whoever gave up (a barrier is in the phase announced last, or past it)
+        if (lane == 0)
+#pragma unroll
+            for (int is_v = 0; is_v < 2; is_v++)
+                for (int i = max(0, asked[is_v] - NB); i < asked[is_v]; i++)
+                    if (!mbar_wait_bounded((is_v ? b_v_full : b_k_full) + (i % NB) * 8, (i / NB) & 1)) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
         TC_DUMP(if (lane == 0) { a.dbg_buf[(size_t)blockIdx.x * 16 + 0] = c_wait; a.dbg_buf[(size_t)blockIdx.x * 16 + 1] = c_issue; a.dbg_buf[(size_t)blockIdx.x * 16 + 15] = n_tiles; });
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
@@ -674,6 +681,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     } else if (!Q8 && warp == 0) {
         // ------------------------------------------------------------ TMA producer
         bool ok = true;
+        int asked = 0;  // stages whose copies have been announced
         long long tprev = TC_NOW(), c_wait = 0, c_issue = 0;
 #pragma unroll 1
         for (int j = 0; j < n_tiles && ok; j++) {
@@ -682,7 +690,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                 if (j >= 2 && !mbar_wait_bounded(b_kv_empty + st * 8, ((j >> 1) - 1) & 1)) ok = false;
                 TC_ACC(c_wait);
                 if (*failed) ok = false;
-                if (ok) mbar_expect_tx(b_kv_full + st * 8, STAGE);
+                if (ok) { mbar_expect_tx(b_kv_full + st * 8, STAGE); asked++; }
                 else { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
             }
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
@@ -696,6 +704,10 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
             }
             if (lane == 0) TC_ACC(c_issue);
         }
+        // never leave with a copy in flight, whoever gave up
+        if (lane == 0)
+            for (int i = max(0, asked - 2); i < asked; i++)
+                if (!mbar_wait_bounded(b_kv_full + (i & 1) * 8, (i >> 1) & 1)) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
         TC_DUMP(if (lane == 0) { a.dbg_buf[(size_t)blockIdx.x * 16 + 0] = c_wait; a.dbg_buf[(size_t)blockIdx.x * 16 + 1] = c_issue; a.dbg_buf[(size_t)blockIdx.x * 16 + 15] = n_tiles; });
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
