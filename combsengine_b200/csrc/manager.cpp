@@ -342,15 +342,22 @@ constexpr float kPairCtaCost = 5.f, kPairSliceCost = 1.f, kPairMergeCost = 1.f; 
 // a tcgen05 launch takes fixed_us, then per wave of one CTA per SM cta_us + tile_us for each K/V tile (head_dim 128:
 // [0] with one query tile, [1] with both); the mma.sync kernel, one warp per item over all its pages, mma_us + page_us
 // for each page of the longest item, `warps` of them per SM at a time; with more items than that, kMmaRounds times as
-// much per round.  Pairs of CTAs (prompts of 40 to 512 tokens, 1 to 8 of them, up to 7680 cached tokens): pair_cta_us and
-// pair_tile_us per wave of one pair per two SMs.
-struct ChunkTimes { float cta_us[2], tile_us[2], mma_us, page_us; int32_t warps; float pair_cta_us, pair_tile_us; };
+// much per round.  Pairs of CTAs (head_dim 128: prompts of 40 to 512 tokens, 1 to 8 of them, up to 7680 cached tokens):
+// pair_cta_us and pair_tile_us per wave of one pair per two SMs.
+//
+// At head_dim 256 the merge of cut items counts too: merge_us[pairs] for each round of loads that the last slice's threads
+// make (four slices and 8 columns of a row per thread and round), which is as long as the tiles where few K/V tiles are
+// cut often.  Fitted over 170 steps (2 to 512 new tokens and mixes of both, 1 to 48 sequences, 0 to 8192 cached tokens, with
+// and without a window, GQA groups of 1, 2 and 8): the estimates are off by 7 % rms, the kernel they choose is within
+// 5 % of the fastest but for prompts of 33 to 65 tokens alone, where it is 1 us off.  us, one tile / pairs: 48 sequences x 2
+// tokens after 2048 74 / 117, 16 x 5 after 8192 94 / 123, 1 x 9 after 8192 45 / 30, a prompt of 512 after 512 49 / 24.
+struct ChunkTimes { float cta_us[2], tile_us[2], mma_us, page_us; int32_t warps; float pair_cta_us, pair_tile_us, merge_us[2]; };
 constexpr float kChunkFixedUs = 1.7f, kMmaRounds = 1.5f;
 ChunkTimes chunk_times(int32_t d) {
     switch (d) {
-        case 64: return {{5.f, 5.f}, {1.f, 1.f}, 11.f, 1.04f, 12, 0.f, 0.f};
-        case 128: return {{5.8f, 10.f}, {2.1f, 2.45f}, 8.f, 0.84f, 8, 9.f, 1.25f};
-        default: return {{6.f, 6.f}, {1.3f, 1.3f}, 7.5f, 0.88f, 4, 11.5f, 1.9f};  // 256
+        case 64: return {{5.f, 5.f}, {1.f, 1.f}, 11.f, 1.04f, 12, 0.f, 0.f, {0.f, 0.f}};
+        case 128: return {{5.8f, 10.f}, {2.1f, 2.45f}, 8.f, 0.84f, 8, 9.f, 1.25f, {0.f, 0.f}};
+        default: return {{6.f, 6.f}, {1.4f, 1.4f}, 7.5f, 0.88f, 4, 8.5f, 1.85f, {1.2f, 1.f}};  // 256
     }
 }
 
@@ -423,7 +430,8 @@ public:
                 const int32_t pages = (int32_t)((q_last >> 4) - (lo_key >> 4) + 1), ppt = cut.kv_tile / 16;
                 const bool both = toks > tile_tokens_;
                 // one query tile per CTA: the same for every item
-                Work w{(pages + ppt - 1) / ppt, both || tile_tokens_ == tokens_ ? 1.f : kHalfTile, (float)toks / (float)tokens_, both ? 1 : 0};
+                Work w{(pages + ppt - 1) / ppt, both || tile_tokens_ == tokens_ ? 1.f : kHalfTile, (float)toks / (float)tokens_, both ? 1 : 0,
+                       std::min(toks, cut.pair ? tokens_ / 2 : tile_tokens_) * a.n_rep()};
                 g.cost = std::max(g.cost, w.per_tile * w.n_tiles);
                 work_.push_back(w);
             }
@@ -459,9 +467,15 @@ public:
     // Expected time of the launch in microseconds, and what it cannot be below however its items are cut.
     float launch_us() {
         const ChunkTimes t = chunk_times(a_.cfg.head_dim);
+        const int threads = cut_.pair ? 512 : 256, row_items = a_.cfg.head_dim / 8;
+        int rounds = 0;  // of the longest merge
         sms_.start(cut_.sm_count);
-        each_cta(how_, [&](const Work& w, int, int, int, int tiles, int, int) { sms_.run(cta_us(t, w, tiles)); modelled_++; });
-        return kChunkFixedUs + sms_.end();
+        each_cta(how_, [&](const Work& w, int, int, int, int tiles, int part, int parts) {
+            if (part == 0 && parts > 1) rounds = std::max(rounds, (parts + 3) / 4 * ((w.tile_rows * row_items + threads - 1) / threads));
+            sms_.run(cta_us(t, w, tiles));
+            modelled_++;
+        });
+        return kChunkFixedUs + sms_.end() + t.merge_us[cut_.pair ? 1 : 0] * (float)rounds;
     }
     float least_us() const {
         const ChunkTimes t = chunk_times(a_.cfg.head_dim);
@@ -492,7 +506,7 @@ public:
     int64_t modelled() const { return modelled_; }
 
 private:
-    struct Work { int32_t n_tiles; float per_tile, rows; int32_t both; };  // an uncut item, the same for every kv head
+    struct Work { int32_t n_tiles; float per_tile, rows; int32_t both, tile_rows; };  // an uncut item, the same for every kv head
     struct Group { int32_t seq, first, n_qt; float cost; };
     // parts of an item: ceil(cost / limit), and for the last `rem` items of the launch order at least rem_parts
     struct How { float limit = 0.f; int64_t rem = 0; int rem_parts = 1; };
@@ -580,14 +594,21 @@ void build_chunk_tile_plan(const Arena& a, int32_t tokens_per_tile, ChunkPlan* p
     p.emit(pl);
 }
 
+// Pairs of SMs take a query tile per CTA, with half of K and V each: a launch that leaves SMs idle ends sooner (a prompt
+// of 512 after 512, 8 kv heads, head_dim 128: 19.5 against 31.0 us), one that fills them does not at head_dim 128 (four of
+// them after 1024: 92 against 73); at head_dim 256, where one CTA has room for K/V tiles of half the size only, prompts do
+// (8 of 512 after 7680: 236 against 338), steps of a few tokens of many sequences, whose second tile is empty, do not.
+//
+// One tcgen05 CTA per SM at a time costs more to start than a few pages take the mma.sync kernel, of which eight warps
+// (items) share an SM: steps with more (sequence, kv head) pairs than SMs over short contexts, and prompts of some tens of
+// tokens.  64 sequences x 2 tokens after 33 (8 kv heads, head_dim 128): 12.7 against 28.7 us, after 600: 45 against 65;
+// 32 x 2 after 600: 43 against 34; a 40-token prompt (4 kv heads) 10.3 against 13.0.
 ChunkLaunch plan_chunk_launch(const Arena& a, const ChunkChoice& c) {
     ChunkLaunch out;
     const float mma_us = c.mma_cols > 0 ? chunk_mma_launch_us(a, c.one.window, c.mma_cols, c.one.sm_count) : INFINITY;
-    // Head_dim 256 takes pairs at every size; see chunk_times for head_dim 128.
-    const bool only_pairs = c.pairs && (c.one_tokens == 0 || a.cfg.head_dim == 256);
     std::unique_ptr<TilePlanner> one, two;
     float least = INFINITY;
-    if (!only_pairs) { one.reset(new TilePlanner(a, c.one_tokens, c.one)); if (c.chooses()) least = one->least_us(); }
+    if (c.one_tokens > 0) { one.reset(new TilePlanner(a, c.one_tokens, c.one)); if (c.chooses()) least = one->least_us(); }
     if (c.pairs) { two.reset(new TilePlanner(a, c.pair_tokens, c.pair)); if (c.chooses()) least = std::min(least, two->least_us()); }
     if (mma_us < least) { out.mma = true; return out; }  // whatever a plan would say
     float us = INFINITY;

@@ -116,7 +116,7 @@ def test_pairs_are_refused_where_there_is_no_such_kernel():
 
 @pytest.mark.parametrize("n_q,n_kv,d,n_seqs,ctx,new,kernel", [
     (32, 8, 128, 1, 512, 512, 6), (28, 4, 128, 1, 400, 40, 6), (32, 8, 128, 4, 1024, 512, 3), (28, 4, 128, 8, 2000, 5, 3), (32, 8, 128, 64, 33, 2, 1),
-    (8, 4, 256, 1, 512, 512, 6), (8, 4, 256, 64, 33, 5, 1)])
+    (8, 4, 256, 1, 512, 512, 6), (8, 4, 256, 1, 2000, 9, 6), (8, 4, 256, 16, 2000, 5, 2), (8, 4, 256, 64, 33, 5, 1)])
 def test_the_default_takes_pairs_where_its_model_expects_them_to_end_sooner(n_q, n_kv, d, n_seqs, ctx, new, kernel):
     # on either side of the line the output is, bit for bit, that of the kernel which the rule names
     from combsengine_b200 import KVArena

@@ -362,12 +362,12 @@ def test_tile_plans_never_need_more_slots_than_the_buffers_have(sms):
 
 
 @pytest.mark.parametrize("n_q,n_kv,d,n_seqs,new,lo,hi,kernel,most", [
-    (32, 8, 128, 64, 3, 40, 100, 1, 0), (8, 4, 256, 64, 3, 100, 1000, 1, 0), (32, 8, 128, 32, 3, 100, 1000, 3, 512),
+    (32, 8, 128, 64, 3, 40, 100, 1, 0), (8, 4, 256, 64, 3, 40, 60, 1, 0), (8, 4, 256, 64, 3, 100, 1000, 2, 800), (32, 8, 128, 32, 3, 100, 1000, 3, 512),
     (28, 4, 128, 64, 5, 100, 3000, 3, 800), (32, 8, 128, 8, 5, 512, 6144, 3, 1496), (32, 8, 128, 1, 512, 512, 512, 6, 800)])
 def test_a_chunk_kernel_is_chosen_without_modelling_every_launch(n_q, n_kv, d, n_seqs, new, lo, hi, kernel, most):
     # CTAs run through the launch model, which the host does in front of a step's first launch: none where the mma.sync
     # kernel is below what any plan could reach, and no more than the plan of one kernel takes when every candidate of its
-    # cut is run (1536, 2084, 1816, 2088, 1496 and 1392; 1024, 1158, 1162, 1426, 928 and 848 more for pairs)
+    # cut is run (1536, 512, 2084, 1816, 2088, 1496 and 1392; 1024, 768, 1158, 1162, 1426, 928 and 848 more for pairs)
     lens = [int(lo + (i + 1) * 0.618 % 1 * (hi - lo)) for i in range(n_seqs)]
     a = KVArena(1, n_q, n_kv, d, 8192, 16, 16384)
     seqs = [a.new_seq() for _ in lens]
@@ -393,3 +393,15 @@ def test_pairs_of_sms_never_need_more_slots_or_tickets_than_the_buffers_have(n_q
             for window in (0, 1024):
                 pl = a.debug_chunk_choice(window, 6, sms)
                 assert pl["kernel"] == 6 and pl["n_slots"] * (1 if d == 128 else 2) <= 4 * sms and 2 * pl["n_cut"] <= 2 * sms
+
+
+@pytest.mark.parametrize("n_seqs,new,ctx,window,fastest", [
+    (48, 2, 2048, 0, 2), (48, 5, 2048, 1024, 2), (48, 9, 8192, 0, 2), (16, 5, 8192, 0, 2), (16, 9, 512, 0, 2), (4, 2, 2048, 0, 2), (4, 9, 8192, 0, 2),
+    (64, 5, 33, 0, 1), (1, 9, 8192, 0, 6), (1, 5, 2048, 1024, 6), (4, 9, 512, 0, 6), (1, 512, 512, 0, 6), (8, 512, 4096, 0, 6), (4, 512, 4096, 1024, 6)])
+def test_head_dim_256_takes_the_kernel_that_was_measured_fastest(n_seqs, new, ctx, window, fastest):
+    # 8 query and 4 kv heads on a B200, one tile / pairs / mma.sync, each row more than 5 % apart
+    a = KVArena(1, 8, 4, 256, 16384, 16, 32768)
+    seqs = [a.new_seq() for _ in range(n_seqs)]
+    a.begin_step_host_only(seqs, [ctx] * n_seqs)
+    a.begin_step_host_only(seqs, [new] * n_seqs)
+    assert a.debug_chunk_choice(window)["kernel"] == fastest
