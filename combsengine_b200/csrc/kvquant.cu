@@ -365,9 +365,13 @@ cudaError_t launch_init_quant(void* arena, size_t n_records, int page_size, int 
 cudaError_t launch_append_quant(const AppendArgs& a, bool bf16, bool overlap, cudaStream_t st) {
     const int64_t rows = 2 * (int64_t)a.step.n_tokens * a.geo.n_kv;
     if (rows <= 0) return cudaSuccess;
-    // 16 bytes a load where k and v allow it; the kernel of one row per warp takes them at any multiple of 8
+    // Token pairs where there is work for them: a lane has 32 divisions to make one after the other, 7 to 9 us however few
+    // rows there are, while a row per warp takes 3 us as long as every row finds a warp (9472 of them) and 1 us per 1700
+    // rows beyond.  us, pairs / rows, at 272, 8192, 16384 and 65536 rows of 128: 6.6 / 2.9, 8.7 / 5.9, 10.1 / 10.0, 19.4 /
+    // 38.2; 1998, 12288 and 24576 of 64: 8.1 / 3.4, 8.6 / 9.1, 9.0 / 16.0; 8192, 16384 of 256: 9.8 / 8.4, 13.7 / 16.0.
+    // And only where k and v allow 16 bytes a load; the other kernel takes them at any multiple of 8.
     const bool aligned16 = ((reinterpret_cast<uintptr_t>(a.k) | reinterpret_cast<uintptr_t>(a.v)) & 15) == 0;
-    if (aligned16 && a.geo.page_size == 16 && (a.geo.d == 64 || a.geo.d == 128 || a.geo.d == 256)) {
+    if (rows >= 12288 && aligned16 && a.geo.page_size == 16 && (a.geo.d == 64 || a.geo.d == 128 || a.geo.d == 256)) {
         const int rpw = 512 / a.geo.d;  // rows or pairs of a warp
         const int64_t warps = (rows / 2 + rpw - 1) / rpw + ((a.step.n_tokens / 2 + a.step.n_seqs) * (int64_t)a.geo.n_kv + rpw - 1) / rpw;
         const int blocks = (int)std::min<int64_t>((warps + 7) / 8, 148 * 8);

@@ -1,4 +1,4 @@
-"""The quantising append over token pairs: sequences that start and end on either side of a pair (needs a B200)."""
+"""The quantising append, by rows and over token pairs: sequences that start and end on either side of a pair (needs a B200)."""
 import pytest
 import torch
 
@@ -29,10 +29,11 @@ def test_rows_that_start_at_8_bytes_fill_the_same_pages(d, k_off, v_off):
     gen = torch.Generator(device="cuda").manual_seed(d)
     rand = lambda n: torch.randn(n, generator=gen, device="cuda", dtype=torch.float16)
     view = lambda x, off: torch.zeros(x.numel() + 16, dtype=x.dtype, device="cuda")[off:off + x.numel()].copy_(x)
-    g = KVArena(1, 8, 2, d, 512, 16, 40, quantize_kv=True)
+    # (801 tokens of 8 heads: over token pairs at a multiple of 16, a row per warp otherwise)
+    g = KVArena(1, 8, 8, d, 1024, 16, 64, quantize_kv=True)
     s = g.new_seq()
-    n = 37
-    q, k, v = (rand(n * h * d) for h in (8, 2, 2))
+    n = 801
+    q, k, v = (rand(n * 8 * d) for _ in range(3))
 
     def pages(kx, vx):
         g.begin_step([s], [n])
@@ -46,3 +47,13 @@ def test_rows_that_start_at_8_bytes_fill_the_same_pages(d, k_off, v_off):
     assert g.device_status() == 0
     assert torch.equal(out, out8)
     assert all((x == y).all() for a, b in zip(rows, rows8) for x, y in zip(a, b))
+
+
+@pytest.mark.parametrize("d", [64, 128, 256])
+def test_large_steps_hold_the_oracles_bytes_whatever_the_parity(d):
+    # 12288 rows and more, over token pairs; the last step is just below, a row per warp
+    p = Pair(1, 8, 8, d, 2048, num_pages=400, seed=d, shuffle_free_list=True, quantize_kv=True)
+    seqs = [p.new_seq() for _ in range(5)]
+    for new in ([1, 2, 333, 16, 433], [2, 301, 1, 3, 512], [417, 316, 5, 33, 1], [160, 161, 1, 160, 286], [160, 160, 1, 160, 286]):
+        p.step(seqs, new)
+        p.assert_state_equal("used")
