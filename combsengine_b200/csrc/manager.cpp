@@ -342,22 +342,27 @@ constexpr float kPairCtaCost = 5.f, kPairSliceCost = 1.f, kPairMergeCost = 1.f; 
 // a tcgen05 launch takes fixed_us, then per wave of one CTA per SM cta_us + tile_us for each K/V tile (head_dim 128:
 // [0] with one query tile, [1] with both); the mma.sync kernel, one warp per item over all its pages, mma_us + page_us
 // for each page of the longest item, `warps` of them per SM at a time; with more items than that, kMmaRounds times as
-// much per round.  Pairs of CTAs (head_dim 128: prompts of 40 to 512 tokens, 1 to 8 of them, up to 7680 cached tokens):
-// pair_cta_us and pair_tile_us per wave of one pair per two SMs.
+// much per round.  Pairs of CTAs: pair_cta_us and pair_tile_us per wave of one pair per two SMs.
 //
-// At head_dim 256 the merge of cut items counts too: merge_us[pairs] for each round of loads that the last slice's threads
-// make (four slices and 8 columns of a row per thread and round), which is as long as the tiles where few K/V tiles are
-// cut often.  Fitted over 170 steps (2 to 512 new tokens and mixes of both, 1 to 48 sequences, 0 to 8192 cached tokens, with
-// and without a window, GQA groups of 1, 2 and 8): the estimates are off by 7 % rms, the kernel they choose is within
-// 5 % of the fastest but for prompts of 33 to 65 tokens alone, where it is 1 us off.  us, one tile / pairs: 48 sequences x 2
-// tokens after 2048 74 / 117, 16 x 5 after 8192 94 / 123, 1 x 9 after 8192 45 / 30, a prompt of 512 after 512 49 / 24.
-struct ChunkTimes { float cta_us[2], tile_us[2], mma_us, page_us; int32_t warps; float pair_cta_us, pair_tile_us, merge_us[2]; };
+// The merge of cut items counts as well (head_dim 128 and 256): merge_us[pairs] for each round of loads that the last
+// slice's threads make (four slices and 8 columns of a row per thread and round), which is as long as the tiles where few
+// K/V tiles are cut often.  Fitted over 384 steps at head_dim 128 and 170 at 256 (2 to 1024 new tokens and mixes of many with
+// one, 1 to 48 sequences, 0 to 8192 cached tokens, with and without a window, GQA groups of 1 to 8): estimates off by 7 to
+// 9 % rms (38 % for the two-tile kernel without the merge), the kernel they choose within 5 % of the fastest of the three
+// but for 24 and 3 steps, the worst 1.36 times (2 prompts of 100 tokens beside 1 to 3 decoding sequences, 25 us).  us, one
+// tile / pairs at head_dim 256: 48 sequences x 2 tokens after 2048 74 / 117, 16 x 5 after 8192 94 / 123, 1 x 9 after 8192 45
+// / 30, a prompt of 512 after 512 49 / 24; two tiles / pairs at 128: 2 prompts of 333 after 1024 (4 kv heads) 35 / 43.
+//
+// pair_margin: pairs are taken where their estimate is below this share of the others'.  At head_dim 128, where the kernels
+// are closer, a tenth, the estimates' own error: 8 sequences x 5 tokens after 512 to 6144 (28 q heads) come out equal and
+// take 29.3 us a layer with two tiles per CTA, 31.6 on pairs.
+struct ChunkTimes { float cta_us[2], tile_us[2], mma_us, page_us; int32_t warps; float pair_cta_us, pair_tile_us, merge_us[2], pair_margin; };
 constexpr float kChunkFixedUs = 1.7f, kMmaRounds = 1.5f;
 ChunkTimes chunk_times(int32_t d) {
     switch (d) {
-        case 64: return {{5.f, 5.f}, {1.f, 1.f}, 11.f, 1.04f, 12, 0.f, 0.f, {0.f, 0.f}};
-        case 128: return {{5.8f, 10.f}, {2.1f, 2.45f}, 8.f, 0.84f, 8, 9.f, 1.25f, {0.f, 0.f}};
-        default: return {{6.f, 6.f}, {1.4f, 1.4f}, 7.5f, 0.88f, 4, 8.5f, 1.85f, {1.2f, 1.f}};  // 256
+        case 64: return {{5.f, 5.f}, {1.f, 1.f}, 11.f, 1.04f, 12, 0.f, 0.f, {0.f, 0.f}, 1.f};
+        case 128: return {{5.8f, 10.f}, {2.1f, 2.45f}, 8.f, 0.84f, 8, 8.f, 1.25f, {0.9f, 1.f}, 0.9f};
+        default: return {{6.f, 6.f}, {1.4f, 1.4f}, 7.5f, 0.88f, 4, 8.5f, 1.85f, {1.2f, 1.f}, 1.f};  // 256
     }
 }
 
@@ -613,10 +618,11 @@ ChunkLaunch plan_chunk_launch(const Arena& a, const ChunkChoice& c) {
     if (mma_us < least) { out.mma = true; return out; }  // whatever a plan would say
     float us = INFINITY;
     if (one) { one->choose(); if (c.chooses()) us = one->launch_us(); }
-    if (two && two->least_us() < us) {
+    const float margin = chunk_times(a.cfg.head_dim).pair_margin;
+    if (two && two->least_us() < margin * us) {
         two->choose();
         const float pair_us = c.chooses() ? two->launch_us() : 0.f;
-        if (pair_us < us) { out.pair = true; us = pair_us; }
+        if (pair_us < margin * us) { out.pair = true; us = pair_us; }
     }
     out.modelled = (one ? one->modelled() : 0) + (two ? two->modelled() : 0);
     out.mma = mma_us < us;

@@ -405,3 +405,14 @@ def test_head_dim_256_takes_the_kernel_that_was_measured_fastest(n_seqs, new, ct
     a.begin_step_host_only(seqs, [ctx] * n_seqs)
     a.begin_step_host_only(seqs, [new] * n_seqs)
     assert a.debug_chunk_choice(window)["kernel"] == fastest
+
+
+@pytest.mark.parametrize("ctx,new,kernel", [
+    ([1024, 1024], [333, 333], 3), ([2378, 921, 4276, 1655, 641, 2975, 1152, 5349], [5] * 8, 3), ([512], [512], 6), ([512], [100], 6)])
+def test_head_dim_128_takes_pairs_only_where_they_are_faster(ctx, new, kernel):
+    # 28 query and 4 kv heads on a B200, two tiles / pairs: 35 / 43 us, 29 / 32 a layer, and pairs faster in the other two
+    a = KVArena(1, 28, 4, 128, 16384, 16, 32768)
+    seqs = [a.new_seq() for _ in ctx]
+    a.begin_step_host_only(seqs, ctx)
+    a.begin_step_host_only(seqs, new)
+    assert a.debug_chunk_choice()["kernel"] == kernel
