@@ -1091,7 +1091,9 @@ int32_t cbkv_attention_rope(cbkv_arena* arena, int32_t layer, const cbkv_rope* r
     if ((rc = materialize(a, layer, st))) return rc;
     const bool quant = d->layers[(size_t)layer].quant;
     const DecodeConfig dc = decode_config(a->cfg.head_dim, a->n_rep(), d->decode_ctas_per_sm, d->decode_stages, d->decode_consumers, quant);
-    if (d->fast && a->step_is_decode && decode_rotates(a->cfg.head_dim, dc.consumers, quant) && !(quant && (debug_flags() & 16))) {
+    const bool normed = norm && (norm->q_weight || norm->k_weight);
+    if (d->fast && a->step_is_decode && !(quant && (debug_flags() & 16)) &&
+        decode_rotates(a->cfg.head_dim, dc.consumers, quant, normed, (int64_t)a->step_meta.size() * a->cfg.n_kv_heads, d->sm_count)) {
         // norm, rotation and append ride inside the decode kernel: one launch instead of two, and its pages are on their
         // way before the previous layer's launch has ended
         RopeDev rd;

@@ -228,9 +228,12 @@ __global__ void resolve_units_kernel(const SegInfo* segs, int n_segs, const int3
 // Warp roles: 0 = producer, 1..C = consumers, C+1 = merger.
 // Q8: the layer holds int8 records; a tile is one record fetched as one box of a byte tensor map.
 // ROPE: q and k_new are normed and rotated here (DecodeArgs::rope); a variant of its own, because the words it holds cost
-// the other ones registers (236 bytes of spills at head_dim 128, int8 pages 60 registers and with them the second CTA).
+// the other ones registers (236 bytes of spills at head_dim 128).  Its own registers are bounded by what a launch has
+// resident, one CTA per SM, over int8 pages of head_dim 64 and 128 two.  Left to itself the compiler took 128 with 268 bytes
+// of spills (16 bits, head_dim 128: 193 now) and 241 (int8: 168 now), which left no room for the second CTA: 32 sequences of
+// 1024 to 4096 tokens, 28/4/128, 28 layers: 1058 -> 957 us, int8 1417 -> 1019 (rotated by a launch of its own 1165, 1047).
 template <int D, int C, bool BF16, bool Q8, bool ROPE>
-__global__ void __launch_bounds__((C + 2) * 32) decode_kernel(const __grid_constant__ CUtensorMap tmap, const DecodeArgs a) {
+__global__ void __launch_bounds__((C + 2) * 32, !ROPE ? 0 : Q8 && D <= 128 ? 2 : 1) decode_kernel(const __grid_constant__ CUtensorMap tmap, const DecodeArgs a) {
     constexpr uint32_t UNIT = Q8 ? (uint32_t)(2 * 16 * D + 2 * 16 * (D / 32) * 2) : 32u * D * 2u;
     constexpr int DP = D + 4;  // row pitch of the merge buffers: the four lanes of a quad land in different banks
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -1071,13 +1074,25 @@ DecodeConfig decode_config(int d, int n_rep, int ctas_per_sm, int stages, int co
     const int bufs = decode_smem_bytes(d, c, stages, comb_cols, 2, q8) <= smem_limit ? 2 : 1;
     return {c, stages, decode_smem_bytes(d, c, stages, comb_cols, bufs, q8), ctas, comb_cols, bufs};
 }
-bool decode_rotates(int d, int consumers, bool q8) {
+// The launch that is saved is worth about 4 us a layer; what it costs is the norm and rotation of q in every consumer warp of
+// every piece, and of k in the one that holds the new row, so it grows with the segments that an SM works through.  Measured
+// us per layer, inside / two launches, 1 to 128 sequences x 2 to 16 kv heads after 300 to 16000 tokens.  Rotation alone, 16
+// bits: faster throughout (1024 segments of head_dim 128 39 / 42, one sequence 7.9 / 14).  int8 pages: head_dim 128 faster
+// up to 512 segments (28 / 32), equal at 1024; 256 faster at 128 (26 / 28), slower at 512 (72 / 67).  With a norm: head_dim
+// 64 faster up to 384 (22 / 23, int8 24 / 26), slower at 1024 (43 / 38); 128 faster up to 256 (21 / 23), slower at 384 (27
+// / 25), int8 equal at 128 (20 / 20), slower at 192 (23 / 22); 256 faster up to 128 (22 / 23), slower at 256 (34 / 29), int8
+// slower from the first (21 / 19).
+bool decode_rotates(int d, int consumers, bool q8, bool norm, int64_t n_segs, int sm_count) {
+    constexpr int64_t ANY = (int64_t)1 << 30;
+    int default_consumers;
+    int64_t per_sm;  // most segments per SM
     switch (d) {
-        case 64: return consumers == (q8 ? DecodeCfg<64>::C8 : DecodeCfg<64>::C);
-        case 128: return consumers == (q8 ? DecodeCfg<128>::C8 : DecodeCfg<128>::C);
-        case 256: return consumers == (q8 ? DecodeCfg<256>::C8 : DecodeCfg<256>::C);
+        case 64: default_consumers = q8 ? DecodeCfg<64>::C8 : DecodeCfg<64>::C; per_sm = norm ? 3 : ANY; break;
+        case 128: default_consumers = q8 ? DecodeCfg<128>::C8 : DecodeCfg<128>::C; per_sm = norm ? (q8 ? 1 : 2) : (q8 ? 5 : ANY); break;
+        case 256: default_consumers = q8 ? DecodeCfg<256>::C8 : DecodeCfg<256>::C; per_sm = norm ? (q8 ? 0 : 1) : (q8 ? 1 : ANY); break;
         default: return false;
     }
+    return consumers == default_consumers && n_segs <= per_sm * sm_count;
 }
 ChunkConfig chunk_config(int d) {
     switch (d) {

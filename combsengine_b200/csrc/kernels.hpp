@@ -189,8 +189,9 @@ struct RopeArgs {
 // Decode kernel configuration for a head_dim (0 warps = not supported by the fast path).
 struct DecodeConfig { int consumers, stages, smem_bytes, ctas_per_sm, comb_cols, comb_bufs; };
 DecodeConfig decode_config(int d, int n_rep, int ctas_per_sm, int stages, int consumers, bool q8 = false);
-// Whether the variant that norms and rotates exists (with the default number of consumer warps).
-bool decode_rotates(int d, int consumers, bool q8);
+// Whether a launch over n_segs (sequence, kv head) pairs takes the variant that rotates (and norms, if `norm`) on the way: where
+// it exists (the default number of consumer warps) and is faster than a launch of its own in front.
+bool decode_rotates(int d, int consumers, bool q8, bool norm, int64_t n_segs, int sm_count);
 struct ChunkConfig { int warps, stages, smem_bytes, cols_per_item; };
 ChunkConfig chunk_config(int d);
 
