@@ -73,7 +73,8 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4 * NB + 5);
     volatile int* failed = reinterpret_cast<volatile int*>(bars + 4 * NB + 6);
     int* s_ticket = reinterpret_cast<int*>(bars + 4 * NB + 7);
-    static_assert(4 * NB + 8 <= 32, "barriers");
+    int* s_asked = reinterpret_cast<int*>(bars + 4 * NB + 8);  // K and V buffers whose copies have been announced
+    static_assert(4 * NB + 9 <= 32, "barriers");
     int* s_pages = reinterpret_cast<int*>(bars + 32);   // [kPageCap] physical pages of the KV range
     float* s_xch = reinterpret_cast<float*>(s_pages + kPageCap);  // [2 buffers][128 rows][2 halves]
     int* s_pair = reinterpret_cast<int*>(s_xch + 2 * 128 * 2);    // [4 pairs of warps][tile parity] a wait ran out
@@ -150,7 +151,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
         // The block-table entries of the whole KV range were staged in shared memory by all threads; one copy per
         // page brings its K, another its V, each issued by the page's lane.
         bool ok = true;
-        int asked[2] = {0, 0};  // K and V buffers whose copies have been announced
+        int asked[2] = {0, 0};
         long long tprev = TC_NOW(), c_wait = 0, c_issue = 0;
 #pragma unroll 1
         for (int j = 0; j < n_tiles && ok; j++) {
@@ -178,12 +179,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
                 if (lane == 0) TC_ACC(c_issue);
             }
         }
-        // never leave with a copy in flight, whoever gave up (a barrier is in the phase announced last, or past it)
-        if (lane == 0)
-#pragma unroll
-            for (int is_v = 0; is_v < 2; is_v++)
-                for (int i = max(0, asked[is_v] - NB); i < asked[is_v]; i++)
-                    if (!mbar_wait_bounded((is_v ? b_v_full : b_k_full) + (i % NB) * 8, (i / NB) & 1)) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
+        if (lane == 0) { s_asked[0] = asked[0]; s_asked[1] = asked[1]; }
         TC_DUMP(if (lane == 0) { a.dbg_buf[(size_t)blockIdx.x * 16 + 0] = c_wait; a.dbg_buf[(size_t)blockIdx.x * 16 + 1] = c_issue; a.dbg_buf[(size_t)blockIdx.x * 16 + 15] = n_tiles; });
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
@@ -404,6 +400,11 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
     // ---- wind down: everybody meets, then the allocating warp frees the tensor memory
     tc_fence_before();
     __syncthreads();
+    // never leave with a copy in flight if somebody gave up (a barrier is in the phase announced last, or past it)
+    if (tid == 0 && *failed)
+        for (int is_v = 0; is_v < 2; is_v++)
+            for (int i = max(0, s_asked[is_v] - NB); i < s_asked[is_v]; i++) mbar_wait_bounded((is_v ? b_v_full : b_k_full) + (i % NB) * 8, (i / NB) & 1);
+    __syncwarp();
     if (warp == 0) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
@@ -486,6 +487,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     const uint32_t b_p_full = smem_u32(bars + 6), b_o_done = smem_u32(bars + 8);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
     volatile int* failed = reinterpret_cast<volatile int*>(bars + 11);
+    int* s_asked = reinterpret_cast<int*>(bars + 12);  // stages whose copies have been announced (float layers)
     int* s_pages = reinterpret_cast<int*>(bars + 16);
     float* s_xch = reinterpret_cast<float*>(s_pages + kPageCap);  // [2 buffers][2 tiles][128 rows][2 halves]
     // Q8 layout of the stage area: K buffers [0, 64 KB), V buffer [64, 96 KB), raw K ring and the first raw V
@@ -681,7 +683,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     } else if (!Q8 && warp == 0) {
         // ------------------------------------------------------------ TMA producer
         bool ok = true;
-        int asked = 0;  // stages whose copies have been announced
+        int asked = 0;
         long long tprev = TC_NOW(), c_wait = 0, c_issue = 0;
 #pragma unroll 1
         for (int j = 0; j < n_tiles && ok; j++) {
@@ -704,10 +706,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
             }
             if (lane == 0) TC_ACC(c_issue);
         }
-        // never leave with a copy in flight, whoever gave up
-        if (lane == 0)
-            for (int i = max(0, asked - 2); i < asked; i++)
-                if (!mbar_wait_bounded(b_kv_full + (i & 1) * 8, (i >> 1) & 1)) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
+        if (lane == 0) *s_asked = asked;
         TC_DUMP(if (lane == 0) { a.dbg_buf[(size_t)blockIdx.x * 16 + 0] = c_wait; a.dbg_buf[(size_t)blockIdx.x * 16 + 1] = c_issue; a.dbg_buf[(size_t)blockIdx.x * 16 + 15] = n_tiles; });
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
@@ -934,6 +933,10 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     }
     tc_fence_before();
     __syncthreads();
+    // never leave with a copy in flight if somebody gave up
+    if (!Q8 && tid == 0 && *failed)
+        for (int i = max(0, *s_asked - 2); i < *s_asked; i++) mbar_wait_bounded(b_kv_full + (i & 1) * 8, (i >> 1) & 1);
+    __syncwarp();
     if (warp == 0) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
