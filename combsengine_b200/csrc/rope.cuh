@@ -1,4 +1,4 @@
-// Device side of the rotation and the QK norm (rope.cu; the decode kernel and the quantising append apply them too).
+// Device side of the rotation and the QK norm (rope.cu; the decode kernel applies them too, its quantising append included).
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>

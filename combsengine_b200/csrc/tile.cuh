@@ -1,5 +1,5 @@
 // Device helpers of the kernels that stream page tiles through a shared-memory ring and do their math with mma.sync
-// (kernels.cu, short_chunk.cu): barriers and copies, one tile against a block of query columns, int8 tiles.
+// (kernels.cu): barriers and copies, one tile against a block of query columns, int8 tiles, norm and rotation on the way.
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>
