@@ -95,21 +95,26 @@ __device__ __forceinline__ void load_page_pair(uint32_t dst, const CUtensorMap* 
 }
 __device__ __forceinline__ void umma_pair_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void umma_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 // arrives on the barrier at this offset in both CTAs when everything issued before is complete
 __device__ __forceinline__ void commit_pair(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(bar), "h"((uint16_t)3) : "memory");
 }
 
 }  // namespace
@@ -194,7 +199,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
     // q, the pages and the partial-result buffers belong to earlier launches until here; everything above runs under their tail
     pdl_wait();
     pdl_launch_dependents();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const uint32_t tS0 = tmem, tP0 = OWN_P ? tmem + 2 * KT : tmem, tO = tmem + 512 - D;
     constexpr uint32_t PSTRIDE = OWN_P ? KT / 2 : KT;
     static_assert(2 * KT + (OWN_P ? KT : 0) + D <= 512, "tensor memory");
@@ -242,7 +247,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
         if (!ok) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (rank == 0 && lane == 0) {
+        if (rank == 0) {
             const uint32_t id_qk = instr_desc(BF16, 256, KT, false);
             const uint32_t id_pv = instr_desc(BF16, 256, D, true);
             const uint64_t dq = smem_desc(smem_u32(sQ), 16, 1024), dk = smem_desc(smem_u32(sK), 16, XB * 1024), dv = smem_desc(smem_u32(sV), 1024, XBV * 1024);
@@ -251,11 +256,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
             auto wait_for = [&](auto&& f) {
                 uint64_t t0 = 0;
                 for (int n = 0; ok; n++) {
-                    if (f()) return;
+                    if (__all_sync(0xffffffffu, f())) return;
                     if ((n & 63) == 63) {
                         if (*failed) ok = false;
                         if (t0 == 0) t0 = global_ns();
                         else if (global_ns() - t0 > 200000000ull) ok = false;
+                        ok = __all_sync(0xffffffffu, ok);
                     }
                 }
             };
@@ -276,8 +282,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
                 // is free: in both CTAs' registers, or, with P over it, read by a P V issued before.
                 wait_for([&] {
                     if (next_qk < n_tiles && next_qk <= j + (OWN_P ? 2 : 1) &&
-                        (!OWN_P || next_qk < 2 || mbar_test_wait(bar(kBSFree + (next_qk & 1)), ((next_qk - 2) >> 1) & 1)) &&
-                        mbar_test_wait(bar(kBKFull + next_qk % NB), (next_qk / NB) & 1))
+                        __all_sync(0xffffffffu, (!OWN_P || next_qk < 2 || mbar_test_wait(bar(kBSFree + (next_qk & 1)), ((next_qk - 2) >> 1) & 1)) &&
+                        mbar_test_wait(bar(kBKFull + next_qk % NB), (next_qk / NB) & 1)))
                         issue_qk(next_qk++);
                     return next_qk > j && mbar_test_wait(bar(kBPFull + (j & 1)), (j >> 1) & 1);
                 });
@@ -292,7 +298,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
                 commit_pair(bar(kBVEmpty + st));
                 commit_pair(bar(kBODone + (j & 1)));
             }
-            if (!ok) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
+            if (!ok && lane == 0) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
         }
     } else {
         // ------------------------------------------------------------ softmax + epilogue

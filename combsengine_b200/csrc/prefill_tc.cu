@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
     // tensor memory, the work record and the block table, which came with the step's upload) runs under their tail
     pdl_wait();
     pdl_launch_dependents();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const uint32_t tS0 = tmem, tQ = tmem + 2 * KT, tO = tmem + 512 - D;
     static_assert(2 * KT + D / 2 + D <= 512, "tensor memory");
     // ---- Q goes to tensor memory (the A operand of S, packed pairs like P): from shared memory the 128-row A and the
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
         TC_DUMP(if (lane == 0) { a.dbg_buf[(size_t)blockIdx.x * 16 + 0] = c_wait; a.dbg_buf[(size_t)blockIdx.x * 16 + 1] = c_issue; a.dbg_buf[(size_t)blockIdx.x * 16 + 15] = n_tiles; });
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
             const uint32_t id_qk = instr_desc(BF16, 128, KT, false);
             const uint32_t id_pv = instr_desc(BF16, 128, D, true);
             // descriptors differ only in the start address field (bits 0-13, address >> 4); 8-token groups of K and V
@@ -207,22 +207,23 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
                 // other: a P V held up by a K that is still on its way would hold up the V buffer it frees.
                 uint64_t t0 = 0;
                 for (int n = 0;; n++) {
-                    if (next_qk <= j + 1 && next_qk < n_tiles && mbar_test_wait(b_k_full + (next_qk % NB) * 8, (next_qk / NB) & 1)) {
+                    if (next_qk <= j + 1 && next_qk < n_tiles && __all_sync(0xffffffffu, mbar_test_wait(b_k_full + (next_qk % NB) * 8, (next_qk / NB) & 1))) {
                         TC_ACC(c_wkv);
                         tc_fence_after();
                         issue_qk(next_qk++);
                         TC_ACC(c_iss);
                     }
-                    if (next_qk > j && mbar_test_wait(b_p_full + (j & 1) * 8, (j >> 1) & 1)) break;
+                    if (next_qk > j && __all_sync(0xffffffffu, mbar_test_wait(b_p_full + (j & 1) * 8, (j >> 1) & 1))) break;
                     if ((n & 63) == 63) {
                         if (*failed) ok = false;
                         if (t0 == 0) t0 = global_ns();
                         else if (global_ns() - t0 > 200000000ull) ok = false;
+                        ok = __all_sync(0xffffffffu, ok);
                         if (!ok) break;
                     }
                 }
                 TC_ACC(c_wp);
-                if (ok) ok = mbar_wait_bounded(b_v_full + (j % NB) * 8, (j / NB) & 1) && !*failed;
+                if (ok) ok = __all_sync(0xffffffffu, mbar_wait_bounded(b_v_full + (j % NB) * 8, (j / NB) & 1) && !*failed);
                 TC_ACC(c_wkv);
                 if (!ok) break;
                 tc_fence_after();
@@ -235,8 +236,8 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
                 umma_commit(b_o_done);
                 TC_ACC(c_iss);
             }
-            if (!ok) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
-            TC_DUMP(a.dbg_buf[(size_t)blockIdx.x * 16 + 2] = c_wkv; a.dbg_buf[(size_t)blockIdx.x * 16 + 3] = c_wp; a.dbg_buf[(size_t)blockIdx.x * 16 + 4] = c_iss;);
+            if (!ok && lane == 0) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
+            TC_DUMP(if (lane == 0) { a.dbg_buf[(size_t)blockIdx.x * 16 + 2] = c_wkv; a.dbg_buf[(size_t)blockIdx.x * 16 + 3] = c_wp; a.dbg_buf[(size_t)blockIdx.x * 16 + 4] = c_iss; });
         }
     } else {
         // ------------------------------------------------------------ softmax + epilogue: two threads per row
@@ -568,7 +569,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
     if (Q8 && warp >= 18) {
         // ------------------------------------------------------------ int8 layer: warp 18 feeds K, warp 19 feeds V
@@ -710,7 +711,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         TC_DUMP(if (lane == 0) { a.dbg_buf[(size_t)blockIdx.x * 16 + 0] = c_wait; a.dbg_buf[(size_t)blockIdx.x * 16 + 1] = c_issue; a.dbg_buf[(size_t)blockIdx.x * 16 + 15] = n_tiles; });
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
             const uint32_t id_qk = instr_desc(BF16, 128, 128, false);
             const uint32_t id_pv = instr_desc(BF16, 128, D, true);
             // float layer: a stage holds pages as they lie in device memory (K and V rows of a page interleaved in
@@ -737,20 +738,20 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                 umma_commit(b_o_done + X * 8);
             };
             long long tprev = TC_NOW(), c_wkv = 0, c_wp = 0, c_iss = 0, c_pv = 0;
-            bool ok = mbar_wait_bounded(b_kv_full, 0);
+            bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(b_kv_full, 0));
             if (ok) { tc_fence_after(); issue_qk(0, 0); if (two) issue_qk(1, 0); }
             for (int j = 0; ok && j < n_tiles; j++) {
                 TC_ACC(c_iss);
-                ok = mbar_wait_bounded(b_p_full, j & 1) && !*failed;
+                ok = __all_sync(0xffffffffu, mbar_wait_bounded(b_p_full, j & 1) && !*failed);
                 TC_ACC(c_wp);
-                if (Q8 && ok) { ok = mbar_wait_bounded(b_v_full, j & 1); TC_ACC(c_wkv); }
+                if (Q8 && ok) { ok = __all_sync(0xffffffffu, mbar_wait_bounded(b_v_full, j & 1)); TC_ACC(c_wkv); }
                 if (!ok) break;
                 tc_fence_after();
                 issue_pv(0, j);
                 TC_ACC(c_pv);
                 if (!two && !Q8) umma_commit(b_kv_empty + (j & 1) * 8);
                 if (j + 1 < n_tiles) {
-                    ok = mbar_wait_bounded(b_kv_full + ((j + 1) & 1) * 8, ((j + 1) >> 1) & 1);
+                    ok = __all_sync(0xffffffffu, mbar_wait_bounded(b_kv_full + ((j + 1) & 1) * 8, ((j + 1) >> 1) & 1));
                     TC_ACC(c_wkv);
                     if (!ok) break;
                     tc_fence_after();
@@ -758,7 +759,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                 }
                 TC_ACC(c_iss);
                 if (two) {
-                    ok = mbar_wait_bounded(b_p_full + 8, j & 1) && !*failed;
+                    ok = __all_sync(0xffffffffu, mbar_wait_bounded(b_p_full + 8, j & 1) && !*failed);
                     TC_ACC(c_wp);
                     if (!ok) break;
                     tc_fence_after();
@@ -769,10 +770,10 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                 if (two || Q8) umma_commit(Q8 ? b_v_empty : b_kv_empty + (j & 1) * 8);
                 if (two && j + 1 < n_tiles) issue_qk(1, j + 1);
             }
-            if (!ok) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
+            if (!ok && lane == 0) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
             (void)c_pv;
-            TC_DUMP(a.dbg_buf[(size_t)blockIdx.x * 16 + 2] = c_wkv; a.dbg_buf[(size_t)blockIdx.x * 16 + 3] = c_wp; a.dbg_buf[(size_t)blockIdx.x * 16 + 4] = c_iss;
-                    a.dbg_buf[(size_t)blockIdx.x * 16 + 11] = c_pv;);
+            TC_DUMP(if (lane == 0) { a.dbg_buf[(size_t)blockIdx.x * 16 + 2] = c_wkv; a.dbg_buf[(size_t)blockIdx.x * 16 + 3] = c_wp; a.dbg_buf[(size_t)blockIdx.x * 16 + 4] = c_iss;
+                    a.dbg_buf[(size_t)blockIdx.x * 16 + 11] = c_pv; });
         }
     } else if (warp >= 2 && warp < (two ? 18 : 10)) {
         // ------------------------------------------------------------ softmax + epilogue of tile X, half H of the keys
