@@ -735,7 +735,7 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
         ProfScope ps(d, st);
         { int32_t frc = flush_uploads(d, st); if (frc) return frc; }
         if (tp->launch.pair) CU_TRY(launch_chunk_pair(KV->map_page, KV->map_vhalf, args, bf16, d->pdl, st));
-        else if (use_tc2) CU_TRY(q8_direct ? launch_chunk_tc2(L.map_k16, L.map_sc, args, bf16, d->pdl, st) : launch_chunk_tc2(KV->map_kv, KV->map_kv, args, bf16, d->pdl, st));
+        else if (use_tc2) CU_TRY(q8_direct ? launch_chunk_tc2(L.map_k16, L.map_sc, args, bf16, d->pdl, st) : launch_chunk_tc2(KV->map_page, KV->map_page, args, bf16, d->pdl, st));
         else CU_TRY(launch_chunk_tc(KV->map_page, args, bf16, d->pdl, st));
         g_launches++;
         d->last_kv_writer = -1;

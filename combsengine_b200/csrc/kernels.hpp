@@ -221,7 +221,7 @@ cudaError_t chunk_tc_init();
 cudaError_t launch_chunk_tc(const CUtensorMap& map, const ChunkArgs& a, bool bf16, bool overlap, cudaStream_t st);
 // two query tiles per CTA, P in tensor memory (head_dim 128)
 bool chunk_tc2_supported(int d);
-// float layer: `map` = the layer's map_kv, map_sc is not used; int8 layer (a.q8_arena non-null): its map_k16 and map_sc
+// float layer: `map` = the layer's map_page, map_sc is not used; int8 layer (a.q8_arena non-null): its map_k16 and map_sc
 cudaError_t launch_chunk_tc2(const CUtensorMap& map, const CUtensorMap& map_sc, const ChunkArgs& a, bool bf16, bool overlap, cudaStream_t st);
 // pairs of SMs (chunk_pair.cu): head_dim 128 or 256; map_k = the layer's map_page, map_v its map_vhalf; one work item per
 // two query tiles

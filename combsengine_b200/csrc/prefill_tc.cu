@@ -425,20 +425,21 @@ static cudaError_t launch_tc(const CUtensorMap& map, const ChunkArgs& a, bool ov
 // memory (it overwrites the first 64 columns of its S tile as packed 16-bit pairs and is the
 // A operand of the P V product), so no shared memory is spent on P.
 //
-//   warp 0        TMA producer: K and V of a tile in one stage, a box of both per page and 64 columns
+//   warp 0        TMA producer: two K and two V buffers, one copy per page of each
 //   warp 1        MMA issuer:  QK_A, QK_B, then per K/V tile  PV_A, QK_A', PV_B, QK_B'
 //   warps 2..9    softmax of tile A        warps 10..17  softmax of tile B
 //
-// A tile's softmax is the longest link of the chain QK -> softmax -> PV, and that chain, not the tensor pipe,
-// set the pace with one thread per row.  Two threads share a row now: the warps of a tile come in pairs that
-// may touch the same quarter of the tensor-memory lanes; one takes keys 0-63 of the tile, the other keys
-// 64-127 (and, when the row maximum moves, the matching half of the O columns).  They exchange their half-row
-// maxima through shared memory once per tile and their half-row sums once at the end.
+// A tile's softmax is the longest link of the chain QK -> softmax -> PV, and that chain sets the pace.  Two threads share
+// a row: the warps of a tile come in pairs that may touch the same quarter of the tensor-memory lanes; H = 0 takes keys
+// 0-31 and 64-95 of the tile, H = 1 the others (and, when the row maximum moves, the matching half of the O columns).
+// They exchange their maxima through shared memory once per tile and their sums once at the end.  P is handed over in two
+// halves, so that P V of keys 0-63 runs under the exponentials of keys 64-127 and only 256 of its 512 cycles are part of the chain.
 //
-// K and V in buffers of their own, as in the kernel above, with the producer started before Q is in place, gain
-// nothing here, where two tiles of work per load hide its wait, and cost another barrier per tile: 8 prompts of 8192
-// tokens over four layers 23.9 ms against 23.5, 6 ragged prompts over int8 pages 4.46 against 4.38, verification of
-// 16 drafts 3.06 against 3.02.
+// K and V have buffers of their own: K of the tile after next is asked for when the scores of this one are computed, and so has
+// one and a half tiles of time to arrive; in one buffer with V, which is read last, it had half of one (without softmax a
+// launch of 512 items of 62 K/V tiles took 546 us with copies, 379 without).  The same launch, softmax and all: 630 us with one
+// buffer, one lane issuing, P handed over whole and a load of the scores at a time, 543 now (981 TFLOP/s; a chain of 3700 cycles
+// per tile, 2048 of them MMA).  Verification of drafts, 8 sequences x 5 tokens after 512 to 6144, 28 layers: 1642 -> 1465 us.
 //
 // Tensor memory: S_A [0,128), S_B [128,256), O_A [256,384), O_B [384,512).
 constexpr int kThreads2 = 576;
@@ -476,20 +477,20 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     static_assert(D == 128, "two-tile kernel: head_dim 128");
     constexpr uint32_t TILE = 128u * D * 2u;   // one Q tile
     constexpr uint32_t BLK = 128u * 128u;      // 64-column block of a Q tile
-    constexpr int XB = D / 64;
-    constexpr uint32_t BLKKV = 8u * 4096u;     // 64-column block of a K/V stage
-    constexpr uint32_t STAGE = 2u * TILE;
+    constexpr int XB = D / 64, NV = Q8 ? 1 : 2;  // column blocks of a row, V buffers
+    constexpr uint32_t KVB = 128u * D * 2u;    // a K or V buffer
+    constexpr uint32_t PGB = 16u * D * 2u;     // a page in it
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sQ = smem;                 // Q_A then Q_B
-    uint8_t* sKV = sQ + 2 * TILE;       // 2 stages
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + 2 * STAGE);
-    // barriers: kv_full[2], kv_empty[2], s_full[A,B], p_full[A,B], o_done[A,B]
-    const uint32_t b_kv_full = smem_u32(bars + 0), b_kv_empty = smem_u32(bars + 2), b_s_full = smem_u32(bars + 4);
-    const uint32_t b_p_full = smem_u32(bars + 6), b_o_done = smem_u32(bars + 8);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
-    volatile int* failed = reinterpret_cast<volatile int*>(bars + 11);
-    int* s_asked = reinterpret_cast<int*>(bars + 12);  // stages whose copies have been announced (float layers)
-    int* s_pages = reinterpret_cast<int*>(bars + 16);
+    uint8_t* sKV = sQ + 2 * TILE;       // two K buffers, two V buffers: [page][8-token group][column block][8 rows of 128 bytes]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + 4 * KVB);
+    const uint32_t b_k_full = smem_u32(bars + 0), b_k_empty = smem_u32(bars + 2), b_v_full = smem_u32(bars + 4), b_v_empty = smem_u32(bars + 6);
+    const uint32_t b_s_full = smem_u32(bars + 8), b_p_full = smem_u32(bars + 10) /* [tile][half of the keys] */, b_o_done = smem_u32(bars + 14);
+    const uint32_t b_q_full = smem_u32(bars + 16);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
+    volatile int* failed = reinterpret_cast<volatile int*>(bars + 18);  // and the ticket
+    int* s_asked = reinterpret_cast<int*>(bars + 19);  // K and V buffers whose copies have been announced (float layers)
+    int* s_pages = reinterpret_cast<int*>(bars + 32);
     float* s_xch = reinterpret_cast<float*>(s_pages + kPageCap);  // [2 buffers][2 tiles][128 rows][2 halves]
     // Q8 layout of the stage area: K buffers [0, 64 KB), V buffer [64, 96 KB), raw K ring and the first raw V
     // slots [96, 128 KB); the other raw V slots and the Q8 barriers follow the exchange area.  A K or V buffer
@@ -498,13 +499,13 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     constexpr uint32_t HALF = 16u * D + 16u * (D / 32) * 2u;              // a record's K or V values with their scales
     static_assert(HALF == (uint32_t)(REC / 2), "half a record");
     constexpr uint32_t QBUF = 128u * D * 2u, QBLK = QBUF / 2;          // one K or V buffer, one 64-column block of it
-    static_assert(!Q8 || kRawK * HALF + kRawVInStage * HALF <= 2 * STAGE - 3 * QBUF, "raw rings in the freed quarter");
+    static_assert(!Q8 || kRawK * HALF + kRawVInStage * HALF <= 4 * KVB - 3 * QBUF, "raw rings in the freed quarter");
     uint8_t* sRawK = sKV + 3 * QBUF;
     uint8_t* sRawV0 = sRawK + kRawK * HALF;
     uint8_t* sRawV1 = reinterpret_cast<uint8_t*>(s_xch + 2 * 2 * 128 * 2) + 128;  // 128-byte aligned, as every slot is
     const uint32_t b_q8 = smem_u32(sRawV1 + (kRawV - kRawVInStage) * HALF);
-    const uint32_t b_v_full = b_q8, b_v_empty = b_q8 + 8, b_rawk = b_q8 + 16, b_rawv = b_rawk + kRawK * 8;
-    (void)sRawK; (void)sRawV0; (void)sRawV1; (void)b_v_full; (void)b_v_empty; (void)b_rawk; (void)b_rawv; (void)REC;
+    const uint32_t b_rawk = b_q8, b_rawv = b_rawk + kRawK * 8;
+    (void)sRawK; (void)sRawV0; (void)sRawV1; (void)b_rawk; (void)b_rawv; (void)REC;
 
     const long long t_entry = TC_NOW();
     (void)t_entry;
@@ -529,13 +530,12 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
 
     if (tid == 0) {
         for (int i = 0; i < 2; i++) {
-            mbar_init(b_kv_full + i * 8, 1); mbar_init(b_kv_empty + i * 8, 1); mbar_init(b_s_full + i * 8, 1);
-            mbar_init(b_p_full + i * 8, 256); mbar_init(b_o_done + i * 8, 1);
+            mbar_init(b_k_full + i * 8, 1); mbar_init(b_k_empty + i * 8, 1); mbar_init(b_v_full + i * 8, 1); mbar_init(b_v_empty + i * 8, 1);
+            mbar_init(b_s_full + i * 8, 1); mbar_init(b_p_full + i * 16, 8); mbar_init(b_p_full + i * 16 + 8, 8); mbar_init(b_o_done + i * 8, 1);
         }
-        if constexpr (Q8) {  // kv_full / kv_empty above are K's here
-            mbar_init(b_v_full, 1); mbar_init(b_v_empty, 1);
+        mbar_init(b_q_full, 16);
+        if constexpr (Q8)
             for (int i = 0; i < kRawK + kRawV; i++) mbar_init(b_rawk + i * 8, 1);
-        }
         *failed = 0;
         for (int i = 0; i < 8; i++) reinterpret_cast<int*>(s_xch + 2 * 2 * 128 * 2)[i] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -547,14 +547,20 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     for (int i = tid; i <= p_hi - p_lo && i < kPageCap; i += (int)blockDim.x) s_pages[i] = a.step.tables[sm.tbl_off + p_lo + i];
+    tc_fence_before();
+    __syncthreads();  // barriers and block table are ready: the producer starts while the softmax warps bring Q
+    tc_fence_after();
     // q, the pages and the partial-result buffers belong to earlier launches until here; everything above (barriers,
     // tensor memory, the work record and the block table, which came with the step's upload) runs under their tail
     pdl_wait();
     pdl_launch_dependents();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+
     // ---- Q tiles: row m of tile X is q head (m / TPT) at token r0 + X TPT + m % TPT
-    {
+    if (warp >= 2 && warp < 18) {
         const uint16_t* qbase = reinterpret_cast<const uint16_t*>(a.q) + (size_t)sm.tok_off * a.geo.n_q * D;
-        for (int c = tid; c < (two ? 256 : 128) * (D / 8); c += (int)blockDim.x) {
+#pragma unroll 4
+        for (int c = tid - 64; c < (two ? 256 : 128) * (D / 8); c += 512) {
             const int mm = c / (D / 8), j = c - mm * (D / 8);
             const int X = mm >> 7, m = mm & 127;
             const int rep = m / TPT, r = r0 + X * TPT + (m - rep * TPT);
@@ -564,12 +570,10 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
             const uint32_t off = X * TILE + (j >> 3) * BLK + m * 128u + (((j & 7) ^ (m & 7)) << 4);
             *reinterpret_cast<uint4*>(sQ + off) = val;
         }
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(b_q_full);
     }
-    fence_proxy_async();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
     if (Q8 && warp >= 18) {
         // ------------------------------------------------------------ int8 layer: warp 18 feeds K, warp 19 feeds V
@@ -632,7 +636,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
             const int j = n >> 3, pg = n & 7;
             if (lane == 0) {
                 if (pg == 0) {  // the buffer this tile goes to must have been read to the end
-                    if (!is_v && j >= 2 && !mbar_wait_bounded(b_kv_empty + (j & 1) * 8, ((j >> 1) - 1) & 1)) ok = false;
+                    if (!is_v && j >= 2 && !mbar_wait_bounded(b_k_empty + (j & 1) * 8, ((j >> 1) - 1) & 1)) ok = false;
                     if (is_v && j >= 1 && !mbar_wait_bounded(b_v_empty, (j - 1) & 1)) ok = false;
                 }
                 if (ok && !mbar_wait_bounded(b_raw + sl * 8, ph)) ok = false;
@@ -667,7 +671,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
             if (lane == 0) {
                 TC_ACC(c_meet);
                 if (issued < n_recs) issue(issued, sl);
-                if (pg == 7) mbar_arrive(is_v ? b_v_full : b_kv_full + (j & 1) * 8);
+                if (pg == 7) mbar_arrive(is_v ? b_v_full : b_k_full + (j & 1) * 8);
                 TC_ACC(c_issue);
             }
             if (issued < n_recs) issued++;
@@ -684,91 +688,93 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     } else if (!Q8 && warp == 0) {
         // ------------------------------------------------------------ TMA producer
         bool ok = true;
-        int asked = 0;
+        int asked[2] = {0, 0};
         long long tprev = TC_NOW(), c_wait = 0, c_issue = 0;
 #pragma unroll 1
         for (int j = 0; j < n_tiles && ok; j++) {
             const int st = j & 1;
-            if (lane == 0) {
-                if (j >= 2 && !mbar_wait_bounded(b_kv_empty + st * 8, ((j >> 1) - 1) & 1)) ok = false;
-                TC_ACC(c_wait);
-                if (*failed) ok = false;
-                if (ok) { mbar_expect_tx(b_kv_full + st * 8, STAGE); asked++; }
-                else { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
-            }
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-            if (!ok) break;
-            for (int bx = lane; bx < 8 * XB; bx += 32) {
-                const int pg = bx / XB, x = bx - pg * XB;
-                const int idx = min(j * 8 + pg, p_hi - p_lo);  // pages past the end repeat the last one (masked)
-                int phys = idx < kPageCap ? s_pages[idx] : a.step.tables[sm.tbl_off + p_lo + idx];
+            // pages past the last visible one repeat it: finite data that the causal mask hides
+            int phys = 0;
+            if (lane < 8) {
+                const int idx = min(j * 8 + lane, p_hi - p_lo);
+                phys = idx < kPageCap ? s_pages[idx] : a.step.tables[sm.tbl_off + p_lo + idx];
                 if (phys < 0 || phys >= a.geo.num_pages) { atomicOr(a.status, ST_BAD_PAGE); phys = 0; }
-                tma_load_2d(smem_u32(sKV + st * STAGE + x * BLKKV + pg * 4096), &tmap32, x * 64, (phys * Hkv + h) * 32, b_kv_full + st * 8);
             }
-            if (lane == 0) TC_ACC(c_issue);
+#pragma unroll
+            for (int is_v = 0; is_v < 2 && ok; is_v++) {
+                const uint32_t full = (is_v ? b_v_full : b_k_full) + st * 8, empty = (is_v ? b_v_empty : b_k_empty) + st * 8;
+                if (lane == 0) {
+                    if (j >= 2 && !mbar_wait_bounded(empty, ((j >> 1) - 1) & 1)) ok = false;
+                    TC_ACC(c_wait);
+                    if (*failed) ok = false;
+                    if (ok) { mbar_expect_tx(full, KVB); asked[is_v]++; }
+                    else { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
+                }
+                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                if (ok && lane < 8) tma_load_page(smem_u32(sKV + (2 * is_v + st) * KVB + lane * PGB), &tmap32, is_v, (phys * Hkv + h) * 2, full);
+                if (lane == 0) TC_ACC(c_issue);
+            }
         }
-        if (lane == 0) *s_asked = asked;
+        if (lane == 0) { s_asked[0] = asked[0]; s_asked[1] = asked[1]; }
         TC_DUMP(if (lane == 0) { a.dbg_buf[(size_t)blockIdx.x * 16 + 0] = c_wait; a.dbg_buf[(size_t)blockIdx.x * 16 + 1] = c_issue; a.dbg_buf[(size_t)blockIdx.x * 16 + 15] = n_tiles; });
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         {
             const uint32_t id_qk = instr_desc(BF16, 128, 128, false);
             const uint32_t id_pv = instr_desc(BF16, 128, D, true);
-            // float layer: a stage holds pages as they lie in device memory (K and V rows of a page interleaved in
-            // groups of eight); int8 layer: the loader warps lay K and V out separately (see the shared memory map)
-            constexpr uint32_t KBUF = Q8 ? QBUF : STAGE, KBLK = Q8 ? QBLK : BLKKV, GRP = Q8 ? 1024u : 2048u, VPAGE = Q8 ? 2048u : 4096u;
+            // 8-token groups of K and V, their 64-wide column blocks, and a page of V are this far apart in a buffer
+            constexpr uint32_t GRP = Q8 ? 1024u : XB * 1024u, CBLK = Q8 ? QBLK : 1024u, VPAGE = Q8 ? 2048u : PGB;
             const uint64_t dq = smem_desc(smem_u32(sQ), 16, 1024), dk = smem_desc(smem_u32(sKV), 16, GRP);
-            const uint64_t dv = smem_desc(smem_u32(sKV) + (Q8 ? 2 * QBUF : 1024u), KBLK, GRP);
+            const uint64_t dv = smem_desc(smem_u32(sKV) + 2 * KVB, CBLK, GRP);
+            const int last_x = two ? 1 : 0;
+            auto wait = [&](uint32_t bar, int parity) -> bool { return __all_sync(0xffffffffu, mbar_wait_unless(bar, parity, failed)); };
             auto issue_qk = [&](int X, int j) {
-                const uint64_t kst = (uint64_t)(((j & 1) * KBUF) >> 4), qst = (uint64_t)((X * TILE) >> 4);
+                const uint64_t kst = (uint64_t)(((j & 1) * KVB) >> 4), qst = (uint64_t)((X * TILE) >> 4);
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ks++) {
                     const uint64_t qoff = (uint64_t)(((ks >> 2) * BLK + (ks & 3) * 32) >> 4);
-                    const uint64_t koff = (uint64_t)(((ks >> 2) * KBLK + (ks & 3) * 32) >> 4);
+                    const uint64_t koff = (uint64_t)(((ks >> 2) * CBLK + (ks & 3) * 32) >> 4);
                     umma(tmem + X * 128, dq + qst + qoff, dk + kst + koff, id_qk, ks > 0);
                 }
                 umma_commit(b_s_full + X * 8);
-                if (Q8 && X == (two ? 1 : 0)) umma_commit(b_kv_empty + (j & 1) * 8);  // all scores of this K buffer have been issued
-            };
-            auto issue_pv = [&](int X, int j) {
-                const uint64_t vst = Q8 ? 0ull : (uint64_t)(((j & 1) * STAGE) >> 4);
-#pragma unroll
-                for (int ks = 0; ks < 8; ks++)  // 16 keys = one page per step; P: 8 packed columns per step
-                    umma_ts(tmem + 256 + X * 128, tmem + X * 128 + ks * 8, dv + vst + (uint64_t)((ks * VPAGE) >> 4), id_pv, (j > 0 || ks > 0));
-                umma_commit(b_o_done + X * 8);
+                if (X == last_x) umma_commit(b_k_empty + (j & 1) * 8);  // all scores of this K buffer have been issued
             };
             long long tprev = TC_NOW(), c_wkv = 0, c_wp = 0, c_iss = 0, c_pv = 0;
-            bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(b_kv_full, 0));
+            bool ok = wait(b_q_full, 0) && wait(b_k_full, 0);
             if (ok) { tc_fence_after(); issue_qk(0, 0); if (two) issue_qk(1, 0); }
+#pragma unroll 1
             for (int j = 0; ok && j < n_tiles; j++) {
                 TC_ACC(c_iss);
-                ok = __all_sync(0xffffffffu, mbar_wait_bounded(b_p_full, j & 1) && !*failed);
-                TC_ACC(c_wp);
-                if (Q8 && ok) { ok = __all_sync(0xffffffffu, mbar_wait_bounded(b_v_full, j & 1)); TC_ACC(c_wkv); }
-                if (!ok) break;
-                tc_fence_after();
-                issue_pv(0, j);
-                TC_ACC(c_pv);
-                if (!two && !Q8) umma_commit(b_kv_empty + (j & 1) * 8);
-                if (j + 1 < n_tiles) {
-                    ok = __all_sync(0xffffffffu, mbar_wait_bounded(b_kv_full + ((j + 1) & 1) * 8, ((j + 1) >> 1) & 1));
-                    TC_ACC(c_wkv);
+                const int vs = NV == 2 ? (j & 1) : 0;
+                const uint64_t vst = (uint64_t)((vs * KVB) >> 4);
+                ok = wait(b_v_full + vs * 8, NV == 2 ? (j >> 1) & 1 : j & 1);
+                TC_ACC(c_wkv);
+#pragma unroll
+                for (int X = 0; X < 2; X++) {
+                    if (X > last_x || !ok) break;
+#pragma unroll
+                    for (int half = 0; half < 2; half++) {  // P of the tile's first 64 keys, of the others
+                        if (ok) ok = wait(b_p_full + X * 16 + half * 8, j & 1);
+                        TC_ACC(c_wp);
+                        if (!ok) break;
+                        tc_fence_after();
+#pragma unroll
+                        for (int ks = half * 4; ks < half * 4 + 4; ks++)  // 16 keys = one page per step; P: 8 packed columns per step
+                            umma_ts(tmem + 256 + X * 128, tmem + X * 128 + ks * 8, dv + vst + (uint64_t)((ks * VPAGE) >> 4), id_pv, (j > 0 || ks > 0));
+                        TC_ACC(c_pv);
+                    }
                     if (!ok) break;
-                    tc_fence_after();
-                    issue_qk(0, j + 1);
+                    if (X == last_x) umma_commit(b_v_empty + vs * 8);  // every read of this V buffer has been issued
+                    if (j + 1 == n_tiles) { umma_commit(b_o_done + X * 8); continue; }
+                    if (X == 0) {
+                        ok = wait(b_k_full + ((j + 1) & 1) * 8, ((j + 1) >> 1) & 1);
+                        TC_ACC(c_wkv);
+                        if (!ok) break;
+                        tc_fence_after();
+                    }
+                    issue_qk(X, j + 1);
+                    TC_ACC(c_iss);
                 }
-                TC_ACC(c_iss);
-                if (two) {
-                    ok = __all_sync(0xffffffffu, mbar_wait_bounded(b_p_full + 8, j & 1) && !*failed);
-                    TC_ACC(c_wp);
-                    if (!ok) break;
-                    tc_fence_after();
-                    issue_pv(1, j);
-                    TC_ACC(c_pv);
-                }
-                // every read of this stage (int8 layer: of the V buffer) has been issued before
-                if (two || Q8) umma_commit(Q8 ? b_v_empty : b_kv_empty + (j & 1) * 8);
-                if (two && j + 1 < n_tiles) issue_qk(1, j + 1);
             }
             if (!ok && lane == 0) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
             (void)c_pv;
@@ -797,33 +803,24 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         const long long tstart = tprev;
 #pragma unroll 1
         for (int j = 0; j < n_tiles; j++) {
-            ok = mbar_wait_bounded(b_s_full + X * 8, j & 1) && !*failed;
+            ok = mbar_wait_unless(b_s_full + X * 8, j & 1, failed);
             ok = __all_sync(0xffffffffu, ok);
             TC_ACC(c_ws);
             if (!ok && lane == 0) *pair_failed = 1;  // the loads below then read stale columns: harmless, nothing is kept
             tc_fence_after();
-            const int kbase = k0 + j * 128 + H * 64;
-            const bool need_mask = (kbase + 63 > qx_min) || (a.window > 0 && kbase + a.window <= max(qx_max, qx_min));
-            // this half of the row of S in registers: maximum, exponentials, packed P back over the S columns
+            // this thread's keys: 32 H .. 32 H + 31 of the tile's first 64 and of its last 64
+            const int kbase = k0 + j * 128 + H * 32;
+            const bool need_mask = (kbase + 95 > qx_min) || (a.window > 0 && kbase + a.window <= max(qx_max, qx_min));
             uint32_t sv[64];
-            tmem_ld_row<64>(tS + H * 64, sv);
+            tmem_ld32x2(tS + H * 32, tS + 64 + H * 32, sv);
             if (need_mask) {
 #pragma unroll
                 for (int e = 0; e < 64; e++) {
-                    const int kp = kbase + e;
+                    const int kp = kbase + e + (e & 32);
                     if (!(kp <= q_pos && (a.window <= 0 || kp + a.window > q_pos))) sv[e] = 0xff800000u;  // -inf
                 }
             }
-            float mx;
-            {
-                float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
-#pragma unroll
-                for (int e = 0; e < 64; e += 4) {
-                    m0 = fmaxf(m0, __uint_as_float(sv[e])); m1 = fmaxf(m1, __uint_as_float(sv[e + 1]));
-                    m2 = fmaxf(m2, __uint_as_float(sv[e + 2])); m3 = fmaxf(m3, __uint_as_float(sv[e + 3]));
-                }
-                mx = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
-            }
+            float mx = max_of(sv);
             // the other half's maximum (double-buffered by tile parity: the partner may still be reading the
             // previous tile's entry when this one is written only if it were two tiles behind, which the
             // barrier of the tile in between rules out)
@@ -839,19 +836,11 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                 m_ref = mx;
             }
             const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
-            float sum = 0.f, sum2 = 0.f;
-#pragma unroll
-            for (int e = 0; e < 64; e += 2) {
-                const float p0 = ex2_approx(fmaf(__uint_as_float(sv[e]), a.scale_log2, -m_use));
-                const float p1 = ex2_approx(fmaf(__uint_as_float(sv[e + 1]), a.scale_log2, -m_use));
-                if (e & 2) sum2 += p0 + p1; else sum += p0 + p1;
-                sv[e >> 1] = pack2<BF16>(p0, p1);  // P pair e/2 reuses a register whose score is already consumed
-            }
-#pragma unroll
-            for (int c = 0; c < 2; c++) tmem_st16(tS + H * 32 + c * 16, sv + c * 16);  // keys 64 H .. 64 H + 63 are packed columns 32 H .. 32 H + 31 of P
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            l_run = l_run * alpha + (sum + sum2);
-            TC_ACC(c_exp);
+            const uint64_t scale2 = f32x2(a.scale_log2, a.scale_log2), neg_ref2 = f32x2(-m_use, -m_use);
+            uint64_t sum[2] = {0ull, 0ull};
+            uint32_t pk[16];
+            exp_pack<32, BF16>(sv, scale2, neg_ref2, sum, pk);
+            tmem_st16(tS + H * 16, pk);  // P of keys 32 H .. : packed columns 16 H ..
             // S_X being full means P V_X of the previous tile has completed (the tensor pipe runs in
             // order), so O_X may be rescaled now: this warp takes the O columns 64 H .. 64 H + 63
             if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
@@ -864,8 +853,18 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                     tmem_st32(tO + H * 64 + c * 32, ov);
                 }
             }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc_fence_before();
-            mbar_arrive(b_p_full + X * 8);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(b_p_full + X * 16);  // P V of the first 64 keys runs under the others' exponentials
+            TC_ACC(c_exp);
+            exp_pack<32, BF16>(sv + 32, scale2, neg_ref2, sum, pk);
+            tmem_st16(tS + 32 + H * 16, pk);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            l_run = l_run * alpha + sum_of(sum);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(b_p_full + X * 16 + 8);
             TC_ACC(c_st);
         }
         TC_DUMP(if (tid == 64) {
@@ -875,8 +874,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         });
         const long long t_loop_end = TC_NOW();
         (void)tstart; (void)c_wo; (void)t_loop_end;
-        // (this tile's last scores were issued after its P V of tile n - 2: the wait is one phase ahead, see chunk_tc_kernel)
-        if (ok) ok = mbar_wait_bounded(b_o_done + X * 8, (n_tiles - 1) & 1) && !*failed;
+        if (ok) ok = mbar_wait_bounded(b_o_done + X * 8, 0) && !*failed;
         ok = __all_sync(0xffffffffu, ok);
         // the row sum is the two halves' sums (exchanged whether or not the wait succeeded: the pair must
         // meet at its barrier the same number of times)
@@ -936,7 +934,8 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     __syncthreads();
     // never leave with a copy in flight if somebody gave up
     if (!Q8 && tid == 0 && *failed)
-        for (int i = max(0, *s_asked - 2); i < *s_asked; i++) mbar_wait_bounded(b_kv_full + (i & 1) * 8, (i >> 1) & 1);
+        for (int is_v = 0; is_v < 2; is_v++)
+            for (int i = max(0, s_asked[is_v] - 2); i < s_asked[is_v]; i++) mbar_wait_bounded((is_v ? b_v_full : b_k_full) + (i & 1) * 8, (i >> 1) & 1);
     __syncwarp();
     if (warp == 0) {
         tc_fence_after();

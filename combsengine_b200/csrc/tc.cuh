@@ -47,6 +47,17 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
         if (global_ns() - t0 > limit_ns) return false;
     }
 }
+// The same in a role's loop: gives up as well when another role of the CTA has (looked at only while the barrier is not there).
+__device__ __forceinline__ bool mbar_wait_unless(uint32_t bar, uint32_t parity, volatile int* failed) {
+    for (int i = 0; i < 64; i++)
+        if (mbar_try_wait(bar, parity)) return true;
+    const uint64_t t0 = global_ns();
+    for (;;) {
+        for (int i = 0; i < 64; i++)
+            if (mbar_try_wait(bar, parity)) return true;
+        if (*failed || global_ns() - t0 > 200000000ull) return false;
+    }
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -180,19 +191,85 @@ __device__ __forceinline__ CtaWork load_work(const ChunkArgs& a) {
     return w;
 }
 
+// Two runs of 32 columns of this thread's lane, both loads in flight before the wait
+__device__ __forceinline__ void tmem_ld32x2(uint32_t first, uint32_t second, uint32_t (&r)[64]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%64];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47,%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%65];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]),
+          "=&r"(r[8]), "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11]), "=&r"(r[12]), "=&r"(r[13]), "=&r"(r[14]), "=&r"(r[15]),
+          "=&r"(r[16]), "=&r"(r[17]), "=&r"(r[18]), "=&r"(r[19]), "=&r"(r[20]), "=&r"(r[21]), "=&r"(r[22]), "=&r"(r[23]),
+          "=&r"(r[24]), "=&r"(r[25]), "=&r"(r[26]), "=&r"(r[27]), "=&r"(r[28]), "=&r"(r[29]), "=&r"(r[30]), "=&r"(r[31]),
+          "=&r"(r[32]), "=&r"(r[33]), "=&r"(r[34]), "=&r"(r[35]), "=&r"(r[36]), "=&r"(r[37]), "=&r"(r[38]), "=&r"(r[39]),
+          "=&r"(r[40]), "=&r"(r[41]), "=&r"(r[42]), "=&r"(r[43]), "=&r"(r[44]), "=&r"(r[45]), "=&r"(r[46]), "=&r"(r[47]),
+          "=&r"(r[48]), "=&r"(r[49]), "=&r"(r[50]), "=&r"(r[51]), "=&r"(r[52]), "=&r"(r[53]), "=&r"(r[54]), "=&r"(r[55]),
+          "=&r"(r[56]), "=&r"(r[57]), "=&r"(r[58]), "=&r"(r[59]), "=&r"(r[60]), "=&r"(r[61]), "=&r"(r[62]), "=&r"(r[63])
+        : "r"(first), "r"(second) : "memory");
+}
 // N consecutive columns of this thread's lane
 template <int N>
 __device__ __forceinline__ void tmem_ld_row(uint32_t taddr, uint32_t (&r)[N]) {
-    if constexpr (N == 32) {
-        tmem_ld32(taddr, r);
-    } else {
-        static_assert(N == 64, "half a KV tile: 32 or 64 tokens");
-        uint32_t lo[32], hi[32];
-        tmem_ld32(taddr, lo);
-        tmem_ld32(taddr + 32, hi);
+    static_assert(N == 32 || N == 64, "half a KV tile: 32 or 64 tokens");
+    if constexpr (N == 32) tmem_ld32(taddr, r);
+    else tmem_ld32x2(taddr, taddr + 32, r);
+}
+__device__ __forceinline__ float max3(float x, float y, float z) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(x), "f"(y), "f"(z));
+    return r;
+}
+template <int N>
+__device__ __forceinline__ float max_of(const uint32_t (&v)[N]) {
+    float m[4] = {__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), __uint_as_float(v[3])};  // four chains
 #pragma unroll
-        for (int e = 0; e < 32; e++) { r[e] = lo[e]; r[32 + e] = hi[e]; }
+    for (int e = 4; e + 8 <= N; e += 8) {
+#pragma unroll
+        for (int c = 0; c < 4; c++) m[c] = max3(m[c], __uint_as_float(v[e + 2 * c]), __uint_as_float(v[e + 2 * c + 1]));
     }
+    static_assert(N % 8 == 0, "the last four");
+    return max3(max3(m[0], __uint_as_float(v[N - 4]), __uint_as_float(v[N - 3])), max3(m[1], __uint_as_float(v[N - 2]), __uint_as_float(v[N - 1])), fmaxf(m[2], m[3]));
+}
+// A pair of 32-bit numbers in one register pair: fma.rn.f32x2 and add.rn.f32x2 do two per issue slot.
+__device__ __forceinline__ uint64_t f32x2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ uint64_t f32x2_bits(uint32_t lo, uint32_t hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 f32x2_split(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t x, uint64_t y, uint64_t z) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t x, uint64_t y) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+    return r;
+}
+// 2^(s * scale - ref) of N scores, packed in pairs in the order of the scores; adds them to `sum` (two pairs of chains).
+template <int N, bool BF16>
+__device__ __forceinline__ void exp_pack(const uint32_t* sv, uint64_t scale2, uint64_t neg_ref2, uint64_t (&sum)[2], uint32_t (&out)[N / 2]) {
+#pragma unroll
+    for (int e = 0; e < N; e += 2) {
+        const float2 x = f32x2_split(fma2(f32x2_bits(sv[e], sv[e + 1]), scale2, neg_ref2));
+        const float p0 = ex2_approx(x.x), p1 = ex2_approx(x.y);
+        sum[(e >> 1) & 1] = add2(sum[(e >> 1) & 1], f32x2(p0, p1));
+        out[e >> 1] = pack2<BF16>(p0, p1);
+    }
+}
+__device__ __forceinline__ float sum_of(const uint64_t (&sum)[2]) {
+    const float2 x = f32x2_split(add2(sum[0], sum[1]));
+    return x.x + x.y;
 }
 // 16 packed columns of this thread's lane (the caller waits)
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
