@@ -691,6 +691,7 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
         args.work_counters = d->work_counters; args.work_slot = (int32_t)(d->launch_seq++ & 3u);
         args.window = (int32_t)w; args.scale_log2 = scale_log2;
         args.n_stages = dc.stages; args.comb_cols = dc.comb_cols; args.comb_bufs = dc.comb_bufs;
+        args.combine_all = pd->host.n_ctas <= d->sm_count ? 1 : 0;
         // the producer may run ahead of earlier work in the stream unless that work wrote what it reads
         args.kv_dep = (d->last_kv_writer == layer || pd->fresh) ? 1 : 0;
         pd->fresh = false;

@@ -199,6 +199,36 @@ __device__ __forceinline__ void merge_parts(const DecodeArgs& a, int base, int n
     }
 }
 
+// One (column, 4 d-values) item of a piece: the C consumers' states (rows of DP floats, ccols of them each; maxima and sums)
+// combined, and the output stored, or the partial of a cut segment.
+template <int D, int C, bool BF16>
+__device__ __forceinline__ void combine_states(const DecodeArgs& a, const float* co, const float* cml, int ccols, int col, int j4, int nparts, int slot, uint16_t* out_row) {
+    constexpr int DP = D + 4;
+    float M = -INFINITY;
+#pragma unroll
+    for (int ww = 0; ww < C; ww++) M = fmaxf(M, cml[(ww * 8 + col) * 2]);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float ls = 0.f;
+#pragma unroll
+    for (int ww = 0; ww < C; ww++) {
+        const float mw = cml[(ww * 8 + col) * 2];
+        const float f = (mw == -INFINITY) ? 0.f : exp2f(mw - M);
+        const float4 v = *reinterpret_cast<const float4*>(co + ((size_t)ww * ccols + col) * DP + j4 * 4);
+        acc.x += f * v.x; acc.y += f * v.y; acc.z += f * v.z; acc.w += f * v.w;
+        ls += f * cml[(ww * 8 + col) * 2 + 1];
+    }
+    if (nparts == 1) {
+        const float inv = 1.f / ls;
+        uint2 pk;
+        pk.x = pack2<BF16>(acc.x * inv, acc.y * inv);
+        pk.y = pack2<BF16>(acc.z * inv, acc.w * inv);
+        *reinterpret_cast<uint2*>(out_row + col * D + j4 * 4) = pk;
+    } else {
+        *reinterpret_cast<float4*>(a.part_o + ((size_t)slot * 8 + col) * D + j4 * 4) = acc;
+        if (j4 == 0) *reinterpret_cast<float2*>(a.part_ml + ((size_t)slot * 8 + col) * 2) = make_float2(M, ls);
+    }
+}
+
 // Record index (page * n_kv + kv head) of every unit of a decode plan, once per step and
 // window: the decode launches of all layers read it instead of chasing the block tables.
 __global__ void resolve_units_kernel(const SegInfo* segs, int n_segs, const int32_t* tables, int n_kv, int num_pages,
@@ -432,6 +462,23 @@ __global__ void __launch_bounds__((C + 2) * 32, !ROPE ? 0 : Q8 && D <= 128 ? 2 :
     };
 
     const int n_rep = a.geo.n_rep;
+    // ALL: the CTA's last piece is combined by all its consumers and the merger, who meet first: nothing is left to overlap with,
+    // and one warp's combine was much of the way from the last tile to the exit.  One sequence of 340 tokens with rotation
+    // (8 segments of 22 pages, 32/8/128) 6.7 -> 5.6 us per launch, 32 sequences of 1024 to 4096 (28/4/128) 34.6 -> 33.5.  Where two
+    // CTAs share an SM (int8 pages) the other one's tiles fill that time, and meeting costs 1.3 %: the merger does it there.  Every
+    // warp passes the same barriers whatever happened to its waits; what a launch that gave up stores is undefined, as its output is.
+    const bool ALL = !Q8 || a.combine_all != 0;
+    auto combine_last = [&](int seg, const int4& x, const int4& y, int first_seg, int first_part, int buf) {
+        consumer_sync((C + 1) * 32);
+        if (warp == C + 1 && lane == 0) CBKV_STAMP(5);
+        const int nparts = y.x, slot = nparts > 1 ? y.y + (seg == first_seg ? first_part : 0) : 0;
+        uint16_t* out_row = reinterpret_cast<uint16_t*>(a.out) + ((size_t)x.w * a.geo.n_q + (size_t)(seg % Hkv) * n_rep) * D;
+        for (int idx = tid - 32; idx < n_rep * (D / 4); idx += (C + 1) * 32) {
+            const int col = idx / (D / 4);
+            combine_states<D, C, BF16>(a, comb_o + (size_t)buf * C * ccols * DP, comb_ml + buf * C * 16, ccols, col, idx - col * (D / 4), nparts, slot, out_row);
+        }
+        consumer_sync((C + 1) * 32);
+    };
     if (warp == C + 1) {
         // -------------------------------------------------------------- merger
         // Combines the consumers' states of each piece, writes the output (or a partial
@@ -472,16 +519,38 @@ __global__ void __launch_bounds__((C + 2) * 32, !ROPE ? 0 : Q8 && D <= 128 ? 2 :
 #ifdef CBKV_MEASURE
         int dbg_tiles = 0, dbg_cut = 0;
 #endif
+        auto draw = [&](int seg, int nparts) {
+            if (lane == 0) {
+                // release: the partial (ordered before by __syncwarp or the CTA's barrier) is visible before the ticket;
+                // acquire: whoever draws the last ticket sees every other part's partial
+                asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(pend_raw) : "l"(a.seg_counter + seg) : "memory");
+            }
+            pend_seg = seg;
+            pend_np = nparts;
+#ifdef CBKV_MEASURE
+            dbg_cut++;
+#endif
+        };
         int4 it;
         bool have = get_item(0, it);
+        int seg = have ? it.z : 0;
 #pragma unroll 1
         while (have) {
-            int seg = it.z, pb = it.x;
+            int pb = it.x;
+            int4 nit;
+            bool more = false;
 #pragma unroll 1
             while (pb < it.y) {
                 const int4* sp = reinterpret_cast<const int4*>(a.segs + seg);
                 const int4 x = __ldg(sp), y = __ldg(sp + 1), z = __ldg(sp + 2);
                 const int pe = min(it.y, z.x);
+#ifdef CBKV_MEASURE
+                dbg_tiles += pe - pb;
+#endif
+                if (pe == it.y) {
+                    more = get_item(k + 1, nit);
+                    if (ALL && !more) break;  // the CTA's last piece is left to all its warps
+                }
                 const int h = seg % Hkv;
                 const int tok_off = x.w, nparts = y.x;
                 const int slot = nparts > 1 ? y.y + (seg == it.z ? it.w : 0) : 0;
@@ -492,8 +561,6 @@ __global__ void __launch_bounds__((C + 2) * 32, !ROPE ? 0 : Q8 && D <= 128 ? 2 :
                     break;
                 }
                 if (lane == 0) CBKV_STAMP(5);
-                const float* co = comb_o + (size_t)buf * C * ccols * DP;
-                const float* cml = comb_ml + buf * C * 16;
                 uint16_t* out_row = reinterpret_cast<uint16_t*>(a.out) + ((size_t)tok_off * a.geo.n_q + (size_t)h * n_rep) * D;
                 // lane owns 4 consecutive d-values (per pass of 128) of every query column
                 constexpr int PASSES = (D + 127) / 128;
@@ -502,60 +569,30 @@ __global__ void __launch_bounds__((C + 2) * 32, !ROPE ? 0 : Q8 && D <= 128 ? 2 :
                     const int j4 = ps * 32 + lane;  // float4 index within a row of D
                     if (j4 * 4 < D) {
 #pragma unroll
-                        for (int col = 0; col < 8; col++) {
-                            if (col < n_rep) {
-                                float M = -INFINITY;
-#pragma unroll
-                                for (int ww = 0; ww < C; ww++) M = fmaxf(M, cml[(ww * 8 + col) * 2]);
-                                float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-                                float ls = 0.f;
-#pragma unroll
-                                for (int ww = 0; ww < C; ww++) {
-                                    const float mw = cml[(ww * 8 + col) * 2];
-                                    const float f = (mw == -INFINITY) ? 0.f : exp2f(mw - M);
-                                    const float4 v = *reinterpret_cast<const float4*>(co + ((size_t)ww * ccols + col) * DP + j4 * 4);
-                                    acc.x += f * v.x; acc.y += f * v.y; acc.z += f * v.z; acc.w += f * v.w;
-                                    ls += f * cml[(ww * 8 + col) * 2 + 1];
-                                }
-                                if (nparts == 1) {
-                                    const float inv = 1.f / ls;
-                                    uint2 pk;
-                                    pk.x = pack2<BF16>(acc.x * inv, acc.y * inv);
-                                    pk.y = pack2<BF16>(acc.z * inv, acc.w * inv);
-                                    *reinterpret_cast<uint2*>(out_row + col * D + j4 * 4) = pk;
-                                } else {
-                                    *reinterpret_cast<float4*>(a.part_o + ((size_t)slot * 8 + col) * D + j4 * 4) = acc;
-                                    if (j4 == 0) *reinterpret_cast<float2*>(a.part_ml + ((size_t)slot * 8 + col) * 2) = make_float2(M, ls);
-                                }
-                            }
-                        }
+                        for (int col = 0; col < 8; col++)
+                            if (col < n_rep) combine_states<D, C, BF16>(a, comb_o + (size_t)buf * C * ccols * DP, comb_ml + buf * C * 16, ccols, col, j4, nparts, slot, out_row);
                     }
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(cempty0 + buf * 8);  // the consumers may store the next piece here
                 settle();  // the previous cut piece's ticket has had a whole piece to come back
-                if (nparts > 1) {
-                    if (lane == 0) {
-                        // release: the warp's partial (ordered before by __syncwarp) is visible before the ticket;
-                        // acquire: whoever draws the last ticket sees every other part's partial
-                        asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(pend_raw) : "l"(a.seg_counter + seg) : "memory");
-                    }
-                    pend_seg = seg;
-                    pend_np = nparts;
-#ifdef CBKV_MEASURE
-                    dbg_cut++;
-#endif
-                }
-#ifdef CBKV_MEASURE
-                dbg_tiles += pe - pb;
-#endif
+                if (nparts > 1) draw(seg, nparts);
                 kk++;
                 seg++;
                 pb = pe;
             }
-            if (failed) break;
+            if (failed || !more) break;
             k++;
-            have = get_item(k, it);
+            it = nit;
+            seg = it.z;
+        }
+        if (ALL) {  // (a CTA whose first item never came falls through with segment 0; its output is undefined)
+            const int4* sp = reinterpret_cast<const int4*>(a.segs + seg);
+            const int4 x = __ldg(sp), y = __ldg(sp + 1);
+            combine_last(seg, x, y, have ? it.z : 0, have ? it.w : 0, NB == 2 ? (kk & 1) : 0);
+            settle();
+            if (y.x > 1 && !failed) draw(seg, y.x);
+            kk++;
         }
         settle();
         // hand the segments to merge to the whole CTA
@@ -741,7 +778,10 @@ __global__ void __launch_bounds__((C + 2) * 32, !ROPE ? 0 : Q8 && D <= 128 ? 2 :
             if (lane == 0) mbar_arrive(empty0 + st * 8);  // the stage may be refilled
         }
 
-        // ---- hand this warp's state for the piece to the merger (double-buffered)
+        // ---- hand this warp's state for the piece to the merger (double-buffered), or leave the CTA's last one to all warps
+        const bool late = !nknown;
+        if (ALL && late) nhave = get_item(k + 1, nit);  // the entry was not there when the piece began: wait for it now
+        const bool last = ALL && !more && !nhave;
         const int buf = NB == 2 ? (kk & 1) : 0, use = NB == 2 ? (kk >> 1) : kk;
         if (vflag[1] != 0) failed = true;  // another warp gave up: stop waiting
         if (use >= 1 && !failed && !mbar_wait_bounded(cempty0 + buf * 8, (use - 1) & 1, 4 * lim)) {
@@ -774,11 +814,12 @@ __global__ void __launch_bounds__((C + 2) * 32, !ROPE ? 0 : Q8 && D <= 128 ? 2 :
             cml[(2 * t) * 2 + 0] = m[0][0]; cml[(2 * t) * 2 + 1] = l[0][0];
             cml[(2 * t + 1) * 2 + 0] = m[0][1]; cml[(2 * t + 1) * 2 + 1] = l[0][1];
         }
+        if (last) break;
         __syncwarp();
         if (lane == 0) mbar_arrive(cfull0 + buf * 8);
         kk++;
-        if (!nknown) {  // the entry was not there when the piece began: wait for it now
-            nhave = get_item(k + 1, nit);
+        if (late) {
+            if (!ALL) nhave = get_item(k + 1, nit);
             if (nhave) {
                 nseg = nit.z;
                 nxt = load_piece(a, nseg);
@@ -811,6 +852,11 @@ __global__ void __launch_bounds__((C + 2) * 32, !ROPE ? 0 : Q8 && D <= 128 ? 2 :
         cur = nxt;
 #pragma unroll
         for (int ks = 0; ks < D / 16; ks++) { qf[0][ks][0] = qf_next[0][ks][0]; qf[0][ks][1] = qf_next[0][ks][1]; }
+    }
+    if (ALL) {
+        const int4* sp = reinterpret_cast<const int4*>(a.segs + seg);
+        const int4 x = __ldg(sp), y = __ldg(sp + 1);
+        combine_last(seg, x, y, have ? it.z : 0, have ? it.w : 0, NB == 2 ? (kk & 1) : 0);
     }
     // idle now: help merge the segments whose last ticket this CTA drew
     consumer_sync((C + 1) * 32);

@@ -117,6 +117,7 @@ struct DecodeArgs {
     int32_t n_stages;   // stages of the CTA's TMA ring
     int32_t comb_cols;  // query columns kept in the merge buffers (n_rep rounded up to even)
     int32_t comb_bufs;  // 1 or 2 merge buffers
+    int32_t combine_all;  // int8 pages: all warps of a CTA combine its last piece (16-bit pages: always)
     int32_t kv_dep;     // 1: earlier work in the stream wrote this layer's pages or unit_row: the producer waits for it
     uint32_t wait_us;   // limit of every bounded wait on a tile, microseconds
     const uint32_t* in_flag;  // non-null: q, k_new, v_new arrive by copies on another stream, which writes in_seq here after them
