@@ -185,6 +185,7 @@ extern "C" {
     // ---- test hooks
     pub fn cbkv_debug_begin_step_host(arena: *mut cbkv_arena, seqs: *const *mut cbkv_seq, new_tokens: *const i64, pos: *const i64, n_seqs: i32) -> i32;
     pub fn cbkv_debug_decode_plan(arena: *mut cbkv_arena, window: i64, n_ctas: i32, tail_pct: i32, min_item: i32, out: *mut i32, cap: i64) -> i64;
+    pub fn cbkv_debug_decode_choice(arena: *mut cbkv_arena, window: i64, int8_pages: i32, consumers: i32, max_ctas: i32, out: *mut i32, cap: i64) -> i64;
     pub fn cbkv_debug_chunk_choice(arena: *mut cbkv_arena, window: i64, mode: i32, sm_count: i32, max_parts: i32, out: *mut i32, cap: i64) -> i64;
     pub fn cbkv_debug_tile_plan(arena: *mut cbkv_arena, window: i64, tokens_per_item: i32, tile_tokens: i32, kv_tile: i32, sm_count: i32, max_parts: i32, out: *mut i32, cap: i64) -> i64;
     pub fn cbkv_debug_set_wait_limit(arena: *mut cbkv_arena, wait_us: i64, fault_tile: i32) -> i32;

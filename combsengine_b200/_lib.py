@@ -103,6 +103,7 @@ PROTOTYPES = {
     "cbkv_debug_tile_plan": (I64, [P, I64, I32, I32, I32, I32, I32, C.POINTER(I32), I64]),
     "cbkv_debug_chunk_choice": (I64, [P, I64, I32, I32, I32, C.POINTER(I32), I64]),
     "cbkv_debug_decode_plan": (I64, [P, I64, I32, I32, I32, C.POINTER(I32), I64]),
+    "cbkv_debug_decode_choice": (I64, [P, I64, I32, I32, I32, C.POINTER(I32), I64]),
     "cbkv_set_decode_split": (I32, [P, I32, I32, I32]),
     "cbkv_debug_set_wait_limit": (I32, [P, I64, I32]),
     "cbkv_static_status": (I32, [P, C.POINTER(I32)]),

@@ -418,29 +418,9 @@ int32_t get_decode_plan(Arena* a, int64_t window, bool quant, cudaStream_t st, D
     auto it = d->decode_plans.find(key);
     if (it != d->decode_plans.end()) { *out = &it->second; return CBKV_OK; }
     DecodePlanDev pd{};
-    // at least one page per consumer warp, at most one resident wave of CTAs
     int max_ctas = d->sm_count * dc.ctas_per_sm;
     if (d->decode_max_ctas > 0) max_ctas = std::min(max_ctas, d->decode_max_ctas);
-    build_decode_plan(*a, window, max_ctas, d->split, &pd.host);
-    {
-        int want = std::max(1, (pd.host.n_units + dc.consumers - 1) / dc.consumers);
-        // Short segments of one length (one sequence's first hundreds of tokens), no more than CTAs, are not cut: a CTA
-        // per segment streams its pages in the time that a cut spends on tickets and the merge.  Measured cut / uncut,
-        // us per launch, 1 to 16 sequences:
-        //   float, head_dim 64:   16 pages 7.9 / 5.1,  40 pages 7.9 / 7.0,   96 pages 7.0 / 10.7
-        //   float, head_dim 128:  16 pages 9.3 / 5.8,  40 pages 9.2 / 8.0,   96 pages 7.9 / 13.4
-        //   float, head_dim 256:  16 pages 11.4 / 7.1, 24 pages 7.5 / 9.4,   40 pages 10.9 / 12.8
-        //   int8,  head_dim 128:  8 pages 7.1 / 6.1,   16 pages 7.3 / 7.5,   40 pages 8.2 / 11.5
-        //   int8,  head_dim 256:  16 pages 12.7 / 10.2, 24 pages 9.7 / 12.5, 40 pages 13.0 / 14.5
-        // Batches of unequal lengths keep the even split: the launch would last as long as the longest segment.
-        const int uncut_pages = !quant && a->cfg.head_dim <= 128 ? 40 : 16;
-        const int per = pd.host.n_segs > 0 ? pd.host.n_units / pd.host.n_segs : 0;
-        bool equal = pd.host.n_segs > 0 && pd.host.n_segs <= max_ctas && per <= uncut_pages;
-        for (int i = 0; equal && i < pd.host.n_segs; i++)
-            equal = pd.host.segs[(size_t)i + 1].unit_begin - pd.host.segs[(size_t)i].unit_begin == per;
-        if (equal) want = std::min(want, pd.host.n_segs);
-        if (want < pd.host.n_ctas) build_decode_plan(*a, window, want, d->split, &pd.host);
-    }
+    choose_decode_plan(*a, window, quant, dc.consumers, max_ctas, d->split, &pd.host);
     // segment and item records in one upload
     const size_t seg_bytes = pd.host.segs.size() * sizeof(SegInfo), item_bytes = pd.host.items.size() * sizeof(ItemInfo);
     std::vector<uint8_t> flat(seg_bytes + item_bytes);
@@ -685,6 +665,7 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
         args.geo = geom(a);
         args.segs = pd->segs; args.items = pd->items; args.unit_row = d->unit_rows + pd->unit_row_off;
         args.n_segs = pd->host.n_segs; args.n_items = pd->host.n_items; args.n_ctas = pd->host.n_ctas;
+        args.aligned = pd->host.aligned ? 1 : 0;
         args.n_units = pd->host.n_units; args.tail_pct = pd->host.levels > 1 ? d->split.tail_pct : 0;
         args.q = q; args.out = out; args.k_new = k_fused; args.v_new = v_fused; args.arena = L.base; args.rope = rope;
         args.part_o = d->part_o; args.part_ml = d->part_ml; args.seg_counter = d->seg_counter; args.status = d->status;
@@ -1632,6 +1613,16 @@ int32_t cbkv_set_chunk_kernel(cbkv_arena* arena, int32_t mode) {
     });
 }
 
+static int64_t flatten_decode_plan(const DecodePlan& pl, int32_t* out, int64_t cap) {
+    std::vector<int32_t> flat = {pl.n_ctas, pl.n_items, pl.n_segs, pl.n_units, pl.n_parts, pl.levels};
+    const int32_t* sp32 = reinterpret_cast<const int32_t*>(pl.segs.data());
+    flat.insert(flat.end(), sp32, sp32 + pl.segs.size() * 8);
+    const int32_t* ip32 = reinterpret_cast<const int32_t*>(pl.items.data());
+    flat.insert(flat.end(), ip32, ip32 + pl.items.size() * 4);
+    for (int64_t i = 0; i < (int64_t)flat.size() && i < cap; i++) out[i] = flat[(size_t)i];
+    return (int64_t)flat.size();
+}
+
 // Host-only view of the decode work split for the step in flight (used by the CPU tests of
 // the partition): out = [n_ctas, n_items, n_segs, n_units, n_parts, levels,
 // segs (n_segs + 1 records of 8 ints), items (n_items records of 4 ints)].
@@ -1645,13 +1636,17 @@ int64_t cbkv_debug_decode_plan(cbkv_arena* arena, int64_t window, int32_t n_ctas
     if (tail_pct >= 0) sp.tail_pct = tail_pct;
     if (min_item >= 0) sp.min_item = min_item;
     build_decode_plan(*a, window, n_ctas, sp, &pl);
-    std::vector<int32_t> flat = {pl.n_ctas, pl.n_items, pl.n_segs, pl.n_units, pl.n_parts, pl.levels};
-    const int32_t* sp32 = reinterpret_cast<const int32_t*>(pl.segs.data());
-    flat.insert(flat.end(), sp32, sp32 + pl.segs.size() * 8);
-    const int32_t* ip32 = reinterpret_cast<const int32_t*>(pl.items.data());
-    flat.insert(flat.end(), ip32, ip32 + pl.items.size() * 4);
-    for (int64_t i = 0; i < (int64_t)flat.size() && i < cap; i++) out[i] = flat[(size_t)i];
-    return (int64_t)flat.size();
+    return flatten_decode_plan(pl, out, cap);
+    });
+}
+// The same for the plan that a decode launch of the step in flight takes.
+int64_t cbkv_debug_decode_choice(cbkv_arena* arena, int64_t window, int32_t int8_pages, int32_t consumers, int32_t max_ctas, int32_t* out, int64_t cap) {
+    return fenced64([&]() -> int64_t {
+    Arena* a = reinterpret_cast<Arena*>(arena);
+    if (!a || a->step_meta.empty() || !out || consumers < 1 || max_ctas < 1) return -1;
+    DecodePlan pl;
+    choose_decode_plan(*a, window, int8_pages != 0, consumers, max_ctas, DecodeSplit{}, &pl);
+    return flatten_decode_plan(pl, out, cap);
     });
 }
 

@@ -339,14 +339,16 @@ __global__ void __launch_bounds__((C + 2) * 32, !ROPE ? 0 : Q8 && D <= 128 ? 2 :
         // The unit range of this CTA's first item follows from the launch's totals (the host cuts the
         // same way, build_decode_plan), so the first copies leave without waiting for its record; the
         // record itself (first segment, part index) is fetched meanwhile for the other warps.
-        int4 cur;
-        {
+        // (A plan whose ranges end where segments do has them in the records only.)
+        int4 cur, rec0;
+        if (a.aligned) {
+            cur = rec0 = fetch(cta);
+        } else {
             const long long rb = (long long)a.n_units * cta / a.n_ctas, re = (long long)a.n_units * (cta + 1) / a.n_ctas;
             const long long len = re - rb;
             cur = make_int4((int)rb, (int)(re - len * a.tail_pct / 100), 0, 0);
+            rec0 = fetch(cta);  // the record and the first rows travel together
         }
-        // the record and the first rows travel together; the other warps get the record the moment it is there
-        const int4 rec0 = fetch(cta);
         int row_first = lane < cur.y - cur.x ? __ldcg(a.unit_row + cur.x + lane) : 0;
         publish(0, rec0);
         int4 nxt = make_int4(-1, -1, 0, 0);

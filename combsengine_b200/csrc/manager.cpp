@@ -225,6 +225,41 @@ void page_stats(const Seq* s, int64_t layers_materialized, cbkv_page_stats_t* ou
     out->layers_sliding = 0;  // windows are masks over pages here; no rolling stores exist
 }
 
+namespace {
+
+// The parts of every segment, the first segment and part of every item: sweeps the items in unit order (range by range,
+// level by level).
+void number_parts(DecodePlan* pl) {
+    const int n_ctas = pl->n_ctas, levels = pl->levels;
+    for (SegInfo& sg : pl->segs) { sg.nparts = 0; sg.part_base = -1; }
+    std::vector<int32_t> order;
+    order.reserve((size_t)pl->n_items);
+    for (int c = 0; c < n_ctas; c++)
+        for (int j = 0; j < levels; j++)
+            if (pl->items[(size_t)j * n_ctas + c].u_end > pl->items[(size_t)j * n_ctas + c].u_begin) order.push_back(j * n_ctas + c);
+    size_t io = 0;
+    int parts = 0;
+    for (int s = 0; s < pl->n_segs; s++) {
+        SegInfo& sg = pl->segs[(size_t)s];
+        const int32_t sb = sg.unit_begin, se = pl->segs[(size_t)s + 1].unit_begin;
+        if (se == sb) continue;
+        while (io < order.size() && pl->items[(size_t)order[io]].u_end <= sb) io++;
+        int cnt = 0;
+        for (size_t k = io; k < order.size() && pl->items[(size_t)order[k]].u_begin < se; k++) {
+            ItemInfo& it = pl->items[(size_t)order[k]];
+            if (it.u_begin >= sb) { it.first_seg = s; it.first_part = cnt; }
+            cnt++;
+        }
+        sg.nparts = cnt;
+        if (cnt > 1) { sg.part_base = parts; parts += cnt; }
+    }
+    pl->n_parts = parts;
+    for (ItemInfo& it : pl->items)  // empty items (possible only when units < items) are never claimed usefully
+        if (it.u_end <= it.u_begin) { it.first_seg = 0; it.first_part = 0; }
+}
+
+}  // namespace
+
 void build_decode_plan(const Arena& a, int64_t window, int32_t n_ctas, const DecodeSplit& split, DecodePlan* pl) {
     const int64_t P = a.cfg.page_size;
     const int Hkv = a.cfg.n_kv_heads;
@@ -288,31 +323,69 @@ void build_decode_plan(const Arena& a, int64_t window, int32_t n_ctas, const Dec
             at += take;
         }
     }
-    // parts of every segment: sweep the items in unit order (range by range, level by level)
-    std::vector<int32_t> order;
-    order.reserve((size_t)pl->n_items);
-    for (int c = 0; c < n_ctas; c++)
-        for (int j = 0; j < levels; j++)
-            if (pl->items[(size_t)j * n_ctas + c].u_end > pl->items[(size_t)j * n_ctas + c].u_begin) order.push_back(j * n_ctas + c);
-    size_t io = 0;
-    int parts = 0;
-    for (int s = 0; s < pl->n_segs; s++) {
-        SegInfo& sg = pl->segs[(size_t)s];
-        const int32_t sb = sg.unit_begin, se = pl->segs[(size_t)s + 1].unit_begin;
-        if (se == sb) continue;
-        while (io < order.size() && pl->items[(size_t)order[io]].u_end <= sb) io++;
-        int cnt = 0;
-        for (size_t k = io; k < order.size() && pl->items[(size_t)order[k]].u_begin < se; k++) {
-            ItemInfo& it = pl->items[(size_t)order[k]];
-            if (it.u_begin >= sb) { it.first_seg = s; it.first_part = cnt; }
-            cnt++;
-        }
-        sg.nparts = cnt;
-        if (cnt > 1) { sg.part_base = parts; parts += cnt; }
+    pl->aligned = false;
+    number_parts(pl);
+}
+
+bool align_decode_plan(int32_t n_kv_heads, int32_t min_pages, int32_t slack, int32_t max_ctas, DecodePlan* pl) {
+    if (pl->levels != 1 || pl->n_units <= 0 || pl->n_segs > max_ctas) return false;
+    auto pages_of = [&](int s) { return pl->segs[(size_t)s + 1].unit_begin - pl->segs[(size_t)s].unit_begin; };
+    int32_t longest = 0;
+    for (int s = 0; s < pl->n_segs; s += n_kv_heads) longest = std::max(longest, pages_of(s));
+    auto fits = [&](int32_t most) {  // the heads of a sequence have the same pages
+        int64_t n = 0;
+        for (int s = 0; s < pl->n_segs; s += n_kv_heads) n += (pages_of(s) + most - 1) / most;
+        return n * n_kv_heads <= max_ctas;
+    };
+    const int32_t even = (pl->n_units + pl->n_ctas - 1) / pl->n_ctas;
+    int32_t lo = std::max(min_pages, 1), hi = std::max(lo, std::min(longest, std::max(even, lo) + slack));
+    if (!fits(hi)) return false;
+    while (lo < hi) {  // the shortest ranges that do
+        const int32_t mid = lo + (hi - lo) / 2;
+        if (fits(mid)) hi = mid; else lo = mid + 1;
     }
-    pl->n_parts = parts;
-    for (ItemInfo& it : pl->items)  // empty items (possible only when units < items) are never claimed usefully
-        if (it.u_end <= it.u_begin) { it.first_seg = 0; it.first_part = 0; }
+    pl->items.clear();
+    for (int s = 0; s < pl->n_segs; s++) {
+        const int32_t p = pages_of(s), n = (p + lo - 1) / lo, begin = pl->segs[(size_t)s].unit_begin;
+        for (int i = 0; i < n; i++) {
+            ItemInfo it{};
+            it.u_begin = begin + (int32_t)((int64_t)p * i / n);
+            it.u_end = begin + (int32_t)((int64_t)p * (i + 1) / n);
+            pl->items.push_back(it);
+        }
+    }
+    pl->n_items = pl->n_ctas = (int32_t)pl->items.size();
+    pl->aligned = true;
+    number_parts(pl);
+    return true;
+}
+
+// A CTA whose range straddles two segments works through two chains one after the other (the second's queries and tiles, its
+// combine, its partial and ticket wait for the first's), and the launch ends with the slowest: 3 to 4 us of the 10 to 15 that
+// decode launches of a few sequences take.  So the ranges end where segments do, unless that makes the longest of them longer
+// than the even cut's by more than it saves: 64 pages at head_dim 64, 48 at 128, 16 at 256; int8 pages, whose tiles are bound by
+// arithmetic, 32, 32 and 8.  Measured even / aligned, us per launch (16 bits; B sequences of lo to hi tokens, kv heads/head_dim):
+//   1 x 1500 3/64 10.7 / 6.6, 4/128 13.2 / 7.4, 4/256 13.8 / 8.0;  4 x 300-2000 3/64 12.1 / 7.9, 4/128 13.3 / 8.8, 4/256 14.3 / 10.5
+//   16 x 4000 4/128 29 / 28, 8/128 47 / 44;  32 x 1024-4096 4/128 33.9 / 33.9 (35.4 with 96 more pages);  16 x 8192 with windows of
+//   1024 4/256 29.7 / 28.1;  8 x 8000 4/256 49 / 52 with 24 more pages
+//   int8: 4 x 300-2000 4/128 24 / 14.6;  32 x 300-1000 8/128 23 / 21;  16 x 4000 8/128 36 / 37, 4/256 48 / 50 with 32 more pages
+//
+// Segments of a few pages are not cut at all: a CTA per segment streams its pages in the time that a cut spends on partials,
+// tickets and the merge.  One sequence, cut into a page per consumer warp / uncut, us per launch:
+//   head_dim  64: 12 pages 5.3 / 4.1, 23 pages 5.6 / 5.4, 27 pages 5.6 / 5.8, 32 pages 5.6 / 6.7
+//   head_dim 128: 12 pages 6.6 / 4.9, 23 pages 6.9 / 6.5, 27 pages 6.9 / 6.7, 32 pages 6.8 / 7.6
+//   head_dim 256: 12 pages 6.5 / 5.6, 16 pages 6.6 / 6.2, 19 pages 6.8 / 7.0, 23 pages 6.9 / 8.1
+//   int8: 64 12 pages 5.8 / 5.1, 26 6.0 / 6.6; 128 19 pages 6.4 / 6.2, 26 6.8 / 7.2; 256 12 pages 7.8 / 7.5, 16 7.6 / 8.2
+void choose_decode_plan(const Arena& a, int64_t window, bool quant, int32_t consumers, int32_t max_ctas, const DecodeSplit& split, DecodePlan* pl) {
+    build_decode_plan(a, window, max_ctas, split, pl);
+    // at least one page per consumer warp, at most one resident wave of CTAs
+    const int32_t want = std::max(1, (pl->n_units + consumers - 1) / consumers);
+    if (want < pl->n_ctas) build_decode_plan(a, window, want, split, pl);
+    const int32_t d = a.cfg.head_dim, at = d <= 64 ? 0 : d <= 128 ? 1 : 2;
+    static constexpr int32_t kSlack[2][3] = {{64, 48, 16}, {32, 32, 8}}, kUncut[2][3] = {{24, 28, 17}, {19, 20, 12}};
+    int32_t longest = 0;
+    for (int s = 0; s < pl->n_segs; s += a.cfg.n_kv_heads) longest = std::max(longest, pl->segs[(size_t)s + 1].unit_begin - pl->segs[(size_t)s].unit_begin);
+    align_decode_plan(a.cfg.n_kv_heads, longest <= kUncut[quant ? 1 : 0][at] ? longest : consumers, kSlack[quant ? 1 : 0][at], max_ctas, pl);
 }
 
 void build_chunk_plan(const Arena& a, int32_t cols_per_item, ChunkPlan* pl) {

@@ -110,6 +110,7 @@ struct ItemInfo {       // 16 bytes
 struct DecodePlan {
     int64_t window = 0;
     int32_t n_ctas = 0, n_items = 0, n_segs = 0, n_units = 0, n_parts = 0, levels = 0;
+    bool aligned = false;         // cut by align_decode_plan: a CTA's range is in its item record only
     std::vector<SegInfo> segs;    // n_segs + 1
     std::vector<ItemInfo> items;  // n_items, in claim order: item c (c < n_ctas) is CTA c's first
 };
@@ -183,6 +184,11 @@ void page_stats(const Seq* s, int64_t layers_materialized, cbkv_page_stats_t* ou
 
 // Builders used by the device layer (pure functions of the step state).
 void build_decode_plan(const Arena& a, int64_t window, int32_t n_ctas, const DecodeSplit& split, DecodePlan* plan);
+// Cuts a plan anew so that no CTA's range holds pages of two segments, where ranges of at least `min_pages` and at most
+// `slack` pages more than the even cut's allow that with no more than max_ctas CTAs.  False: the plan stays as it was.
+bool align_decode_plan(int32_t n_kv_heads, int32_t min_pages, int32_t slack, int32_t max_ctas, DecodePlan* plan);
+// The plan that the decode launches of a step take: `consumers` warps per CTA, one resident wave of at most max_ctas CTAs.
+void choose_decode_plan(const Arena& a, int64_t window, bool quant, int32_t consumers, int32_t max_ctas, const DecodeSplit& split, DecodePlan* plan);
 void build_chunk_plan(const Arena& a, int32_t cols_per_item, ChunkPlan* plan);
 // Work list of the tcgen05 chunk kernel: one item per (sequence, kv head, tile of
 // `tokens_per_tile` new tokens); `cols_per_item` records tokens_per_tile.

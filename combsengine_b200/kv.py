@@ -355,9 +355,16 @@ class KVArena:
     def debug_decode_plan(self, window: int, n_ctas: int, tail_pct: int = -1, min_item: int = -1) -> dict:
         """The decode work split of the step in flight (host only): counts, `segs` [n_segs + 1, 8] and
         `items` [n_items, 4] in claim order (see include/combs_kv.h for the columns)."""
+        return self._decode_plan(self._lib.cbkv_debug_decode_plan, window, n_ctas, tail_pct, min_item)
+
+    def debug_decode_choice(self, window: int = 0, int8_pages: bool = False, consumers: int = 6, max_ctas: int = 148) -> dict:
+        """The same for the plan that decode launches of the step in flight take."""
+        return self._decode_plan(self._lib.cbkv_debug_decode_choice, window, 1 if int8_pages else 0, consumers, max_ctas)
+
+    def _decode_plan(self, call, *args) -> dict:
         cap = 1 << 20
         buf = (C.c_int32 * cap)()
-        n = self._lib.cbkv_debug_decode_plan(self._h, window, n_ctas, tail_pct, min_item, buf, cap)
+        n = call(self._h, *args, buf, cap)
         if n < 0 or n > cap:
             raise CbkvError(-6, "no step in flight or plan too large")
         a = np.frombuffer(buf, dtype=np.int32, count=n).copy()

@@ -279,6 +279,46 @@ def test_decode_plan_covers_every_page_once(window, n_ctas, tail_pct, min_item):
     assert parts == pl["n_parts"]
 
 
+@pytest.mark.parametrize("d,int8,lens,window", [
+    (64, False, [385, 300, 20], 0), (64, False, [384, 300, 20], 0), (128, False, [449], 0), (128, False, [448, 448], 0),   # uncut or not
+    (128, False, [300, 800, 1400, 2000], 0), (256, False, [1001, 3000], 0), (256, False, [8192] * 16, 1024),
+    (128, True, [300, 2000, 17, 5000], 0), (256, True, [193, 192], 0), (128, False, [5] * 37, 0), (128, False, [5] * 38, 0),
+    (128, False, [32000] + [40] * 30, 0), (64, False, [1, 16, 17], 0)])
+def test_decode_ranges_end_where_segments_do_when_that_costs_little(d, int8, lens, window):
+    Hkv, C = 4, 4 if int8 and d <= 128 else 6
+    most = 296 if int8 and d <= 128 else 148
+    slack = {64: 32, 128: 32, 256: 8}[d] if int8 else {64: 64, 128: 48, 256: 16}[d]
+    uncut = {64: 19, 128: 20, 256: 12}[d] if int8 else {64: 24, 128: 28, 256: 17}[d]
+    a = KVArena(1, 8, Hkv, d, 33000, 16, 1 << 15)
+    seqs = [a.new_seq() for _ in lens]
+    if max(lens) > 1:
+        old = [(s, n - 1) for s, n in zip(seqs, lens) if n > 1]
+        a.begin_step_host_only([s for s, _ in old], [n for _, n in old])
+    a.begin_step_host_only(seqs, [1] * len(seqs))
+    pl = a.debug_decode_choice(window, int8, C, most)
+    sub, items, U = pl["segs"][:, 0], pl["items"], pl["n_units"]
+    pages = np.diff(sub)
+    size = items[:, 1] - items[:, 0]
+    assert pl["n_ctas"] == pl["n_items"] == len(items) <= most and size.min() >= 1
+    assert items[0, 0] == 0 and items[-1, 1] == U and np.array_equal(items[1:, 0], items[:-1, 1])
+    first = np.searchsorted(sub, items[:, 0], side="right") - 1
+    aligned = bool(np.all(items[:, 1] <= sub[first + 1]))
+    even = -(-U // min(most, max(1, -(-U // C))))
+    limit = max(even, pages.max() if pages.max() <= uncut else C) + slack
+    # ranges of at most `limit` pages that end where segments do exist exactly when the library takes such
+    possible = int(np.sum(-(-pages // min(limit, pages.max())))) <= most
+    assert aligned == possible or (aligned and pl["n_ctas"] == -(-U // even))
+    if possible:
+        assert size.max() <= limit
+        if pages.max() <= uncut:
+            assert len(items) == len(pages)
+        for s in range(len(pages)):
+            mine = np.flatnonzero(first == s)
+            assert pl["segs"][s, 4] == len(mine) and np.ptp(size[mine]) <= 1
+            assert np.array_equal(items[mine, 2], np.full(len(mine), s)) and np.array_equal(items[mine, 3], np.arange(len(mine)))
+    assert pl["n_parts"] == int(np.sum(pl["segs"][:-1, 4][pl["segs"][:-1, 4] > 1]))
+
+
 @pytest.mark.skipif(torch.cuda.is_available(), reason="checks the behaviour on a machine without a GPU")
 def test_compute_fails_loudly_without_a_gpu():
     a = arena()
