@@ -262,8 +262,10 @@ __global__ void resolve_units_kernel(const SegInfo* segs, int n_segs, const int3
 // resident, one CTA per SM, over int8 pages of head_dim 64 and 128 two.  Left to itself the compiler took 128 with 268 bytes
 // of spills (16 bits, head_dim 128: 193 now) and 241 (int8: 168 now), which left no room for the second CTA: 32 sequences of
 // 1024 to 4096 tokens, 28/4/128, 28 layers: 1058 -> 957 us, int8 1417 -> 1019 (rotated by a launch of its own 1165, 1047).
+// 16-bit pages: one CTA per SM, whose ring takes its shared memory, so its registers are not held to what two would have
+// (head_dim 128: 128, with 144 bytes of spills, 1949 us for 28 layers of 32 sequences, two steps; 176 and 1882 now).
 template <int D, int C, bool BF16, bool Q8, bool ROPE>
-__global__ void __launch_bounds__((C + 2) * 32, !ROPE ? 0 : Q8 && D <= 128 ? 2 : 1) decode_kernel(const __grid_constant__ CUtensorMap tmap, const DecodeArgs a) {
+__global__ void __launch_bounds__((C + 2) * 32, !Q8 ? 1 : !ROPE ? 0 : D <= 128 ? 2 : 1) decode_kernel(const __grid_constant__ CUtensorMap tmap, const DecodeArgs a) {
     constexpr uint32_t UNIT = Q8 ? (uint32_t)(2 * 16 * D + 2 * 16 * (D / 32) * 2) : 32u * D * 2u;
     constexpr int DP = D + 4;  // row pitch of the merge buffers: the four lanes of a quad land in different banks
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -701,6 +703,28 @@ __global__ void __launch_bounds__((C + 2) * 32, !ROPE ? 0 : Q8 && D <= 128 ? 2 :
         const int n0 = nbase + (pb - it.x);  // the piece's first tile, counted over the CTA's items
         const int n1 = n0 + (pe - pb);
         int T = n0 + (cw - n0 % C + C) % C;  // this warp's first tile of the piece
+        // Short pieces: the step's new row and the page it goes to, for the warp that has the segment's last page, are asked for
+        // here and arrive under the wait for the tiles and the products of the warp's earlier ones (us per launch, 2
+        // sequences of 1000 to 3000, 4/256, 10.4 -> 9.4; 8 of 500 to 2000, 8/128, 12.2 -> 10.9; 16 of 8192 with windows of 1024,
+        // 4/256, 28.1 -> 27.0).  In long pieces other warps are busy meanwhile and it costs 0.5 % (32 of 1024 to 4096); the
+        // rotating variant gains nothing.
+        constexpr int NROW = (2 * (D / 8) + 31) / 32;
+        uint4 row_new[NROW];
+        int rec_new = -1;
+        bool early = false;
+        if constexpr (!Q8 && !ROPE) {
+            const int u_last = cur.sb + cur.page_last - cur.page_lo;
+            early = a.k_new != nullptr && pe - pb <= 8 * C && u_last >= pb && u_last < pe && (n0 + u_last - pb) % C == cw;
+            if (early) {
+                rec_new = __ldcg(a.unit_row + u_last);
+                const size_t rowi = (size_t)cur.tok_off * Hkv + cur.h;
+#pragma unroll
+                for (int i = 0; i < NROW; i++) {
+                    const int c = lane + 32 * i, kv = c / (D / 8), j = c - kv * (D / 8);
+                    if (c < 2 * (D / 8)) row_new[i] = __ldcg(reinterpret_cast<const uint4*>(kv ? a.v_new : a.k_new) + rowi * (D / 8) + j);
+                }
+            }
+        }
         // stage and revolution parity of this warp's tiles, advanced by C per tile (NS is a multiple of C)
         int st = T % NS, par = (T / NS) & 1;
 #pragma unroll 1
@@ -723,27 +747,39 @@ __global__ void __launch_bounds__((C + 2) * 32, !ROPE ? 0 : Q8 && D <= 128 ? 2 :
                 if (!Q8 && a.k_new != nullptr && lp == cur.page_last) {
                     // fused append: put the new K/V row into the tile just fetched and into its page
                     const int slot = cur.q_pos & 15;
-                    const int rec = __ldcg(a.unit_row + u);
+                    const int rec = early ? rec_new : __ldcg(a.unit_row + u);
                     const size_t rowi = (size_t)cur.tok_off * Hkv + cur.h;
                     const uint16_t* krow = reinterpret_cast<const uint16_t*>(a.k_new) + rowi * D;
                     float inv_rms = 0.f;
                     if constexpr (ROPE) { if (a.rope.k_weight) inv_rms = inv_rms_of(row_sumsq<D, BF16>(krow, lane), D, a.rope.eps); }
-                    for (int c = lane; c < 2 * (D / 8); c += 32) {
-                        int kv = c / (D / 8), j = c - kv * (D / 8);
-                        uint4 val;
-                        if (ROPE && kv == 0) {
-                            uint32_t o4[4];
-                            rope_k_words<D, BF16, 4>(a.rope, reinterpret_cast<const uint32_t*>(krow), 4 * j, cur.q_pos, inv_rms, o4);
-                            val = make_uint4(o4[0], o4[1], o4[2], o4[3]);
-                        } else {
-                            val = *(reinterpret_cast<const uint4*>(kv ? a.v_new : a.k_new) + rowi * (D / 8) + j);
-                        }
+                    auto put = [&](int kv, int j, const uint4& val) {
                         uint32_t row = page_row(kv, slot, 16, true);
                         uint32_t addr = stage + (j >> 3) * 4096u + swz(row, j & 7);
                         asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(val.x), "r"(val.y), "r"(val.z), "r"(val.w) : "memory");
                         if (rec >= 0) {
                             size_t drow = (size_t)rec * 32 + row;
                             reinterpret_cast<uint4*>(a.arena)[drow * (D / 8) + j] = val;
+                        }
+                    };
+                    if constexpr (ROPE) {
+                        for (int c = lane; c < 2 * (D / 8); c += 32) {
+                            int kv = c / (D / 8), j = c - kv * (D / 8);
+                            uint4 val;
+                            if (kv == 0) {
+                                uint32_t o4[4];
+                                rope_k_words<D, BF16, 4>(a.rope, reinterpret_cast<const uint32_t*>(krow), 4 * j, cur.q_pos, inv_rms, o4);
+                                val = make_uint4(o4[0], o4[1], o4[2], o4[3]);
+                            } else {
+                                val = *(reinterpret_cast<const uint4*>(a.v_new) + rowi * (D / 8) + j);
+                            }
+                            put(kv, j, val);
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < NROW; i++) {
+                            const int c = lane + 32 * i, kv = c / (D / 8), j = c - kv * (D / 8);
+                            if (c >= 2 * (D / 8)) break;
+                            put(kv, j, early ? row_new[i] : *(reinterpret_cast<const uint4*>(kv ? a.v_new : a.k_new) + rowi * (D / 8) + j));
                         }
                     }
                     fence_proxy_async();

@@ -355,7 +355,9 @@ bool align_decode_plan(int32_t n_kv_heads, int32_t min_pages, int32_t slack, int
         }
     }
     pl->n_items = pl->n_ctas = (int32_t)pl->items.size();
-    pl->aligned = true;
+    pl->aligned = false;  // one sequence, or several of one length: the even cut of as many CTAs, which the kernel computes
+    for (int64_t c = 0; c < pl->n_ctas && !pl->aligned; c++)
+        pl->aligned = pl->items[(size_t)c].u_begin != (int64_t)pl->n_units * c / pl->n_ctas;
     number_parts(pl);
     return true;
 }
@@ -385,7 +387,9 @@ void choose_decode_plan(const Arena& a, int64_t window, bool quant, int32_t cons
     static constexpr int32_t kSlack[2][3] = {{64, 48, 16}, {32, 32, 8}}, kUncut[2][3] = {{24, 28, 17}, {19, 20, 12}};
     int32_t longest = 0;
     for (int s = 0; s < pl->n_segs; s += a.cfg.n_kv_heads) longest = std::max(longest, pl->segs[(size_t)s + 1].unit_begin - pl->segs[(size_t)s].unit_begin);
-    align_decode_plan(a.cfg.n_kv_heads, longest <= kUncut[quant ? 1 : 0][at] ? longest : consumers, kSlack[quant ? 1 : 0][at], max_ctas, pl);
+    // (Launches of an arena of one or two layers have nothing to overlap with: one of 33 pages, 3/64, 13.9 / 14.5 us cut.)
+    const int32_t uncut = a.cfg.num_layers <= 2 && !quant && d <= 128 ? 40 : kUncut[quant ? 1 : 0][at];
+    align_decode_plan(a.cfg.n_kv_heads, longest <= uncut ? longest : consumers, kSlack[quant ? 1 : 0][at], max_ctas, pl);
 }
 
 void build_chunk_plan(const Arena& a, int32_t cols_per_item, ChunkPlan* pl) {

@@ -110,7 +110,7 @@ struct ItemInfo {       // 16 bytes
 struct DecodePlan {
     int64_t window = 0;
     int32_t n_ctas = 0, n_items = 0, n_segs = 0, n_units = 0, n_parts = 0, levels = 0;
-    bool aligned = false;         // cut by align_decode_plan: a CTA's range is in its item record only
+    bool aligned = false;         // cut by align_decode_plan so that a CTA's range is in its item record only
     std::vector<SegInfo> segs;    // n_segs + 1
     std::vector<ItemInfo> items;  // n_items, in claim order: item c (c < n_ctas) is CTA c's first
 };

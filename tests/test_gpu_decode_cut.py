@@ -31,7 +31,7 @@ def quantised(x):
 def test_one_segment_per_cta(d, n_kv, n_rep, int8, lens, window):
     dt, n_q, B = torch.float16, n_kv * n_rep, len(lens)
     torch.manual_seed(sum(lens) + d)
-    a = KVArena(1, n_q, n_kv, d, max(lens) + 16, 16, sum(-(-n // 16) for n in lens) + 4, [window], dt, sliding_popn_refuses=False, quantize_kv=int8)
+    a = KVArena(4, n_q, n_kv, d, max(lens) + 16, 16, sum(-(-n // 16) for n in lens) + 4, [window] * 4, dt, sliding_popn_refuses=False, quantize_kv=int8)
     a.set_free_list(torch.randperm(a.num_pages).numpy())
     seqs = [a.new_seq() for _ in lens]
     kv = [torch.randn(2, n_kv, n, d, device="cuda", dtype=dt) for n in lens]

@@ -289,7 +289,7 @@ def test_decode_ranges_end_where_segments_do_when_that_costs_little(d, int8, len
     most = 296 if int8 and d <= 128 else 148
     slack = {64: 32, 128: 32, 256: 8}[d] if int8 else {64: 64, 128: 48, 256: 16}[d]
     uncut = {64: 19, 128: 20, 256: 12}[d] if int8 else {64: 24, 128: 28, 256: 17}[d]
-    a = KVArena(1, 8, Hkv, d, 33000, 16, 1 << 15)
+    a = KVArena(4, 8, Hkv, d, 33000, 16, 1 << 15)
     seqs = [a.new_seq() for _ in lens]
     if max(lens) > 1:
         old = [(s, n - 1) for s, n in zip(seqs, lens) if n > 1]
