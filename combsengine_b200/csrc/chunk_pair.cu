@@ -335,7 +335,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
         bool ok = true;
 #pragma unroll 1
         for (int j = X; j < n_tiles; j += 2) {
-            ok = mbar_wait_bounded(bar(kBSFull + X), (j >> 1) & 1) && !*failed;
+            ok = mbar_wait_unless(bar(kBSFull + X), (j >> 1) & 1, failed);
             ok = __all_sync(0xffffffffu, ok);
             tc_fence_after();
             const int kbase = k0 + j * KT + H * HK;
@@ -354,16 +354,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
                     if (!(kp <= q_pos && (a.window <= 0 || kp + a.window > q_pos))) sv[e] = 0xff800000u;  // -inf
                 }
             }
-            float mx;
-            {
-                float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
-#pragma unroll
-                for (int e = 0; e < HK; e += 4) {
-                    m0 = fmaxf(m0, __uint_as_float(sv[e])); m1 = fmaxf(m1, __uint_as_float(sv[e + 1]));
-                    m2 = fmaxf(m2, __uint_as_float(sv[e + 2])); m3 = fmaxf(m3, __uint_as_float(sv[e + 3]));
-                }
-                mx = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
-            }
+            float mx = max_of(sv);
             const int turn = (j >> 1) & 1;
             volatile int* pair_failed = s_pair + pair_id * 2 + turn;
             float* xrow = s_xch + ((X * 2 + turn) * 128 + m) * 2;
@@ -400,7 +391,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
             }
             // the P V that read this P buffer last, two tiles ago, is complete
             if (j > 1) {
-                bool done = mbar_wait_bounded(bar(kBODone + X), ((j - 2) >> 1) & 1) && !*failed;
+                bool done = mbar_wait_unless(bar(kBODone + X), ((j - 2) >> 1) & 1, failed);
                 if (!__all_sync(0xffffffffu, done) && lane == 0) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
                 tc_fence_after();
             }

@@ -256,9 +256,9 @@ __device__ __forceinline__ uint64_t add2(uint64_t x, uint64_t y) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
     return r;
 }
-// 2^(s * scale - ref) of N scores, packed in pairs in the order of the scores; adds them to `sum` (two pairs of chains).
+// 2^(s * scale - ref) of N scores, packed in pairs in the order of the scores (out may be sv); adds them to `sum` (two pairs of chains).
 template <int N, bool BF16>
-__device__ __forceinline__ void exp_pack(const uint32_t* sv, uint64_t scale2, uint64_t neg_ref2, uint64_t (&sum)[2], uint32_t (&out)[N / 2]) {
+__device__ __forceinline__ void exp_pack(const uint32_t* sv, uint64_t scale2, uint64_t neg_ref2, uint64_t (&sum)[2], uint32_t* out) {
 #pragma unroll
     for (int e = 0; e < N; e += 2) {
         const float2 x = f32x2_split(fma2(f32x2_bits(sv[e], sv[e + 1]), scale2, neg_ref2));
