@@ -312,12 +312,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
         // ---- Q to shared memory, rows past the data are zero
         {
             const uint16_t* qbase = reinterpret_cast<const uint16_t*>(a.q) + (size_t)sm.tok_off * a.geo.n_q * D;
-            for (int c = tid - 64; c < 128 * (D / 8); c += 512) {
-                const int mm = c / (D / 8), jj = c - mm * (D / 8), rr = mm / TPT, ii = mm - rr * TPT;
-                uint4 val = make_uint4(0, 0, 0, 0);
-                if (rr < n_rep && ii < nv) val = *reinterpret_cast<const uint4*>(qbase + ((size_t)(h * n_rep + rr) * sm.snew + r0 + ii) * D + jj * 8);
-                *reinterpret_cast<uint4*>(sQ + (jj >> 3) * QBLK + mm * 128u + (((jj & 7) ^ (mm & 7)) << 4)) = val;
+#pragma unroll
+            for (int u = 0; u < D / 32; u++) {  // all of a thread's copies are in flight together
+                const int c = tid - 64 + u * 512, mm = c / (D / 8), jj = c - mm * (D / 8), rr = mm / TPT, ii = mm - rr * TPT;
+                const bool there = rr < n_rep && ii < nv;
+                cp_async16(smem_u32(sQ) + (jj >> 3) * QBLK + mm * 128u + (((jj & 7) ^ (mm & 7)) << 4),
+                           there ? qbase + ((size_t)(h * n_rep + rr) * sm.snew + r0 + ii) * D + jj * 8 : qbase, there);
             }
+            cp_async_wait_all();
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) arrive_cluster_release(at_rank0(bar(kBQFull)));

@@ -559,17 +559,15 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     // ---- Q tiles: row m of tile X is q head (m / TPT) at token r0 + X TPT + m % TPT
     if (warp >= 2 && warp < 18) {
         const uint16_t* qbase = reinterpret_cast<const uint16_t*>(a.q) + (size_t)sm.tok_off * a.geo.n_q * D;
-#pragma unroll 4
-        for (int c = tid - 64; c < (two ? 256 : 128) * (D / 8); c += 512) {
-            const int mm = c / (D / 8), j = c - mm * (D / 8);
-            const int X = mm >> 7, m = mm & 127;
-            const int rep = m / TPT, r = r0 + X * TPT + (m - rep * TPT);
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if (rep < n_rep && r < sm.snew)
-                val = *reinterpret_cast<const uint4*>(qbase + ((size_t)(h * n_rep + rep) * sm.snew + r) * D + j * 8);
-            const uint32_t off = X * TILE + (j >> 3) * BLK + m * 128u + (((j & 7) ^ (m & 7)) << 4);
-            *reinterpret_cast<uint4*>(sQ + off) = val;
+#pragma unroll
+        for (int u = 0; u < 2 * (D / 32); u++) {  // all of a thread's copies are in flight together
+            const int X = u / (D / 32), c = tid - 64 + (u - X * (D / 32)) * 512, m = c / (D / 8), j = c - m * (D / 8), rep = m / TPT, r = r0 + X * TPT + (m - rep * TPT);
+            if (X == 1 && !two) break;
+            const bool there = rep < n_rep && r < sm.snew;
+            cp_async16(smem_u32(sQ) + X * TILE + (j >> 3) * BLK + m * 128u + (((j & 7) ^ (m & 7)) << 4),
+                       there ? qbase + ((size_t)(h * n_rep + rep) * sm.snew + r) * D + j * 8 : qbase, there);
         }
+        cp_async_wait_all();
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(b_q_full);

@@ -58,6 +58,11 @@ __device__ __forceinline__ bool mbar_wait_unless(uint32_t bar, uint32_t parity, 
         if (*failed || global_ns() - t0 > 200000000ull) return false;
     }
 }
+// 16 bytes to shared memory without a register in between; zeros if not `there` (src is valid either way)
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool there) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(there ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
