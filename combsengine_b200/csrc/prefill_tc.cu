@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
         for (int i = 0; i < NB; i++) {
             mbar_init(b_k_full + i * 8, 1); mbar_init(b_k_empty + i * 8, 1); mbar_init(b_v_full + i * 8, 1); mbar_init(b_v_empty + i * 8, 1);
         }
-        for (int i = 0; i < 2; i++) { mbar_init(b_s_full + i * 8, 1); mbar_init(b_p_full + i * 8, 256); }
+        for (int i = 0; i < 2; i++) { mbar_init(b_s_full + i * 8, 1); mbar_init(b_p_full + i * 8, D == 64 ? 8 : 256); }
         mbar_init(b_o_done, 1);
         *failed = 0;
         for (int i = 0; i < 8; i++) s_pair[i] = 0;
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
         const long long tstart = tprev;
 #pragma unroll 1
         for (int j = 0; j < n_tiles; j++) {
-            ok = mbar_wait_bounded(b_s_full + (j & 1) * 8, (j >> 1) & 1) && !*failed;
+            ok = D == 64 ? mbar_wait_unless(b_s_full + (j & 1) * 8, (j >> 1) & 1, failed) : mbar_wait_bounded(b_s_full + (j & 1) * 8, (j >> 1) & 1) && !*failed;
             ok = __all_sync(0xffffffffu, ok);
             TC_ACC(c_ws);
             volatile int* pair_failed = s_pair + (warp & 3) * 2 + (j & 1);
@@ -282,7 +282,9 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
                 }
             }
             float mx;
-            {
+            if constexpr (D == 64) {
+                mx = max_of(sv);
+            } else {
                 float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
 #pragma unroll
                 for (int e = 0; e < HK; e += 4) {
@@ -303,18 +305,26 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
                 m_ref = mx;
             }
             const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
-            float sum = 0.f, sum2 = 0.f;
+            float sum_all;
+            if constexpr (D == 64) {
+                uint64_t sum[2] = {0ull, 0ull};
+                exp_pack<HK, BF16>(sv, f32x2(a.scale_log2, a.scale_log2), f32x2(-m_use, -m_use), sum, sv);  // a pair reuses a register whose score is consumed
+                sum_all = sum_of(sum);
+            } else {  // (two at a time, and maxima of three above, spill at head_dim 256: verification there was 2 % slower with them)
+                float sum = 0.f, sum2 = 0.f;
 #pragma unroll
-            for (int e = 0; e < HK; e += 2) {
-                const float p0 = ex2_approx(fmaf(__uint_as_float(sv[e]), a.scale_log2, -m_use));
-                const float p1 = ex2_approx(fmaf(__uint_as_float(sv[e + 1]), a.scale_log2, -m_use));
-                if (e & 2) sum2 += p0 + p1; else sum += p0 + p1;  // two chains
-                sv[e >> 1] = pack2<BF16>(p0, p1);  // P pair e/2 reuses a register whose score is already consumed
+                for (int e = 0; e < HK; e += 2) {
+                    const float p0 = ex2_approx(fmaf(__uint_as_float(sv[e]), a.scale_log2, -m_use));
+                    const float p1 = ex2_approx(fmaf(__uint_as_float(sv[e + 1]), a.scale_log2, -m_use));
+                    if (e & 2) sum2 += p0 + p1; else sum += p0 + p1;  // two chains
+                    sv[e >> 1] = pack2<BF16>(p0, p1);
+                }
+                sum_all = sum + sum2;
             }
 #pragma unroll
             for (int c = 0; c < HK / 32; c++) tmem_st16(tS + H * (HK / 2) + c * 16, sv + c * 16);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            l_run = l_run * alpha + (sum + sum2);
+            l_run = l_run * alpha + sum_all;
             TC_ACC(c_exp);
             // O may be rescaled once the previous P V is complete.  A parity wait cannot tell a phase from the one two
             // before it, so it holds only where the phase before the awaited one is known to be complete.  Here: the
@@ -338,7 +348,12 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
                 }
             }
             tc_fence_before();     // the tensor-memory traffic above is ordered before the hand-over
-            mbar_arrive(b_p_full + (j & 1) * 8);
+            if constexpr (D == 64) {
+                __syncwarp();
+                if (lane == 0) mbar_arrive(b_p_full + (j & 1) * 8);
+            } else {
+                mbar_arrive(b_p_full + (j & 1) * 8);
+            }
             TC_ACC(c_st);
         }
         TC_DUMP(if (tid == 64) {
