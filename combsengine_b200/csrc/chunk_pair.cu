@@ -1,10 +1,10 @@
 // Chunk (prefill) attention on pairs of SMs: the one-tile kernel of prefill_tc.cu with cta_group::2.
 // Reference math: attend() with seq > 1, kv.rs:243-268.
 //
-// What bounds the one-SM kernels: an MMA of 16 deep costs 70 cycles with A in shared memory and 86 with A in tensor memory
-// whatever its N up to 128, and 128 with N = 256 (measured, one thread issuing back to back, either cta_group); and shared
+// What bounds the one-SM kernels: an MMA of 16 deep takes the tensor pipe 64 cycles at N = 128, 128 at N = 256, and hardly
+// less than 50 with a smaller N (measured, back to back, either cta_group, A in shared or tensor memory); and shared
 // memory delivers 128 bytes a cycle, which two query tiles of head_dim 128 use up (128-row Q and 128 keys per MMA, and the
-// copies), while at head_dim 256 K, V and Q leave room for KV tiles of 64 keys only, at the price of 128.  A pair of CTAs,
+// copies), while at head_dim 256 K, V and Q leave room for KV tiles of 64 keys only, at that price.  A pair of CTAs,
 // one query tile each, runs M = 256 MMAs for which each CTA holds half of K and half of V: half of the operand bytes, half
 // of the L2 reads per query tile, and KV tiles of 128 keys at both head_dims.
 //

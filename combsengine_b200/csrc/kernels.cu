@@ -36,14 +36,12 @@ namespace cbkv {
 // ------------------------------------------------------------------ append
 template <typename T>
 __global__ void append_kernel(const AppendArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
     const int D8 = a.geo.d / 8;
-    const int64_t total = (int64_t)a.step.n_tokens * a.geo.n_kv * 2 * D8;
-    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (int64_t)gridDim.x * blockDim.x) {
-        int c = (int)(idx % D8);
-        int64_t rem = idx / D8;
-        int kv = (int)(rem & 1);
+    const int64_t total = (int64_t)a.step.n_tokens * a.geo.n_kv * 2 * D8, stride = (int64_t)gridDim.x * blockDim.x;
+    // where 16 bytes go, in vectors of the arena; -1: the table entry is not a page
+    auto place_of = [&](int64_t idx) -> int64_t {
+        const int64_t rem = idx / D8;
+        const int kv = (int)(rem & 1), c = (int)(idx - rem * D8);
         int64_t row = rem >> 1;  // packed row: sequence blocks of [n_kv][snew] rows
         int lo = 0, hi = a.step.n_seqs - 1;  // last sequence whose first row is <= row
         while (lo < hi) {
@@ -56,10 +54,20 @@ __global__ void append_kernel(const AppendArgs a) {
         int gpos = sm.pos + r;                         // global = pos + written, kv.rs:725
         int phys = a.step.tables[sm.tbl_off + gpos / a.geo.page_size];  // kv.rs:728
         int slot = gpos % a.geo.page_size;             // kv.rs:726
-        if (phys < 0 || phys >= a.geo.num_pages) { atomicOr(a.status, ST_BAD_PAGE); continue; }
-        const uint4* src = reinterpret_cast<const uint4*>(kv ? a.v : a.k) + row * D8 + c;
-        int64_t drow = ((int64_t)phys * a.geo.n_kv + h) * 2 * a.geo.page_size + page_row(kv, slot, a.geo.page_size, a.geo.tiled != 0);
-        reinterpret_cast<uint4*>(a.arena)[drow * D8 + c] = *src;
+        if (phys < 0 || phys >= a.geo.num_pages) { atomicOr(a.status, ST_BAD_PAGE); return -1; }
+        return (((int64_t)phys * a.geo.n_kv + h) * 2 * a.geo.page_size + page_row(kv, slot, a.geo.page_size, a.geo.tiled != 0)) * D8 + c;
+    };
+    // The first look-up, a chain of loads, runs under the tail of the launch before: the records and block tables came with
+    // the step's upload, which no kernel overlaps.
+    int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    int64_t to = idx < total ? place_of(idx) : -1;
+    pdl_wait();
+    pdl_launch_dependents();
+    while (idx < total) {
+        const int64_t rem = idx / D8;
+        if (to >= 0) reinterpret_cast<uint4*>(a.arena)[to] = *(reinterpret_cast<const uint4*>((rem & 1) ? a.v : a.k) + (rem >> 1) * D8 + (idx - rem * D8));
+        idx += stride;
+        if (idx < total) to = place_of(idx);
     }
 }
 

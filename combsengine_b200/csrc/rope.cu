@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(256) rope_append_kernel(const RopeArgs a) {
 constexpr int ROPE_SEQ_SMEM = 1024;
 
 template <bool BF16, int T>
-__global__ void __launch_bounds__(256) rope_append_vec_kernel(const RopeArgs a) {
+__global__ void __launch_bounds__(256, 5) rope_append_vec_kernel(const RopeArgs a) {
     __shared__ int s_tok[ROPE_SEQ_SMEM];
     const int n_seqs = a.step.n_seqs;
     const bool in_smem = n_seqs <= ROPE_SEQ_SMEM;
@@ -205,61 +205,62 @@ __global__ void __launch_bounds__(256) rope_append_vec_kernel(const RopeArgs a) 
         for (int i = threadIdx.x; i < n_seqs; i += blockDim.x) s_tok[i] = a.step.seq_meta[i].tok_off;
         __syncthreads();
     }
-    pdl_wait();  // the sequence records above came with the step's upload, which no kernel overlaps
-    pdl_launch_dependents();
     const int lane = threadIdx.x & 31, t = lane % T, sub = lane / T;
     constexpr int RPW = 32 / T;  // rows per warp per round
     // row counts fit 32 bits (the launcher checks)
     const uint32_t warp0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t q_rows = (uint32_t)a.step.n_tokens * a.geo.n_q, kv_rows = (uint32_t)a.step.n_tokens * a.geo.n_kv;
     const uint32_t total = q_rows + (a.k_out ? 1u : 2u) * kv_rows;
-    for (uint32_t R0 = warp0 * RPW; R0 < total; R0 += nwarps * RPW) {
-        const uint32_t R = R0 + sub;
-        const bool live = R < total;
-        const uint32_t Rc = live ? R : total - 1;
+    struct Row { int kind; uint32_t row; };                 // q, k or v; its row among them
+    struct Place { uint4* dst; uint4 tc, ts; bool ok; };    // where it goes, its cosines and sines
+    auto row_of = [&](uint32_t R) -> Row {
+        const uint32_t Rc = R < total ? R : total - 1;
         const int kind = Rc < q_rows ? 0 : (Rc < q_rows + kv_rows ? 1 : 2);
-        const uint32_t row = kind == 0 ? Rc : (kind == 1 ? Rc - q_rows : Rc - q_rows - kv_rows);
-        const uint32_t heads = kind == 0 ? a.geo.n_q : a.geo.n_kv;
-        // data first: its address does not depend on the sequence look-up
-        const uint4* src = reinterpret_cast<const uint4*>(kind == 0 ? a.q : (kind == 1 ? a.k : a.v)) + (size_t)row * (2 * T);
-        const uint4 xa = src[t], xb = src[T + t];
+        return {kind, kind == 0 ? Rc : (kind == 1 ? Rc - q_rows : Rc - q_rows - kv_rows)};
+    };
+    auto place_of = [&](const Row& x, bool live) -> Place {
+        const uint32_t heads = x.kind == 0 ? a.geo.n_q : a.geo.n_kv;
         int b;
         if (in_smem) {
             int lo = 0, hi = n_seqs - 1;
             while (lo < hi) {
                 const int mid = (lo + hi + 1) >> 1;
-                if ((uint32_t)s_tok[mid] * heads <= row) lo = mid; else hi = mid - 1;
+                if ((uint32_t)s_tok[mid] * heads <= x.row) lo = mid; else hi = mid - 1;
             }
             b = lo;
         } else {
-            b = seq_of_row(a.step, row, (int)heads);
+            b = seq_of_row(a.step, x.row, (int)heads);
         }
         const SeqMeta sm = a.step.seq_meta[b];
-        const uint32_t local = row - (uint32_t)sm.tok_off * heads;
+        const uint32_t local = x.row - (uint32_t)sm.tok_off * heads;
         const uint32_t h = local / (uint32_t)sm.snew, r = local - h * (uint32_t)sm.snew;
         const int gpos = sm.pos + (int)r;
-        uint4 tc = make_uint4(0, 0, 0, 0), ts = tc;
-        if (kind != 2) {
+        Place p;
+        p.tc = p.ts = make_uint4(0, 0, 0, 0);
+        p.ok = live;
+        if (x.kind != 2) {
             const int tpos = min(gpos, (int)a.rope.max_position - 1);
             const uint4* trow = reinterpret_cast<const uint4*>(a.rope.table) + (size_t)tpos * (2 * T);
-            tc = trow[t]; ts = trow[T + t];
+            p.tc = trow[t]; p.ts = trow[T + t];
         }
-        uint4* dst;
-        bool ok = live;
-        if (kind == 0) {
-            dst = reinterpret_cast<uint4*>(a.q_out) + (size_t)row * (2 * T);
+        if (x.kind == 0) {
+            p.dst = reinterpret_cast<uint4*>(a.q_out) + (size_t)x.row * (2 * T);
         } else if (a.k_out) {
-            dst = reinterpret_cast<uint4*>(a.k_out) + (size_t)row * (2 * T);
+            p.dst = reinterpret_cast<uint4*>(a.k_out) + (size_t)x.row * (2 * T);
         } else {
             int phys = a.step.tables[sm.tbl_off + gpos / a.geo.page_size];
-            if (phys < 0 || phys >= a.geo.num_pages) { if (live && t == 0) atomicOr(a.status, ST_BAD_PAGE); phys = 0; ok = false; }
+            if (phys < 0 || phys >= a.geo.num_pages) { if (live && t == 0) atomicOr(a.status, ST_BAD_PAGE); phys = 0; p.ok = false; }
             const int slot = gpos % a.geo.page_size;
             const int64_t drow = ((int64_t)phys * a.geo.n_kv + h) * 2 * a.geo.page_size +
-                                 page_row(kind == 2, slot, a.geo.page_size, a.geo.tiled != 0);
-            dst = reinterpret_cast<uint4*>(a.arena) + drow * (2 * T);
+                                 page_row(x.kind == 2, slot, a.geo.page_size, a.geo.tiled != 0);
+            p.dst = reinterpret_cast<uint4*>(a.arena) + drow * (2 * T);
         }
+        return p;
+    };
+    auto src_of = [&](const Row& x) { return reinterpret_cast<const uint4*>(x.kind == 0 ? a.q : (x.kind == 1 ? a.k : a.v)) + (size_t)x.row * (2 * T); };
+    auto finish = [&](const Row& x, const Place& p, const uint4& xa, const uint4& xb) {
         uint32_t A[4] = {xa.x, xa.y, xa.z, xa.w}, B[4] = {xb.x, xb.y, xb.z, xb.w};
-        const void* wv = kind == 0 ? a.rope.q_weight : (kind == 1 ? a.rope.k_weight : nullptr);
+        const void* wv = x.kind == 0 ? a.rope.q_weight : (x.kind == 1 ? a.rope.k_weight : nullptr);
         if (wv) {
             float ss = 0.f;
 #pragma unroll
@@ -279,15 +280,34 @@ __global__ void __launch_bounds__(256) rope_append_vec_kernel(const RopeArgs a) 
                 B[j] = norm2<BF16>(B[j], WB[j], inv_rms, a.rope.gemma != 0);
             }
         }
-        if (kind != 2) {
-            const uint32_t TC[4] = {tc.x, tc.y, tc.z, tc.w}, TS[4] = {ts.x, ts.y, ts.z, ts.w};
+        if (x.kind != 2) {
+            const uint32_t TC[4] = {p.tc.x, p.tc.y, p.tc.z, p.tc.w}, TS[4] = {p.ts.x, p.ts.y, p.ts.z, p.ts.w};
 #pragma unroll
             for (int j = 0; j < 4; j++) rotate2<BF16>(A[j], B[j], TC[j], TS[j]);
         }
-        if (ok) {
-            dst[t] = make_uint4(A[0], A[1], A[2], A[3]);
-            dst[T + t] = make_uint4(B[0], B[1], B[2], B[3]);
+        if (p.ok) {
+            p.dst[t] = make_uint4(A[0], A[1], A[2], A[3]);
+            p.dst[T + t] = make_uint4(B[0], B[1], B[2], B[3]);
         }
+    };
+    // The first round's look-ups run under the tail of the launch before: the records, the block tables (they came with
+    // the step's upload, which no kernel overlaps) and the rotary table are no kernel's work; q, k and v may be.
+    uint32_t R0 = warp0 * RPW;
+    const Row first = row_of(R0 + sub);
+    Place place{};
+    if (R0 < total) place = place_of(first, R0 + sub < total);
+    pdl_wait();
+    pdl_launch_dependents();
+    if (R0 >= total) return;
+    {
+        const uint4* src = src_of(first);
+        finish(first, place, src[t], src[T + t]);
+    }
+    for (R0 += nwarps * RPW; R0 < total; R0 += nwarps * RPW) {
+        const Row x = row_of(R0 + sub);
+        const uint4* src = src_of(x);  // data first: its address does not depend on the sequence look-up
+        const uint4 xa = src[t], xb = src[T + t];
+        finish(x, place_of(x, R0 + sub < total), xa, xb);
     }
 }
 
