@@ -453,8 +453,8 @@ static cudaError_t launch_tc(const CUtensorMap& map, const ChunkArgs& a, bool ov
 // K and V have buffers of their own: K of the tile after next is asked for when the scores of this one are computed, and so has
 // one and a half tiles of time to arrive; in one buffer with V, which is read last, it had half of one (without softmax a
 // launch of 512 items of 62 K/V tiles took 546 us with copies, 379 without).  The same launch, softmax and all: 630 us with one
-// buffer, one lane issuing, P handed over whole and a load of the scores at a time, 543 now (981 TFLOP/s; a chain of 3700 cycles
-// per tile, 2048 of them MMA).  Verification of drafts, 8 sequences x 5 tokens after 512 to 6144, 28 layers: 1642 -> 1465 us.
+// buffer, one lane issuing, P handed over whole and a load of the scores at a time, 528 now (1008 TFLOP/s; a chain of 3700 cycles
+// per tile, 2048 of them MMA).  Verification of drafts, 8 sequences x 5 tokens after 512 to 6144, 28 layers: 1642 -> 1461 us.
 //
 // Tensor memory: S_A [0,128), S_B [128,256), O_A [256,384), O_B [384,512).
 constexpr int kThreads2 = 576;

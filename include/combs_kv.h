@@ -393,7 +393,7 @@ int64_t cbkv_debug_chunk_choice(cbkv_arena* arena, int64_t window, int32_t mode,
                                 int32_t* out, int64_t cap);
 
 /* Tuning (no reference counterpart): the share of a CTA's range that is cut into dynamically
- * claimed tail items (percent), the smallest item (pages; 0 = no tail, a static equal split) and
+ * claimed tail items (percent), the smallest item (pages; 0 = no tail, a static split: even, or ranges that end where segments do) and
  * the number of halvings + 2.  Negative / < 2 = keep. */
 int32_t cbkv_set_decode_split(cbkv_arena* arena, int32_t tail_pct, int32_t min_item, int32_t max_levels);
 
