@@ -41,11 +41,9 @@ __global__ void __launch_bounds__(256) append_quant_kernel(const AppendArgs a) {
     const int64_t kv_rows = (int64_t)a.step.n_tokens * Hkv;
     uint8_t* arena = reinterpret_cast<uint8_t*>(a.arena);
     const size_t rec = qrec_bytes(P, d);
-    pdl_wait();
-    pdl_launch_dependents();
-    for (int64_t R = warp0; R < 2 * kv_rows; R += nwarps) {
-        const int is_v = R >= kv_rows;
-        const int64_t row = is_v ? R - kv_rows : R;
+    struct Place { uint8_t* recp; int slot; };  // null: the table entry is not a page
+    auto place_of = [&](int64_t R) -> Place {
+        const int64_t row = R >= kv_rows ? R - kv_rows : R;
         int lo = 0, hi = a.step.n_seqs - 1;
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
@@ -55,10 +53,23 @@ __global__ void __launch_bounds__(256) append_quant_kernel(const AppendArgs a) {
         const int64_t local = row - (int64_t)sm.tok_off * Hkv;
         const int h = (int)(local / sm.snew), r = (int)(local - (int64_t)h * sm.snew);
         const int gpos = sm.pos + r;                            // kv.rs:749
-        int phys = a.step.tables[sm.tbl_off + gpos / P];        // kv.rs:752
-        if (phys < 0 || phys >= a.geo.num_pages) { if (lane == 0) atomicOr(a.status, ST_BAD_PAGE); continue; }
-        const int slot = gpos % P;                              // kv.rs:750
-        uint8_t* recp = arena + ((size_t)phys * Hkv + h) * rec;
+        const int phys = a.step.tables[sm.tbl_off + gpos / P];  // kv.rs:752
+        if (phys < 0 || phys >= a.geo.num_pages) { if (lane == 0) atomicOr(a.status, ST_BAD_PAGE); return {nullptr, 0}; }
+        return {arena + ((size_t)phys * Hkv + h) * rec, gpos % P};  // kv.rs:750
+    };
+    // the first row's look-up runs under the tail of the launch before: the records and block tables came with the step's
+    // upload, which no kernel overlaps
+    Place next{nullptr, 0};
+    if (warp0 < 2 * kv_rows) next = place_of(warp0);
+    pdl_wait();
+    pdl_launch_dependents();
+    for (int64_t R = warp0; R < 2 * kv_rows; R += nwarps) {
+        const int is_v = R >= kv_rows;
+        const int64_t row = is_v ? R - kv_rows : R;
+        if (R != warp0) next = place_of(R);
+        uint8_t* recp = next.recp;
+        const int slot = next.slot;
+        if (recp == nullptr) continue;
         const uint2* src = reinterpret_cast<const uint2*>(is_v ? a.v : a.k) + row * words;
         // every lane runs every round (the shuffles below name the full warp)
         for (int c0 = 0; c0 < words; c0 += 32) {
