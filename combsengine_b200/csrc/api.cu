@@ -707,6 +707,7 @@ int32_t run_attention(Arena* a, int layer, const void* q, const void* k_fused, c
         args.rep_slots = 128 / tile_tokens;
         args.q8_arena = q8_direct ? L.base : nullptr;
         args.split_o = d->split_o; args.split_ml = d->split_ml; args.split_counter = d->split_counter;
+        args.fault_tile = d->fault_tile;
 #ifdef CBKV_MEASURE
         if (debug_flags() & 8) {  // per-role cycle counters of the first 4096 CTAs
             if (!d->dbg_buf) { CU_TRY(cudaMalloc(&d->dbg_buf, 4096 * 16 * sizeof(unsigned long long))); }
@@ -1704,9 +1705,10 @@ int32_t cbkv_set_decode_split(cbkv_arena* arena, int32_t tail_pct, int32_t min_i
 
 // Test hook for the kernels' failure path.  wait_us > 0 replaces the limit of the decode kernel's
 // bounded waits (default 100000); fault_tile >= 0 makes the producer of CTA 0 skip the copy of that
-// tile, so the consumer that owns it finds its wait running out, the status word gets
-// ST_WAIT_TIMEOUT and the launch returns without a result; -1 switches the hook off.  Nothing is
-// read or written outside the kernel's own buffers either way.
+// tile (tcgen05 chunk kernels: of that K/V tile, and their limits stay 0.1 and 0.2 s), so whoever
+// needs it finds its wait running out, the status word gets ST_WAIT_TIMEOUT and the launch returns
+// without a result; -1 switches the hook off.  Nothing is read or written outside the kernel's own
+// buffers either way.
 int32_t cbkv_debug_set_wait_limit(cbkv_arena* arena, int64_t wait_us, int32_t fault_tile) {
     return fenced([&]() -> int32_t {
     Arena* a = reinterpret_cast<Arena*>(arena);

@@ -231,7 +231,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
                 if (!ok) break;
                 asked[is_v]++;
                 const uint32_t full0 = at_rank0(full);
-                if (is_v) {
+                if (j == a.fault_tile && blockIdx.x == 0) {  // the copies are announced and not made
+                } else if (is_v) {
                     if (lane < PPT) load_page_pair(smem_u32(sV + st * HALF) + lane * PGV, &tmap_v, rank * XBV, 1, (phys * Hkv + h) * 2, full0);
                 } else if (lane >= rank * (PPT / 2) && lane < (rank + 1) * (PPT / 2)) {
                     load_page_pair(smem_u32(sK + st * HALF) + (lane - rank * (PPT / 2)) * PGK, &tmap_k, 0, 0, (phys * Hkv + h) * 2, full0);

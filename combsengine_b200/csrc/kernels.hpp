@@ -149,6 +149,7 @@ struct ChunkArgs {
     float* split_o;         // float4 [slot][query tile][column group D / 4][row 128]; rows: q head * valid tokens + token
     float2* split_ml;       // [slot][query tile][row 128]
     int32_t* split_counter; // per cut item, zero between launches
+    int32_t fault_tile;     // test hook, tcgen05 kernels: the copies of this K/V tile of CTA 0 are never issued (-1 = none)
 #ifdef CBKV_MEASURE
     unsigned long long* dbg_buf;  // per-CTA cycle counters of the tcgen05 kernel
 #endif

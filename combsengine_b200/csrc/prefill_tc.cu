@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
                     else { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
                 }
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-                if (ok && lane < PPT)
+                if (ok && lane < PPT && (j != a.fault_tile || blockIdx.x != 0))
                     tma_load_page(smem_u32((is_v ? sV : sK) + st * KVB + lane * PGB), &tmap, is_v, (phys * Hkv + h) * 2, full);
                 if (lane == 0) TC_ACC(c_issue);
             }
@@ -507,6 +507,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     int* s_asked = reinterpret_cast<int*>(bars + 19);  // K and V buffers whose copies have been announced (float layers)
     int* s_pages = reinterpret_cast<int*>(bars + 32);
     float* s_xch = reinterpret_cast<float*>(s_pages + kPageCap);  // [2 buffers][2 tiles][128 rows][2 halves]
+    int* s_pair = reinterpret_cast<int*>(s_xch + 2 * 2 * 128 * 2);  // [2 tiles][4 pairs of warps][parity of the K/V tile] a wait ran out
     // Q8 layout of the stage area: K buffers [0, 64 KB), V buffer [64, 96 KB), raw K ring and the first raw V
     // slots [96, 128 KB); the other raw V slots and the Q8 barriers follow the exchange area.  A K or V buffer
     // is [64-column block][page][8-token group][8 rows of 128 bytes], 128-byte swizzle.
@@ -517,7 +518,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     static_assert(!Q8 || kRawK * HALF + kRawVInStage * HALF <= 4 * KVB - 3 * QBUF, "raw rings in the freed quarter");
     uint8_t* sRawK = sKV + 3 * QBUF;
     uint8_t* sRawV0 = sRawK + kRawK * HALF;
-    uint8_t* sRawV1 = reinterpret_cast<uint8_t*>(s_xch + 2 * 2 * 128 * 2) + 128;  // 128-byte aligned, as every slot is
+    uint8_t* sRawV1 = reinterpret_cast<uint8_t*>(s_pair) + 128;  // 128-byte aligned, as every slot is
     const uint32_t b_q8 = smem_u32(sRawV1 + (kRawV - kRawVInStage) * HALF);
     const uint32_t b_rawk = b_q8, b_rawv = b_rawk + kRawK * 8;
     (void)sRawK; (void)sRawV0; (void)sRawV1; (void)b_rawk; (void)b_rawv; (void)REC;
@@ -552,7 +553,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         if constexpr (Q8)
             for (int i = 0; i < kRawK + kRawV; i++) mbar_init(b_rawk + i * 8, 1);
         *failed = 0;
-        for (int i = 0; i < 8; i++) reinterpret_cast<int*>(s_xch + 2 * 2 * 128 * 2)[i] = 0;
+        for (int i = 0; i < 16; i++) s_pair[i] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap32) : "memory");
         if constexpr (Q8) asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_sc) : "memory");
@@ -609,6 +610,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
             const int row0 = (phys * Hkv + h) * (int)(REC / 128u);
             const uint32_t dst = smem_u32(slot_ptr(sl)), bar = b_raw + sl * 8;
             mbar_expect_tx(bar, HALF);
+            if (n >> 3 == a.fault_tile && blockIdx.x == 0) return;
             tma_load_2d(dst, &tmap32, 0, row0 + (is_v ? 16 : 0), bar);
             tma_load_2d(dst + 16u * D, &tmap_sc, 0, row0 + 32 + (is_v ? 1 : 0), bar);
         };
@@ -724,7 +726,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                     else { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
                 }
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-                if (ok && lane < 8) tma_load_page(smem_u32(sKV + (2 * is_v + st) * KVB + lane * PGB), &tmap32, is_v, (phys * Hkv + h) * 2, full);
+                if (ok && lane < 8 && (j != a.fault_tile || blockIdx.x != 0)) tma_load_page(smem_u32(sKV + (2 * is_v + st) * KVB + lane * PGB), &tmap32, is_v, (phys * Hkv + h) * 2, full);
                 if (lane == 0) TC_ACC(c_issue);
             }
         }
@@ -808,8 +810,9 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         const int pair_bar = 1 + X * 4 + (warp & 3);  // named barrier of the two warps that share this quarter of tile X
         auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory"); };
         // A named barrier has no time limit, so the two warps of a pair must leave the loop in the same
-        // iteration: whichever sees a wait run out says so here before the pair's barrier, both read it after.
-        volatile int* pair_failed = reinterpret_cast<volatile int*>(s_xch + 2 * 2 * 128 * 2) + X * 4 + (warp & 3);
+        // iteration: whichever sees a wait run out says so before the pair's barrier, both read it after.  Two flags
+        // in turn: once another role has given up, a wait for the next tile's scores ends at once, and a warp may be
+        // there before the other has read this tile's flag.
         float m_ref = -INFINITY, l_run = 0.f;  // l_run: this half's share of the row sum
         bool ok = true;
         long long tprev = TC_NOW(), c_ws = 0, c_ld = 0, c_exp = 0, c_wo = 0, c_st = 0;
@@ -819,6 +822,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
             ok = mbar_wait_unless(b_s_full + X * 8, j & 1, failed);
             ok = __all_sync(0xffffffffu, ok);
             TC_ACC(c_ws);
+            volatile int* pair_failed = s_pair + X * 8 + (warp & 3) * 2 + (j & 1);
             if (!ok && lane == 0) *pair_failed = 1;  // the loads below then read stale columns: harmless, nothing is kept
             tc_fence_after();
             // this thread's keys: 32 H .. 32 H + 31 of the tile's first 64 and of its last 64

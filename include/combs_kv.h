@@ -400,8 +400,8 @@ int32_t cbkv_set_decode_split(cbkv_arena* arena, int32_t tail_pct, int32_t min_i
 /* Test hook for the kernels' failure path (the reference has no device-side failure path; its
  * host-side one is the panic fence above).  wait_us > 0 replaces the limit of the decode
  * kernel's bounded waits (default 100000 us).  fault_tile >= 0: the producer of CTA 0 never
- * issues the copy of that tile, so the wait of the warp that owns it runs out: the launch
- * returns, ST_WAIT_TIMEOUT (2) shows in cbkv_device_status, its output is undefined, and the
+ * issues the copy of that tile (tcgen05 chunk kernels: of that K/V tile; their limits stay 0.1
+ * and 0.2 s), so the wait of the warp that owns it runs out: the launch returns, ST_WAIT_TIMEOUT (2) shows in cbkv_device_status, its output is undefined, and the
  * next step runs normally.  fault_tile = -1 switches the hook off.  Nothing is read or written
  * outside the kernel's own buffers either way. */
 int32_t cbkv_debug_set_wait_limit(cbkv_arena* arena, int64_t wait_us, int32_t fault_tile);

@@ -73,3 +73,43 @@ def test_ticket_counters_are_clean_after_a_failed_launch():
     assert g.device_status() & 2   # the word still remembers the failed launch; now it is read and cleared
     assert g.device_status() == 0
     p.assert_state_equal(pages="used")
+
+
+# One launch of every tcgen05 chunk kernel that never receives one of its K/V tiles: the first, one in the middle (the softmax
+# warps are then in different tiles) and the last; whole items, and items cut along K/V.
+@pytest.mark.parametrize("mode,n_q,n_kv,d,int8", [(2, 9, 3, 64, False), (2, 28, 4, 128, False), (2, 8, 4, 256, False), (3, 28, 4, 128, False),
+                                                  (4, 28, 4, 128, True), (6, 28, 4, 128, False), (6, 8, 4, 256, False)])
+@pytest.mark.parametrize("parts,new", [(1, 100), (64, 5)])
+def test_a_chunk_launch_whose_copy_never_comes_returns_and_the_next_one_is_correct(mode, n_q, n_kv, d, int8, parts, new):
+    from combsengine_b200 import KVArena
+
+    ctx, rand = [900, 1300], lambda n: torch.randn(n, device="cuda", dtype=torch.float16)
+    torch.manual_seed(d + mode)
+    g = KVArena(1, n_q, n_kv, d, 2048, 16, 256, quantize_kv=int8)
+    g.set_chunk_kernel(mode)
+    g.set_chunk_split(parts)
+    seqs = [g.new_seq() for _ in ctx]
+    g.begin_step(seqs, ctx)
+    g.append(0, rand(sum(ctx) * n_kv * d), rand(sum(ctx) * n_kv * d))
+    q, k, v = (rand(len(ctx) * new * h * d) for h in (n_q, n_kv, n_kv))
+
+    def step(fault_tile):
+        g.debug_set_wait_limit(fault_tile=fault_tile)
+        g.begin_step(seqs, [new] * len(ctx))
+        out = g.attention(0, q, k, v, d ** -0.5)
+        torch.cuda.synchronize()
+        for s in seqs:
+            s.popn(new)
+        return out, g.device_status()
+
+    first, status = step(-1)
+    assert status == 0
+    keys = 64 if mode == 2 and d == 256 else 128
+    last = -(-(ctx[1] + new) // keys) - 1
+    seen = 0
+    for tile in (0, 1, 4, last):
+        seen += step(tile)[1]              # a CTA with fewer tiles withholds nothing
+        again, status = step(-1)
+        assert status == 0 and torch.equal(first, again)
+    assert seen >= (6 if parts == 1 else 2) and seen % 2 == 0
+    g.close()
