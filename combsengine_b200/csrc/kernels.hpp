@@ -140,6 +140,7 @@ struct ChunkArgs {
     int32_t* status;
     int32_t window;
     float scale_log2;
+    int32_t fault_tile; // test hook, tcgen05 kernels: the copies of this K/V tile of CTA 0 are never issued (-1 = none)
     int32_t rep_slots;  // tcgen05 kernel: q heads per kv head rounded up to a power of two (rows per token in a tile)
     const void* q8_arena;  // two-tile tcgen05 kernel: non-null = the layer's int8 records, read and converted by the kernel itself
     // tcgen05 kernels: one record per CTA (n_items of them).  The CTAs of an item that is cut along K/V write their
@@ -149,7 +150,6 @@ struct ChunkArgs {
     float* split_o;         // float4 [slot][query tile][column group D / 4][row 128]; rows: q head * valid tokens + token
     float2* split_ml;       // [slot][query tile][row 128]
     int32_t* split_counter; // per cut item, zero between launches
-    int32_t fault_tile;     // test hook, tcgen05 kernels: the copies of this K/V tile of CTA 0 are never issued (-1 = none)
 #ifdef CBKV_MEASURE
     unsigned long long* dbg_buf;  // per-CTA cycle counters of the tcgen05 kernel
 #endif

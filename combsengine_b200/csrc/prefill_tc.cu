@@ -462,7 +462,7 @@ constexpr int kThreads2 = 576;
 template <int D>
 constexpr int tc2_smem_bytes() {
     return 2 * 128 * D * 2 /* Q_A, Q_B */ + 2 * 2 * 128 * D * 2 /* two K/V stages */ + 256 + kPageCap * 4 +
-           2 * 2 * 128 * 2 * 4 /* half-row maxima of both tiles, double-buffered */ + 64 /* the pairs' failure flags */;
+           2 * 2 * 128 * 2 * 4 /* half-row maxima of both tiles, double-buffered */;
 }
 
 // Q8: the layer holds int8 records (kernels.hpp, qrec_*) and the kernel converts them itself
@@ -485,7 +485,7 @@ constexpr int kRawVInStage = 7;            // V slots that fit behind the K ring
 template <int D>
 constexpr int tc2_half_rec() { return 16 * D + 16 * (D / 32) * 2; }  // values + scales of K or of V
 template <int D>
-constexpr int tc2_smem_bytes_q8() { return tc2_smem_bytes<D>() + 64 + (kRawV - kRawVInStage) * tc2_half_rec<D>() + (kRawK + kRawV + 2) * 8; }
+constexpr int tc2_smem_bytes_q8() { static_assert(kPageCap % 32 == 0, "128-byte aligned slots"); return tc2_smem_bytes<D>() + (kRawV - kRawVInStage) * tc2_half_rec<D>() + (kRawK + kRawV + 2) * 8; }
 
 template <int D, bool BF16, bool Q8>
 __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel(const __grid_constant__ CUtensorMap tmap32, const __grid_constant__ CUtensorMap tmap_sc, const ChunkArgs a) {
@@ -507,7 +507,6 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     int* s_asked = reinterpret_cast<int*>(bars + 19);  // K and V buffers whose copies have been announced (float layers)
     int* s_pages = reinterpret_cast<int*>(bars + 32);
     float* s_xch = reinterpret_cast<float*>(s_pages + kPageCap);  // [2 buffers][2 tiles][128 rows][2 halves]
-    int* s_pair = reinterpret_cast<int*>(s_xch + 2 * 2 * 128 * 2);  // [2 tiles][4 pairs of warps][parity of the K/V tile] a wait ran out
     // Q8 layout of the stage area: K buffers [0, 64 KB), V buffer [64, 96 KB), raw K ring and the first raw V
     // slots [96, 128 KB); the other raw V slots and the Q8 barriers follow the exchange area.  A K or V buffer
     // is [64-column block][page][8-token group][8 rows of 128 bytes], 128-byte swizzle.
@@ -518,7 +517,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     static_assert(!Q8 || kRawK * HALF + kRawVInStage * HALF <= 4 * KVB - 3 * QBUF, "raw rings in the freed quarter");
     uint8_t* sRawK = sKV + 3 * QBUF;
     uint8_t* sRawV0 = sRawK + kRawK * HALF;
-    uint8_t* sRawV1 = reinterpret_cast<uint8_t*>(s_pair) + 128;  // 128-byte aligned, as every slot is
+    uint8_t* sRawV1 = reinterpret_cast<uint8_t*>(s_xch + 2 * 2 * 128 * 2);  // 128-byte aligned, as every slot is
     const uint32_t b_q8 = smem_u32(sRawV1 + (kRawV - kRawVInStage) * HALF);
     const uint32_t b_rawk = b_q8, b_rawv = b_rawk + kRawK * 8;
     (void)sRawK; (void)sRawV0; (void)sRawV1; (void)b_rawk; (void)b_rawv; (void)REC;
@@ -553,7 +552,6 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         if constexpr (Q8)
             for (int i = 0; i < kRawK + kRawV; i++) mbar_init(b_rawk + i * 8, 1);
         *failed = 0;
-        for (int i = 0; i < 16; i++) s_pair[i] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap32) : "memory");
         if constexpr (Q8) asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_sc) : "memory");
@@ -808,11 +806,10 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         const uint32_t lane_addr = (uint32_t)lane_base << 16;
         const uint32_t tS = tmem + X * 128 + lane_addr, tO = tmem + 256 + X * 128 + lane_addr;
         const int pair_bar = 1 + X * 4 + (warp & 3);  // named barrier of the two warps that share this quarter of tile X
-        auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory"); };
-        // A named barrier has no time limit, so the two warps of a pair must leave the loop in the same
-        // iteration: whichever sees a wait run out says so before the pair's barrier, both read it after.  Two flags
-        // in turn: once another role has given up, a wait for the next tile's scores ends at once, and a warp may be
-        // there before the other has read this tile's flag.
+        // A named barrier has no time limit, so the two warps of a pair must leave the loop in the same iteration.  Whether
+        // one saw a wait run out travels with the pair's barrier: a flag in shared memory could be raised for the next tile
+        // (once another role has given up, that wait ends at once) before the other has read it for this one, and two
+        // flags in turn cost 0.4 to 1.2 % (26 sequences of a mixed step 4626 us, this way 4496; one flag 4586).
         float m_ref = -INFINITY, l_run = 0.f;  // l_run: this half's share of the row sum
         bool ok = true;
         long long tprev = TC_NOW(), c_ws = 0, c_ld = 0, c_exp = 0, c_wo = 0, c_st = 0;
@@ -822,9 +819,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
             ok = mbar_wait_unless(b_s_full + X * 8, j & 1, failed);
             ok = __all_sync(0xffffffffu, ok);
             TC_ACC(c_ws);
-            volatile int* pair_failed = s_pair + X * 8 + (warp & 3) * 2 + (j & 1);
-            if (!ok && lane == 0) *pair_failed = 1;  // the loads below then read stale columns: harmless, nothing is kept
-            tc_fence_after();
+            tc_fence_after();  // (without the scores the loads below read stale columns: harmless, nothing is kept)
             // this thread's keys: 32 H .. 32 H + 31 of the tile's first 64 and of its last 64
             const int kbase = k0 + j * 128 + H * 32;
             const bool need_mask = (kbase + 95 > qx_min) || (a.window > 0 && kbase + a.window <= max(qx_max, qx_min));
@@ -843,9 +838,9 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
             // barrier of the tile in between rules out)
             float* xrow = s_xch + (((j & 1) * 2 + X) * 128 + m) * 2;
             xrow[H] = mx;
-            pair_sync();  // also: both warps have their S columns in registers, so P may overwrite them
+            const bool gave_up = bar_any(pair_bar, 64, !ok);  // also: both warps have their S columns in registers, so P may overwrite them
             mx = fmaxf(mx, xrow[H ^ 1]) * a.scale_log2;
-            if (*pair_failed) { ok = false; break; }  // both warps of the pair, in the same iteration
+            if (gave_up) { ok = false; break; }  // both warps of the pair, in the same iteration
             TC_ACC(c_ld);
             float alpha = 1.f;
             if (mx > m_ref + 8.f || m_ref == -INFINITY) {  // both halves see the same mx: the same decision
@@ -897,7 +892,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
         // meet at its barrier the same number of times)
         float* xrow = s_xch + ((n_tiles & 1) * 2 + X) * 256 + m * 2;
         xrow[H] = l_run;
-        pair_sync();
+        bar_sync(pair_bar, 64);
         const float l_row = l_run + xrow[H ^ 1];
         if (!ok && lane == 0) {
             *failed = 1;
