@@ -43,7 +43,7 @@ constexpr int kPairBufs = 5;
 // barriers, each 8 bytes
 constexpr int kBKFull = 0, kBVFull = kBKFull + kPairBufs, kBKEmpty = kBVFull + kPairBufs, kBVEmpty = kBKEmpty + kPairBufs;
 constexpr int kBSFull = kBVEmpty + kPairBufs, kBPFull = kBSFull + 2, kBODone = kBPFull + 2, kBQFull = kBODone + 2;
-constexpr int kPairWords = 4 + 8;  // 8-byte words after the barriers: tensor memory, failed and ticket, then the 16 flags of the pairs of warps
+constexpr int kPairWords = 4 + 8;  // 8-byte words after the barriers: tensor memory, failed, ticket, the issuer's last barrier, then the 16 flags of the pairs of warps
 constexpr int kBSFree = kBQFull + 1, kBRef = kBSFree + 2 /* [2 buffers][4 quarters] */, kBCount = kBRef + 8;
 
 template <int D>
@@ -116,6 +116,13 @@ __device__ __forceinline__ void commit_pair(uint32_t bar) {
         "elect.sync _|q, 0xffffffff;\n\t"
         "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(bar), "h"((uint16_t)3) : "memory");
 }
+// the same on this CTA's barrier alone
+__device__ __forceinline__ void commit_own(uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
+}
 
 }  // namespace
 
@@ -139,6 +146,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kBCount);
     volatile int* failed = reinterpret_cast<volatile int*>(bars + kBCount + 1);
     int* s_ticket = reinterpret_cast<int*>(bars + kBCount + 2);
+    const uint32_t b_drain = bar(kBCount + 3);
     int* s_pair = reinterpret_cast<int*>(bars + kBCount + 4);      // [8 pairs of warps][parity of the group's tile] a wait ran out
     int* s_pages = reinterpret_cast<int*>(bars + kBCount + kPairWords);  // [kPageCap] physical pages of the KV range
     float* s_xch = reinterpret_cast<float*>(s_pages + kPageCap);   // [S buffer][parity of the group's tile][128 rows][2 halves]
@@ -181,6 +189,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
         mbar_init(bar(kBQFull), 32);
         for (int i = 0; i < 2; i++) mbar_init(bar(kBSFree + i), 16);
         for (int i = 0; i < 8; i++) mbar_init(bar(kBRef + i), 1);
+        mbar_init(b_drain, 1);
         *failed = 0;
         for (int i = 0; i < 16; i++) s_pair[i] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -207,6 +216,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
         bool ok = true;
+        const int withheld = blockIdx.x == 0 ? a.fault_tile : -1;  // announced and not made
         int asked[2] = {0, 0};  // K and V buffers that this CTA has asked copies for
 #pragma unroll 1
         for (int j = 0; j < n_tiles && ok; j++) {
@@ -231,10 +241,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
                 if (!ok) break;
                 asked[is_v]++;
                 const uint32_t full0 = at_rank0(full);
-                if (j == a.fault_tile && blockIdx.x == 0) {  // the copies are announced and not made
-                } else if (is_v) {
-                    if (lane < PPT) load_page_pair(smem_u32(sV + st * HALF) + lane * PGV, &tmap_v, rank * XBV, 1, (phys * Hkv + h) * 2, full0);
-                } else if (lane >= rank * (PPT / 2) && lane < (rank + 1) * (PPT / 2)) {
+                if (is_v) {
+                    if (lane < PPT && j != withheld) load_page_pair(smem_u32(sV + st * HALF) + lane * PGV, &tmap_v, rank * XBV, 1, (phys * Hkv + h) * 2, full0);
+                } else if (lane >= rank * (PPT / 2) && lane < (rank + 1) * (PPT / 2) && j != withheld) {
                     load_page_pair(smem_u32(sK + st * HALF) + (lane - rank * (PPT / 2)) * PGK, &tmap_k, 0, 0, (phys * Hkv + h) * 2, full0);
                 }
             }
@@ -299,7 +308,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads) chunk_
                 commit_pair(bar(kBVEmpty + st));
                 commit_pair(bar(kBODone + (j & 1)));
             }
-            if (!ok && lane == 0) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
+            if (!ok) {  // what has been issued ends before the tensor memory is given back
+                if (lane == 0) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
+                commit_own(b_drain);
+                mbar_wait_bounded(b_drain, 0);
+            }
         }
     } else {
         // ------------------------------------------------------------ softmax + epilogue

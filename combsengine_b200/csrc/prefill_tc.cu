@@ -74,7 +74,8 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
     volatile int* failed = reinterpret_cast<volatile int*>(bars + 4 * NB + 6);
     int* s_ticket = reinterpret_cast<int*>(bars + 4 * NB + 7);
     int* s_asked = reinterpret_cast<int*>(bars + 4 * NB + 8);  // K and V buffers whose copies have been announced
-    static_assert(4 * NB + 9 <= 32, "barriers");
+    const uint32_t b_drain = smem_u32(bars + 4 * NB + 9);
+    static_assert(4 * NB + 10 <= 32, "barriers");
     int* s_pages = reinterpret_cast<int*>(bars + 32);   // [kPageCap] physical pages of the KV range
     float* s_xch = reinterpret_cast<float*>(s_pages + kPageCap);  // [2 buffers][128 rows][2 halves]
     int* s_pair = reinterpret_cast<int*>(s_xch + 2 * 128 * 2);    // [4 pairs of warps][tile parity] a wait ran out
@@ -102,6 +103,7 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
         }
         for (int i = 0; i < 2; i++) { mbar_init(b_s_full + i * 8, 1); mbar_init(b_p_full + i * 8, D == 64 ? 8 : 256); }
         mbar_init(b_o_done, 1);
+        mbar_init(b_drain, 1);
         *failed = 0;
         for (int i = 0; i < 8; i++) s_pair[i] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -236,7 +238,10 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
                 umma_commit(b_o_done);
                 TC_ACC(c_iss);
             }
-            if (!ok && lane == 0) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
+            if (!ok) {
+                if (lane == 0) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
+                umma_commit(b_drain);  // waited for below
+            }
             TC_DUMP(if (lane == 0) { a.dbg_buf[(size_t)blockIdx.x * 16 + 2] = c_wkv; a.dbg_buf[(size_t)blockIdx.x * 16 + 3] = c_wp; a.dbg_buf[(size_t)blockIdx.x * 16 + 4] = c_iss; });
         }
     } else {
@@ -416,10 +421,13 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
     // ---- wind down: everybody meets, then the allocating warp frees the tensor memory
     tc_fence_before();
     __syncthreads();
-    // never leave with a copy in flight if somebody gave up (a barrier is in the phase announced last, or past it)
-    if (tid == 0 && *failed)
+    // Never leave with a product or a copy in flight if somebody gave up (a copy's barrier is in the phase announced last, or
+    // past it).  If the issuer was not the one, its last product has the limit of the first wait to end.
+    if (tid == 0 && *failed) {
+        mbar_wait_bounded(b_drain, 0);
         for (int is_v = 0; is_v < 2; is_v++)
             for (int i = max(0, s_asked[is_v] - NB); i < s_asked[is_v]; i++) mbar_wait_bounded((is_v ? b_v_full : b_k_full) + (i % NB) * 8, (i / NB) & 1);
+    }
     __syncwarp();
     if (warp == 0) {
         tc_fence_after();
@@ -505,6 +513,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
     volatile int* failed = reinterpret_cast<volatile int*>(bars + 18);  // and the ticket
     int* s_asked = reinterpret_cast<int*>(bars + 19);  // K and V buffers whose copies have been announced (float layers)
+    const uint32_t b_drain = smem_u32(bars + 20);
     int* s_pages = reinterpret_cast<int*>(bars + 32);
     float* s_xch = reinterpret_cast<float*>(s_pages + kPageCap);  // [2 buffers][2 tiles][128 rows][2 halves]
     // Q8 layout of the stage area: K buffers [0, 64 KB), V buffer [64, 96 KB), raw K ring and the first raw V
@@ -549,6 +558,7 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
             mbar_init(b_s_full + i * 8, 1); mbar_init(b_p_full + i * 16, 8); mbar_init(b_p_full + i * 16 + 8, 8); mbar_init(b_o_done + i * 8, 1);
         }
         mbar_init(b_q_full, 16);
+        mbar_init(b_drain, 1);
         if constexpr (Q8)
             for (int i = 0; i < kRawK + kRawV; i++) mbar_init(b_rawk + i * 8, 1);
         *failed = 0;
@@ -789,7 +799,10 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
                     TC_ACC(c_iss);
                 }
             }
-            if (!ok && lane == 0) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
+            if (!ok) {
+                if (lane == 0) { *failed = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
+                umma_commit(b_drain);  // waited for below
+            }
             (void)c_pv;
             TC_DUMP(if (lane == 0) { a.dbg_buf[(size_t)blockIdx.x * 16 + 2] = c_wkv; a.dbg_buf[(size_t)blockIdx.x * 16 + 3] = c_wp; a.dbg_buf[(size_t)blockIdx.x * 16 + 4] = c_iss;
                     a.dbg_buf[(size_t)blockIdx.x * 16 + 11] = c_pv; });
@@ -944,10 +957,12 @@ __global__ void __launch_bounds__(Q8 ? kThreads2Q8 : kThreads2) chunk_tc2_kernel
     }
     tc_fence_before();
     __syncthreads();
-    // never leave with a copy in flight if somebody gave up
-    if (!Q8 && tid == 0 && *failed)
-        for (int is_v = 0; is_v < 2; is_v++)
+    // never leave with a product or a copy in flight if somebody gave up (as above)
+    if (tid == 0 && *failed) {
+        mbar_wait_bounded(b_drain, 0);
+        for (int is_v = 0; is_v < 2 && !Q8; is_v++)
             for (int i = max(0, s_asked[is_v] - 2); i < s_asked[is_v]; i++) mbar_wait_bounded((is_v ? b_v_full : b_k_full) + (i & 1) * 8, (i >> 1) & 1);
+    }
     __syncwarp();
     if (warp == 0) {
         tc_fence_after();
