@@ -366,11 +366,18 @@ bool align_decode_plan(int32_t n_kv_heads, int32_t min_pages, int32_t slack, int
 // combine, its partial and ticket wait for the first's), and the launch ends with the slowest: 3 to 4 us of the 10 to 15 that
 // decode launches of a few sequences take.  So the ranges end where segments do, unless that makes the longest of them longer
 // than the even cut's by more than it saves: 64 pages at head_dim 64, 48 at 128, 16 at 256; int8 pages, whose tiles are bound by
-// arithmetic, 32, 32 and 8.  Measured even / aligned, us per launch (16 bits; B sequences of lo to hi tokens, kv heads/head_dim):
+// arithmetic, 20, 16 and 8.  Measured even / aligned, us per launch (16 bits; B sequences of lo to hi tokens, kv heads/head_dim):
 //   1 x 1500 3/64 10.7 / 6.6, 4/128 13.2 / 7.4, 4/256 13.8 / 8.0;  4 x 300-2000 3/64 12.1 / 7.9, 4/128 13.3 / 8.8, 4/256 14.3 / 10.5
 //   16 x 4000 4/128 29 / 28, 8/128 47 / 44;  32 x 1024-4096 4/128 33.9 / 33.9 (35.4 with 96 more pages);  16 x 8192 with windows of
 //   1024 4/256 29.7 / 28.1;  8 x 8000 4/256 49 / 52 with 24 more pages
 //   int8: 4 x 300-2000 4/128 24 / 14.6;  32 x 300-1000 8/128 23 / 21;  16 x 4000 8/128 36 / 37, 4/256 48 / 50 with 32 more pages
+// The lines are where batches of nearly as many segments as CTAs break even, all of one length but one sequence, which a range
+// then holds whole (pages of the others + of that one; with half of the batch longer the ranges that end with segments win by more):
+//   3/64 5 + 69 10.2 / 9.5, 5 + 120 11.1 / 12.9, 80 + 144 15.7 / 15.5, 200 + 264 26.2 / 26.3;  8/128 5 + 53 11.4 / 9.7, 40 + 88
+//   14.6 / 14.9, 120 + 168 28.3 / 29.4;  4/256 5 + 21 11.5 / 10.0, 40 + 56 22.9 / 24.2, 200 + 216 78 / 79
+//   int8: 3/64 5 + 25 12.3 / 10.9, 5 + 36 12.3 / 12.7, 40 + 60 18.7 / 18.0, 40 + 80 18.9 / 21.1;  4/128 5 + 36 14.5 / 14.8, 40 + 56
+//   24.7 / 21.6, 40 + 80 25.3 / 26.4;  8/128 (the long one in two) 5 + 36 12.8 / 13.3, 5 + 69 14.0 / 17.0, 40 + 140 25.0 / 27.2;
+//   4/256 5 + 13 14.7 / 12.8, 40 + 48 27.0 / 22.2, 40 + 80 27.8 / 31.7
 //
 // Segments of a few pages are not cut at all: a CTA per segment streams its pages in the time that a cut spends on partials,
 // tickets and the merge.  One sequence, cut into a page per consumer warp / uncut, us per launch:
@@ -384,7 +391,7 @@ void choose_decode_plan(const Arena& a, int64_t window, bool quant, int32_t cons
     const int32_t want = std::max(1, (pl->n_units + consumers - 1) / consumers);
     if (want < pl->n_ctas) build_decode_plan(a, window, want, split, pl);
     const int32_t d = a.cfg.head_dim, at = d <= 64 ? 0 : d <= 128 ? 1 : 2;
-    static constexpr int32_t kSlack[2][3] = {{64, 48, 16}, {32, 32, 8}}, kUncut[2][3] = {{24, 28, 17}, {19, 20, 12}};
+    static constexpr int32_t kSlack[2][3] = {{64, 48, 16}, {20, 16, 8}}, kUncut[2][3] = {{24, 28, 17}, {19, 20, 12}};
     int32_t longest = 0;
     for (int s = 0; s < pl->n_segs; s += a.cfg.n_kv_heads) longest = std::max(longest, pl->segs[(size_t)s + 1].unit_begin - pl->segs[(size_t)s].unit_begin);
     // (Launches of an arena of one or two layers have nothing to overlap with: one of 33 pages, 3/64, 13.9 / 14.5 us cut.)
