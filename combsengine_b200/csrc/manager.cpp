@@ -385,6 +385,13 @@ bool align_decode_plan(int32_t n_kv_heads, int32_t min_pages, int32_t slack, int
 //   head_dim 128: 12 pages 6.6 / 4.9, 23 pages 6.9 / 6.5, 27 pages 6.9 / 6.7, 32 pages 6.8 / 7.6
 //   head_dim 256: 12 pages 6.5 / 5.6, 16 pages 6.6 / 6.2, 19 pages 6.8 / 7.0, 23 pages 6.9 / 8.1
 //   int8: 64 12 pages 5.8 / 5.1, 26 6.0 / 6.6; 128 19 pages 6.4 / 6.2, 26 6.8 / 7.2; 256 12 pages 7.8 / 7.5, 16 7.6 / 8.2
+// An arena of one layer launches once a step, behind that step's upload and unit table: no launch runs under another's tail, and
+// an upload of more than 1 KB, which a cut makes of many a short one, takes 5 us longer.  So segments of up to 40 pages stay whole
+// there, up to 16 of them; with more, both uploads are that long.  16 bits, us per step, cut / uncut at 33 and 40 pages:
+//   1 sequence:  3/64 12.7 / 12.7, 12.8 / 12.6;  1/128 12.5 / 12.6, 12.3 / 13.4;  4/128 12.7 / 12.8, 13.1 / 13.7;  8/128 18.7 / 13.4, 17.4 / 14.5
+//   2 sequences: 3/64 19.2 / 12.8, 18.6 / 13.0;  1/128 12.5 / 12.5, 12.7 / 13.5;  4/128 18.9 / 13.5, 18.6 / 14.5;  8/128 18.5 / 19.7, 17.4 / 21.1
+//   4 sequences: 3/64 17.6 / 17.2, 17.6 / 19.7;  1/128 17.6 / 13.1, 17.5 / 13.9;  4/128 17.4 / 17.0, 17.7 / 18.5;  8/128 19.2 / 19.7, 18.5 / 20.4
+// With two layers one sequence is equal at 33 pages and better cut at 40 (3/64 17.6 / 17.6, 17.6 / 19.3; 4/128 18.4 / 18.6, 19.0 / 19.7).
 void choose_decode_plan(const Arena& a, int64_t window, bool quant, int32_t consumers, int32_t max_ctas, const DecodeSplit& split, DecodePlan* pl) {
     build_decode_plan(a, window, max_ctas, split, pl);
     // at least one page per consumer warp, at most one resident wave of CTAs
@@ -394,8 +401,7 @@ void choose_decode_plan(const Arena& a, int64_t window, bool quant, int32_t cons
     static constexpr int32_t kSlack[2][3] = {{64, 48, 16}, {20, 16, 8}}, kUncut[2][3] = {{24, 28, 17}, {19, 20, 12}};
     int32_t longest = 0;
     for (int s = 0; s < pl->n_segs; s += a.cfg.n_kv_heads) longest = std::max(longest, pl->segs[(size_t)s + 1].unit_begin - pl->segs[(size_t)s].unit_begin);
-    // (Launches of an arena of one or two layers have nothing to overlap with: one of 33 pages, 3/64, 13.9 / 14.5 us cut.)
-    const int32_t uncut = a.cfg.num_layers <= 2 && !quant && d <= 128 ? 40 : kUncut[quant ? 1 : 0][at];
+    const int32_t uncut = a.cfg.num_layers == 1 && pl->n_segs <= 16 && !quant && d <= 128 ? 40 : kUncut[quant ? 1 : 0][at];
     align_decode_plan(a.cfg.n_kv_heads, longest <= uncut ? longest : consumers, kSlack[quant ? 1 : 0][at], max_ctas, pl);
 }
 

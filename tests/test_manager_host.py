@@ -321,6 +321,21 @@ def test_decode_ranges_end_where_segments_do_when_that_costs_little(d, int8, len
     assert pl["n_parts"] == int(np.sum(pl["segs"][:-1, 4][pl["segs"][:-1, 4] > 1]))
 
 
+# the longest segments that stay whole: one layer (up to 16 segments of 16-bit pages, head_dim up to 128), two, and more
+@pytest.mark.parametrize("layers", [1, 2, 3])
+@pytest.mark.parametrize("d,int8,n_kv,seqs,one,more", [(64, False, 3, 2, 40, 24), (128, False, 8, 2, 40, 28), (128, False, 8, 3, 28, 28), (128, False, 1, 4, 40, 28),
+                                                       (256, False, 4, 1, 17, 17), (64, True, 3, 2, 19, 19), (128, True, 4, 1, 20, 20), (256, True, 4, 1, 12, 12)])
+def test_short_segments_stay_whole(layers, d, int8, n_kv, seqs, one, more):
+    limit = one if layers == 1 else more
+    for pages in (limit, limit + 1):
+        a = KVArena(layers, 2 * n_kv, n_kv, d, 1024, 16, 256)
+        s = [a.new_seq() for _ in range(seqs)]
+        a.begin_step_host_only(s, [16 * pages - 1] * seqs)
+        a.begin_step_host_only(s, [1] * seqs)
+        pl = a.debug_decode_choice(0, int8, 4 if int8 and d <= 128 else 6, 296 if int8 and d <= 128 else 148)
+        assert (pl["n_ctas"] == seqs * n_kv) == (pages == limit) and pl["n_ctas"] >= seqs * n_kv
+
+
 @pytest.mark.skipif(torch.cuda.is_available(), reason="checks the behaviour on a machine without a GPU")
 def test_compute_fails_loudly_without_a_gpu():
     a = arena()
