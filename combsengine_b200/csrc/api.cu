@@ -96,7 +96,7 @@ struct DeviceState {
     int cur = 0;
     uint64_t uploaded_step = 0;
     StepDev step{};
-    std::map<std::pair<int64_t, int>, DecodePlanDev> decode_plans;  // by (window, consumer warps)
+    std::map<std::pair<int64_t, bool>, DecodePlanDev> decode_plans;  // by (window, int8 pages)
     int32_t* unit_rows = nullptr;  // unit_row arrays of the step's plans, one after the other
     size_t unit_rows_cap = 0, unit_rows_used = 0;
     int32_t* work_counters = nullptr;  // four claim counters of the decode kernel, rotating per launch
@@ -416,7 +416,7 @@ GeomDev geom(const Arena* a) {
 int32_t get_decode_plan(Arena* a, int64_t window, bool quant, cudaStream_t st, DecodePlanDev** out) {
     DeviceState* d = dev_of(a);
     DecodeConfig dc = decode_config(a->cfg.head_dim, a->n_rep(), d->decode_ctas_per_sm, d->decode_stages, d->decode_consumers, quant);
-    const auto key = std::make_pair(window, dc.consumers);
+    const auto key = std::make_pair(window, quant);  // the cut is another for int8 pages, also with the same number of consumer warps
     auto it = d->decode_plans.find(key);
     if (it != d->decode_plans.end()) { *out = &it->second; return CBKV_OK; }
     DecodePlanDev pd{};

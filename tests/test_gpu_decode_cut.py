@@ -1,5 +1,5 @@
-"""Decode launches whose CTAs hold one segment each (ranges that end where segments do, short segments uncut, the last piece
-combined by all warps) against attention in float64, at the sizes where the plan changes."""
+"""Decode launches whose CTAs hold one segment each (ranges that end where segments do, short segments uncut, rings of the
+ranges' size, the last piece combined by all warps) against attention in float64, at the sizes where the plan changes."""
 import pytest
 import torch
 
@@ -29,21 +29,9 @@ def quantised(x):
 @pytest.mark.parametrize("lens,window", [([1, 16, 17], None), ([272, 273], None), ([384, 385], None), ([448], None), ([449], None), ([320, 321], None),
                                          ([1500, 40, 700], None), ([3000, 1000], 1024), ([100 + 37 * i for i in range(20)], None), ([900] * 36, None)])
 def test_one_segment_per_cta(d, n_kv, n_rep, int8, lens, window):
-    check(d, n_kv, n_rep, int8, lens, window, 4)
-
-
-# arenas of one layer keep longer segments whole, those of two do not
-@pytest.mark.parametrize("layers", [1, 2])
-@pytest.mark.parametrize("d,n_kv,n_rep", [(64, 3, 3), (128, 4, 7), (128, 1, 4)])
-@pytest.mark.parametrize("lens", [[384, 385], [448, 449], [640], [641, 300], [640] * 20])
-def test_arenas_of_few_layers(d, n_kv, n_rep, lens, layers):
-    check(d, n_kv, n_rep, False, lens, None, layers)
-
-
-def check(d, n_kv, n_rep, int8, lens, window, layers):
     dt, n_q, B = torch.float16, n_kv * n_rep, len(lens)
     torch.manual_seed(sum(lens) + d)
-    a = KVArena(layers, n_q, n_kv, d, max(lens) + 16, 16, sum(-(-n // 16) for n in lens) + 4, [window] * layers, dt, sliding_popn_refuses=False, quantize_kv=int8)
+    a = KVArena(4, n_q, n_kv, d, max(lens) + 16, 16, sum(-(-n // 16) for n in lens) + 4, [window] * 4, dt, sliding_popn_refuses=False, quantize_kv=int8)
     a.set_free_list(torch.randperm(a.num_pages).numpy())
     seqs = [a.new_seq() for _ in lens]
     kv = [torch.randn(2, n_kv, n, d, device="cuda", dtype=dt) for n in lens]
