@@ -1,5 +1,5 @@
-"""Decode launches whose CTAs hold one segment each (ranges that end where segments do, short segments uncut, rings of the
-ranges' size, the last piece combined by all warps) against attention in float64, at the sizes where the plan changes."""
+"""Decode launches whose CTAs hold one segment each (ranges that end where segments do, short segments uncut, the last piece
+combined by all warps) against attention in float64, at the sizes where the plan changes."""
 import pytest
 import torch
 
@@ -29,9 +29,21 @@ def quantised(x):
 @pytest.mark.parametrize("lens,window", [([1, 16, 17], None), ([272, 273], None), ([384, 385], None), ([448], None), ([449], None), ([320, 321], None),
                                          ([1500, 40, 700], None), ([3000, 1000], 1024), ([100 + 37 * i for i in range(20)], None), ([900] * 36, None)])
 def test_one_segment_per_cta(d, n_kv, n_rep, int8, lens, window):
+    check(d, n_kv, n_rep, int8, lens, window, 4)
+
+
+# arenas of one layer keep longer segments whole, those of two do not
+@pytest.mark.parametrize("layers", [1, 2])
+@pytest.mark.parametrize("d,n_kv,n_rep", [(64, 3, 3), (128, 4, 7), (128, 1, 4)])
+@pytest.mark.parametrize("lens", [[384, 385], [448, 449], [640], [641, 300], [640] * 20])
+def test_arenas_of_few_layers(d, n_kv, n_rep, lens, layers):
+    check(d, n_kv, n_rep, False, lens, None, layers)
+
+
+def check(d, n_kv, n_rep, int8, lens, window, layers):
     dt, n_q, B = torch.float16, n_kv * n_rep, len(lens)
     torch.manual_seed(sum(lens) + d)
-    a = KVArena(4, n_q, n_kv, d, max(lens) + 16, 16, sum(-(-n // 16) for n in lens) + 4, [window] * 4, dt, sliding_popn_refuses=False, quantize_kv=int8)
+    a = KVArena(layers, n_q, n_kv, d, max(lens) + 16, 16, sum(-(-n // 16) for n in lens) + 4, [window] * layers, dt, sliding_popn_refuses=False, quantize_kv=int8)
     a.set_free_list(torch.randperm(a.num_pages).numpy())
     seqs = [a.new_seq() for _ in lens]
     kv = [torch.randn(2, n_kv, n, d, device="cuda", dtype=dt) for n in lens]
@@ -53,4 +65,31 @@ def test_one_segment_per_cta(d, n_kv, n_rep, int8, lens, window):
         for o in (out[b], again[b]):
             err = (o.to(torch.float64) - ref).abs()
             assert bool((err <= 2e-3 + 1e-2 * ref.abs()).all()), (b, lens[b], float(err.max()))
+    a.close()
+
+
+# A layer with a window of its own keeps 16-bit pages in an arena of int8 ones, and an int8 layer may be called with the same
+# window: each has its own cut, whichever comes first in the step (16-bit segments of 16 or 24 pages stay whole, int8 ones are cut).
+@pytest.mark.parametrize("d,consumers,n", [(256, 0, 251), (128, 6, 380)])
+def test_layers_of_both_kinds_under_one_window(d, consumers, n):
+    n_kv, n_q, dt, window, ctx = 4, 8, torch.float16, 512, [n, n - 11]
+    torch.manual_seed(d)
+    a = KVArena(4, n_q, n_kv, d, 1024, 16, 64, [window, None, None, None], dt, sliding_popn_refuses=False, quantize_kv=True)
+    a.set_decode_tuning(consumers=consumers)
+    seqs = [a.new_seq() for _ in ctx]
+    rand = lambda n: torch.randn(n, device="cuda", dtype=dt)
+    a.begin_step(seqs, ctx)
+    for layer in range(2):
+        a.append(layer, rand(sum(ctx) * n_kv * d), rand(sum(ctx) * n_kv * d))
+    q, k, v = (rand(2 * h * d) for h in (n_q, n_kv, n_kv))
+    outs = []
+    for order in ((0,), (1,), (0, 1), (1, 0)):
+        a.begin_step(seqs, [1, 1])
+        outs.append({layer: a.attention(layer, q, k, v, d ** -0.5, window=window) for layer in order})
+        for s in seqs:
+            s.popn(1)
+    assert a.device_status() == 0
+    for both in outs[2:]:
+        for layer in range(2):
+            assert torch.equal(both[layer], outs[layer][layer])
     a.close()
