@@ -1137,6 +1137,32 @@ template <> struct ChunkCfg<256> { static constexpr int W = 4, S = 2, NT = 1; };
 
 template <int D> constexpr int chunk_smem() { return ChunkCfg<D>::W * ChunkCfg<D>::S * 32 * D * 2 + ChunkCfg<D>::W * ChunkCfg<D>::S * 8; }
 
+template <int D, int C, bool BF16, bool Q8>
+static int decode_resident() {
+    static const int n = [] {  // asked once
+        int r = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, decode_kernel<D, C, BF16, Q8, false>, (C + 2) * 32, 0) == cudaSuccess) return std::max(r, 1);
+        cudaGetLastError();  // no device: nothing will be launched
+        return 8;
+    }();
+    return n;
+}
+template <int D, bool BF16, bool Q8>
+static int decode_resident(int consumers) {
+    return consumers == 4 ? decode_resident<D, 4, BF16, Q8>() : consumers == 6 ? decode_resident<D, 6, BF16, Q8>() : consumers == 8 ? decode_resident<D, 8, BF16, Q8>() : decode_resident<D, 12, BF16, Q8>();
+}
+// CTAs of the decode kernel whose registers an SM holds at a time.  The variants over 16-bit pages are compiled for one (176
+// registers at head_dim 128): two CTAs per SM that do not fit share the ring's memory and run one after the other (28 layers of 32
+// sequences, two steps, 28/4/128: 3700 us; 2320 with 128 registers and both resident, 1840 with one).
+static int decode_resident(int d, int consumers, bool q8) {
+    auto least = [&](auto f, auto b) { return std::min(f(consumers), b(consumers)); };
+    switch (d) {
+        case 64: return q8 ? least(decode_resident<64, false, true>, decode_resident<64, true, true>) : least(decode_resident<64, false, false>, decode_resident<64, true, false>);
+        case 128: return q8 ? least(decode_resident<128, false, true>, decode_resident<128, true, true>) : least(decode_resident<128, false, false>, decode_resident<128, true, false>);
+        default: return q8 ? least(decode_resident<256, false, true>, decode_resident<256, true, true>) : least(decode_resident<256, false, false>, decode_resident<256, true, false>);
+    }
+}
+
 // Stage count: the largest multiple of the consumer count that fits next to the merge
 // buffers when `ctas_per_sm` CTAs share the SM's shared memory (1 KB per CTA is
 // reserved by the system), at most 8 stages per consumer.  Bytes in flight matter
@@ -1155,7 +1181,7 @@ DecodeConfig decode_config(int d, int n_rep, int ctas_per_sm, int stages, int co
     // other's tiles; measured 0.80 ms per cfg2 step against 0.85 with one CTA of eight
     if (q8 && d <= 128) { c = DecodeCfg<128>::C8; ctas = 2; }
     if (consumers == 4 || consumers == 6 || consumers == 8 || (consumers == 12 && d <= 128)) c = consumers;  // 12 warps of head_dim 256 spill
-    if (ctas_per_sm > 0) ctas = ctas_per_sm;
+    if (ctas_per_sm > 0) ctas = ctas_per_sm == 1 ? 1 : std::min(ctas_per_sm, decode_resident(d, c, q8));
     const int comb_cols = std::min(8, (n_rep + 1) & ~1);
     const int smem_limit = std::min(227 * 1024, (228 * 1024) / ctas - 1024);
     if (stages <= 0) {

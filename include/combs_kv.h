@@ -325,7 +325,7 @@ int64_t cbkv_launch_count(void);
 int32_t cbkv_profile_enable(cbkv_arena* arena, int32_t on);
 int32_t cbkv_profile_read(cbkv_arena* arena, double* total_ms, int64_t* launches);
 /* Tuning knobs for measurements and tests (0 = built-in default): CTAs per SM of the
- * decode kernel, stages of its TMA ring (rounded down to a multiple of the consumer
+ * decode kernel (at most as many as its registers let run at a time), stages of its TMA ring (rounded down to a multiple of the consumer
  * count), consumer warps per CTA (4, 6, 8 or 12), an upper bound on the CTAs launched,
  * and whether consecutive launches, of any of the library's kernels, may overlap
  * (programmatic dependent launch; 1 = default). */

@@ -93,3 +93,27 @@ def test_layers_of_both_kinds_under_one_window(d, consumers, n):
         for layer in range(2):
             assert torch.equal(both[layer], outs[layer][layer])
     a.close()
+
+
+@pytest.mark.parametrize("d,int8", [(64, False), (128, False), (256, False), (128, True)])
+def test_no_more_ctas_are_planned_than_run_at_a_time(d, int8):
+    # two CTAs per SM asked for: the cut is that of one where the kernel has the registers of one
+    n_kv, n_q, dt, ctx = 4, 8, torch.float16, [900 + 61 * i for i in range(40)]
+    torch.manual_seed(d)
+    a = KVArena(3, n_q, n_kv, d, max(ctx) + 16, 16, sum(n // 16 + 2 for n in ctx), None, dt, quantize_kv=int8)
+    seqs = [a.new_seq() for _ in ctx]
+    rand = lambda n: torch.randn(n, device="cuda", dtype=dt)
+    a.begin_step(seqs, ctx)
+    a.append(0, rand(sum(ctx) * n_kv * d), rand(sum(ctx) * n_kv * d))
+    q, k, v = (rand(len(ctx) * h * d) for h in (n_q, n_kv, n_kv))
+    sms, outs = torch.cuda.get_device_properties(0).multi_processor_count, []
+    for per_sm, max_ctas in ((1, 0), (2, 0), (2, sms)):
+        a.set_decode_tuning(ctas_per_sm=per_sm, max_ctas=max_ctas)
+        a.begin_step(seqs, [1] * len(ctx))
+        outs.append(a.attention(0, q, k, v, d ** -0.5))
+        for s in seqs:
+            s.popn(1)
+    assert a.device_status() == 0
+    assert torch.equal(outs[0], outs[2])
+    assert torch.equal(outs[0], outs[1]) != int8  # int8 pages: two run at a time, and the launch is cut for them
+    a.close()
