@@ -1648,7 +1648,7 @@ int64_t cbkv_debug_decode_choice(cbkv_arena* arena, int64_t window, int32_t int8
     Arena* a = reinterpret_cast<Arena*>(arena);
     if (!a || a->step_meta.empty() || !out || consumers < 1 || max_ctas < 1) return -1;
     DecodePlan pl;
-    choose_decode_plan(*a, window, int8_pages != 0, consumers, max_ctas, DecodeSplit{}, &pl);
+    choose_decode_plan(*a, window, int8_pages != 0, consumers, max_ctas, a->dev ? dev_of(a)->split : DecodeSplit{}, &pl);
     return flatten_decode_plan(pl, out, cap);
     });
 }

@@ -373,7 +373,8 @@ int32_t cbkv_debug_raise(int32_t kind);
 int64_t cbkv_debug_decode_plan(cbkv_arena* arena, int64_t window, int32_t n_ctas, int32_t tail_pct, int32_t min_item,
                                int32_t* out, int64_t cap);
 /* The same for the plan that the library's own decode launches of the step take, with `consumers` consumer
- * warps per CTA and at most `max_ctas` CTAs: the even split, or ranges that end where segments do. */
+ * warps per CTA, at most `max_ctas` CTAs and the arena's cbkv_set_decode_split: the even split, or ranges
+ * that end where segments do. */
 int64_t cbkv_debug_decode_choice(cbkv_arena* arena, int64_t window, int32_t int8_pages, int32_t consumers,
                                  int32_t max_ctas, int32_t* out, int64_t cap);
 

@@ -117,3 +117,16 @@ def test_no_more_ctas_are_planned_than_run_at_a_time(d, int8):
     assert torch.equal(outs[0], outs[2])
     assert torch.equal(outs[0], outs[1]) != int8  # int8 pages: two run at a time, and the launch is cut for them
     a.close()
+
+
+def test_the_plan_that_is_shown_follows_the_arenas_split():
+    a = KVArena(3, 8, 4, 128, 8192, 16, 2048)
+    seqs = [a.new_seq() for _ in range(4)]
+    a.begin_step(seqs, [6000, 300, 4000, 2000])
+    a.begin_step(seqs, [1] * 4)
+    assert a.debug_decode_choice()["n_items"] == a.debug_decode_choice()["n_ctas"]
+    a.set_decode_split(tail_pct=25, min_item=2)
+    shown, asked = a.debug_decode_choice(), a.debug_decode_plan(0, 148, 25, 2)
+    assert shown["n_items"] > shown["n_ctas"]
+    assert (shown["items"] == asked["items"]).all() and (shown["segs"] == asked["segs"]).all()
+    a.close()
