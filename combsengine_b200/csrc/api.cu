@@ -321,9 +321,10 @@ int32_t alloc_float_layer(Arena* a, LayerArena* Lp, cudaStream_t st) {
 // upload; returns the device address.
 int32_t slot_upload(DeviceState* d, const void* src, size_t bytes, cudaStream_t st, const void** dev_out) {
     StepSlot& s = d->slots[d->cur];
-    // 16 bytes is the widest load of a record.  A copy of up to 1 KB is cheaper by 5 us, and a short step's pieces fit in that
-    // unless they are padded (one layer, 2 sequences of 320 tokens, 3/64, cut: 19.8 us per step with pieces 256 bytes apart, 12.7 now).
-    size_t off = (s.used + 15) & ~(size_t)15;
+    // A record of 32 bytes in a sector of its own (16 bytes apart: 26 sequences with windows, 28 layers, 4/256, 1203 us, 1191 now).
+    // Not more: a copy of up to 1 KB is cheaper by 5 us, and a short step's pieces fit in that unless they are padded (one layer, 2
+    // sequences of 320 tokens, 3/64, cut: 19.8 us per step with pieces 256 bytes apart, 12.7 so).
+    size_t off = (s.used + 31) & ~(size_t)31;
     if (off + bytes > s.cap) {
         // grow: nothing of this slot may still be in flight
         CU_TRY(cudaStreamSynchronize(st));
