@@ -443,9 +443,9 @@ constexpr float kPairCtaCost = 5.f, kPairSliceCost = 1.f, kPairMergeCost = 1.f; 
 // tile / pairs at head_dim 256: 48 sequences x 2 tokens after 2048 74 / 117, 16 x 5 after 8192 94 / 123, 1 x 9 after 8192 45
 // / 30, a prompt of 512 after 512 49 / 24; two tiles / pairs at 128: 2 prompts of 333 after 1024 (4 kv heads) 35 / 43.
 //
-// The tcgen05 kernels are 5 to 15 % faster than when this was fitted, all by about as much, and the ratios are what decides: over 92
-// steps (1 to 64 sequences, 1 to 512 new tokens and mixes, four geometries) the kernel taken was within 7 % of the fastest, but
-// for one (a prompt of 100 tokens at head_dim 256, 12.6 us against 11.1).
+// The tcgen05 kernels are 5 to 15 % faster than when this was fitted, all by about as much; the mma.sync kernel is not, so near
+// its line it is taken a little too often.  Over 92 steps (1 to 64 sequences, 1 to 512 new tokens and mixes, four geometries) the
+// kernel taken was within 7 % of the fastest, but for one (a prompt of 100 tokens at head_dim 256, 12.6 us against 11.1).
 //
 // pair_margin: pairs are taken where their estimate is below this share of the others'.  At head_dim 128, where the kernels
 // are closer, a tenth, the estimates' own error: 8 sequences x 5 tokens after 512 to 6144 (28 q heads) come out equal and

@@ -10,8 +10,8 @@
 // two), so the K/V tiles are shared by the whole q-head group.
 //
 //   warp 0        TMA producer: one copy per page and operand
-//   warp 1        one thread issues tcgen05.mma: S = Q K^T (two S buffers), O += P V, whichever
-//                 has its operands first
+//   warp 1        converged, one elected lane issues tcgen05.mma: S = Q K^T (two S buffers), O += P V,
+//                 whichever has its operands first
 //   warps 2..9    softmax: two threads per TMEM lane (row), one for each half of a tile's keys; P goes back to
 //                 tensor memory over its S columns (16-bit pairs) and is the A operand of P V; O rescaled in
 //                 TMEM when a row max moves
@@ -315,7 +315,8 @@ __global__ void __launch_bounds__(kThreads) chunk_tc_kernel(const __grid_constan
                 uint64_t sum[2] = {0ull, 0ull};
                 exp_pack<HK, BF16>(sv, f32x2(a.scale_log2, a.scale_log2), f32x2(-m_use, -m_use), sum, sv);  // a pair reuses a register whose score is consumed
                 sum_all = sum_of(sum);
-            } else {  // (two at a time, and maxima of three above, spill at head_dim 256: verification there was 2 % slower with them)
+            } else {  // (two at a time, and maxima of three above, spill at head_dim 256: verification there was 2 % slower with
+                      // them; 128 comes here only when asked for, 4 % slower on long prompts, 600 / 576 us, and equal on short steps)
                 float sum = 0.f, sum2 = 0.f;
 #pragma unroll
                 for (int e = 0; e < HK; e += 2) {
@@ -461,15 +462,15 @@ static cudaError_t launch_tc(const CUtensorMap& map, const ChunkArgs& a, bool ov
 // K and V have buffers of their own: K of the tile after next is asked for when the scores of this one are computed, and so has
 // one and a half tiles of time to arrive; in one buffer with V, which is read last, it had half of one (without softmax a
 // launch of 512 items of 62 K/V tiles took 546 us with copies, 379 without).  The same launch, softmax and all: 630 us with one
-// buffer, one lane issuing, P handed over whole and a load of the scores at a time, 528 now (1008 TFLOP/s; a chain of 3700 cycles
-// per tile, 2048 of them MMA).  Verification of drafts, 8 sequences x 5 tokens after 512 to 6144, 28 layers: 1642 -> 1461 us.
+// buffer, one lane issuing, P handed over whole and a load of the scores at a time, 518 now (1028 TFLOP/s; a chain of 3600 cycles
+// per tile, 2048 of them MMA; without the exponentials 485, without copies 508, with neither 465).  Verification of drafts, 8 sequences x 5 tokens after 512 to 6144, 28 layers: 1642 -> 1461 us.
 //
 // Tensor memory: S_A [0,128), S_B [128,256), O_A [256,384), O_B [384,512).
 constexpr int kThreads2 = 576;
 
 template <int D>
 constexpr int tc2_smem_bytes() {
-    return 2 * 128 * D * 2 /* Q_A, Q_B */ + 2 * 2 * 128 * D * 2 /* two K/V stages */ + 256 + kPageCap * 4 +
+    return 2 * 128 * D * 2 /* Q_A, Q_B */ + 2 * 2 * 128 * D * 2 /* two K and two V buffers */ + 256 + kPageCap * 4 +
            2 * 2 * 128 * 2 * 4 /* half-row maxima of both tiles, double-buffered */;
 }
 

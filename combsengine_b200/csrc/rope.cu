@@ -196,6 +196,8 @@ __global__ void __launch_bounds__(256) rope_append_kernel(const RopeArgs a) {
 // block-table look-up overlaps its data loads.
 constexpr int ROPE_SEQ_SMEM = 1024;
 
+// Five blocks per SM: a warp waits on memory nearly all its time, so what counts is rows in flight.  48 registers without spills; left
+// alone the compiler takes 59, for four blocks (ragged prefill at head_dim 256 with norms 11.08 -> 10.99 ms, a mixed step 4557 -> 4542 us).
 template <bool BF16, int T>
 __global__ void __launch_bounds__(256, 5) rope_append_vec_kernel(const RopeArgs a) {
     __shared__ int s_tok[ROPE_SEQ_SMEM];

@@ -349,7 +349,7 @@ class KVArena:
         check(self._lib.cbkv_set_decode_split(self._h, tail_pct, min_item, max_levels))
 
     def debug_set_wait_limit(self, wait_us: int = 0, fault_tile: int = -1) -> None:
-        """Test hook: limit of the decode kernel's bounded waits, and a tile of CTA 0 whose copy is withheld."""
+        """Test hook: limit of the decode kernel's bounded waits, and a tile of CTA 0 (decode and tcgen05 chunk kernels) whose copy is withheld."""
         check(self._lib.cbkv_debug_set_wait_limit(self._h, wait_us, fault_tile))
 
     def debug_decode_plan(self, window: int, n_ctas: int, tail_pct: int = -1, min_item: int = -1) -> dict:
